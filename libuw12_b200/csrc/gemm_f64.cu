@@ -1,6 +1,6 @@
-// FP64 DMMA GEMM for sm_100a: 128x128x16 CTA tiles, 8 warps of 64x32,
-// 4-stage cp.async pipeline (16-byte copies when the operand allows it),
-// grouped CTA raster for L2 reuse, m16n8k4 f64 tensor-core MMAs.
+// FP64 GEMM engine for sm_100a: picks the CTA tile and the split of every
+// launch (the kernels are dgemm_tile.cuh's), reduces split-K partials, and holds
+// the profiler and the split-K autotuner.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include "dgemm_tile.cuh"
 #include "gemm_f64.cuh"
 #include "ozaki.cuh"
 
@@ -18,336 +19,26 @@ namespace uw12b {
 
 namespace {
 
-// k tile 16 with 4 stages measured 1.5% faster than 32 with 3 (and than 16
-// with 5, 32 with 2) on a full evaluation with N = 500 AO, M = 1500 DF and
-// R = 2000 RI functions; both are compile-time settings.
-#ifndef UW12_DMMA_BK
-#define UW12_DMMA_BK 16
-#endif
-#ifndef UW12_DMMA_STAGES
-#define UW12_DMMA_STAGES 4
-#endif
-constexpr int BM = 128;
-constexpr int BN = 128;
-constexpr int BK = UW12_DMMA_BK;          // 16 or 32 (k extent of a pipeline stage)
-constexpr int STAGES = UW12_DMMA_STAGES;  // stages in flight; shared memory <= 227 KiB
-static_assert(BK == 16 || BK == 32, "k tile of 16 or 32");
-constexpr int THREADS = 256;
-constexpr int LDW = BM + 4;  // [k][m] / [k][n] tile rows (doubles); 132 % 16 == 4
-constexpr int LDK = BK + 4;  // [m][k] / [n][k] tile rows (doubles); 20 (or 36) % 16 == 4, even
-constexpr int STAGE_ELEMS = (BM * LDK > BK * LDW) ? BM * LDK : BK * LDW;  // 2560
-constexpr size_t SMEM_BYTES = size_t(STAGES) * 2 * STAGE_ELEMS * sizeof(double);  // 160 KiB
-static_assert(SMEM_BYTES <= 227 * 1024, "pipeline stages exceed shared memory");
-constexpr int GROUP_N = 8;   // CTAs that run together share A panels across 8 n-tiles
+constexpr int BK = kDgemmBK;
 constexpr long long kSMs = 148;
 
-struct KParams {
-  const double* A;
-  const double* B;
-  double* C;
-  double* work;  // split > 1: partial tiles [split][nbo][m*n]
-  long long lda, ldb, ldc;
-  long long m, n, k;
-  double alpha, beta;
-  long long nbo1, nbo;
-  long long sAo1, sAo2, sBo1, sBo2, sCo1, sCo2;
-  long long nbr1;
-  long long sAr1, sAr2, sBr1, sBr2;
-  long long tiles_m, tiles_n, tiles_mn;
-  long long ktiles_pb, ktiles_total;
-  int split;
-};
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) {
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-
-// 8- or 16-byte asynchronous global -> shared copy; bytes beyond src_bytes
-// are zero-filled (src_bytes = 0 reads nothing).
-template <int BYTES>
-__device__ __forceinline__ void cp_async(double* dst, const double* src, int src_bytes) {
-  if (BYTES == 16)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst)),
-                 "l"(src), "r"(src_bytes));
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(smem_u32(dst)),
-                 "l"(src), "r"(src_bytes));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
-}
-
-__device__ __forceinline__ void dmma(double (&c)[4], double a0, double a1, double b0) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
-      "{%0,%1,%2,%3};\n"
-      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-      : "d"(a0), "d"(a1), "d"(b0));
-}
-
-__device__ __forceinline__ void dmma16(double (&c)[4], const double (&a)[8], const double (&b)[4]) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, "
-      "{%4,%5,%6,%7,%8,%9,%10,%11}, {%12,%13,%14,%15}, {%0,%1,%2,%3};\n"
-      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]),
-        "d"(b[0]), "d"(b[1]), "d"(b[2]), "d"(b[3]));
-}
-
-// Loader of one operand tile (BK deep, 128 wide) into shared memory.
-//   KC  : the operand is contiguous along k in global memory ([w][k] tile,
-//         row LDK) -- otherwise along the 128-wide dimension ([k][w], row LDW);
-//   VEC : copies of two consecutive doubles (16 bytes) along the contiguous
-//         dimension; requires even leading dimension / offsets.
-// Thread mapping: the contiguous index is the fastest-varying across threads.
-template <bool KC, bool VEC>
-struct TileLoader {
-  static constexpr int W = VEC ? 2 : 1;                       // doubles per copy
-  static constexpr int CONTIG = KC ? BK : 128;                // contiguous extent
-  static constexpr int TPC = CONTIG / W;                      // threads along it
-  static constexpr int OTHER_STEP = THREADS / TPC;            // other-dim stride
-  static constexpr int OTHER = KC ? 128 : BK;                 // other extent
-  static constexpr int COPIES = OTHER / OTHER_STEP;           // copies per thread
-
-  int c0;   // contiguous index of this thread's first element
-  int o0;   // other index of this thread's first copy
-
-  __device__ __forceinline__ explicit TileLoader(int tid)
-      : c0((tid % TPC) * W), o0(tid / TPC) {}
-
-  // Element (w, kk) of the 128-wide x BK tile lives at global offset
-  // w + ld*kk (not KC) or kk + ld*w (KC).
-  __device__ __forceinline__ long long base(long long w0, long long ld) const {
-    return KC ? (c0 + ld * (w0 + o0)) : (w0 + c0 + ld * o0);
-  }
-  __device__ __forceinline__ long long step(long long ld) const { return OTHER_STEP * ld; }
-  __device__ __forceinline__ long long kstep(long long ld) const { return KC ? BK : BK * ld; }
-
-  // Copies this thread's share of a tile.  wlim = extent left along the
-  // 128-wide dimension from the tile start, klim = extent left along k.
-  __device__ __forceinline__ void load(double* s, const double* g, const double* dummy,
-                                       long long wlim, long long klim, long long ld) const {
-#pragma unroll
-    for (int r = 0; r < COPIES; ++r) {
-      const int o = o0 + r * OTHER_STEP;
-      const long long lim_c = KC ? klim : wlim;  // limit along the contiguous dim
-      const long long lim_o = KC ? wlim : klim;  // limit along the other dim
-      int bytes = 0;
-      if (o < lim_o) {
-        const long long left = lim_c - c0;
-        bytes = left >= W ? 8 * W : (left > 0 ? 8 * static_cast<int>(left) : 0);
-      }
-      double* dst = KC ? s + o * LDK + c0 : s + o * LDW + c0;
-      const double* src = bytes ? g + r * OTHER_STEP * ld : dummy;
-      cp_async<8 * W>(dst, src, bytes);
-    }
-  }
-};
-
-template <bool AK, bool BNC, bool VA, bool VB>
-__global__ void __launch_bounds__(THREADS, 1) dgemm_dmma(const KParams p) {
-  extern __shared__ __align__(16) double smem[];
-  double* As = smem;
-  double* Bs = smem + STAGES * STAGE_ELEMS;
-
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  const int warp = tid >> 5;
-  const int g = lane >> 2;  // groupID
-  const int t = lane & 3;   // thread in group
-  const int wm = (warp & 1) * 64;
-  const int wn = (warp >> 1) * 32;
-
-  // Block -> (tile, output batch, split).  Tiles are visited in groups of
-  // GROUP_N n-tiles, m-tile outermost inside a group, so the ~148 CTAs that
-  // run at once touch a few A panels and GROUP_N B panels.
-  long long bid = blockIdx.x;
-  const long long tile = bid % p.tiles_mn;
-  bid /= p.tiles_mn;
-  const long long bo = bid % p.nbo;
-  const int sp = static_cast<int>(bid / p.nbo);
-  const long long per_group = p.tiles_m * GROUP_N;
-  const long long grp = tile / per_group;
-  const long long gn0 = grp * GROUP_N;
-  const long long gsize = (p.tiles_n - gn0) < GROUP_N ? (p.tiles_n - gn0) : GROUP_N;
-  const long long local = tile - grp * per_group;
-  const long long tn = gn0 + local % gsize;
-  const long long tm = local / gsize;
-  const long long m0 = tm * BM;
-  const long long n0 = tn * BN;
-  const long long bo1 = bo % p.nbo1;
-  const long long bo2 = bo / p.nbo1;
-  const double* Ab = p.A + bo1 * p.sAo1 + bo2 * p.sAo2;
-  const double* Bb = p.B + bo1 * p.sBo1 + bo2 * p.sBo2;
-
-  const long long kt_begin = p.ktiles_total * sp / p.split;
-  const long long kt_end = p.ktiles_total * (sp + 1) / p.split;
-
-  const TileLoader<AK, VA> la(tid);
-  const TileLoader<!BNC, VB> lb(tid);
-  const long long a_base = la.base(m0, p.lda);
-  const long long b_base = lb.base(n0, p.ldb);
-  const long long a_kstep = la.kstep(p.lda);
-  const long long b_kstep = lb.kstep(p.ldb);
-  const long long a_wlim = p.m - m0;
-  const long long b_wlim = p.n - n0;
-
-  // Incremental (reduction batch, k offset) iterator of the next stage to
-  // load: no integer division inside the main loop.
-  long long it_kin, it_br1;
-  const double* itA;
-  const double* itB;
-  {
-    const long long br = kt_begin / p.ktiles_pb;
-    const long long kt_in = kt_begin - br * p.ktiles_pb;
-    it_kin = kt_in * BK;
-    it_br1 = br % p.nbr1;
-    const long long br2 = br / p.nbr1;
-    itA = Ab + it_br1 * p.sAr1 + br2 * p.sAr2 + kt_in * a_kstep;
-    itB = Bb + it_br1 * p.sBr1 + br2 * p.sBr2 + kt_in * b_kstep;
-  }
-  const long long k_pad = p.ktiles_pb * BK;
-
-  auto load_stage = [&](int slot) {
-    const long long klim = p.k - it_kin;
-    la.load(As + slot * STAGE_ELEMS, itA + a_base, p.A, a_wlim, klim, p.lda);
-    lb.load(Bs + slot * STAGE_ELEMS, itB + b_base, p.B, b_wlim, klim, p.ldb);
-    it_kin += BK;
-    itA += a_kstep;
-    itB += b_kstep;
-    if (it_kin >= k_pad) {
-      it_kin = 0;
-      itA += p.sAr1 - p.ktiles_pb * a_kstep;
-      itB += p.sBr1 - p.ktiles_pb * b_kstep;
-      if (++it_br1 == p.nbr1) {
-        it_br1 = 0;
-        itA += p.sAr2 - p.nbr1 * p.sAr1;
-        itB += p.sBr2 - p.nbr1 * p.sBr1;
-      }
-    }
-  };
-
-  double acc[4][4][4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[a][b][c] = 0.0;
-
-#pragma unroll
-  for (int s = 0; s < STAGES - 1; ++s) {
-    if (kt_begin + s < kt_end) load_stage(s);
-    cp_async_commit();
-  }
-
-  int slot = 0;
-  int load_slot = STAGES - 1;
-  for (long long kt = kt_begin; kt < kt_end; ++kt) {
-    cp_async_wait<STAGES - 2>();
-    __syncthreads();
-    if (kt + STAGES - 1 < kt_end) load_stage(load_slot);
-    cp_async_commit();
-    load_slot = (load_slot + 1 == STAGES) ? 0 : load_slot + 1;
-
-    const double* as = As + slot * STAGE_ELEMS;
-    const double* bs = Bs + slot * STAGE_ELEMS;
-#if UW12_DMMA_K16
-    // m16n8k16: A fragment element q sits at row g + 8 (q & 1), k = t + 4 (q >> 1);
-    // B fragment element q at k = t + 4 q, column g.
-#pragma unroll
-    for (int kh = 0; kh < BK / 16; ++kh) {
-      double bf[4][4];
-#pragma unroll
-      for (int ni = 0; ni < 4; ++ni) {
-        const int col = wn + ni * 8 + g;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int kk = kh * 16 + t + 4 * q;
-          bf[ni][q] = BNC ? bs[kk * LDW + col] : bs[col * LDK + kk];
-        }
-      }
-#pragma unroll
-      for (int mi = 0; mi < 4; ++mi) {
-        double af[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int row = wm + mi * 16 + g + 8 * (q & 1);
-          const int kk = kh * 16 + t + 4 * (q >> 1);
-          af[q] = AK ? as[row * LDK + kk] : as[kk * LDW + row];
-        }
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni) dmma16(acc[mi][ni], af, bf[ni]);
-      }
-    }
-#else
-#pragma unroll
-    for (int kq = 0; kq < BK / 4; ++kq) {
-      const int kk = kq * 4 + t;
-      double af[4][2], bf[4];
-#pragma unroll
-      for (int mi = 0; mi < 4; ++mi) {
-        const int row = wm + mi * 16 + g;
-        af[mi][0] = AK ? as[row * LDK + kk] : as[kk * LDW + row];
-        af[mi][1] = AK ? as[(row + 8) * LDK + kk] : as[kk * LDW + row + 8];
-      }
-#pragma unroll
-      for (int ni = 0; ni < 4; ++ni) {
-        const int col = wn + ni * 8 + g;
-        bf[ni] = BNC ? bs[kk * LDW + col] : bs[col * LDK + kk];
-      }
-#pragma unroll
-      for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni) dmma(acc[mi][ni], af[mi][0], af[mi][1], bf[ni]);
-    }
-#endif
-    slot = (slot + 1 == STAGES) ? 0 : slot + 1;
-  }
-  cp_async_wait<0>();
-
-  // Epilogue: C = alpha acc + beta C, or the raw partial tile for split-K.
-  double* Cb = p.split == 1 ? p.C + bo1 * p.sCo1 + bo2 * p.sCo2
-                            : p.work + (static_cast<long long>(sp) * p.nbo + bo) * (p.m * p.n);
-  const long long ldc = p.split == 1 ? p.ldc : p.m;
-#pragma unroll
-  for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-    for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const long long r = m0 + wm + mi * 16 + g + 8 * h;
-        if (r >= p.m) continue;
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const long long c = n0 + wn + ni * 8 + 2 * t + q;
-          if (c >= p.n) continue;
-          double* dst = Cb + r + ldc * c;
-          if (p.split == 1) {
-            const double v = p.alpha * acc[mi][ni][2 * h + q];
-            *dst = (p.beta == 0.0) ? v : v + p.beta * (*dst);
-          } else {
-            *dst = acc[mi][ni][2 * h + q];
-          }
-        }
-      }
-}
-
-// C = alpha * sum_s work[s] + beta * C (fixed summation order).
-__global__ void splitk_reduce(const double* __restrict__ work, int split, long long m, long long n,
-                              long long nbo, long long nbo1, double alpha, double beta, double* C,
-                              long long ldc, long long sCo1, long long sCo2) {
-  const long long total = m * n * nbo;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long mn = m * n;
-    const long long bo = idx / mn;
-    const long long e = idx - bo * mn;
-    const long long r = e % m, c = e / m;
+// C = alpha * sum_s work[s] + beta * C (fixed summation order).  Bound by the
+// latency of the partials' loads at the small outputs that split: eight are in
+// flight per thread.  I: index type (32-bit divisions where the output allows).
+template <typename I>
+__global__ void splitk_reduce(const double* __restrict__ work, int split, I m, I mn, I total,
+                              I nbo1, double alpha, double beta, double* C, long long ldc,
+                              long long sCo1, long long sCo2) {
+  const I step = static_cast<I>(gridDim.x) * blockDim.x;
+  for (I idx = static_cast<I>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total; idx += step) {
+    const I bo = idx / mn;
+    const I e = idx - bo * mn;
+    const I c = e / m;
+    const I r = e - c * m;
+    const double* w = work + idx;
     double s = 0.0;
-    for (int q = 0; q < split; ++q) s += work[(q * nbo + bo) * mn + e];
+#pragma unroll 8
+    for (int q = 0; q < split; ++q) s += w[static_cast<long long>(q) * total];
     double* dst = C + (bo % nbo1) * sCo1 + (bo / nbo1) * sCo2 + r + ldc * c;
     const double v = alpha * s;
     *dst = (beta == 0.0) ? v : v + beta * (*dst);
@@ -368,67 +59,94 @@ __global__ void scale_only(long long m, long long n, long long nbo, long long nb
   }
 }
 
-// Split-K factor: the CTAs of one launch run in waves of 148 (one per SM), so
-// a launch with few output tiles, or with a last wave that is mostly empty,
-// splits the contraction to fill the waves.  A split keeps >= 512 of k per
-// CTA so the partial-tile round trip stays small against the MMA work.
-int choose_split(long long ctas, long long ktiles_total) {
-  auto eff = [&](long long c) {
-    const long long waves = (c + kSMs - 1) / kSMs;
-    return double(c) / double(waves * kSMs);
-  };
-  if (ctas >= 8 * kSMs) return 1;
-  int best = 1;
-  double best_eff = eff(ctas);
-  for (int s = 2; s <= 64; ++s) {
-    if (ktiles_total / s < 512 / BK) break;
-    const double e = eff(ctas * s);
-    if (e > best_eff + 0.05) {
-      best = s;
-      best_eff = e;
+// The tile and the split of a launch come from a cost model of the kernel,
+// fitted to a sweep of every tile and split over 41 shapes (outputs from 24 x 24
+// to 160000 x 600, contractions from 24 to 1.08 million terms, all layouts): its
+// pick is within 5 % of the measured best on 37 of them and within 16 % on 40.
+// In cycles, for a CTA on one SM:
+//   mma   its k tile at the tensor pipe's 64 multiply-adds per cycle, over the
+//         share of that rate which the tile reaches with all its CTAs resident
+//         (what is lost is operand traffic: 33.6, 31.5 and 30.1 TFLOP/s of 37.2
+//         for 64 x 64, 64 x 32 and 32 x 32 at 45000 x 9000 x 900);
+//   lone  its k tile when it has the SM to itself (fragment and barrier latency);
+//   lsu   its k tile's 8-byte copies where an operand does not allow 16-byte ones.
+// A split adds the partials' round trip and one launch.  The old rule, one
+// 128 x 128 tile, left 95 % of the tensor pipe idle at 360 x 360 x 360 and
+// computed 64 % padding at 300 x 300.
+struct TileCost {
+  const DgemmTile* tile;
+  double eff, lone;
+};
+const TileCost kTiles[] = {{&kTile64x64, 0.905, 1500.0},
+                           {&kTile64x32, 0.86, 900.0},
+                           {&kTile32x32, 0.82, 600.0},
+                           {&kTile128x16, 0.78, 1180.0},
+                           {&kTile128x8, 0.62, 940.0}};
+constexpr int kSplits[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64};
+constexpr double kCtaStart = 2500.0;    // prologue, epilogue and launch of a wave
+constexpr double kSplitLaunch = 5500.0; // the reduction's launch
+constexpr double kSplitBytes = 1600.0;  // partial bytes per cycle through L2 / HBM
+// Partial tiles of an automatic split: at most 256 MiB.
+constexpr double kMaxPartials = double(1LL << 25);
+
+struct Plan {
+  const DgemmTile* tile = nullptr;
+  int split = 1;
+};
+
+// Fewest predicted cycles over the tiles and, when `split` is 0, over the
+// splits whose partials stay within max_partials doubles and leave every CTA
+// two k tiles.
+Plan choose_plan(const GemmDesc& d, bool va, bool vb, int split, double max_partials) {
+  const long long nbo = d.nbo1 * d.nbo2;
+  const long long kt = (d.k + BK - 1) / BK * d.nbr1 * d.nbr2;
+  const double out = double(d.m) * double(d.n) * double(nbo);
+  Plan best;
+  double best_cost = 1e300;
+  for (const TileCost& t : kTiles) {
+    const DgemmTile& g = *t.tile;
+    const long long tiles = ((d.m + g.bm - 1) / g.bm) * ((d.n + g.bn - 1) / g.bn) * nbo;
+    double mma = g.bm * g.bn * BK / 64.0 / t.eff;
+    const double lsu = (va ? 0.0 : g.bm * (d.a_kcontig ? 6.5 : 5.0)) +
+                       (vb ? 0.0 : g.bn * (d.b_ncontig ? 5.0 : 6.5));
+    mma = std::max(mma, lsu);
+    const double occ = g.ctas_per_sm;
+    for (const int s : kSplits) {
+      if (split > 0 ? s != kSplits[0] : (s > 1 && (kt / s < 2 || out * s > max_partials))) break;
+      const int sp = split > 0 ? split : s;
+      const long long ctas = tiles * sp;
+      if (ctas > 0x7fffffffLL) break;
+      const double ktl = double((kt + sp - 1) / sp);
+      const long long per_sm = (ctas + kSMs - 1) / kSMs;
+      const long long full = per_sm / g.ctas_per_sm, rem = per_sm % g.ctas_per_sm;
+      double cost;
+      if (full >= 4)  // many waves: the CTAs of an SM drift apart and its last ones overlap
+        cost = ktl * (double(ctas) / kSMs + 0.5 * occ) * std::max(mma, t.lone / occ) + kCtaStart;
+      else
+        cost = ktl * (double(full) * std::max(occ * mma, t.lone) +
+                      (rem ? std::max(double(rem) * mma, t.lone) : 0.0)) +
+               kCtaStart * double(full + (rem ? 1 : 0));
+      if (sp > 1) cost += kSplitLaunch + (sp + 1) * out * 8.0 / kSplitBytes;
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = Plan{t.tile, sp};
+      }
     }
   }
+  if (!best.tile) throw Error(kErrInvalid, "gemm: too many output tiles for one launch");
   return best;
 }
 
 // A 16-byte copy needs the operand base, leading dimension and every batch
-// stride to be even (in doubles); tile origins are multiples of 32.
+// stride to be even (in doubles); tile origins are multiples of 8.
 bool vec_ok(const double* base, long long ld, long long s1, long long s2, long long s3,
             long long s4) {
   return (reinterpret_cast<std::uintptr_t>(base) % 16 == 0) && (ld % 2 == 0) && (s1 % 2 == 0) &&
          (s2 % 2 == 0) && (s3 % 2 == 0) && (s4 % 2 == 0);
 }
 
-template <bool AK, bool BNC, bool VA, bool VB>
-void launch_kernel(const KParams& p, long long grid, cudaStream_t s) {
-  static bool attr_set[64] = {};
-  static std::mutex mu;
-  int dev = 0;
-  UW12_CUDA(cudaGetDevice(&dev));
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    if (dev < 64 && !attr_set[dev]) {
-      UW12_CUDA(cudaFuncSetAttribute(dgemm_dmma<AK, BNC, VA, VB>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(SMEM_BYTES)));
-      attr_set[dev] = true;
-    }
-  }
-  dgemm_dmma<AK, BNC, VA, VB><<<static_cast<unsigned>(grid), THREADS, SMEM_BYTES, s>>>(p);
-  UW12_LAUNCHED();
-}
-
-template <bool AK, bool BNC>
-void launch_layout(const KParams& p, bool va, bool vb, long long grid, cudaStream_t s) {
-  if (va && vb) launch_kernel<AK, BNC, true, true>(p, grid, s);
-  else if (va) launch_kernel<AK, BNC, true, false>(p, grid, s);
-  else if (vb) launch_kernel<AK, BNC, false, true>(p, grid, s);
-  else launch_kernel<AK, BNC, false, false>(p, grid, s);
-}
-
-// Fills the kernel parameters and chooses the split-K factor.  Returns false
-// for an empty output; *empty_k is set when the contraction is empty
-// (C = beta C).
+// Fills the kernel parameters up to the tile and the split.  Returns false for
+// an empty output; *empty_k is set when the contraction is empty (C = beta C).
 bool prepare(const GemmDesc& d, KParams& p, bool* empty_k) {
   const long long nbo = d.nbo1 * d.nbo2;
   const long long nbr = d.nbr1 * d.nbr2;
@@ -449,15 +167,20 @@ bool prepare(const GemmDesc& d, KParams& p, bool* empty_k) {
   p.sCo1 = d.sCo1; p.sCo2 = d.sCo2;
   p.nbr1 = d.nbr1;
   p.sAr1 = d.sAr1; p.sAr2 = d.sAr2; p.sBr1 = d.sBr1; p.sBr2 = d.sBr2;
-  p.tiles_m = (d.m + BM - 1) / BM;
-  p.tiles_n = (d.n + BN - 1) / BN;
-  p.tiles_mn = p.tiles_m * p.tiles_n;
   p.ktiles_pb = (d.k + BK - 1) / BK;
   p.ktiles_total = p.ktiles_pb * nbr;
-  int split = d.split;
-  if (split <= 0) split = choose_split(p.tiles_mn * nbo, p.ktiles_total);
-  p.split = static_cast<int>(std::max<long long>(1, std::min<long long>(split, p.ktiles_total)));
   return true;
+}
+
+bool a_vec(const GemmDesc& d) { return vec_ok(d.A, d.lda, d.sAo1, d.sAo2, d.sAr1, d.sAr2); }
+bool b_vec(const GemmDesc& d) { return vec_ok(d.B, d.ldb, d.sBo1, d.sBo2, d.sBr1, d.sBr2); }
+
+// The plan for a given split (at most one per k tile), or for the rule's own
+// choice (split 0).
+Plan make_plan(const GemmDesc& d, const KParams& p, long long split,
+               double max_partials = kMaxPartials) {
+  return choose_plan(d, a_vec(d), b_vec(d),
+                     static_cast<int>(std::min<long long>(split, p.ktiles_total)), max_partials);
 }
 
 void launch_scale_only(const GemmDesc& d, cudaStream_t s) {
@@ -469,21 +192,43 @@ void launch_scale_only(const GemmDesc& d, cudaStream_t s) {
   UW12_LAUNCHED();
 }
 
-// Launches the GEMM (and the split-K reduction when p.split > 1, with
+// Makes the layout's kernels of every tile resident on the current device at
+// the layout's first use there, so that no later size of it loads a kernel.
+void load_layout(int layout) {
+  static bool loaded[64][16] = {};
+  static std::mutex mu;
+  int dev = 0;
+  UW12_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  if (dev < 64 && loaded[dev][layout]) return;
+  for (const TileCost& t : kTiles) t.tile->load(layout);
+  if (dev < 64) loaded[dev][layout] = true;
+}
+
+// Launches the GEMM (and the split-K reduction when the plan splits, with
 // partial tiles in p.work).
-void launch(const GemmDesc& d, const KParams& p, cudaStream_t s) {
-  const long long grid = p.tiles_mn * p.nbo * p.split;
-  const bool va = vec_ok(d.A, d.lda, d.sAo1, d.sAo2, d.sAr1, d.sAr2);
-  const bool vb = vec_ok(d.B, d.ldb, d.sBo1, d.sBo2, d.sBr1, d.sBr2);
-  if (!d.a_kcontig && !d.b_ncontig) launch_layout<false, false>(p, va, vb, grid, s);
-  else if (!d.a_kcontig && d.b_ncontig) launch_layout<false, true>(p, va, vb, grid, s);
-  else if (d.a_kcontig && !d.b_ncontig) launch_layout<true, false>(p, va, vb, grid, s);
-  else launch_layout<true, true>(p, va, vb, grid, s);
+void launch(const GemmDesc& d, KParams p, const Plan& plan, cudaStream_t s) {
+  const DgemmTile& t = *plan.tile;
+  p.tiles_m = (d.m + t.bm - 1) / t.bm;
+  p.tiles_n = (d.n + t.bn - 1) / t.bn;
+  p.tiles_mn = p.tiles_m * p.tiles_n;
+  p.split = plan.split;
+  const int layout = int(d.a_kcontig) | int(d.b_ncontig) << 1 | int(a_vec(d)) << 2 |
+                     int(b_vec(d)) << 3;
+  load_layout(layout);
+  t.launch(p, layout, p.tiles_mn * p.nbo * p.split, s);
   if (p.split > 1) {
     const long long total = d.m * d.n * p.nbo;
     const int blocks = static_cast<int>(std::min<long long>((total + 255) / 256, kSMs * 16));
-    splitk_reduce<<<blocks, 256, 0, s>>>(p.work, p.split, d.m, d.n, p.nbo, d.nbo1, d.alpha,
-                                         d.beta, d.C, d.ldc, d.sCo1, d.sCo2);
+    if (total < (1LL << 31))
+      splitk_reduce<unsigned><<<blocks, 256, 0, s>>>(
+          p.work, p.split, static_cast<unsigned>(d.m), static_cast<unsigned>(d.m * d.n),
+          static_cast<unsigned>(total), static_cast<unsigned>(d.nbo1), d.alpha, d.beta, d.C,
+          d.ldc, d.sCo1, d.sCo2);
+    else
+      splitk_reduce<long long><<<blocks, 256, 0, s>>>(p.work, p.split, d.m, d.m * d.n, total,
+                                                      d.nbo1, d.alpha, d.beta, d.C, d.ldc, d.sCo1,
+                                                      d.sCo2);
     UW12_LAUNCHED();
   }
 }
@@ -554,18 +299,18 @@ void profile_record(int kind, cudaEvent_t a, cudaEvent_t b, double work, std::st
 
 // ---- split-K autotuner ------------------------------------------------------
 //
-// choose_split's wave heuristic picks the split-K factor of a launch from its
-// output CTA count alone.  The autotuner replaces it by measurement: a shape
-// class is (output CTAs = tiles x output batches, power-of-two bucket of the
-// k tiles over all reduction batches); in tuning mode the first automatic-split
-// GEMM of a class not yet in the table is launched once with every candidate
-// split (1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64 while each CTA keeps >= 4 k
-// tiles and the partial tiles stay within 256 MiB or the rule's), each timed with CUDA events on the current stream, and the fastest
-// is recorded and launched last, so C holds its result.  Only GEMMs with
-// beta = 0 are tuned (their repeated launches overwrite C); the others, and
-// every GEMM in "use" mode, take the table's split for their class when it has
-// one and the heuristic otherwise.  Output CTA counts of at least 8 waves never
-// split and are not tuned.
+// choose_plan predicts the split-K factor of a launch.  The autotuner replaces
+// it by measurement: a shape class is (output CTAs = 128 x 128 output tiles x
+// output batches, power-of-two bucket of the k tiles over all reduction
+// batches); in tuning mode the first automatic-split GEMM of a class not yet in
+// the table is launched once with every candidate split (1, 2, 3, 4, 6, 8, 12,
+// 16, 24, 32, 48, 64 while each CTA keeps >= 4 k tiles and the partial tiles stay
+// within 256 MiB or the rule's), each with the tile the cost model picks for it
+// and timed with CUDA events on the current stream, and the fastest is recorded
+// and launched last, so C holds its result.  Only GEMMs with beta = 0 are tuned
+// (their repeated launches overwrite C); the others, and every GEMM in "use"
+// mode, take the table's split for their class when it has one and the rule's
+// otherwise.  Outputs of at least 8 waves of 128 x 128 tiles are not tuned.
 namespace {
 struct TuneKey {
   long long ctas;
@@ -589,35 +334,39 @@ int kbucket_of(long long ktiles_total) {
 }
 
 TuneKey tune_key(long long m, long long n, long long k, long long nbo, long long nbr) {
-  const long long tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN);
+  const long long tiles = ((m + 127) / 128) * ((n + 127) / 128);
   return TuneKey{tiles * nbo, kbucket_of(((k + BK - 1) / BK) * nbr)};
 }
+TuneKey tune_key(const GemmDesc& d) {
+  return tune_key(d.m, d.n, d.k, d.nbo1 * d.nbo2, d.nbr1 * d.nbr2);
+}
 
-// the table's split for p's class, or 0
-int tuned_split(const KParams& p) {
+// the table's split for d's class, or 0
+int tuned_split(const GemmDesc& d) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
   if (g_tune_mode == 0) return 0;
-  auto it = g_tune.find(TuneKey{p.tiles_mn * p.nbo, kbucket_of(p.ktiles_total)});
+  auto it = g_tune.find(tune_key(d));
   return it == g_tune.end() ? 0 : it->second.split;
 }
 
-bool tuning_wanted(const GemmDesc& d, const KParams& p) {
+bool tuning_wanted(const GemmDesc& d) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
   if (g_tune_mode != 1 || d.split > 0 || d.beta != 0.0) return false;
-  if (p.tiles_mn * p.nbo >= 8 * kSMs) return false;
-  return g_tune.find(TuneKey{p.tiles_mn * p.nbo, kbucket_of(p.ktiles_total)}) == g_tune.end();
+  const TuneKey key = tune_key(d);
+  if (key.ctas >= 8 * kSMs) return false;
+  return g_tune.find(key) == g_tune.end();
 }
 
 // Times every candidate split of d (beta = 0) on stream s, records the fastest
 // for the class and leaves C with the result of a launch with it.
 void tune_and_launch(const GemmDesc& d, KParams p, cudaStream_t s) {
-  const int heuristic = choose_split(p.tiles_mn * p.nbo, p.ktiles_total);
+  const int heuristic = make_plan(d, p, 0).split;
   // a candidate's partial tiles stay within 2^25 doubles (256 MiB) or the
   // rule's own, so tuning needs no more memory than the evaluation around it
   const double per_split = double(p.nbo) * double(d.m) * double(d.n);
   const double cap = std::max(double(1LL << 25), per_split * heuristic);
   std::vector<int> cands;
-  for (int c : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64})
+  for (int c : kSplits)
     if (c == 1 || (p.ktiles_total / c >= 4 && per_split * c <= cap)) cands.push_back(c);
   if (std::find(cands.begin(), cands.end(), heuristic) == cands.end()) cands.push_back(heuristic);
   struct Events {  // destroyed on every exit, a failed launch included
@@ -633,16 +382,16 @@ void tune_and_launch(const GemmDesc& d, KParams p, cudaStream_t s) {
   int best = heuristic;
   double best_ms = 1e300;
   for (int c : cands) {
-    p.split = c;
+    const Plan plan = make_plan(d, p, c);
     DevBuf work;
     if (c > 1) {
       work.alloc(static_cast<size_t>(c) * p.nbo * d.m * d.n, s);
       p.work = work.get();
     }
-    launch(d, p, s);  // warm-up (caches, first-launch set-up)
+    launch(d, p, plan, s);  // warm-up (caches, first-launch set-up)
     UW12_CUDA(cudaEventRecord(e0, s));
-    launch(d, p, s);
-    launch(d, p, s);
+    launch(d, p, plan, s);
+    launch(d, p, plan, s);
     UW12_CUDA(cudaEventRecord(e1, s));
     UW12_CUDA(cudaEventSynchronize(e1));
     float ms = 0.f;
@@ -654,15 +403,14 @@ void tune_and_launch(const GemmDesc& d, KParams p, cudaStream_t s) {
   }
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune[TuneKey{p.tiles_mn * p.nbo, kbucket_of(p.ktiles_total)}] = TuneEntry{best, best_ms};
+    g_tune[tune_key(d)] = TuneEntry{best, best_ms};
   }
-  p.split = best;
   DevBuf work;
   if (best > 1) {
     work.alloc(static_cast<size_t>(best) * p.nbo * d.m * d.n, s);
     p.work = work.get();
   }
-  launch(d, p, s);
+  launch(d, p, make_plan(d, p, best), s);
 }
 }  // namespace
 
@@ -748,17 +496,14 @@ void gemm_dmma(const GemmDesc& d) {
     return;
   }
   const bool prof = profile_enabled();
-  if (d.split <= 0) {
-    if (!prof && tuning_wanted(d, p)) {
-      tune_and_launch(d, p, s);
-      return;
-    }
-    if (const int t = tuned_split(p))
-      p.split = static_cast<int>(std::min<long long>(t, p.ktiles_total));
+  if (d.split <= 0 && !prof && tuning_wanted(d)) {
+    tune_and_launch(d, p, s);
+    return;
   }
+  const Plan plan = make_plan(d, p, d.split > 0 ? d.split : tuned_split(d));
   DevBuf work;
-  if (p.split > 1) {
-    work.alloc(static_cast<size_t>(p.split) * p.nbo * d.m * d.n, s);
+  if (plan.split > 1) {
+    work.alloc(static_cast<size_t>(plan.split) * p.nbo * d.m * d.n, s);
     p.work = work.get();
   }
   cudaEvent_t ev_a = nullptr, ev_b = nullptr;
@@ -767,15 +512,14 @@ void gemm_dmma(const GemmDesc& d) {
     UW12_CUDA(cudaEventCreate(&ev_b));
     UW12_CUDA(cudaEventRecord(ev_a, s));
   }
-  launch(d, p, s);
+  launch(d, p, plan, s);
   if (prof) {
     UW12_CUDA(cudaEventRecord(ev_b, s));
     std::lock_guard<std::mutex> lk(g_prof_mu);
     char shape[256];
-    std::snprintf(shape, sizeof(shape), "%lld %lld %lld %lld %lld %d %d%d %d%d", d.m, d.n, d.k,
-                  p.nbo, d.nbr1 * d.nbr2, p.split, int(d.a_kcontig), int(d.b_ncontig),
-                  int(vec_ok(d.A, d.lda, d.sAo1, d.sAo2, d.sAr1, d.sAr2)),
-                  int(vec_ok(d.B, d.ldb, d.sBo1, d.sBo2, d.sBr1, d.sBr2)));
+    std::snprintf(shape, sizeof(shape), "%lld %lld %lld %lld %lld %d %d%d %d%d %dx%d", d.m, d.n,
+                  d.k, p.nbo, d.nbr1 * d.nbr2, plan.split, int(d.a_kcontig), int(d.b_ncontig),
+                  int(a_vec(d)), int(b_vec(d)), plan.tile->bm, plan.tile->bn);
     g_prof_recs.push_back({ev_a, ev_b, 2.0 * double(d.m) * double(d.n) * double(d.k) *
                                            double(p.nbo) * double(d.nbr1 * d.nbr2),
                            shape, kProfDgemm});
@@ -819,18 +563,16 @@ void gemm_noalloc(const GemmDesc& d) {
     return;
   }
   const double per_split = double(p.nbo) * double(d.m) * double(d.n);
-  if (d.split > 1 && per_split * p.split > double(kNoAllocScratchDoubles))
+  // an automatic split keeps its partial tiles within the array (split 1 needs none)
+  const Plan plan = make_plan(d, p, std::max(0, d.split), double(kNoAllocScratchDoubles));
+  if (d.split > 1 && per_split * plan.split > double(kNoAllocScratchDoubles))
     throw Error(kErrInvalid,
                 "gemm_noalloc: split * batches * m * n = " +
-                    std::to_string(static_cast<long long>(per_split * p.split)) +
+                    std::to_string(static_cast<long long>(per_split * plan.split)) +
                     " doubles exceeds the fixed scratch of " +
                     std::to_string(kNoAllocScratchDoubles) + " doubles (16 MiB)");
-  if (p.split > 1 && per_split * p.split > double(kNoAllocScratchDoubles)) {
-    // automatic split: shrink it until the partial tiles fit (split 1 needs none)
-    p.split = static_cast<int>(std::max(1.0, std::floor(kNoAllocScratchDoubles / per_split)));
-  }
-  if (p.split > 1) p.work = noalloc_scratch_for_current_device();
-  launch(d, p, s);
+  if (plan.split > 1) p.work = noalloc_scratch_for_current_device();
+  launch(d, p, plan, s);
 }
 
 }  // namespace uw12b
