@@ -77,6 +77,30 @@ cudaMemPool_t library_pool() {
   return g_pools[dev];
 }
 
+namespace {
+thread_local Arena* t_arena = nullptr;
+}  // namespace
+
+Arena::Arena() {
+  if (t_arena) return;
+  s_ = current_stream();
+  void* p = nullptr;
+  if (cudaMallocFromPoolAsync(&p, kDoubles * sizeof(double), library_pool(), s_) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  base_ = static_cast<double*>(p);
+  t_arena = this;
+}
+
+Arena::~Arena() {
+  if (t_arena != this) return;
+  t_arena = nullptr;
+  cudaFreeAsync(base_, s_);
+}
+
+Arena* Arena::current() { return t_arena; }
+
 void trim_pools() {
   std::lock_guard<std::mutex> lk(g_pool_mu);
   for (int d = 0; d < 64; ++d)
@@ -211,10 +235,27 @@ void run_form_fock(const uw12c_integrals* W, const uw12c_integrals* V, const uw1
   rq.allreduce = uw12b::g_allreduce;
   rq.allreduce_user = uw12b::g_allreduce_user;
   DeviceGuard dg(w.device);
+  auto evaluate = [&] {
+    uw12b::Arena arena;
+    if (adjoint)
+      uw12b::form_fock_adjoint(rq, *adjoint);
+    else
+      uw12b::form_fock(rq);
+  };
+  // an evaluation that hands out gradient blocks or joins collectives is not repeated
+  bool streamed = false;
   if (adjoint)
-    uw12b::form_fock_adjoint(rq, *adjoint);
-  else
-    uw12b::form_fock(rq);
+    for (int i = 0; i < 3; ++i)
+      streamed = streamed || adjoint->sink3[i] || (i < 2 && adjoint->sink3_ri[i]);
+  rq.assume_memory = !streamed && rq.n_shards <= 1;
+  try {
+    evaluate();
+  } catch (const Error& e) {
+    if (e.code != UW12C_ERR_ALLOC || !rq.assume_memory || rq.mem_budget) throw;
+    cudaGetLastError();  // the failed allocation's, which the next launch check would see
+    rq.assume_memory = false;
+    evaluate();
+  }
   check_split_pipeline();
 }
 
@@ -772,7 +813,27 @@ int uw12c_fock_batched(const uw12c_molecule* mols, size_t n, int indirect_term,
     const int moduli = uw12b::split_moduli();
     const double min_flops = uw12b::split_min_flops();
     size_t total_budget = uw12b::g_budget.load();
-    if (!total_budget) {
+    // small molecules: each worker's share of the memory that an evaluation may
+    // assume holds any of them whole, without asking for the free memory
+    // (engine.cuh); a worker that then runs out of memory asks for itself
+    const size_t assumed = uw12b::assumed_doubles() * sizeof(double) / workers;
+    size_t largest = 0;
+    for (size_t i = 0; i < n; ++i) {
+      const uw12c_molecule& m = mols[i];
+      if (!m.W || !m.W->h || !m.V || !m.V->h || !m.WV || !m.WV->h || !m.n_occ || m.n_spin > 2)
+        continue;  // refused by its own evaluation
+      uw12b::FockRequest rq;
+      rq.W = m.W->h.get();
+      rq.V = m.V->h.get();
+      rq.WV = m.WV->h.get();
+      rq.n_ao = m.n_ao;
+      rq.n_occ.assign(m.n_occ, m.n_occ + m.n_spin);
+      rq.indirect = indirect_term != 0;
+      rq.calc_fock = calculate_fock != 0;
+      largest = std::max(largest, uw12b::budget_need(rq, false, false) * sizeof(double));
+    }
+    const bool assume = !total_budget && largest <= assumed;
+    if (!total_budget && !assume) {
       size_t free_b = 0, total_b = 0;
       UW12_CUDA(cudaMemGetInfo(&free_b, &total_b));
       total_budget = static_cast<size_t>(0.45 * double(free_b));
@@ -787,7 +848,7 @@ int uw12c_fock_batched(const uw12c_molecule* mols, size_t n, int indirect_term,
       int dev = -1;
       uw12b::set_split_moduli(moduli);
       uw12b::set_split_min_flops(min_flops);
-      uw12b::g_budget_override = worker_budget;
+      uw12b::g_budget_override = assume ? 0 : worker_budget;
       for (size_t q; (q = next.fetch_add(1)) < n;) {
         const size_t i = order[q];
         const uw12c_molecule& m = mols[i];

@@ -56,16 +56,58 @@ void set_current_stream(cudaStream_t s);
 cudaMemPool_t library_pool();
 void trim_pools();
 
-// Device memory from the library's stream-ordered pool of the current device.
+// One block of the pool that serves the small buffers of an evaluation on this
+// host thread and its current stream: a buffer from it costs no driver call (a
+// stream-ordered allocation and its release cost about 1.5 us of host time, and
+// the smallest evaluations make 80 of them in 0.65 ms).  Buffers are laid one
+// after the other; the last one laid is taken back when it is released, the
+// others with the arena.  All of them are used on the arena's stream only, so
+// memory given out again is reused in stream order.  An arena inside another on
+// the same thread and stream does nothing; without memory for its block it
+// leaves every buffer to the pool.
+class Arena {
+ public:
+  Arena();
+  ~Arena();
+  Arena(const Arena&) = delete;
+  Arena& operator=(const Arena&) = delete;
+
+  // The calling thread's arena (null: none).
+  static Arena* current();
+  // n doubles for stream s, or null when they do not fit.
+  double* take(size_t n_doubles, cudaStream_t s) {
+    const size_t n = (n_doubles + 31) / 32 * 32;  // 256-byte aligned
+    if (s != s_ || n > kDoubles - off_) return nullptr;
+    double* p = base_ + off_;
+    off_ += n;
+    return p;
+  }
+  void give(const double* p, size_t n_doubles) {
+    const size_t n = (n_doubles + 31) / 32 * 32;
+    if (p + n == base_ + off_) off_ -= n;
+  }
+
+ private:
+  static constexpr size_t kDoubles = (size_t(32) << 20) / sizeof(double);  // 32 MiB
+  double* base_ = nullptr;
+  size_t off_ = 0;
+  cudaStream_t s_ = nullptr;
+};
+
+// Device memory from the calling thread's arena, when it fits there, or from the
+// library's stream-ordered pool of the current device.
 class DevBuf {
  public:
   DevBuf() = default;
   explicit DevBuf(size_t n_doubles, cudaStream_t s = nullptr) { alloc(n_doubles, s); }
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
-  DevBuf(DevBuf&& o) noexcept : p_(o.p_), n_(o.n_), s_(o.s_) { o.p_ = nullptr; o.n_ = 0; }
+  DevBuf(DevBuf&& o) noexcept { take(o); }
   DevBuf& operator=(DevBuf&& o) noexcept {
-    if (this != &o) { release(); p_ = o.p_; n_ = o.n_; s_ = o.s_; o.p_ = nullptr; o.n_ = 0; }
+    if (this != &o) {
+      release();
+      take(o);
+    }
     return *this;
   }
   ~DevBuf() { release(); }
@@ -74,25 +116,41 @@ class DevBuf {
     release();
     s_ = s ? s : current_stream();
     n_ = n_doubles;
-    if (n_)
-      UW12_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p_), n_ * sizeof(double),
-                                        library_pool(), s_));
+    if (!n_) return;
+    if (Arena* a = Arena::current()) {
+      p_ = a->take(n_, s_);
+      if (p_) {
+        arena_ = a;
+        return;
+      }
+    }
+    UW12_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p_), n_ * sizeof(double),
+                                      library_pool(), s_));
   }
   void zero() {
     if (n_) UW12_CUDA(cudaMemsetAsync(p_, 0, n_ * sizeof(double), s_));
   }
   void release() noexcept {
-    if (p_) cudaFreeAsync(p_, s_);
+    if (p_ && arena_)
+      arena_->give(p_, n_);
+    else if (p_)
+      cudaFreeAsync(p_, s_);
     p_ = nullptr;
+    arena_ = nullptr;
     n_ = 0;
   }
   double* get() const { return p_; }
   size_t size() const { return n_; }
 
  private:
+  void take(DevBuf& o) noexcept {
+    p_ = o.p_; n_ = o.n_; s_ = o.s_; arena_ = o.arena_;
+    o.p_ = nullptr; o.n_ = 0; o.arena_ = nullptr;
+  }
   double* p_ = nullptr;
   size_t n_ = 0;
   cudaStream_t s_ = nullptr;
+  Arena* arena_ = nullptr;
 };
 
 inline size_t packed_size(size_t n) { return n * (n + 1) / 2; }

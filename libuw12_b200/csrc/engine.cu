@@ -179,23 +179,51 @@ void eigh(double* A, size_t n, double* w) {
   if (hinfo != 0) throw_runtime("eigen-decomposition failed");
 }
 
-// Chunk budget in doubles: the caller's, or `fraction` (45% by default) of
-// the device memory available now (free memory plus what the library's pool
-// holds unused).  The evaluations re-read it at the start of each chunked
-// phase, after the phase's persistent intermediates are allocated.
-size_t auto_budget_doubles(size_t requested_bytes, double fraction = 0.45) {
-  if (requested_bytes)  // an explicit budget may be small (many small chunks)
-    return std::max<size_t>(requested_bytes, size_t(64) << 10) / sizeof(double);
-  size_t free_b = 0, total_b = 0;
-  UW12_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  unsigned long long reserved = 0, used = 0;  // 64-bit pool attributes
-  UW12_CUDA(cudaMemPoolGetAttribute(library_pool(), cudaMemPoolAttrReservedMemCurrent, &reserved));
-  UW12_CUDA(cudaMemPoolGetAttribute(library_pool(), cudaMemPoolAttrUsedMemCurrent, &used));
-  const double avail = double(free_b) + (reserved > used ? double(reserved - used) : 0.0);
-  // the automatic budget never drops below 64 MiB
-  return std::max<size_t>(static_cast<size_t>(fraction * avail), size_t(64) << 20) /
-         sizeof(double);
-}
+// Chunk budget of one evaluation, in doubles: the caller's, or `fraction` (45% by
+// default, at least 64 MiB) of the device memory available now (free memory
+// plus what the library's pool holds unused).  Re-read at the start of each
+// chunked phase, after the phase's persistent intermediates are allocated.
+//
+// Asking for the free memory (cudaMemGetInfo) enters the kernel driver: 90 us on
+// a quiet host, tens of milliseconds while other processes of the host are in
+// it, against 2.5 us for a launch.  So:
+//  * it is asked at most once per evaluation; afterwards the pool's own counters
+//    say how much of that free memory the evaluation has taken;
+//  * an evaluation whose chunks all fit whole in 64 MiB, or in 1/32 of the
+//    device's memory where it may be repeated (assume_memory), asks nothing
+//    (`need`: an upper bound of every size that is compared with a budget, so any
+//    larger budget would give the same chunks).  Should an allocation of the
+//    latter fail, the caller runs it again without the assumption.
+class Budget {
+ public:
+  Budget(size_t requested_bytes, size_t need, bool assume_memory)
+      : requested_(requested_bytes), need_(need) {
+    if (!requested_ && assume_memory) whole_ = std::max(whole_, assumed_doubles());
+  }
+
+  size_t doubles(double fraction = 0.45) {
+    if (requested_)  // an explicit budget may be small (many small chunks)
+      return std::max<size_t>(requested_, size_t(64) << 10) / sizeof(double);
+    if (need_ <= whole_) return whole_;
+    unsigned long long reserved = 0, used = 0;  // 64-bit pool attributes
+    UW12_CUDA(cudaMemPoolGetAttribute(library_pool(), cudaMemPoolAttrReservedMemCurrent, &reserved));
+    UW12_CUDA(cudaMemPoolGetAttribute(library_pool(), cudaMemPoolAttrUsedMemCurrent, &used));
+    if (free0_ < 0.0) {
+      size_t free_b = 0, total_b = 0;
+      UW12_CUDA(cudaMemGetInfo(&free_b, &total_b));
+      free0_ = double(free_b);
+      reserved0_ = double(reserved);
+    }
+    const double free_now = std::max(0.0, free0_ - (double(reserved) - reserved0_));
+    const double avail = free_now + (reserved > used ? double(reserved - used) : 0.0);
+    return std::max<size_t>(static_cast<size_t>(fraction * avail) / sizeof(double), kFloor);
+  }
+
+ private:
+  static constexpr size_t kFloor = (size_t(64) << 20) / sizeof(double);
+  size_t requested_, need_, whole_ = kFloor;
+  double free0_ = -1.0, reserved0_ = 0.0;
+};
 
 inline long long LL(size_t v) { return static_cast<long long>(v); }
 
@@ -286,6 +314,20 @@ size_t aux_step(const IntegralsHandle& X, bool ri, size_t budget) {
 }
 
 }  // namespace
+
+size_t assumed_doubles() {
+  static std::mutex mu;
+  static size_t total[64] = {};
+  int dev = 0;
+  UW12_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return 0;
+  std::lock_guard<std::mutex> lk(mu);
+  if (!total[dev]) {
+    size_t free_b = 0;
+    UW12_CUDA(cudaMemGetInfo(&free_b, &total[dev]));
+  }
+  return total[dev] / 32 / sizeof(double);
+}
 
 // --------------------------------------------------------------------------
 // handles
@@ -582,17 +624,17 @@ void transform_ao(const IntegralsHandle& X, const double* Cm, size_t nc, double*
 
 // Chunk size c <= max_chunk (in units of `unit` GEMM columns) for a loop over
 // `total` units: the chunked GEMMs have n = unit * c columns, so c is chosen
-// to fill the 128-wide column tiles over the whole loop (fewest wasted
-// columns, then the largest chunk).
+// to fill 64-wide column tiles over the whole loop (fewest wasted columns, then
+// the largest chunk).
 size_t tile_chunk(size_t total, size_t unit, size_t max_chunk) {
   max_chunk = std::max<size_t>(1, std::min(max_chunk, total));
-  auto tiles = [](size_t cols) { return (cols + 127) / 128; };
+  auto tiles = [](size_t cols) { return (cols + 63) / 64; };
   size_t best = max_chunk;
   double best_fill = -1.0;
   for (size_t c = max_chunk; c >= std::max<size_t>(1, max_chunk / 2); --c) {
     const size_t full = total / c, rem = total % c;
     const size_t used = full * tiles(unit * c) + (rem ? tiles(unit * rem) : 0);
-    const double fill = double(total * unit) / double(used * 128);
+    const double fill = double(total * unit) / double(used * 64);
     if (fill > best_fill + 1e-9) {
       best_fill = fill;
       best = c;
@@ -608,12 +650,11 @@ struct SpinDims {
 
 // Occupation-weighted occupied orbitals Co (utils.hpp:289-310) of both spins side
 // by side (N x o_tot) and their active (last n_active) columns Ca (freeze_core,
-// utils.hpp:235-253; N x a_tot), on the device.
+// utils.hpp:235-253; N x a_tot), one after the other on the device.
 void upload_orbitals(const FockRequest& rq, std::vector<SpinDims>& sd, size_t& o_tot,
-                     size_t& a_tot, DevBuf& Co, DevBuf& Ca) {
+                     size_t& a_tot, DevBuf& C) {
   const int ns = rq.n_spin;
   const size_t N = rq.n_ao;
-  cudaStream_t st = current_stream();
   sd.assign(ns, SpinDims{});
   o_tot = a_tot = 0;
   for (int s = 0; s < ns; ++s) {
@@ -625,27 +666,22 @@ void upload_orbitals(const FockRequest& rq, std::vector<SpinDims>& sd, size_t& o
     o_tot += sd[s].o;
     a_tot += sd[s].a;
   }
-  Co.alloc(N * o_tot);
-  Ca.alloc(N * a_tot);
-  DevBuf wts(o_tot);
-  std::vector<double> w(o_tot);
+  // [Co | Ca] is weighted on the host and copied at once
+  std::vector<double> c(N * (o_tot + a_tot));
   const double per = (ns == 1) ? 2.0 : 1.0;
   for (int s = 0; s < ns; ++s)
-    for (size_t k = 0; k < sd[s].o; ++k) w[sd[s].ooff + k] = std::sqrt(rq.occ[s][k] / per);
-  if (o_tot)
-    UW12_CUDA(cudaMemcpyAsync(wts.get(), w.data(), o_tot * sizeof(double), cudaMemcpyHostToDevice,
-                              st));
-  for (int s = 0; s < ns; ++s) {
-    if (!sd[s].o) continue;
-    UW12_CUDA(cudaMemcpy2DAsync(Co.get() + N * sd[s].ooff, N * sizeof(double), rq.C[s],
-                                rq.ldc[s] * sizeof(double), N * sizeof(double), sd[s].o,
-                                cudaMemcpyHostToDevice, st));
-  }
-  if (o_tot) scale_rc(Co.get(), LL(N), LL(N), LL(o_tot), nullptr, wts.get(), 1.0, Co.get(), LL(N));
-  for (int s = 0; s < ns; ++s)
-    if (sd[s].a)
-      UW12_CUDA(cudaMemcpyAsync(Ca.get() + N * sd[s].aoff, Co.get() + N * (sd[s].ooff + sd[s].c),
-                                N * sd[s].a * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    for (size_t k = 0; k < sd[s].o; ++k) {
+      const double w = std::sqrt(rq.occ[s][k] / per);
+      const double* src = rq.C[s] + rq.ldc[s] * k;
+      double* dst = c.data() + N * (sd[s].ooff + k);
+      for (size_t i = 0; i < N; ++i) dst[i] = w * src[i];
+      if (k >= sd[s].c)
+        std::copy(dst, dst + N, c.data() + N * (o_tot + sd[s].aoff + k - sd[s].c));
+    }
+  C.alloc(c.size());
+  if (!c.empty())
+    UW12_CUDA(cudaMemcpyAsync(C.get(), c.data(), c.size() * sizeof(double),
+                              cudaMemcpyHostToDevice, current_stream()));
 }
 
 }  // namespace
@@ -653,6 +689,31 @@ void upload_orbitals(const FockRequest& rq, std::vector<SpinDims>& sd, size_t& o
 // --------------------------------------------------------------------------
 // form_fock
 // --------------------------------------------------------------------------
+size_t budget_need(const FockRequest& rq, bool adjoint, bool streamed) {
+  const size_t N = rq.n_ao, np = packed_size(N), R = rq.W->n_ri, Rp = N + R;
+  const size_t M = std::max({rq.W->n_df, rq.V->n_df, rq.WV->n_df});
+  bool stored = rq.W->J3_0.get() && rq.V->J3_0.get() && rq.WV->J3_0.get() &&
+                rq.W->J3_ri_0.get() && rq.V->J3_ri_0.get();
+  size_t o = 0, o1 = 0;  // occupied orbitals of all spins, of the larger spin
+  for (size_t n : rq.n_occ) {
+    o += n;
+    o1 = std::max(o1, n);
+  }
+  // aux blocks of unstored tensors and of streamed gradients
+  const size_t blocks = stored && !streamed ? 0 : 16 * (np + R * N) * M;
+  size_t need = blocks + 2 * (N * N + np) * M;                           // unpacked AO blocks
+  need = std::max(need, (2 * (N + o1) + 3 * Rp) * o * M);                // whole transforms
+  if (rq.calc_fock) need = std::max(need, blocks + (4 * N * N + Rp * N + 2 * R * N + np) * M);
+  if (rq.indirect) {
+    need = std::max(need, (3 * Rp * o1 + M) * o1 * o1);                  // pair products of energies
+    if (rq.calc_fock)
+      need = std::max(need, blocks + o1 * o1 * (2 * Rp * N + N * N + R * N + np));
+  }
+  if (adjoint)
+    need = std::max({need, 2 * (N + R + 2 * (o1 + 2 * Rp)) * o * M, (4 * N * N + N * o) * M});
+  return need;
+}
+
 void form_fock(const FockRequest& rq) {
   const IntegralsHandle& W = *rq.W;
   const IntegralsHandle& V = *rq.V;
@@ -670,7 +731,8 @@ void form_fock(const FockRequest& rq) {
   const double two = (ns == 1) ? 2.0 : 1.0;
   const double kap4 = 2.0 * half;
   cudaStream_t st = current_stream();
-  size_t budget = auto_budget_doubles(rq.mem_budget);
+  Budget budgets(rq.mem_budget, budget_need(rq, false, false), rq.assume_memory);
+  size_t budget = budgets.doubles();
   // Sharding: aux functions and occupied orbitals are dealt out in
   // contiguous, balanced ranges (part).  The fitted densities, the MO
   // transforms and the 2-el Fock run over this shard's aux range, and the
@@ -700,9 +762,11 @@ void form_fock(const FockRequest& rq) {
   size_t o_tot = 0, a_tot = 0;
   PhaseClock clock;
   clock.mark("orbitals");
-  DevBuf Co, Ca;
-  upload_orbitals(rq, sd, o_tot, a_tot, Co, Ca);
-  auto Ca_s = [&](int s) { return Ca.get() + N * sd[s].aoff; };
+  DevBuf orbs;
+  upload_orbitals(rq, sd, o_tot, a_tot, orbs);
+  const double* const Co = orbs.get();
+  const double* const Ca = Co + N * o_tot;
+  auto Ca_s = [&](int s) { return Ca + N * sd[s].aoff; };
 
   DevBuf acc(kSlots);
   acc.zero();
@@ -760,7 +824,7 @@ void form_fock(const FockRequest& rq) {
       // B1 of the active orbitals: the shard's aux range of sq(J3_0) Ca times
       // the matching rows of P2, summed over the shards
       DevBuf H(N * a_tot * (xhi - xlo));
-      transform_ao(WV, Ca.get(), a_tot, H.get(), budget / 2, xlo, xhi);
+      transform_ao(WV, Ca, a_tot, H.get(), budget / 2, xlo, xhi);
       for (int s = 0; s < ns; ++s) {
         const size_t a = sd[s].a;
         if (!a) continue;
@@ -801,7 +865,7 @@ void form_fock(const FockRequest& rq) {
   // direct Fock, which are sums over orbitals: when the whole intermediates
   // (B1, B2, Wst of W and V, S^-1 Wst_V) exceed the chunk budget they are
   // formed for a chunk of orbitals at a time instead (orbital_chunked).
-  budget = auto_budget_doubles(rq.mem_budget);
+  budget = budgets.doubles();
   size_t whole = 0;
   for (int s = 0; s < ns; ++s)
     whole += 2 * (N * sd[s].o * MW + sd[s].a * sd[s].o * MW) + 3 * Rp * sd[s].a * MW;
@@ -821,7 +885,7 @@ void form_fock(const FockRequest& rq) {
     const IntegralsHandle& X = which == 0 ? W : V;
     PerX& P = which == 0 ? XW : XV;
     const size_t M = X.n_df;
-    budget = auto_budget_doubles(rq.mem_budget);
+    budget = budgets.doubles();
     P.B1.resize(ns);
     P.B2.resize(ns);
     P.Wst.resize(ns);
@@ -831,7 +895,7 @@ void form_fock(const FockRequest& rq) {
     const auto [xlo, xhi] = part(M);
     {
       DevBuf H(N * o_tot * (xhi - xlo));
-      transform_ao(X, Co.get(), o_tot, H.get(), budget / 2, xlo, xhi);
+      transform_ao(X, Co, o_tot, H.get(), budget / 2, xlo, xhi);
       for (int s = 0; s < ns; ++s) {
         const size_t o = sd[s].o;
         if (!o) continue;
@@ -842,7 +906,7 @@ void form_fock(const FockRequest& rq) {
       }
     }
     DevBuf H2(R * a_tot * (xhi - xlo));
-    if (a_tot) ri_transform(X, Ca.get(), a_tot, H2.get(), budget, xlo, xhi);
+    if (a_tot) ri_transform(X, Ca, a_tot, H2.get(), budget, xlo, xhi);
     for (int s = 0; s < ns; ++s) {
       const size_t o = sd[s].o, a = sd[s].a, c = sd[s].c;
       if (!a) continue;
@@ -886,7 +950,7 @@ void form_fock(const FockRequest& rq) {
   auto b1_chunk = [&](const IntegralsHandle& X, int s, size_t k0, size_t nk, DevBuf& out) {
     const size_t M = X.n_df;
     DevBuf H(N * nk * M);
-    transform_ao(X, Co.get() + N * (sd[s].ooff + k0), nk, H.get(), budget / 2);
+    transform_ao(X, Co + N * (sd[s].ooff + k0), nk, H.get(), budget / 2);
     out.alloc(N * nk * M);
     gemm(gemm_nn(LL(N * nk), LL(M), LL(M), 1.0, H.get(), LL(N * nk), X.P2.get(), LL(M), 0.0,
                  out.get(), LL(N * nk)));
@@ -924,7 +988,7 @@ void form_fock(const FockRequest& rq) {
           St[which].alloc(Rp * nj * M);
           // AO rows of orbital j: sq(J3_0) Co[:, c + j] P2, into rows [0, N) of its block
           DevBuf H(N * nj * M);
-          transform_ao(X, Co.get() + N * (sd[s].ooff + c + j0), nj, H.get(), budget / 2);
+          transform_ao(X, Co + N * (sd[s].ooff + c + j0), nj, H.get(), budget / 2);
           GemmDesc ga = gemm_nn(LL(N), LL(M), LL(M), 1.0, H.get(), LL(N * nj), X.P2.get(), LL(M),
                                 0.0, St[which].get(), LL(Rp * nj));
           ga.nbo1 = LL(nj);
@@ -1123,7 +1187,7 @@ void form_fock(const FockRequest& rq) {
       // contraction length of the p GEMM, whose output is large), its AO
       // blocks up to a sixteenth, the chunk the rest; unstored W blocks add
       // to the chunk's share.
-      budget = auto_budget_doubles(rq.mem_budget, 0.7);
+      budget = budgets.doubles(0.7);
       const size_t vstep = aux_step(V, false, budget / 4), vrstep = aux_step(V, true, budget);
       const size_t vscr = (V.J3_0.get() ? 0 : np * vstep) + (V.J3_ri_0.get() ? 0 : R * N * vrstep);
       const size_t per_a = 2 * N * N + Rp * N + R * N + (W.J3_0.get() ? 0 : np);
@@ -1227,7 +1291,7 @@ void form_fock(const FockRequest& rq) {
       clock.mark("ss_3el_energy");
       // ---- 3-el indirect energy (indirect_utils.cpp:101-133), chunked over k
       {
-        budget = auto_budget_doubles(rq.mem_budget);
+        budget = budgets.doubles();
         const size_t per_k = 2 * Rp * a * a;
         const auto [klo, khi] = part(o);
         const size_t kc = tile_chunk(khi - klo, a,
@@ -1298,7 +1362,7 @@ void form_fock(const FockRequest& rq) {
                     xhV.get(), LL(MV));
         g.b_ncontig = true;
         gemm(g);
-        budget = auto_budget_doubles(rq.mem_budget);
+        budget = budgets.doubles();
         // unstored W / V blocks (accumulated over, for every k chunk) take at
         // most an eighth of the budget each
         size_t xscr = 0;
@@ -1500,16 +1564,21 @@ void form_fock_adjoint(const FockRequest& rq_in, const AdjointOutputs& out) {
   const size_t R = W.n_ri, Rp = N + R;
   const double two = (ns == 1) ? 2.0 : 1.0;
   cudaStream_t st = current_stream();
-  size_t budget = auto_budget_doubles(rq.mem_budget);
+  const bool streamed = out.sink3[0] || out.sink3[1] || out.sink3[2] || out.sink3_ri[0] ||
+                        out.sink3_ri[1];
+  Budget budgets(rq.mem_budget, budget_need(rq, true, streamed), rq.assume_memory);
+  size_t budget = budgets.doubles();
   double F[2][2] = {{0, 0}, {0, 0}};
   for (int s = 0; s < ns; ++s)
     for (int sp = 0; sp < ns; ++sp) F[s][sp] = spin_factor(ns, s, sp, rq.s_os, rq.s_ss);
 
   std::vector<SpinDims> sd;
   size_t o_tot = 0, a_tot = 0;
-  DevBuf Co, Ca;
-  upload_orbitals(rq, sd, o_tot, a_tot, Co, Ca);
-  auto Ca_s = [&](int s) { return Ca.get() + N * sd[s].aoff; };
+  DevBuf orbs;
+  upload_orbitals(rq, sd, o_tot, a_tot, orbs);
+  const double* const Co = orbs.get();
+  const double* const Ca = Co + N * o_tot;
+  auto Ca_s = [&](int s) { return Ca + N * sd[s].aoff; };
 
   // output targets: the caller's device buffers, or device staging for host outputs
   std::vector<std::pair<DevBuf, double*>> staged;
@@ -1540,13 +1609,13 @@ void form_fock_adjoint(const FockRequest& rq_in, const AdjointOutputs& out) {
   size_t whole = (N * o_tot + R * a_tot) * Mmax;
   for (int s = 0; s < ns; ++s)
     whole += 2 * (sd[s].a * sd[s].o + 2 * Rp * sd[s].a) * Mmax;
-  const bool orbital_chunked = !same_spin && whole > auto_budget_doubles(rq.mem_budget, 0.9);
+  const bool orbital_chunked = !same_spin && whole > budgets.doubles(0.9);
   // B1 (N*nk x M) of occupied orbitals [k0, k0 + nk) of spin s for potential X:
   // sq(J3_0[:, A]) Co[:, k] P2
   auto b1_chunk = [&](const IntegralsHandle& X, int s, size_t k0, size_t nk, DevBuf& dst) {
     const size_t M = X.n_df;
     DevBuf H(N * nk * M);
-    transform_ao(X, Co.get() + N * (sd[s].ooff + k0), nk, H.get(), budget / 2);
+    transform_ao(X, Co + N * (sd[s].ooff + k0), nk, H.get(), budget / 2);
     dst.alloc(N * nk * M);
     gemm(gemm_nn(LL(N * nk), LL(M), LL(M), 1.0, H.get(), LL(N * nk), X.P2.get(), LL(M), 0.0,
                  dst.get(), LL(N * nk)));
@@ -1558,7 +1627,7 @@ void form_fock_adjoint(const FockRequest& rq_in, const AdjointOutputs& out) {
     const size_t M = X.n_df;
     {
       DevBuf H(N * nj * M);
-      transform_ao(X, Co.get() + N * (sd[s].ooff + sd[s].c + j0), nj, H.get(), budget / 2);
+      transform_ao(X, Co + N * (sd[s].ooff + sd[s].c + j0), nj, H.get(), budget / 2);
       GemmDesc ga = gemm_nn(LL(N), LL(M), LL(M), 1.0, H.get(), LL(N * nj), X.P2.get(), LL(M),
                             0.0, St, LL(Rp * nj));
       ga.nbo1 = LL(nj);
@@ -1593,11 +1662,11 @@ void form_fock_adjoint(const FockRequest& rq_in, const AdjointOutputs& out) {
     P.B2.resize(ns);
     P.Wst.resize(ns);
     P.SW.resize(ns);
-    budget = auto_budget_doubles(rq.mem_budget);
+    budget = budgets.doubles();
     DevBuf H(N * o_tot * M);
-    transform_ao(X, Co.get(), o_tot, H.get(), budget / 2);
+    transform_ao(X, Co, o_tot, H.get(), budget / 2);
     DevBuf H2(R * a_tot * M);
-    if (a_tot) ri_transform(X, Ca.get(), a_tot, H2.get(), budget);
+    if (a_tot) ri_transform(X, Ca, a_tot, H2.get(), budget);
     for (int s = 0; s < ns; ++s) {
       const size_t o = sd[s].o, a = sd[s].a, c = sd[s].c;
       if (!a) continue;
@@ -1754,7 +1823,7 @@ void form_fock_adjoint(const FockRequest& rq_in, const AdjointOutputs& out) {
                LL(ao));
       // three-electron, chunks of occupied orbitals k
       {
-        budget = auto_budget_doubles(rq.mem_budget);
+        budget = budgets.doubles();
         const size_t per_k = 3 * Ra * a + a * std::max(MW, MV);
         const size_t kc = tile_chunk(o, a, std::max<size_t>(1, std::min(o, budget / per_k)));
         DevBuf TY(Ra * MW), TZ(Ra * MV), Tmp(Ra * a * kc), GY(Ra * a * kc), GZ(Ra * a * kc),
@@ -1861,7 +1930,7 @@ void form_fock_adjoint(const FockRequest& rq_in, const AdjointOutputs& out) {
     DevBuf Bb1(N * o_tot * M), Bbri;
     Bb1.zero();  // the columns of spins without active orbitals stay zero
     if (want_ri && a_tot) Bbri.alloc(R * a_tot * M);
-    budget = auto_budget_doubles(rq.mem_budget);
+    budget = budgets.doubles();
     for (int s = 0; s < ns; ++s) {
       const size_t o = sd[s].o, a = sd[s].a, c = sd[s].c;
       if (!a) continue;
@@ -1925,7 +1994,7 @@ void form_fock_adjoint(const FockRequest& rq_in, const AdjointOutputs& out) {
                               X.P2.get() + a0, LL(M), 0.0, Bb10.get(), LL(N * o_tot));
         gp.b_ncontig = true;
         gemm(gp);
-        GemmDesc g = gemm_nn(LL(N), LL(N), LL(o_tot), 1.0, Bb10.get(), LL(N), Co.get(), LL(N), 0.0,
+        GemmDesc g = gemm_nn(LL(N), LL(N), LL(o_tot), 1.0, Bb10.get(), LL(N), Co, LL(N), 0.0,
                              G.get(), LL(N));
         g.b_ncontig = true;
         g.nbo1 = LL(na);
@@ -1960,7 +2029,7 @@ void form_fock_adjoint(const FockRequest& rq_in, const AdjointOutputs& out) {
         for (size_t b0 = 0; b0 < M; b0 += step) {
           const size_t nb = std::min(step, M - b0);
           GemmDesc g = gemm_nn(LL(R), LL(N), LL(a_tot), 1.0, Bbri0.get() + R * a_tot * b0, LL(R),
-                               Ca.get(), LL(N), 0.0, g3ri ? g3ri + rows * b0 : Rk.get(), LL(R));
+                               Ca, LL(N), 0.0, g3ri ? g3ri + rows * b0 : Rk.get(), LL(R));
           g.b_ncontig = true;
           g.nbo1 = LL(nb);
           g.sAo1 = LL(R * a_tot);
@@ -1980,7 +2049,7 @@ void form_fock_adjoint(const FockRequest& rq_in, const AdjointOutputs& out) {
     const GradSink& s3 = out.sink3[which];
     const GradSink& s3ri = out.sink3_ri[which];
     if (!g3 && !g3ri && !s3 && !s3ri) continue;
-    budget = auto_budget_doubles(rq.mem_budget);
+    budget = budgets.doubles();
     DevBuf Bb1(N * o_tot * M), Bbri(R * a_tot * M);
     Bb1.zero();
     for (int s = 0; s < ns; ++s) {
@@ -2044,7 +2113,7 @@ void form_fock_adjoint(const FockRequest& rq_in, const AdjointOutputs& out) {
       for (size_t a0 = 0; a0 < M; a0 += ac) {
         const size_t na = std::min(ac, M - a0);
         GemmDesc g = gemm_nn(LL(N), LL(N), LL(o_tot), 1.0, Bb10.get() + N * o_tot * a0, LL(N),
-                             Co.get(), LL(N), 0.0, G.get(), LL(N));
+                             Co, LL(N), 0.0, G.get(), LL(N));
         g.b_ncontig = true;
         g.nbo1 = LL(na);
         g.sAo1 = LL(N * o_tot);
@@ -2077,7 +2146,7 @@ void form_fock_adjoint(const FockRequest& rq_in, const AdjointOutputs& out) {
         for (size_t b0 = 0; b0 < M; b0 += step) {
           const size_t nb = std::min(step, M - b0);
           GemmDesc g = gemm_nn(LL(R), LL(N), LL(a_tot), 1.0, Bbri0.get() + R * a_tot * b0, LL(R),
-                               Ca.get(), LL(N), 0.0, g3ri ? g3ri + rows * b0 : Rk.get(), LL(R));
+                               Ca, LL(N), 0.0, g3ri ? g3ri + rows * b0 : Rk.get(), LL(R));
           g.b_ncontig = true;
           g.nbo1 = LL(nb);
           g.sAo1 = LL(R * a_tot);
@@ -2164,9 +2233,9 @@ void form_fock_adjoint(const FockRequest& rq_in, const AdjointOutputs& out) {
     const double gs = two * rq.s_ss;
     ssAX.alloc(MX * MX);
     ssAX.zero();
-    budget = auto_budget_doubles(rq.mem_budget);
+    budget = budgets.doubles();
     DevBuf H(N * a_tot * MX);
-    transform_ao(WV, Ca.get(), a_tot, H.get(), budget / 2);
+    transform_ao(WV, Ca, a_tot, H.get(), budget / 2);
     for (int s = 0; s < ns; ++s) {
       const size_t a = sd[s].a;
       if (!a) continue;

@@ -99,6 +99,9 @@ struct FockRequest {
   bool fock_device = false;         // fock points to device memory
   double* terms = nullptr;          // host: {E2, E3, E4} or null
   size_t mem_budget = 0;            // bytes for chunked intermediates (0 = auto)
+  // Chunks that fit assumed_doubles() whole are laid out without asking for the
+  // free memory; on a failed allocation the caller evaluates again with false.
+  bool assume_memory = false;
   size_t shard = 0, n_shards = 1;   // partial evaluation: this shard's share only
   // Sum over the shards of a device buffer (in place, ordered on `stream`),
   // called at the same points, with the same counts, on every shard; needed
@@ -108,6 +111,15 @@ struct FockRequest {
 };
 
 void form_fock(const FockRequest& rq);
+
+// Memory (doubles) that an evaluation may assume to be there: 1/32 of the
+// current device's.
+size_t assumed_doubles();
+// An upper bound (doubles) of every size that form_fock and form_fock_adjoint
+// compare with a chunk budget: the largest of what each chunked phase would
+// hold unchunked, times the share of the budget it is given.  `streamed`: some
+// three-index gradient leaves in blocks.
+size_t budget_need(const FockRequest& rq, bool adjoint, bool streamed);
 
 // Reverse mode of form_fock: the gradient of its energy (the direct terms, and
 // with rq.indirect the same-spin terms too) with respect to the stored
