@@ -552,7 +552,7 @@ class PhaseClock {
   std::vector<std::pair<std::string, cudaEvent_t>> marks_;
 };
 
-enum Slot { kE2d = 0, kE2i = 1, kE3d = 2, kE3i = 3, kE4d = 4, kE4i = 5, kSlots = 8 };
+enum Slot { kE2d = 0, kE2i = 1, kE3d = 2, kE3i = 3, kE4d = 4, kE4i = 5 };
 
 double spin_factor(int ns, int s, int sp, double s_os, double s_ss) {
   // four_electron_utils.cpp:9-30
@@ -768,7 +768,7 @@ void form_fock(const FockRequest& rq) {
   const double* const Ca = Co + N * o_tot;
   auto Ca_s = [&](int s) { return Ca + N * sd[s].aoff; };
 
-  DevBuf acc(kSlots);
+  DevBuf acc(kAccDoubles);
   acc.zero();
   std::vector<DevBuf> Fp(ns);
   for (int s = 0; s < ns; ++s) {
@@ -1461,7 +1461,7 @@ void form_fock(const FockRequest& rq) {
   // energies and the symmetrised Fock matrix
   // =====================================================================
   clock.mark("finish");
-  double e[kSlots];
+  double e[kAccSlots];
   UW12_CUDA(cudaMemcpyAsync(e, acc.get(), sizeof(e), cudaMemcpyDeviceToHost, st));
   if (rq.fock && calc) {
     double* dst = rq.fock;

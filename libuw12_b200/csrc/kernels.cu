@@ -15,20 +15,60 @@ inline int grid_for(long long total, int per_sm = 16) {
 
 __device__ __forceinline__ long long tri(long long i) { return i * (i + 1) / 2; }
 
-__global__ void k_unpack_sym(const double* __restrict__ P, long long ldp, long long n,
-                             long long ncols, double* out, long long ldo, long long so,
-                             double alpha, double beta) {
-  const long long nn = n * n;
-  const long long total = nn * ncols;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long c = idx / nn;
-    const long long e = idx - c * nn;
-    const long long i = e % n, j = e / n;
-    const long long pi = (i >= j) ? tri(i) + j : tri(j) + i;
-    const double v = alpha * P[pi + ldp * c];
-    double* dst = out + i + ldo * j + so * c;
-    *dst = (beta == 0.0) ? v : v + beta * (*dst);
+// Tile t of the lower triangle of a matrix of 32 x 32 tiles -> tile row and
+// column (tj <= ti), t = ti (ti + 1) / 2 + tj.
+__device__ __forceinline__ void lower_tile(int t, int& ti, int& tj) {
+  ti = static_cast<int>((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
+  while (ti * (ti + 1) / 2 > t) --ti;
+  while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
+  tj = t - ti * (ti + 1) / 2;
+}
+
+// Bound by HBM: every packed element is read once and written to both halves.
+// A block takes one 32 x 32 tile of the lower triangle of one column: its rows
+// are contiguous in the packed storage and in the upper half of the output, and
+// go to the lower half through shared memory, so all three streams are
+// coalesced (an element per thread instead reads the packed rows of half of the
+// output at a stride, and divides twice in 64 bits per element: 300 x 300 x 900
+// 0.34 -> 0.19 ms, 5.1 TB/s).
+__global__ void __launch_bounds__(256) k_unpack_sym(const double* __restrict__ P, long long ldp,
+                                                    int n, long long ncols, double* out,
+                                                    long long ldo, long long so, double alpha,
+                                                    double beta) {
+  __shared__ double tile[32][33];
+  int ti, tj;
+  lower_tile(blockIdx.x, ti, tj);
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int i0 = ti * 32, j0 = tj * 32;
+  for (long long c = blockIdx.y; c < ncols; c += gridDim.y) {
+    const double* p = P + ldp * c;
+    double* o = out + so * c;
+    double v[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int i = i0 + ty + 8 * r, j = j0 + tx;
+      v[r] = (i < n && j <= i) ? alpha * p[tri(i) + j] : 0.0;
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int i = i0 + ty + 8 * r, j = j0 + tx;
+      tile[ty + 8 * r][tx] = v[r];
+      if (i < n && j <= i) {
+        double* d = o + j + ldo * i;
+        *d = beta == 0.0 ? v[r] : v[r] + beta * *d;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int i = i0 + tx, j = j0 + ty + 8 * r;
+      if (i < n && j < i) {
+        const double w = tile[tx][ty + 8 * r];
+        double* d = o + i + ldo * j;
+        *d = beta == 0.0 ? w : w + beta * *d;
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -48,13 +88,14 @@ __global__ void k_pack_density(const double* __restrict__ C, long long ldc, long
   }
 }
 
+template <typename I>
 __global__ void k_scale_rc(const double* __restrict__ X, long long ldx, long long rows,
                            long long cols, const double* __restrict__ r,
                            const double* __restrict__ c, double alpha, double* Y, long long ldy) {
-  const long long total = rows * cols;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long i = idx % rows, j = idx / rows;
+  const I nr = static_cast<I>(rows), total = nr * static_cast<I>(cols);
+  for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
+       idx += static_cast<I>(gridDim.x) * blockDim.x) {
+    const I j = idx / nr, i = idx - j * nr;
     double v = alpha * X[i + ldx * j];
     if (r) v *= r[i];
     if (c) v *= c[j];
@@ -62,15 +103,16 @@ __global__ void k_scale_rc(const double* __restrict__ X, long long ldx, long lon
   }
 }
 
+template <typename I>
 __global__ void k_copy3d(const double* __restrict__ src, long long s1, long long s2, double* dst,
                          long long d1, long long d2, long long n0, long long n1, long long n2,
                          double alpha, double beta) {
-  const long long total = n0 * n1 * n2;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long i = idx % n0;
-    const long long rest = idx / n0;
-    const long long j = rest % n1, l = rest / n1;
+  const I m0 = static_cast<I>(n0), m1 = static_cast<I>(n1);
+  const I total = m0 * m1 * static_cast<I>(n2);
+  for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
+       idx += static_cast<I>(gridDim.x) * blockDim.x) {
+    const I rest = idx / m0, i = idx - rest * m0;
+    const I l = rest / m1, j = rest - l * m1;
     double* d = dst + i + d1 * j + d2 * l;
     const double v = alpha * src[i + s1 * j + s2 * l];
     *d = beta != 0.0 ? v + beta * *d : v;
@@ -93,49 +135,71 @@ __device__ __forceinline__ double block_sum(double v) {
   return s;
 }
 
+// acc[slot] += coef * (sum of every block's s): the block that takes the last
+// ticket adds the partial sums in a fixed order and hands the ticket back.  One
+// launch instead of a second single-thread kernel whose serial sum of up to 592
+// partials took longer (7.6 us) than the products (4.1 us at 500 x 500).
+__device__ __forceinline__ void finish_reduction(double s, double* partials, double coef,
+                                                 double* acc, int slot) {
+  __shared__ bool last;
+  unsigned* ticket = reinterpret_cast<unsigned*>(acc + kAccSlots);
+  s = block_sum(s);
+  if (threadIdx.x == 0) {
+    partials[blockIdx.x] = s;
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double v = 0.0;
+  for (unsigned q = threadIdx.x; q < gridDim.x; q += kT) v += __ldcg(partials + q);
+  v = block_sum(v);
+  if (threadIdx.x == 0) {
+    acc[slot] += coef * v;
+    *ticket = 0u;
+  }
+}
+
+template <typename I>
 __global__ void k_wdot(const double* __restrict__ x, long long ldx, const double* __restrict__ y,
                        long long ldy, long long rows, long long cols, const double* __restrict__ rw,
-                       const double* __restrict__ cw, double* partials) {
-  const long long total = rows * cols;
+                       const double* __restrict__ cw, double* partials, double coef, double* acc,
+                       int slot) {
+  const I nr = static_cast<I>(rows), total = nr * static_cast<I>(cols);
   double s = 0.0;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long i = idx % rows, j = idx / rows;
+  for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
+       idx += static_cast<I>(gridDim.x) * blockDim.x) {
+    const I j = idx / nr, i = idx - j * nr;
     double v = x[i + ldx * j] * y[i + ldy * j];
     if (rw) v *= rw[i];
     if (cw) v *= cw[j];
     s += v;
   }
-  s = block_sum(s);
-  if (threadIdx.x == 0) partials[blockIdx.x] = s;
+  finish_reduction(s, partials, coef, acc, slot);
 }
 
-__global__ void k_finish(const double* partials, int n, double coef, double* acc, int slot) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (int q = 0; q < n; ++q) s += partials[q];
-    acc[slot] += coef * s;
-  }
-}
-
+template <typename I>
 __global__ void k_permdot_4el(const double* __restrict__ X, const double* __restrict__ Y,
-                              long long a, long long o, double* partials) {
+                              long long a, long long o, double* partials, double coef,
+                              double* acc, int slot) {
+  const I na = static_cast<I>(a), nao = na * static_cast<I>(o);
+  const I total = nao * nao;  // (i, l, j, k)
   const long long ao = a * o;
-  const long long total = ao * ao;  // (i, l, j, k)
   double s = 0.0;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long row = idx % ao, col = idx / ao;  // row = i + a*l, col = j + a*k
-    const long long i = row % a, l = row / a, j = col % a, k = col / a;
+  for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
+       idx += static_cast<I>(gridDim.x) * blockDim.x) {
+    const I col = idx / nao, row = idx - col * nao;  // row = i + a*l, col = j + a*k
+    const I l = row / na, i = row - l * na, k = col / na, j = col - k * na;
     s += X[row + ao * col] * Y[(i + a * k) + ao * (j + a * l)];
   }
-  s = block_sum(s);
-  if (threadIdx.x == 0) partials[blockIdx.x] = s;
+  finish_reduction(s, partials, coef, acc, slot);
 }
 
 // One warp per (i, j, k) triple, summing the contiguous p index.
 __global__ void k_permdot_3el(const double* __restrict__ Yw, const double* __restrict__ Zv,
-                              long long rp, long long a, long long kc, double* partials) {
+                              long long rp, long long a, long long kc, double* partials,
+                              double coef, double* acc, int slot) {
   const long long triples = a * a * kc;
   const int lane = threadIdx.x & 31;
   const long long warp_global = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
@@ -150,8 +214,7 @@ __global__ void k_permdot_3el(const double* __restrict__ Yw, const double* __res
     const double* z = Zv + rp * j + ra * (i + a * k);
     for (long long p = lane; p < rp; p += 32) s += y[p] * z[p];
   }
-  s = block_sum(s);
-  if (threadIdx.x == 0) partials[blockIdx.x] = s;
+  finish_reduction(s, partials, coef, acc, slot);
 }
 
 __global__ void k_symmetrise(const double* __restrict__ G, long long ldg, long long n, double* F,
@@ -208,12 +271,13 @@ struct CombineArgs {
   double cX[2];
 };
 
+template <typename I>
 __global__ void k_combine_y(double* Y, long long m, CombineArgs a, int nq,
                             const double* __restrict__ r, const double* __restrict__ c) {
-  const long long total = m * m;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long i = idx % m, j = idx / m;
+  const I nr = static_cast<I>(m), total = nr * nr;
+  for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
+       idx += static_cast<I>(gridDim.x) * blockDim.x) {
+    const I j = idx / nr, i = idx - j * nr;
     double t = 0.0, x = 0.0;
     for (int q = 0; q < nq; ++q) {
       if (a.cT[q] != 0.0) t += a.cT[q] * a.T[q][idx];
@@ -246,12 +310,13 @@ struct LincombArgs {
   int scaled[kMaxLincomb];
 };
 
+template <typename I>
 __global__ void k_lincomb(double* Y, long long m, long long n, int nt, LincombArgs a,
                           const double* __restrict__ r, const double* __restrict__ c) {
-  const long long total = m * n;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long i = idx % m, j = idx / m;
+  const I nr = static_cast<I>(m), total = nr * static_cast<I>(n);
+  for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
+       idx += static_cast<I>(gridDim.x) * blockDim.x) {
+    const I j = idx / nr, i = idx - j * nr;
     const double rc = (r ? r[i] : 1.0) * (c ? c[j] : 1.0);
     double plain = 0.0, sc = 0.0;
     for (int q = 0; q < nt; ++q) {
@@ -266,20 +331,24 @@ __global__ void k_lincomb(double* Y, long long m, long long n, int nt, LincombAr
 }
 
 // out[i(i+1)/2 + j, a] = G[i, j, a] + G[j, i, a] (j < i), G[i, i, a] (j = i):
-// the gradient of a function of sq(x) with respect to the packed x.
-__global__ void k_pack_sym_sum(const double* __restrict__ G, long long n, long long na,
-                               double* out, long long ldo, double beta) {
-  const long long np = n * (n + 1) / 2;
-  const long long total = np * na;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long p = idx % np, a = idx / np;
+// the gradient of a function of sq(x) with respect to the packed x.  Bound by
+// HBM and L2 (G[i, j] is read at a stride; its lines serve the neighbouring rows
+// from L2).  One packed element per thread with 32-bit indices (0.34 -> 0.26 ms
+// over the four launches of an open-shell gradient at N = 200, M = 600); tiles
+// through shared memory as in k_unpack_sym took 0.36 ms, two dependent phases
+// for no fewer bytes.
+template <typename I>
+__global__ void k_pack_sym_sum(const double* __restrict__ G, I n, I np, I total, double* out,
+                               long long ldo, double beta) {
+  for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
+       idx += static_cast<I>(gridDim.x) * blockDim.x) {
+    const I a = idx / np, p = idx - a * np;
     // row i of the packed index: i(i+1)/2 <= p < (i+1)(i+2)/2
-    long long i = static_cast<long long>((sqrt(8.0 * double(p) + 1.0) - 1.0) * 0.5);
+    I i = static_cast<I>((sqrtf(8.0f * static_cast<float>(p) + 1.0f) - 1.0f) * 0.5f);
     while (i * (i + 1) / 2 > p) --i;
     while ((i + 1) * (i + 2) / 2 <= p) ++i;
-    const long long j = p - i * (i + 1) / 2;
-    const double* g = G + n * n * a;
+    const I j = p - i * (i + 1) / 2;
+    const double* g = G + static_cast<long long>(n) * n * a;
     const double v = (i == j) ? g[i + n * i] : g[i + n * j] + g[j + n * i];
     double* o = out + p + ldo * a;
     *o = beta != 0.0 ? beta * *o + v : v;
@@ -289,34 +358,33 @@ __global__ void k_pack_sym_sum(const double* __restrict__ G, long long n, long l
 // out[p + rp*i + rp*a*(j + a*kk)] = alpha * Z[p + rp*j + rp*a*(i + a*kk)]:
 // the two active-orbital indices of the same-spin three-electron products
 // exchanged (the permutation under which YW and ZV are contracted).
+template <typename I>
 __global__ void k_perm_3el(const double* __restrict__ Z, double* __restrict__ out,
                            long long rp, long long a, long long kc, double alpha) {
-  const long long total = rp * a * a * kc;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long p = idx % rp;
-    long long t = idx / rp;
-    const long long i = t % a;
-    t /= a;
-    const long long j = t % a;
-    const long long kk = t / a;
-    out[idx] = alpha * Z[p + rp * (j + a * (i + a * kk))];
+  const I nr = static_cast<I>(rp), na = static_cast<I>(a);
+  const I total = nr * na * na * static_cast<I>(kc);
+  for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
+       idx += static_cast<I>(gridDim.x) * blockDim.x) {
+    I t = idx / nr;
+    const I p = idx - t * nr;
+    const I t1 = t / na, i = t - t1 * na;
+    const I kk = t1 / na, j = t1 - kk * na;
+    out[idx] = alpha * Z[p + rp * (j + a * (i + a * static_cast<long long>(kk)))];
   }
 }
 
 // out[i + a*l + ao*(j + a*k)] = alpha * V[i + a*k + ao*(j + a*l)], ao = a*o:
 // the occupied indices of rows and columns of (ik|jl) exchanged.
+template <typename I>
 __global__ void k_perm_4el(const double* __restrict__ V, double* __restrict__ out,
                            long long a, long long o, double alpha) {
-  const long long ao = a * o, total = ao * ao;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long i = idx % a;
-    long long t = idx / a;
-    const long long l = t % o;
-    t /= o;
-    const long long j = t % a;
-    const long long k = t / a;
+  const I na = static_cast<I>(a), no = static_cast<I>(o), total = na * no * na * no;
+  const long long ao = a * o;
+  for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
+       idx += static_cast<I>(gridDim.x) * blockDim.x) {
+    const I t0 = idx / na, i = idx - t0 * na;
+    const I t1 = t0 / no, l = t0 - t1 * no;
+    const I k = t1 / na, j = t1 - k * na;
     out[idx] = alpha * V[i + a * k + ao * (j + a * l)];
   }
 }
@@ -350,11 +418,17 @@ __global__ void k_gather_scale_cols(const double* __restrict__ src, long long ro
   }
 }
 
-void finish_reduction(const double* partials, int n, double coef, double* acc, int slot,
-                      cudaStream_t s) {
-  k_finish<<<1, 32, 0, s>>>(partials, n, coef, acc, slot);
-  UW12_LAUNCHED();
+// Grid of k_unpack_sym: lower-triangle tiles x columns.
+inline dim3 tile_grid(long long n, long long ncols) {
+  const long long t = (n + 31) / 32;
+  return dim3(static_cast<unsigned>(t * (t + 1) / 2),
+              static_cast<unsigned>(std::min<long long>(ncols, 65535)));
 }
+
+// Index arithmetic in 32 bits where the element count allows it: the divisions
+// that turn an element's number into its indices otherwise take longer than
+// the element's traffic.
+inline bool small_index(long long total) { return total < (1LL << 31); }
 
 }  // namespace
 
@@ -362,8 +436,8 @@ void unpack_sym(const double* P, long long ldp, long long n, long long ncols, do
                 long long ldo, long long so, double alpha, double beta) {
   const long long total = n * n * ncols;
   if (total <= 0) return;
-  k_unpack_sym<<<grid_for(total), kT, 0, current_stream()>>>(P, ldp, n, ncols, out, ldo, so,
-                                                              alpha, beta);
+  k_unpack_sym<<<tile_grid(n, ncols), kT, 0, current_stream()>>>(
+      P, ldp, static_cast<int>(n), ncols, out, ldo, so, alpha, beta);
   UW12_LAUNCHED();
 }
 
@@ -379,7 +453,11 @@ void scale_rc(const double* X, long long ldx, long long rows, long long cols, co
               const double* c, double alpha, double* Y, long long ldy) {
   const long long total = rows * cols;
   if (total <= 0) return;
-  k_scale_rc<<<grid_for(total), kT, 0, current_stream()>>>(X, ldx, rows, cols, r, c, alpha, Y,
+  if (small_index(total))
+    k_scale_rc<unsigned><<<grid_for(total), kT, 0, current_stream()>>>(X, ldx, rows, cols, r, c, alpha, Y,
+                                                            ldy);
+  else
+    k_scale_rc<long long><<<grid_for(total), kT, 0, current_stream()>>>(X, ldx, rows, cols, r, c, alpha, Y,
                                                             ldy);
   UW12_LAUNCHED();
 }
@@ -388,7 +466,11 @@ void copy3d(const double* src, long long s1, long long s2, double* dst, long lon
             long long d2, long long n0, long long n1, long long n2, double alpha, double beta) {
   const long long total = n0 * n1 * n2;
   if (total <= 0) return;
-  k_copy3d<<<grid_for(total), kT, 0, current_stream()>>>(src, s1, s2, dst, d1, d2, n0, n1, n2,
+  if (small_index(total))
+    k_copy3d<unsigned><<<grid_for(total), kT, 0, current_stream()>>>(src, s1, s2, dst, d1, d2, n0, n1, n2,
+                                                          alpha, beta);
+  else
+    k_copy3d<long long><<<grid_for(total), kT, 0, current_stream()>>>(src, s1, s2, dst, d1, d2, n0, n1, n2,
                                                           alpha, beta);
   UW12_LAUNCHED();
 }
@@ -401,9 +483,13 @@ void wdot(const double* x, long long ldx, const double* y, long long ldy, long l
   cudaStream_t s = current_stream();
   const int blocks = grid_for(total, 4);
   DevBuf part(blocks, s);
-  k_wdot<<<blocks, kT, 0, s>>>(x, ldx, y, ldy, rows, cols, rw, cw, part.get());
+  if (small_index(total))
+    k_wdot<unsigned><<<blocks, kT, 0, s>>>(x, ldx, y, ldy, rows, cols, rw, cw, part.get(), coef,
+                                           acc, slot);
+  else
+    k_wdot<long long><<<blocks, kT, 0, s>>>(x, ldx, y, ldy, rows, cols, rw, cw, part.get(), coef,
+                                            acc, slot);
   UW12_LAUNCHED();
-  finish_reduction(part.get(), blocks, coef, acc, slot, s);
 }
 
 void permdot_4el(const double* X, const double* Y, long long a, long long o, double coef,
@@ -413,9 +499,11 @@ void permdot_4el(const double* X, const double* Y, long long a, long long o, dou
   cudaStream_t s = current_stream();
   const int blocks = grid_for(total, 4);
   DevBuf part(blocks, s);
-  k_permdot_4el<<<blocks, kT, 0, s>>>(X, Y, a, o, part.get());
+  if (small_index(total))
+    k_permdot_4el<unsigned><<<blocks, kT, 0, s>>>(X, Y, a, o, part.get(), coef, acc, slot);
+  else
+    k_permdot_4el<long long><<<blocks, kT, 0, s>>>(X, Y, a, o, part.get(), coef, acc, slot);
   UW12_LAUNCHED();
-  finish_reduction(part.get(), blocks, coef, acc, slot, s);
 }
 
 void permdot_3el(const double* Y, const double* Z, long long rp, long long a, long long kc,
@@ -425,9 +513,8 @@ void permdot_3el(const double* Y, const double* Z, long long rp, long long a, lo
   cudaStream_t s = current_stream();
   const int blocks = grid_for(triples * 32, 8);
   DevBuf part(blocks, s);
-  k_permdot_3el<<<blocks, kT, 0, s>>>(Y, Z, rp, a, kc, part.get());
+  k_permdot_3el<<<blocks, kT, 0, s>>>(Y, Z, rp, a, kc, part.get(), coef, acc, slot);
   UW12_LAUNCHED();
-  finish_reduction(part.get(), blocks, coef, acc, slot, s);
 }
 
 void symmetrise(const double* G, long long ldg, long long n, double* F, long long ldf) {
@@ -457,7 +544,10 @@ void combine_y(double* Y, long long m, const double* const* T, const double* coe
   for (int q = 0; q < nq; ++q) {
     a.T[q] = T[q]; a.X[q] = X[q]; a.cT[q] = coefT[q]; a.cX[q] = coefX[q];
   }
-  k_combine_y<<<grid_for(total), kT, 0, current_stream()>>>(Y, m, a, nq, r, c);
+  if (small_index(total))
+    k_combine_y<unsigned><<<grid_for(total), kT, 0, current_stream()>>>(Y, m, a, nq, r, c);
+  else
+    k_combine_y<long long><<<grid_for(total), kT, 0, current_stream()>>>(Y, m, a, nq, r, c);
   UW12_LAUNCHED();
 }
 
@@ -481,7 +571,10 @@ void lincomb(double* Y, long long m, long long n, int nt, const double* const* m
     a.coef[q] = coefs[q];
     a.scaled[q] = scaled ? scaled[q] : 0;
   }
-  k_lincomb<<<grid_for(total), kT, 0, current_stream()>>>(Y, m, n, nt, a, r, c);
+  if (small_index(total))
+    k_lincomb<unsigned><<<grid_for(total), kT, 0, current_stream()>>>(Y, m, n, nt, a, r, c);
+  else
+    k_lincomb<long long><<<grid_for(total), kT, 0, current_stream()>>>(Y, m, n, nt, a, r, c);
   UW12_LAUNCHED();
 }
 
@@ -489,7 +582,14 @@ void pack_sym_sum(const double* G, long long n, long long na, double* out, long 
                   double beta) {
   const long long total = n * (n + 1) / 2 * na;
   if (total <= 0) return;
-  k_pack_sym_sum<<<grid_for(total), kT, 0, current_stream()>>>(G, n, na, out, ldo, beta);
+  const long long np = n * (n + 1) / 2;
+  if (small_index(std::max(total, n * n)))
+    k_pack_sym_sum<unsigned><<<grid_for(total), kT, 0, current_stream()>>>(
+        G, static_cast<unsigned>(n), static_cast<unsigned>(np), static_cast<unsigned>(total), out,
+        ldo, beta);
+  else
+    k_pack_sym_sum<long long><<<grid_for(total), kT, 0, current_stream()>>>(G, n, np, total, out,
+                                                                            ldo, beta);
   UW12_LAUNCHED();
 }
 
@@ -497,14 +597,20 @@ void perm_3el(const double* Z, double* out, long long rp, long long a, long long
               double alpha) {
   const long long total = rp * a * a * kc;
   if (total <= 0) return;
-  k_perm_3el<<<grid_for(total), kT, 0, current_stream()>>>(Z, out, rp, a, kc, alpha);
+  if (small_index(total))
+    k_perm_3el<unsigned><<<grid_for(total), kT, 0, current_stream()>>>(Z, out, rp, a, kc, alpha);
+  else
+    k_perm_3el<long long><<<grid_for(total), kT, 0, current_stream()>>>(Z, out, rp, a, kc, alpha);
   UW12_LAUNCHED();
 }
 
 void perm_4el(const double* V, double* out, long long a, long long o, double alpha) {
   const long long total = a * o * a * o;
   if (total <= 0) return;
-  k_perm_4el<<<grid_for(total), kT, 0, current_stream()>>>(V, out, a, o, alpha);
+  if (small_index(total))
+    k_perm_4el<unsigned><<<grid_for(total), kT, 0, current_stream()>>>(V, out, a, o, alpha);
+  else
+    k_perm_4el<long long><<<grid_for(total), kT, 0, current_stream()>>>(V, out, a, o, alpha);
   UW12_LAUNCHED();
 }
 

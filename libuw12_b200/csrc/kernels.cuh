@@ -28,8 +28,14 @@ void copy3d(const double* src, long long s1, long long s2, double* dst, long lon
             long long d2, long long n0, long long n1, long long n2, double alpha = 1.0,
             double beta = 0.0);
 
+// Sums of wdot, permdot_4el and permdot_3el: acc is a device array of
+// kAccDoubles, zeroed before its first use; slots below kAccSlots hold sums, the
+// last double is the ticket of the reductions' last block.
+constexpr int kAccSlots = 8;
+constexpr int kAccDoubles = kAccSlots + 1;
+
 // acc[slot] += coef * sum_{i<rows, j<cols} x[i + ldx*j] * y[i + ldy*j] * rw[i] * cw[j]
-// (rw / cw may be null).  Two-pass, fixed-order reduction.
+// (rw / cw may be null).  Fixed-order reduction.
 void wdot(const double* x, long long ldx, const double* y, long long ldy, long long rows,
           long long cols, const double* rw, const double* cw, double coef, double* acc, int slot);
 
