@@ -689,6 +689,40 @@ void upload_orbitals(const FockRequest& rq, std::vector<SpinDims>& sd, size_t& o
 // --------------------------------------------------------------------------
 // form_fock
 // --------------------------------------------------------------------------
+namespace {
+// Whether the t~ dX Fock term takes fewer operations over orbital pairs than over
+// aux functions (halves of the FLOPs of both forms' products; a tie goes to
+// the pairs).  Over aux functions: S^-1 G_W, and per spin J3^V T2^T and the sum
+// over a.  Over pairs: S^-1 G_V and D, and without the same-spin terms (which
+// form them anyway) G_W and G_V; with them Y_W is used twice and S^-1 Wst_W is
+// not needed.  With 3 DF and 4 RI functions per AO and closed shell the pairs
+// win up to a o = 0.8 M without and 4 M with the same-spin terms.
+bool pair_form_cheaper(const FockRequest& rq, const std::vector<SpinDims>& sd, bool same_spin) {
+  const int ns = rq.n_spin;
+  const double N = double(rq.n_ao), R = double(rq.W->n_ri), Rp = N + R;
+  const double MW = double(rq.W->n_df), MV = double(rq.V->n_df);
+  const double J = 0.5 * N * (N + 1.0) + R * N;  // rows of a three-index tensor
+  double aux = 0.0, pairs = 0.0;
+  for (int sp = 0; sp < ns; ++sp) {
+    bool any = false;
+    for (int s = 0; s < ns; ++s)
+      any = any || (spin_factor(ns, s, sp, rq.s_os, rq.s_ss) != 0.0 && sd[s].a > 0);
+    if (any) aux += J * MW * MV + N * N * Rp * MW + MW * MV * (MW + MV);
+  }
+  if (aux == 0.0) return false;
+  aux += Rp * Rp * N * MW;
+  for (int s = 0; s < ns; ++s) {
+    const double a = double(sd[s].a), ao = a * double(sd[s].o);
+    pairs += ao * (Rp * Rp * N + (same_spin && ns == 1 ? 0.0 : N * N * Rp));
+    if (same_spin)
+      aux += a * a * N * Rp * MW + Rp * Rp * a * MW;
+    else
+      pairs += ao * (J * (MW + MV) + MW * MW + MV * MV);
+  }
+  return pairs <= aux;
+}
+}  // namespace
+
 size_t budget_need(const FockRequest& rq, bool adjoint, bool streamed) {
   const size_t N = rq.n_ao, np = packed_size(N), R = rq.W->n_ri, Rp = N + R;
   const size_t M = std::max({rq.W->n_df, rq.V->n_df, rq.WV->n_df});
@@ -706,9 +740,8 @@ size_t budget_need(const FockRequest& rq, bool adjoint, bool streamed) {
   if (rq.calc_fock) need = std::max(need, blocks + (4 * N * N + Rp * N + 2 * R * N + np) * M);
   if (rq.indirect) {
     need = std::max(need, (3 * Rp * o1 + M) * o1 * o1);                  // pair products of energies
-    if (rq.calc_fock)
-      need = std::max(need, blocks + o1 * o1 * (2 * Rp * N + N * N + R * N + np));
   }
+  if (rq.calc_fock) need = std::max(need, blocks + o1 * o1 * (4 * Rp * N + np));  // pair products
   if (adjoint)
     need = std::max({need, 2 * (N + R + 2 * (o1 + 2 * Rp)) * o * M, (4 * N * N + N * o) * M});
   return need;
@@ -860,7 +893,10 @@ void form_fock(const FockRequest& rq) {
     std::vector<DevBuf> B1, B2, Wst, SV;
   };
   PerX XW, XV;
-  const bool need_sv_w = calc && do_ind;
+  // The t~ dX Fock term through orbital pairs (below) or aux functions; the
+  // pairs need B2 whole.
+  const bool pairs_cheaper = calc && pair_form_cheaper(rq, sd, do_ind);
+  const bool need_sv_w = calc && do_ind && !pairs_cheaper;
   // Without same-spin terms the stacked transforms serve only X_AB, t and the
   // direct Fock, which are sums over orbitals: when the whole intermediates
   // (B1, B2, Wst of W and V, S^-1 Wst_V) exceed the chunk budget they are
@@ -881,6 +917,7 @@ void form_fock(const FockRequest& rq) {
     UW12_CUDA(cudaStreamSynchronize(st));
     orbital_chunked = any > 0.0;
   }
+  const bool fold = pairs_cheaper && !orbital_chunked;
   for (int which = 0; which < 2 && !orbital_chunked; ++which) {
     const IntegralsHandle& X = which == 0 ? W : V;
     PerX& P = which == 0 ? XW : XV;
@@ -1144,11 +1181,12 @@ void form_fock(const FockRequest& rq) {
         gemm(gf);
       }
     }
-    if (!do_ind && !orbital_chunked)  // B1 and B2 serve only the direct Fock and the same-spin terms
+    if (!do_ind && !orbital_chunked)  // B1 and B2 serve the direct Fock and the pair terms only
       for (int s = 0; s < ns; ++s) {
         XW.B1[s].release();
-        XW.B2[s].release();
         XV.B1[s].release();
+        if (fold) continue;
+        XW.B2[s].release();
         XV.B2[s].release();
       }
     // t~ dX: F[sigma'] -= sum_ab T2[a,b] G_W[a]^T S^-1 G_V[b] with
@@ -1156,10 +1194,10 @@ void form_fock(const FockRequest& rq) {
     // (R' x N).  L[a] = S^-1 G_W[a] does not depend on sigma', so it is formed
     // once per aux chunk and contracted with H[a] = sum_b T2[a,b] G_V[b] of
     // every spin.
-    clock.mark("tdx_fock");
+    if (!fold) clock.mark("tdx_fock");
     std::vector<int> tdx_spins;
     std::vector<DevBuf> T2s;
-    for (int sp = 0; sp < ns; ++sp) {
+    for (int sp = 0; sp < ns && !fold; ++sp) {
       const double* Tq[2] = {ttl[0].get(), ns > 1 ? ttl[1].get() : nullptr};
       double cT[2] = {0, 0}, cX[2] = {0, 0};
       bool any = false;
@@ -1264,16 +1302,18 @@ void form_fock(const FockRequest& rq) {
   }
 
   // =====================================================================
-  // same-spin (indirect) terms
+  // terms over orbital pairs: the same-spin (indirect) terms, and t~ dX when
+  // it is cheaper there
   // =====================================================================
-  if (do_ind) {
+  if (do_ind || fold) {
     for (int s = 0; s < ns; ++s) {
       const size_t o = sd[s].o, a = sd[s].a, c = sd[s].c;
       if (a == 0 || o == 0) continue;
       const size_t ao = a * o, No = N * o;
-      DevBuf b2wl(ao * MW), b2vl(ao * MV);
+      DevBuf b2wl(ao * MW), b2vl(ao * MV), b1wl, b1vl;
       scale_rc(XW.B2[s].get(), LL(ao), LL(ao), LL(MW), nullptr, W.lam.get(), 1.0, b2wl.get(), LL(ao));
       scale_rc(XV.B2[s].get(), LL(ao), LL(ao), LL(MV), nullptr, V.lam.get(), 1.0, b2vl.get(), LL(ao));
+      if (do_ind) {
       clock.mark("ss_4el_energy");
       // ---- 4-el indirect energy (four_electron.cpp:143-179)
       if (lead) {
@@ -1311,7 +1351,8 @@ void form_fock(const FockRequest& rq) {
         }
       }
       if (!calc) continue;
-      DevBuf b1wl(No * MW), b1vl(No * MV);
+      b1wl.alloc(No * MW);
+      b1vl.alloc(No * MV);
       scale_rc(XW.B1[s].get(), LL(No), LL(No), LL(MW), nullptr, W.lam.get(), 1.0, b1wl.get(), LL(No));
       scale_rc(XV.B1[s].get(), LL(No), LL(No), LL(MV), nullptr, V.lam.get(), 1.0, b1vl.get(), LL(No));
       clock.mark("ss_4el_fock");
@@ -1350,108 +1391,172 @@ void form_fock(const FockRequest& rq) {
           gemm(gf);
         }
       }
-      clock.mark("ss_3el_fock");
-      // ---- 3-el indirect Fock (indirect_utils.cpp:139-345), chunked over k
-      {
-        DevBuf xhW(MW * ao), xhV(MV * ao);
-        GemmDesc g = gemm_nn(LL(MW), LL(ao), LL(MW), 1.0, W.P2.get(), LL(MW), b2wl.get(), LL(ao),
-                             0.0, xhW.get(), LL(MW));
-        g.b_ncontig = true;
-        gemm(g);
-        g = gemm_nn(LL(MV), LL(ao), LL(MV), 1.0, V.P2.get(), LL(MV), b2vl.get(), LL(ao), 0.0,
-                    xhV.get(), LL(MV));
-        g.b_ncontig = true;
-        gemm(g);
-        budget = budgets.doubles();
-        // unstored W / V blocks (accumulated over, for every k chunk) take at
-        // most an eighth of the budget each
-        size_t xscr = 0;
-        for (const IntegralsHandle* Xi : {&W, &V})
-          xscr = std::max(xscr, (Xi->J3_0.get() ? 0 : np * aux_step(*Xi, false, budget / 2)) +
-                                    (Xi->J3_ri_0.get() ? 0 : R * N * aux_step(*Xi, true, budget / 2)));
-        // two R' a N buffers per k: Z_W (term 1, done first), then W_k of the
-        // k-term in the same memory; Z_V (term 0) lives until the k-term
-        const size_t per_k = 2 * Rp * a * N + a * (N * N + R * N + np);
-        const auto [klo, khi] = part(o);
-        const size_t kavail = budget > xscr ? budget - xscr : 0;
-        const size_t kc = tile_chunk(khi - klo, a,
-                                     std::max<size_t>(1, std::min(khi - klo, kavail / per_k)));
-        DevBuf ZYV(Rp * a * N * kc), ZYW(Rp * a * N * kc), gpk(np * a * kc), Gao(N * N * a * kc),
-            gri(R * N * a * kc), scrX, scrXr;
-        double* const Wk = ZYW.get();  // after term 1 has used Z_W
-        for (size_t k0 = klo; k0 < khi; k0 += kc) {
-          const size_t nk = std::min(kc, khi - k0);
-          for (int term : {1, 0}) {
-            // term 0: fock_i(W, V) over (j, k); term 1: fock_i(V, W) over (i, k)
-            const IntegralsHandle& Xi = term == 0 ? W : V;
-            const double* xh = term == 0 ? xhW.get() : xhV.get();
-            const size_t MXi = Xi.n_df;
-            const double* SVy = term == 0 ? XV.SV[s].get() : XW.SV[s].get();
-            const double* b1yl = term == 0 ? b1vl.get() : b1wl.get();
-            const size_t MY = term == 0 ? MV : MW;
-            double* ZY = term == 0 ? ZYV.get() : ZYW.get();
-            GemmDesc gz = gemm_nn(LL(Rp * a), LL(N * nk), LL(MY), 1.0, SVy, LL(Rp * a),
-                                  b1yl + N * k0, LL(No), 0.0, ZY, LL(Rp * a));
-            gz.b_ncontig = true;
-            gemm(gz);
-            // gpk = J3_0 xh, gri = J3_ri_0 xh, accumulated over Xi's aux blocks
-            const size_t st_ao = aux_step(Xi, false, budget / 2);
-            const size_t st_ri = aux_step(Xi, true, budget / 2);
-            for (size_t b0 = 0; b0 < MXi; b0 += st_ao) {
-              const size_t nb = std::min(st_ao, MXi - b0);
-              gemm(gemm_nn(LL(np), LL(a * nk), LL(nb), 1.0, aux_block(Xi, false, b0, nb, scrX),
-                           LL(np), xh + MXi * a * k0 + b0, LL(MXi), b0 ? 1.0 : 0.0, gpk.get(),
-                           LL(np)));
-            }
-            unpack_sym(gpk.get(), LL(np), LL(N), LL(a * nk), Gao.get(), LL(N), LL(N * N));
-            for (size_t b0 = 0; b0 < MXi; b0 += st_ri) {
-              const size_t nb = std::min(st_ri, MXi - b0);
-              gemm(gemm_nn(LL(R * N), LL(a * nk), LL(nb), 1.0, aux_block(Xi, true, b0, nb, scrXr),
-                           LL(R * N), xh + MXi * a * k0 + b0, LL(MXi), b0 ? 1.0 : 0.0, gri.get(),
-                           LL(R * N)));
-            }
-            GemmDesc fa = gemm_nn(LL(N), LL(N), LL(N), s_ss, Gao.get(), LL(N), ZY, LL(Rp * a),
-                                  1.0, Fp[s].get(), LL(N));
-            fa.nbr1 = LL(a);
-            fa.nbr2 = LL(nk);
-            fa.sAr1 = LL(N * N);
-            fa.sAr2 = LL(N * N * a);
-            fa.sBr1 = LL(Rp);
-            fa.sBr2 = LL(Rp * a * N);
-            gemm(fa);
-            GemmDesc fr = gemm_nn(LL(N), LL(N), LL(R), s_ss, gri.get(), LL(R), ZY + N, LL(Rp * a),
-                                  1.0, Fp[s].get(), LL(N));
-            fr.a_kcontig = true;
-            fr.nbr1 = LL(a);
-            fr.nbr2 = LL(nk);
-            fr.sAr1 = LL(R * N);
-            fr.sAr2 = LL(R * N * a);
-            fr.sBr1 = LL(Rp);
-            fr.sBr2 = LL(Rp * a * N);
-            gemm(fr);
+      }  // do_ind
+      clock.mark("pair_fock");
+      // ---- Fock terms over pairs of an active orbital j and an occupied
+      // orbital k, in chunks of k.  With G_X[jk] = sum_A [sq(J3_0^X[:,A]);
+      // J3ri_0^X[:,A]] x^_X[A;jk], x^_X = P2_X L_X B2_X^T, and
+      // Y_X[jk] = Wst_X[j] L_X B1_X[k]^T (both R' x N):
+      //   same-spin 3-el (indirect_utils.cpp:139-345)
+      //     s_ss sum_jk (G_W^T S^-1 Y_V + G_V^T S^-1 Y_W)
+      //     + s_ss sum_ij Y_W[i,c+j]^T S^-1 Y_V[j,c+i]
+      //   t~ dX (direct_utils.cpp:256-347), T2 = sum_s x^_W x^_V^T:
+      //     F[sigma'] -= half f(s, sigma') D, D = sum_jk G_W^T S^-1 G_V.
+      // t~ has the rank of the pairs, so D needs S^-1 on N a o columns instead
+      // of S^-1 G_W on the N M of all aux functions and J3^V T2^T (M x M); with
+      // the same-spin terms G_W and G_V are there already, S^-1 G_V also
+      // replaces S^-1 Y_W (Y_W then serves the k-term as it is), and no
+      // product has an aux x aux operand.  pair_form_cheaper counts both forms.
+      // One B200, against the form over aux functions and k-chunked Y_W (same GEMM
+      // kernels): closed shell N=300, M=900, R=1200, o=30 in FP64 229 -> 176 ms; open
+      // shell N=200, M=600, R=800, o=16/15 53.3 -> 35.3 ms.
+      double cD[2] = {0.0, 0.0};
+      for (int sp = 0; sp < ns && fold; ++sp) cD[sp] = half * spin_factor(ns, s, sp, s_os, s_ss);
+      if (!do_ind && cD[0] == 0.0 && cD[1] == 0.0) continue;
+      DevBuf xhW(MW * ao), xhV(MV * ao);
+      GemmDesc g = gemm_nn(LL(MW), LL(ao), LL(MW), 1.0, W.P2.get(), LL(MW), b2wl.get(), LL(ao),
+                           0.0, xhW.get(), LL(MW));
+      g.b_ncontig = true;
+      gemm(g);
+      g = gemm_nn(LL(MV), LL(ao), LL(MV), 1.0, V.P2.get(), LL(MV), b2vl.get(), LL(ao), 0.0,
+                  xhV.get(), LL(MV));
+      g.b_ncontig = true;
+      gemm(g);
+      budget = budgets.doubles();
+      // unstored W / V blocks (accumulated over, for every k chunk) take at
+      // most an eighth of the budget each
+      size_t xscr = 0;
+      for (const IntegralsHandle* Xi : {&W, &V})
+        xscr = std::max(xscr, (Xi->J3_0.get() ? 0 : np * aux_step(*Xi, false, budget / 2)) +
+                                  (Xi->J3_ri_0.get() ? 0 : R * N * aux_step(*Xi, true, budget / 2)));
+      const size_t pair = Rp * N;  // doubles of one pair's matrix
+      const size_t per_k = a * (pair * (do_ind ? (fold ? 4 : 3) : 2) + np + std::max(MW, MV));
+      const auto [klo, khi] = part(o);
+      const size_t kavail = budget > xscr ? budget - xscr : 0;
+      const size_t kc = tile_chunk(khi - klo, a,
+                                   std::max<size_t>(1, std::min(khi - klo, kavail / per_k)));
+      const bool whole_k = kc == o;
+      // pair (j, k) of a chunk of nk orbitals is matrix (k - k0) + nk j of a buffer
+      const size_t nbuf = pair * a * kc;
+      DevBuf gpk(np * a * kc), xk(std::max(MW, MV) * a * kc), bufG(nbuf), bufS(nbuf),
+          bufY(do_ind ? nbuf : 0), bufZ(do_ind && fold ? nbuf : 0), scrX, scrXr;
+      // dst = G_X of the chunk, over X's aux blocks
+      auto form_g = [&](const IntegralsHandle& X, const double* xh, size_t k0, size_t nk,
+                        double* dst) {
+        const size_t M = X.n_df;
+        copy3d(xh + M * a * k0, LL(M), LL(M * a), xk.get(), LL(M * nk), LL(M), LL(M), LL(a),
+               LL(nk));
+        const size_t st_ao = aux_step(X, false, budget / 2);
+        const size_t st_ri = aux_step(X, true, budget / 2);
+        for (size_t b0 = 0; b0 < M; b0 += st_ao) {
+          const size_t nb = std::min(st_ao, M - b0);
+          gemm(gemm_nn(LL(np), LL(a * nk), LL(nb), 1.0, aux_block(X, false, b0, nb, scrX), LL(np),
+                       xk.get() + b0, LL(M), b0 ? 1.0 : 0.0, gpk.get(), LL(np)));
+        }
+        unpack_sym(gpk.get(), LL(np), LL(N), LL(a * nk), dst, LL(Rp), LL(pair));
+        for (size_t b0 = 0; b0 < M; b0 += st_ri) {
+          const size_t nb = std::min(st_ri, M - b0);
+          GemmDesc gr = gemm_nn(LL(R), LL(a * nk), LL(nb), 1.0, aux_block(X, true, b0, nb, scrXr),
+                                LL(R * N), xk.get() + b0, LL(M), b0 ? 1.0 : 0.0, dst + N,
+                                LL(pair));
+          gr.nbo1 = LL(N);
+          gr.sAo1 = LL(R);
+          gr.sCo1 = LL(Rp);
+          gemm(gr);
+        }
+      };
+      // dst = St[j] L B1[k]^T of the chunk (St: R' a x M)
+      auto form_y = [&](const double* St, const double* b1l, size_t M, size_t k0, size_t nk,
+                        double* dst) {
+        GemmDesc gy = gemm_nn(LL(Rp), LL(N * nk), LL(M), 1.0, St, LL(Rp * a), b1l + N * k0,
+                              LL(No), 0.0, dst, LL(Rp));
+        gy.b_ncontig = true;
+        gy.nbo1 = LL(a);
+        gy.sAo1 = LL(Rp);
+        gy.sCo1 = LL(pair * nk);
+        gemm(gy);
+      };
+      // F += coef sum_pairs A[pair]^T B[pair]
+      auto add_pairs = [&](double coef, const double* A, const double* B, size_t n_pairs, double beta,
+                           double* F) {
+        GemmDesc gf = gemm_nn(LL(N), LL(N), LL(Rp), coef, A, LL(Rp), B, LL(Rp), beta, F, LL(N));
+        gf.a_kcontig = true;
+        gf.nbr1 = LL(n_pairs);
+        gf.sAr1 = LL(pair);
+        gf.sBr1 = LL(pair);
+        gemm(gf);
+      };
+      for (size_t k0 = klo; k0 < khi; k0 += kc) {
+        const size_t nk = std::min(kc, khi - k0), n_pairs = a * nk;
+        const double* z = nullptr;   // S^-1 Y_V
+        const double* yw = nullptr;  // Y_W, when the whole of it is held
+        if (fold) {
+          form_g(V, xhV.get(), k0, nk, bufG.get());
+          gemm(gemm_nn(LL(Rp), LL(N * n_pairs), LL(Rp), 1.0, AB.Sinv.get(), LL(Rp), bufG.get(),
+                       LL(Rp), 0.0, bufS.get(), LL(Rp)));
+          if (do_ind) {
+            form_y(XW.Wst[s].get(), b1wl.get(), MW, k0, nk, bufY.get());
+            add_pairs(s_ss, bufS.get(), bufY.get(), n_pairs, 1.0, Fp[s].get());
+            if (whole_k) yw = bufY.get();
           }
-          // k-term (fock_k) for active orbitals c+i inside this chunk
-          const long long i0 = std::max<long long>(0, LL(k0) - LL(c));
-          const long long i1 = LL(k0 + nk) - LL(c);
+          form_g(W, xhW.get(), k0, nk, bufG.get());
+        } else {
+          form_g(V, xhV.get(), k0, nk, bufG.get());
+          form_y(XW.SV[s].get(), b1wl.get(), MW, k0, nk, bufY.get());
+          add_pairs(s_ss, bufG.get(), bufY.get(), n_pairs, 1.0, Fp[s].get());
+          form_g(W, xhW.get(), k0, nk, bufG.get());
+        }
+        if (do_ind) {
+          double* zbuf = fold ? bufZ.get() : bufS.get();
+          form_y(XV.SV[s].get(), b1vl.get(), MV, k0, nk, zbuf);
+          z = zbuf;
+          // k-term (fock_k) for active orbitals c + i inside this chunk
+          const size_t i0 = std::max(k0, c) - c, i1 = std::max(k0 + nk, c) - c;
           if (i1 > i0) {
-            const size_t ni = static_cast<size_t>(i1 - i0);
-            GemmDesc gw = gemm_nn(LL(Rp * ni), LL(N * a), LL(MW), 1.0,
-                                  XW.Wst[s].get() + Rp * i0, LL(Rp * a), b1wl.get() + N * c,
-                                  LL(No), 0.0, Wk, LL(Rp * ni));
-            gw.b_ncontig = true;
-            gemm(gw);
-            GemmDesc fk = gemm_nn(LL(N), LL(N), LL(Rp), s_ss, Wk, LL(Rp * ni),
-                                  ZYV.get() + Rp * a * N * (c + i0 - k0), LL(Rp * a), 1.0,
-                                  Fp[s].get(), LL(N));
+            const size_t ni = i1 - i0;
+            GemmDesc fk = gemm_nn(LL(N), LL(N), LL(Rp), s_ss, yw, LL(Rp),
+                                  z + pair * (c + i0 - k0), LL(Rp), 1.0, Fp[s].get(), LL(N));
             fk.a_kcontig = true;
             fk.nbr1 = LL(ni);
             fk.nbr2 = LL(a);
-            fk.sAr1 = LL(Rp);
-            fk.sAr2 = LL(Rp * ni * N);
-            fk.sBr1 = LL(Rp * a * N);
-            fk.sBr2 = LL(Rp);
+            fk.sBr1 = LL(pair);
+            fk.sBr2 = LL(pair * nk);
+            if (yw) {
+              fk.A = yw + pair * c;
+              fk.sAr1 = LL(pair * nk);
+              fk.sAr2 = LL(pair);
+            } else {
+              // Y_W[i, c + j] of the chunk's i and all j
+              GemmDesc gw = gemm_nn(LL(Rp * ni), LL(N * a), LL(MW), 1.0,
+                                    XW.Wst[s].get() + Rp * i0, LL(Rp * a), b1wl.get() + N * c,
+                                    LL(No), 0.0, bufY.get(), LL(Rp * ni));
+              gw.b_ncontig = true;
+              gemm(gw);
+              fk.A = bufY.get();
+              fk.lda = LL(Rp * ni);
+              fk.sAr1 = LL(Rp);
+              fk.sAr2 = LL(Rp * ni * N);
+            }
             gemm(fk);
           }
+        }
+        if (!fold) {
+          add_pairs(s_ss, bufG.get(), z, n_pairs, 1.0, Fp[s].get());
+        } else if (ns == 1) {
+          // one product for t~ dX and the same-spin term: G_W^T (s_ss S^-1 Y_V - cD S^-1 G_V)
+          if (do_ind) {
+            const double* mats[2] = {z, bufS.get()};
+            const double coefs[2] = {s_ss, -cD[0]};
+            lincomb(bufS.get(), LL(pair), LL(n_pairs), 2, mats, coefs, nullptr, nullptr, nullptr);
+          }
+          add_pairs(do_ind ? 1.0 : -cD[0], bufG.get(), bufS.get(), n_pairs, 1.0, Fp[s].get());
+        } else {
+          if (do_ind) add_pairs(s_ss, bufG.get(), z, n_pairs, 1.0, Fp[s].get());
+          DevBuf D(N * N);
+          add_pairs(1.0, bufG.get(), bufS.get(), n_pairs, 0.0, D.get());
+          for (int sp = 0; sp < ns; ++sp)
+            if (cD[sp] != 0.0)
+              copy3d(D.get(), LL(N), 0, Fp[sp].get(), LL(N), 0, LL(N), LL(N), 1, -cD[sp], 1.0);
         }
       }
     }

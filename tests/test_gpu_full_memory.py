@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 def test_evaluation_with_little_memory_left(uw12lib, cuda_device):
     import torch
     L = uw12lib
-    c = Case("full", 96, 288, 384, (10,), (9,), "baseline", 5, 8.0)
+    c = Case("full", 96, 288, 384, (20,), (19,), "baseline", 5, 8.0)
     d = make_case(c)
     W = L.setup_base_integrals(d.W3, d.W2, d.W3_ri)
     V = L.setup_base_integrals(d.V3, d.V2, d.V3_ri)
@@ -29,7 +29,7 @@ def test_evaluation_with_little_memory_left(uw12lib, cuda_device):
     torch.cuda.synchronize()
     L.trim_memory()
     torch.cuda.empty_cache()
-    left = 220 << 20  # the unchunked evaluation takes about 300 MiB
+    left = 400 << 20  # the unchunked evaluation takes about 700 MiB
     fill = []
     try:
         free, _ = torch.cuda.mem_get_info()
