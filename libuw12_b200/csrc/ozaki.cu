@@ -7,13 +7,14 @@
 //                 that every element is below 2^beta in magnitude;
 //   k_residues    FP64 -> rint(x 2^shift) -> L int8 residue planes, K-major
 //                 (row r of plane (l, p) is K_pad contiguous bytes);
-//   k_i8_mma      persistent, one CTA per SM; work item = one 128 x 256
-//                 output tile of one modulus and one K chunk: TMA (128-byte
-//                 swizzled boxes, 4-stage ring) -> shared memory ->
-//                 tcgen05.mma.kind::i8 with the int32 accumulator in TMEM (two
-//                 256-column buffers) -> tcgen05.ld -> residue mod p -> uint8
-//                 rows in HBM.  Warp roles: 0 TMA producer, 1 TMEM owner + MMA
-//                 issuer, 2..5 epilogue (TMEM lane quarter = warp % 4);
+//   k_i8_mma      persistent, one CTA pair (or CTA) per SM pair (SM); work item =
+//                 one 256 x 256 (128 x 256) output tile of one modulus and one K
+//                 chunk: TMA (128-byte swizzled boxes, ring of stages) -> shared
+//                 memory -> tcgen05.mma.cta_group::2 (::1) kind::i8 with the int32
+//                 accumulator in TMEM (two 256-column buffers) -> tcgen05.ld ->
+//                 residue mod p -> uint8 rows in HBM.  Warp roles: 0 TMA producer,
+//                 1 TMEM owner + MMA issuer, 2..5 epilogue (TMEM lane quarter =
+//                 warp % 4);
 //   k_crt         per output element: sum the K-chunk residues mod p, CRT on
 //                 <= 41-bit chunks in FP64 (exact integer arithmetic), join the
 //                 chunks error-free (TwoSum), scale by 2^-(sa+sb), apply
@@ -50,7 +51,6 @@ struct Consts {
   int L = 0, nch = 0, cw = 0, beta = 0;
   uint32_t p[kOzakiMaxModuli];
   uint32_t barrett[kOzakiMaxModuli];  // floor(2^32 / p)
-  uint32_t off[kOzakiMaxModuli];      // multiple of p, >= 2^30
   double pd[kOzakiMaxModuli], inv_p[kOzakiMaxModuli];
   double w[kOzakiMaxModuli][kMaxChunks];  // chunks of (M/p_l) * ((M/p_l)^-1 mod p_l) mod M
   double mc[kMaxChunks];                  // chunks of M
@@ -82,7 +82,6 @@ Consts make_consts(int L) {
     c.log2_m += std::log2(double(p));
     c.p[l] = p;
     c.barrett[l] = static_cast<uint32_t>((1ULL << 32) / p);
-    c.off[l] = static_cast<uint32_t>(((1ULL << 30) + p - 1) / p * p);
     c.pd[l] = double(p);
     c.inv_p[l] = 1.0 / double(p);
   }
@@ -323,7 +322,7 @@ __device__ __forceinline__ uint32_t residue_low(int vl, double v, double inv_p, 
 
 // Tile of 32 rows x 128 k of one plane -> L residue rows per row: row r of
 // modulus l of a plane is out row ((plane * tiles + r / T) * L + l) * T + r % T
-// (T = 2^tile_log2, the MMA tile height of this operand; tiles = rows_pad / T),
+// (T = tile_rows, the MMA tile height of this operand; tiles = rows_pad / T),
 // each k_pad bytes; zeros in padding.  The L residue rows of a tile are
 // T * k_pad bytes apart.  Thread (row pair rr, rr + 16; lane t of 16) converts
 // the 8 consecutive k 8t .. 8t+7 of each of its rows and stores 8 residue bytes
@@ -332,7 +331,7 @@ __device__ __forceinline__ uint32_t residue_low(int vl, double v, double inv_p, 
 // immediate constant-bank operands.  Grid: (row tiles, k tiles, planes).
 template <bool KCONTIG, int LM>
 __global__ void __launch_bounds__(256) k_residues(OperandView v, const int* __restrict__ shift,
-                                                  ResidueMods mods, int tile_log2,
+                                                  ResidueMods mods, int tile_rows,
                                                   long long tiles, long long k_pad,
                                                   uint8_t* __restrict__ out) {
   __shared__ __align__(16) double tile[32 * 128];
@@ -345,8 +344,7 @@ __global__ void __launch_bounds__(256) k_residues(OperandView v, const int* __re
   load_tile<KCONTIG>(v, plane, row0, koff, tile);
   __syncthreads();
   const int t = threadIdx.x & 15;
-  const long long tmask = (1LL << tile_log2) - 1;
-  const long long lstep = k_pad << tile_log2;  // next modulus of the same row
+  const long long lstep = k_pad * tile_rows;  // next modulus of the same row
 #pragma unroll 1
   for (int it = 0; it < 2; ++it) {
     const int r = (threadIdx.x >> 4) + 16 * it;
@@ -366,8 +364,9 @@ __global__ void __launch_bounds__(256) k_residues(OperandView v, const int* __re
 #pragma unroll
     for (int q = 0; q < 8; ++q) vl[q] = int_of(x[q]);
     // row of modulus 0 in the residue layout
+    const unsigned ti = static_cast<unsigned>(row) / static_cast<unsigned>(tile_rows);
     const long long base_row =
-        (((plane * tiles + (row >> tile_log2)) * mods.L) << tile_log2) + (row & tmask);
+        ((plane * tiles + ti) * mods.L) * tile_rows + (static_cast<unsigned>(row) - ti * tile_rows);
     uint8_t* dst = out + base_row * k_pad + k0 + 8 * t;
 #pragma unroll
     for (int l = 0; l < (LM ? LM : kOzakiMaxModuli); ++l) {
@@ -392,35 +391,45 @@ __global__ void __launch_bounds__(256) k_residues(OperandView v, const int* __re
 // ---------------------------------------------------------------------------
 // tcgen05 int8 product kernel
 // ---------------------------------------------------------------------------
-// Work-item tile: kJHalves x 128 output columns j by 256 output rows i.  One
-// half: the two 256-column TMEM accumulators are double-buffered across items;
-// two halves: both accumulators belong to one item (two MMAs per K step share
-// the i operand), so each K step moves 64 KiB for twice the products.
-#ifndef UW12_I8_JHALVES
-#define UW12_I8_JHALVES 1
-#endif
-constexpr int kJHalves = UW12_I8_JHALVES;
-static_assert(kJHalves == 1 || kJHalves == 2, "one or two j halves per work item");
-constexpr int kTileJ = 128;  // MMA M (TMEM lanes): output columns j
-constexpr int kItemJ = kTileJ * kJHalves;  // output columns j per work item
-constexpr int kTileI = 256;  // MMA N (TMEM columns): output rows i
-constexpr int kTileK = 128;  // bytes of K per pipeline stage (one 128-byte swizzle row)
-constexpr int kBytesJ = kItemJ * kTileK;  // 16 or 32 KiB
-constexpr int kBytesI = kTileI * kTileK;  // 32 KiB
+// Work item: TJ = 128 (one CTA) or 256 (a CTA pair) output columns j by tile_i
+// <= 256 output rows i of one modulus and one K chunk.  A CTA holds 128 columns j
+// in its 128 TMEM lanes; the two 256-column TMEM accumulators are double-buffered
+// across items.
+//
+// What bounds it: at K = 1500 the int8 tensor pipe under the power cap (1.59 ms for
+// 20000 x 6000 x 1500 and 14 moduli with no epilogue at all, 3.16 POPS) and, below
+// about K = 1000, the epilogue's arithmetic and stores.  The single critical thread
+// of each role must stay off that path: items advance without divisions, and the
+// epilogue reduces with one conversion, FMA and multiply-add per accumulator and
+// stores whole sectors.  A CTA pair (cta_group::2) shares both operands of its
+// 256 x 256 tile: each CTA loads its own 128 columns j and half of the rows i, 32
+// instead of 48 KiB from L2 per 512 tensor cycles.  Measured (one CTA, decoding
+// every item, remainders in [0, p), 16-byte stores -> now): 20000 x 6000 x 1500 2.05
+// -> 1.78 ms, 2500 x 200000 x 2000 11.7 -> 9.9, 2500 x 200000 x 500 5.0 -> 4.2,
+// 1200 x 900 x 900 in 64 batches 1.06 -> 0.88.  Eight epilogue warps instead of four
+// gain 3 % at K = 500 and lose 2 % at K = 1500.
+constexpr int kLanes = 128;     // TMEM lanes: output columns j per CTA
+constexpr int kMaxTileI = 256;  // MMA N (TMEM columns): output rows i
+constexpr int kTileK = 128;     // bytes of K per pipeline stage (one 128-byte swizzle row)
+constexpr int kBytesJ = kLanes * kTileK;  // 16 KiB
 constexpr int kMmaK = 32;                 // K of one kind::i8 MMA
-constexpr int kAccBufs = 2 / kJHalves;    // accumulator sets (2 x 256 TMEM columns in all)
-constexpr int kEpiWarps = 4 * kJHalves;   // one per TMEM lane quarter and j half
+constexpr int kEpiWarps = 4;              // one per TMEM lane quarter
 constexpr int kThreads = 64 + 32 * kEpiWarps;
+// stages of 48 (one CTA) or 32 KiB (pair)
+constexpr int stages_of(bool pair) { return pair ? 6 : 4; }
+constexpr int bytes_i_of(bool pair) { return (pair ? kMaxTileI / 2 : kMaxTileI) * kTileK; }
 constexpr unsigned long long kWaitLimitNs = 4000000000ULL;  // 4 s
 
 struct MmaArgs {
-  int tiles_j, tiles_i, L, splits, nbatch, nbo1;
-  long long n_items;
+  int tiles_j, tiles_i, tile_j, tile_i, L, splits, nbatch, nbo1;
+  unsigned n_items;
+  int step[6];  // mixed-radix digits (tj, ti, l, split, b1, b2) of the number of groups
   int a_var1, a_var2, b_var1, b_var2;  // operand planes vary with bo1 / bo2
   int planes_a, planes_b;
   long long m_pad, n_pad;
   int kb_per_split, kb_total;
-  uint32_t p[kOzakiMaxModuli], barrett[kOzakiMaxModuli], off[kOzakiMaxModuli];
+  int p[kOzakiMaxModuli], c16[kOzakiMaxModuli], mode[kOzakiMaxModuli];
+  float inv_p[kOzakiMaxModuli];
   uint8_t* R;
   int* err;
 };
@@ -470,13 +479,38 @@ __device__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_fla
     }
   }
 }
+// 2-D box load into this CTA's shared memory; bytes are counted on the barrier
+// at the shared::cluster address bar (the pair's leader's when PAIR).
+template <bool PAIR>
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y,
                                             uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-      : "memory");
+  if (PAIR)
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        ".cta_group::2 [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+  else
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
+// shared::cluster address of this CTA's shared address `a` in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t map_rank(uint32_t a, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tc_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -491,25 +525,46 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
          (static_cast<uint64_t>(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
 // Instruction descriptor of kind::i8: s32 accumulator, signed int8 A and B,
-// both K-major, N = kTileI, M = kTileJ.
-constexpr uint32_t kIdesc = (2u << 4) | (1u << 7) | (1u << 10) |
-                            (static_cast<uint32_t>(kTileI >> 3) << 17) |
-                            (static_cast<uint32_t>(kTileJ >> 4) << 24);
-
-__device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                       uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(
-          tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
-      : "memory");
+// both K-major, N = tile_i, M = 128 (one CTA) or 256 (pair).
+__device__ __forceinline__ uint32_t i8_idesc(int tile_i, int m) {
+  return (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(tile_i >> 3) << 17) |
+         (static_cast<uint32_t>(m >> 4) << 24);
 }
+
+template <bool PAIR>
+__device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                       uint32_t idesc, uint32_t accumulate) {
+  if (PAIR)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, "
+        "p;\n\t}" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(
+            tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u)
+        : "memory");
+}
+// Arrives on the barrier (of both CTAs of a pair) when the MMAs issued so far
+// have completed.
+template <bool PAIR>
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   bar)
-               : "memory");
+  if (PAIR)
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 "
+        "[%0], %1;" ::"r"(bar),
+        "h"(static_cast<uint16_t>(3))
+        : "memory");
+  else
+    asm volatile(
+        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
+        : "memory");
 }
 
 #define UW12_TMEM_LD32(taddr, v)                                                               \
@@ -533,59 +588,115 @@ __device__ __forceinline__ long long residue_offset(const MmaArgs& a, int split,
   return (((static_cast<long long>(split) * a.nbatch + b) * a.n_pad + j) * a.L + l) * a.m_pad;
 }
 
+// Residue bytes of an accumulator v (|v| <= 2^30) modulo p: r = v - q p with
+// q = rint(float(v) / p) taken from the low bits of fma(float(v), 1/p, 1.5 2^23), as
+// a signed byte stored with 128 added.  float(v) and 1/p are each off by 2^-24, so
+// |r| <= p / 2 + |v| 2^-23: below 128 for short enough K chunks (kFast).  Where it
+// may not be, v is first replaced by (v mod 2^16) + floor(v / 2^16) (2^16 mod p), at
+// most 2^21.04, congruent modulo p (kFold).  p = 256: the low byte (kMask).  A
+// conversion, an FMA and a multiply-add per accumulator, against seven integer
+// instructions at half rate for a remainder in [0, p).
+enum ResidueMode { kMask = 0, kFast = 1, kFold = 2 };
+
+template <int MODE>
+__device__ __forceinline__ uint32_t residue_of(uint32_t acc, int p, int c16, float inv_p) {
+  int v = static_cast<int>(acc);
+  if (MODE == kMask) return acc;
+  if (MODE == kFold) v = (v & 0xffff) + (v >> 16) * c16;
+  const int q = __float_as_int(fmaf(__int2float_rn(v), inv_p, 12582912.0f));
+  return static_cast<uint32_t>(v - q * p);  // low byte: the offset 1.5 2^23 has none
+}
+
+// Four residues to one word of bytes, 128 added to each.
+template <int MODE>
+__device__ __forceinline__ uint32_t residue_word(const uint32_t* v, int p, int c16, float inv_p) {
+  const uint32_t b01 = __byte_perm(residue_of<MODE>(v[0], p, c16, inv_p),
+                                   residue_of<MODE>(v[1], p, c16, inv_p), 0x0040);
+  const uint32_t b23 = __byte_perm(residue_of<MODE>(v[2], p, c16, inv_p),
+                                   residue_of<MODE>(v[3], p, c16, inv_p), 0x0040);
+  return __byte_perm(b01, b23, 0x5410) ^ 0x80808080u;
+}
+
 __device__ __forceinline__ uint32_t mod_u32(uint32_t u, uint32_t p, uint32_t barrett) {
   uint32_t r = u - __umulhi(u, barrett) * p;
   return r >= p ? r - p : r;
 }
 
-// One work item = one 128 x 256 output tile of one modulus, one K chunk and
-// one batch; items are numbered tile fastest, then modulus, K chunk, batch.
+// One work item = one tile_j x tile_i output tile of one modulus, one K chunk and
+// one batch; items are numbered tile fastest (j, then i), then modulus, K chunk,
+// batch: the digits of a mixed-radix number.  A role decodes its first item and
+// then adds the digits of the step (the number of groups) with carries: decoding
+// every item took five 64-bit divisions, about 3000 cycles of each role's single
+// critical thread per item of 2048 (K = 512) to 6144 (K = 1536) tensor cycles.
 struct WorkItem {
-  int tj, ti, l, split, b, kb0, nkb, yj, yi;
+  int tj, ti, l, split, b1, b2;
+
+  __device__ __forceinline__ WorkItem(const MmaArgs& a, unsigned w) {
+    tj = static_cast<int>(w % a.tiles_j);
+    w /= a.tiles_j;
+    ti = static_cast<int>(w % a.tiles_i);
+    w /= a.tiles_i;
+    l = static_cast<int>(w % a.L);
+    w /= a.L;
+    split = static_cast<int>(w % a.splits);
+    w /= a.splits;
+    b1 = static_cast<int>(w % a.nbo1);
+    b2 = static_cast<int>(w / a.nbo1);
+  }
+  __device__ __forceinline__ void advance(const MmaArgs& a) {
+    int carry = 0;
+    auto add = [&](int& digit, int step, int radix) {
+      digit += step + carry;
+      carry = digit >= radix;
+      digit -= carry ? radix : 0;
+    };
+    add(tj, a.step[0], a.tiles_j);
+    add(ti, a.step[1], a.tiles_i);
+    add(l, a.step[2], a.L);
+    add(split, a.step[3], a.splits);
+    add(b1, a.step[4], a.nbo1);
+    b2 += a.step[5] + carry;
+  }
+  __device__ __forceinline__ int kb0(const MmaArgs& a) const { return split * a.kb_per_split; }
+  __device__ __forceinline__ int nkb(const MmaArgs& a) const {
+    return min(a.kb_per_split, a.kb_total - kb0(a));
+  }
+  // first residue row of the tile: ((plane * tiles + tile) * L + l) * tile rows
+  __device__ __forceinline__ int row_j(const MmaArgs& a) const {
+    const int pb = (a.b_var1 ? b1 : 0) + (a.b_var1 ? a.nbo1 : 1) * (a.b_var2 ? b2 : 0);
+    return ((pb * a.tiles_j + tj) * a.L + l) * a.tile_j;
+  }
+  __device__ __forceinline__ int row_i(const MmaArgs& a) const {
+    const int pa = (a.a_var1 ? b1 : 0) + (a.a_var1 ? a.nbo1 : 1) * (a.a_var2 ? b2 : 0);
+    return ((pa * a.tiles_i + ti) * a.L + l) * a.tile_i;
+  }
 };
 
-__device__ __forceinline__ WorkItem decode_item(const MmaArgs& a, long long w) {
-  WorkItem it;
-  const long long tiles = static_cast<long long>(a.tiles_j) * a.tiles_i;
-  const long long tile = w % tiles;
-  long long rest = w / tiles;
-  it.tj = static_cast<int>(tile % a.tiles_j);
-  it.ti = static_cast<int>(tile / a.tiles_j);
-  it.l = static_cast<int>(rest % a.L);
-  rest /= a.L;
-  it.split = static_cast<int>(rest % a.splits);
-  it.b = static_cast<int>(rest / a.splits);
-  const int b1 = it.b % a.nbo1, b2 = it.b / a.nbo1;
-  const int pa = (a.a_var1 ? b1 : 0) + (a.a_var1 ? a.nbo1 : 1) * (a.a_var2 ? b2 : 0);
-  const int pb = (a.b_var1 ? b1 : 0) + (a.b_var1 ? a.nbo1 : 1) * (a.b_var2 ? b2 : 0);
-  it.kb0 = it.split * a.kb_per_split;
-  it.nkb = min(a.kb_per_split, a.kb_total - it.kb0);
-  // residue rows: ((plane * tiles + tile) * L + l) * tile_rows + row in tile
-  it.yj = static_cast<int>(
-      ((static_cast<long long>(pb) * (a.n_pad / kItemJ) + it.tj) * a.L + it.l) * kItemJ);
-  it.yi = static_cast<int>(
-      ((static_cast<long long>(pa) * (a.m_pad / kTileI) + it.ti) * a.L + it.l) * kTileI);
-  return it;
+// Arrive on the barrier at a shared::cluster address.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar)
+               : "memory");
 }
 
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
-// Persistent: one CTA per SM walks the work items blockIdx.x, + gridDim.x, ...
-// through a STAGES-deep TMA ring; with one j half per item the two TMEM
-// accumulators (2 x 256 columns) let the epilogue of one item overlap the MMAs
-// of the next, with two halves they hold the item's two halves.
-template <int STAGES>
+// Persistent: one CTA (or CTA pair) per SM (pair) walks the work items group id,
+// + number of groups, ... through a ring of TMA stages.  Warp roles in every
+// CTA: 0 TMA producer, 1 TMEM owner and, in the pair's leader (cluster rank 0),
+// MMA issuer, 2.. epilogue.  Barriers: full (the leader's; bytes of both CTAs),
+// empty and acc_full (each CTA's, arrived by the commits), acc_empty (the
+// leader's, arrived by the epilogue warps of both).
+template <bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
     k_i8_mma(const __grid_constant__ CUtensorMap tm_j, const __grid_constant__ CUtensorMap tm_i,
              const MmaArgs a) {
+  constexpr int STAGES = stages_of(PAIR);
+  constexpr int BYTES_I = bytes_i_of(PAIR);
+  constexpr int CTAS = PAIR ? 2 : 1;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  uint8_t* sj = base;                            // STAGES x kBytesJ
-  uint8_t* si = base + STAGES * kBytesJ;         // STAGES x 32 KiB
-  uint64_t* bars = reinterpret_cast<uint64_t*>(si + STAGES * kBytesI);
+  uint8_t* sj = base;                            // STAGES x 16 KiB
+  uint8_t* si = base + STAGES * kBytesJ;         // STAGES x BYTES_I
+  uint64_t* bars = reinterpret_cast<uint64_t*>(si + STAGES * BYTES_I);
   uint64_t* full = bars;
   uint64_t* empty = bars + STAGES;
   uint64_t* acc_full = bars + 2 * STAGES;       // [2]
@@ -594,6 +705,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const uint32_t rank = PAIR ? cluster_rank() : 0u;
+  const unsigned group = blockIdx.x / CTAS, groups = gridDim.x / CTAS;
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(smem_u32(&full[s]), 1);
@@ -601,147 +714,176 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&acc_full[b]), 1);
-      mbar_init(smem_u32(&acc_empty[b]), kEpiWarps);  // one arrival per epilogue warp
+      mbar_init(smem_u32(&acc_empty[b]), CTAS * kEpiWarps);  // one arrival per epilogue warp
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(tmem_slot)),
-                 "r"(static_cast<uint32_t>(2 * kTileI))
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                       smem_u32(tmem_slot)),
+                   "r"(static_cast<uint32_t>(2 * kMaxTileI))
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                       smem_u32(tmem_slot)),
+                   "r"(static_cast<uint32_t>(2 * kMaxTileI))
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();  // the peer's barriers are initialised
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0 && lane == 0) {
-    // ---- TMA producer
-    long long pos = 0;  // ring position, continued across items
+    // ---- TMA producer: this CTA's 128 columns j and its share of the rows i
+    const int rows_i = a.tile_i / CTAS;
+    const uint32_t bytes = static_cast<uint32_t>(CTAS * (kBytesJ + rows_i * kTileK));
+    int s = 0;        // ring slot and its phase, continued across items
+    uint32_t ph = 0;
     bool ok = true;
-    for (long long w = blockIdx.x; ok && w < a.n_items; w += gridDim.x) {
-      const WorkItem it = decode_item(a, w);
-      for (int kb = 0; kb < it.nkb; ++kb) {
-        const int s = static_cast<int>(pos % STAGES);
-        const uint32_t ph = static_cast<uint32_t>(pos / STAGES) & 1;
+    WorkItem it(a, group);
+    for (unsigned w = group; ok && w < a.n_items; w += groups, it.advance(a)) {
+      const int yj = it.row_j(a) + static_cast<int>(rank) * kLanes;
+      const int yi = it.row_i(a) + static_cast<int>(rank) * rows_i;
+      const int kb0 = it.kb0(a), nkb = it.nkb(a);
+      for (int kb = 0; kb < nkb; ++kb) {
         if (!mbar_wait(smem_u32(&empty[s]), ph ^ 1, abort_flag, a.err, 1)) {
           ok = false;
           break;
         }
-        const uint32_t fb = smem_u32(&full[s]);
-        mbar_expect_tx(fb, kBytesJ + kBytesI);
-        const int x = (it.kb0 + kb) * kTileK;
-        tma_load_2d(smem_u32(sj + s * kBytesJ), &tm_j, x, it.yj, fb);
-        tma_load_2d(smem_u32(si + s * kBytesI), &tm_i, x, it.yi, fb);
-        ++pos;
+        uint32_t fb = smem_u32(&full[s]);
+        if (rank == 0) mbar_expect_tx(fb, bytes);
+        if (PAIR) fb = map_rank(fb, 0);
+        const int x = (kb0 + kb) * kTileK;
+        tma_load_2d<PAIR>(smem_u32(sj + s * kBytesJ), &tm_j, x, yj, fb);
+        tma_load_2d<PAIR>(smem_u32(si + s * BYTES_I), &tm_i, x, yi, fb);
+        if (++s == STAGES) {
+          s = 0;
+          ph ^= 1;
+        }
       }
     }
     if (!ok) {
-      // let the copies already issued land before the CTA exits
-      for (long long q = pos > STAGES ? pos - STAGES : 0; q < pos; ++q)
-        (void)mbar_wait(smem_u32(&full[q % STAGES]), static_cast<uint32_t>(q / STAGES) & 1,
-                        abort_flag, a.err, 1);
+      // the copies already issued land before the CTA exits: they count on barriers
+      // whose phase may never complete now, so give them a millisecond
+      for (const unsigned long long t0 = global_ns(); global_ns() - t0 < 1000000ULL;) {
+      }
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1 && lane == 0 && rank == 0) {
     // ---- MMA issuer
-    long long pos = 0;
-    int t = 0, last_buf = -1;
-    uint32_t last_use = 0;
-    for (long long w = blockIdx.x; w < a.n_items; w += gridDim.x, ++t) {
-      const WorkItem it = decode_item(a, w);
-      const int buf = t % kAccBufs;
-      const uint32_t use = static_cast<uint32_t>(t / kAccBufs);
+    const uint32_t idesc = i8_idesc(a.tile_i, CTAS * kLanes);
+    int s = 0, t = 0, last_buf = -1;
+    uint32_t ph = 0, last_use = 0;
+    WorkItem it(a, group);
+    for (unsigned w = group; w < a.n_items; w += groups, it.advance(a), ++t) {
+      const int buf = t & 1;
+      const uint32_t use = static_cast<uint32_t>(t >> 1);
       if (!mbar_wait(smem_u32(&acc_empty[buf]), (use & 1) ^ 1, abort_flag, a.err, 2)) break;
       tc_fence_after();
-      const uint32_t d = tmem + static_cast<uint32_t>(buf * kJHalves * kTileI);
+      const uint32_t d = tmem + static_cast<uint32_t>(buf * kMaxTileI);
       bool ok = true;
-      for (int kb = 0; kb < it.nkb; ++kb) {
-        const int s = static_cast<int>(pos % STAGES);
-        const uint32_t ph = static_cast<uint32_t>(pos / STAGES) & 1;
+      const int nkb = it.nkb(a);
+      for (int kb = 0; kb < nkb; ++kb) {
         if (!mbar_wait(smem_u32(&full[s]), ph, abort_flag, a.err, 2)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint64_t di = sw128_desc(smem_u32(si + s * kBytesI));
+        const uint64_t dj = sw128_desc(smem_u32(sj + s * kBytesJ));
+        const uint64_t di = sw128_desc(smem_u32(si + s * BYTES_I));
 #pragma unroll
-        for (int h = 0; h < kJHalves; ++h) {
-          // j half h: rows 128 h .. of the stage, accumulator columns 256 h ..
-          const uint64_t dj = sw128_desc(smem_u32(sj + s * kBytesJ + h * kTileJ * kTileK));
-#pragma unroll
-          for (int kk = 0; kk < kTileK / kMmaK; ++kk) {
-            // advance along K inside the swizzle row: +32 bytes = +2 in the
-            // 16-byte address field
-            mma_i8(d + static_cast<uint32_t>(h * kTileI), dj + 2 * kk, di + 2 * kk,
-                   (kb | kk) != 0);
-          }
+        for (int kk = 0; kk < kTileK / kMmaK; ++kk) {
+          // advance along K inside the swizzle row: +32 bytes = +2 in the
+          // 16-byte address field
+          mma_i8<PAIR>(d, dj + 2 * kk, di + 2 * kk, idesc, (kb | kk) != 0);
         }
-        mma_commit(smem_u32(&empty[s]));
-        ++pos;
+        mma_commit<PAIR>(smem_u32(&empty[s]));
+        if (++s == STAGES) {
+          s = 0;
+          ph ^= 1;
+        }
       }
-      mma_commit(smem_u32(&acc_full[buf]));  // also on failure, so the epilogue wakes
+      mma_commit<PAIR>(smem_u32(&acc_full[buf]));  // also on failure, so the epilogue wakes
       last_buf = buf;
       last_use = use;
       if (!ok) break;
     }
-    if (last_buf >= 0)  // every MMA of this CTA has completed before TMEM is released
+    if (last_buf >= 0)  // every MMA of this CTA (pair) has completed before TMEM is released
       (void)mbar_wait(smem_u32(&acc_full[last_buf]), last_use & 1, abort_flag, a.err, 4);
   } else if (warp >= 2) {
     // ---- epilogue: TMEM -> residues mod p -> uint8 rows
-    const int q = warp & 3;          // TMEM lane quarter this warp may access
-    const int h = (warp - 2) / 4;    // j half
+    const int q = warp & 3;               // TMEM lane quarter this warp may access
     int t = 0;
-    for (long long w = blockIdx.x; w < a.n_items; w += gridDim.x, ++t) {
-      const WorkItem it = decode_item(a, w);
-      const int buf = t % kAccBufs;
-      const uint32_t use = static_cast<uint32_t>(t / kAccBufs);
+    WorkItem it(a, group);
+    for (unsigned w = group; w < a.n_items; w += groups, it.advance(a), ++t) {
+      const int buf = t & 1;
+      const uint32_t use = static_cast<uint32_t>(t >> 1);
       // warp-uniform, so that the .sync.aligned TMEM loads below are convergent
       const bool ok =
           __all_sync(0xffffffffu, mbar_wait(smem_u32(&acc_full[buf]), use & 1, abort_flag, a.err, 3));
       tc_fence_after();
       if (!ok) break;
-      const uint32_t p = a.p[it.l], bm = a.barrett[it.l], off = a.off[it.l];
-      const long long j = static_cast<long long>(it.tj) * kItemJ + h * kTileJ + q * 32 + lane;
-      uint8_t* rowp = a.R + residue_offset(a, it.split, it.b, j, it.l) +
-                      static_cast<long long>(it.ti) * kTileI;
-      const uint32_t tq = tmem + static_cast<uint32_t>((buf * kJHalves + h) * kTileI) +
+      const int p = a.p[it.l], c16 = a.c16[it.l], mode = a.mode[it.l];
+      const float inv_p = a.inv_p[it.l];
+      const long long j = static_cast<long long>(it.tj) * a.tile_j + rank * kLanes + q * 32 + lane;
+      uint8_t* rowp = a.R + residue_offset(a, it.split, it.b1 + a.nbo1 * it.b2, j, it.l) +
+                      static_cast<long long>(it.ti) * a.tile_i;
+      const uint32_t tq = tmem + static_cast<uint32_t>(buf * kMaxTileI) +
                           (static_cast<uint32_t>(q * 32) << 16);
 #pragma unroll 1
-      for (int c = 0; c < kTileI / 32; ++c) {
+      for (int c = 0; c < a.tile_i / 32; ++c) {
         uint32_t v[32];
         UW12_TMEM_LD32(tq + c * 32, v);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         uint32_t wd[8];
+        if (mode == kFast) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          uint32_t word = 0;
+          for (int e = 0; e < 8; ++e) wd[e] = residue_word<kFast>(v + 4 * e, p, c16, inv_p);
+        } else if (mode == kFold) {
 #pragma unroll
-          for (int u = 0; u < 4; ++u) word |= mod_u32(v[4 * e + u] + off, p, bm) << (8 * u);
-          wd[e] = word;
+          for (int e = 0; e < 8; ++e) wd[e] = residue_word<kFold>(v + 4 * e, p, c16, inv_p);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) wd[e] = residue_word<kMask>(v + 4 * e, p, c16, inv_p);
         }
-        uint4* dst = reinterpret_cast<uint4*>(rowp + c * 32);
-        dst[0] = make_uint4(wd[0], wd[1], wd[2], wd[3]);
-        dst[1] = make_uint4(wd[4], wd[5], wd[6], wd[7]);
+        // one whole 32-byte sector per lane
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(rowp + c * 32),
+                     "r"(wd[0]), "r"(wd[1]), "r"(wd[2]), "r"(wd[3]), "r"(wd[4]), "r"(wd[5]),
+                     "r"(wd[6]), "r"(wd[7])
+                     : "memory");
       }
       // this warp's TMEM reads are done: release the accumulator
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&acc_empty[buf]));
+      if (lane == 0) {
+        const uint32_t bar = smem_u32(&acc_empty[buf]);
+        mbar_arrive_cluster(PAIR ? map_rank(bar, 0) : bar);
+      }
     }
   }
 
   tc_fence_before();
+  __syncwarp();
   __syncthreads();
+  if (PAIR) cluster_sync();  // no MMA, copy or arrival of the pair is outstanding
   if (warp == 1) {
     tc_fence_after();
     __syncwarp();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(static_cast<uint32_t>(2 * kTileI))
-                 : "memory");
+    if (PAIR)
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                   "r"(static_cast<uint32_t>(2 * kMaxTileI))
+                   : "memory");
+    else
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                   "r"(static_cast<uint32_t>(2 * kMaxTileI))
+                   : "memory");
   }
 }
 
@@ -760,7 +902,9 @@ struct CrtArgs {
   long long ldc, sCo1, sCo2;
   double alpha, beta;
   uint32_t p[kOzakiMaxModuli], barrett[kOzakiMaxModuli];
+  uint32_t red_off[kOzakiMaxModuli];  // REDUCE: undoes the 128 added to each K chunk's residue
   double w[kOzakiMaxModuli][kMaxChunks];
+  double s0[kMaxChunks];  // -128 sum_l w: undoes the 128 added to each residue (exact)
   double mc[kMaxChunks];
   double inv_m;
   int cw;          // CRT chunk width in bits
@@ -840,8 +984,9 @@ __device__ __forceinline__ uint32_t load_residues(const uint8_t* p) {
   return __ldg(reinterpret_cast<const unsigned short*>(p));
 }
 
-// REDUCE: several K chunks, whose residue sums are reduced mod p; with one K
-// chunk the stored residues (already in [0, p)) enter the CRT sum directly.
+// Stored residues are bytes in [0, 255], 128 more than a residue in [-128, 127].
+// REDUCE: several K chunks (at most 257), whose byte sums are reduced mod p; with
+// one K chunk the bytes enter the CRT sum directly, which starts at s0.
 template <int NCH, bool REDUCE>
 __global__ void __launch_bounds__(256, REDUCE ? 2 : kCrtMinBlocks) k_crt(const CrtArgs a) {
   constexpr int E = kCrtElems;
@@ -891,9 +1036,9 @@ __global__ void __launch_bounds__(256, REDUCE ? 2 : kCrtMinBlocks) k_crt(const C
 #pragma unroll
     for (int e = 0; e < E; ++e)
 #pragma unroll
-      for (int c = 0; c < NCH; ++c) S[e][c] = 0.0;
+      for (int c = 0; c < NCH; ++c) S[e][c] = REDUCE ? 0.0 : a.s0[c];
     if (!REDUCE) {
-      // one K chunk: the stored residues (in [0, p)) enter the CRT sum directly
+      // one K chunk: the stored residues enter the CRT sum directly
 #pragma unroll
       for (int l = 0; l < kOzakiMaxModuli; ++l) {
         if (l < a.L) {
@@ -932,7 +1077,7 @@ __global__ void __launch_bounds__(256, REDUCE ? 2 : kCrtMinBlocks) k_crt(const C
           const uint32_t u[4] = {s02[l] & 0xffffu, s13[l] & 0xffffu, s02[l] >> 16, s13[l] >> 16};
 #pragma unroll
           for (int e = 0; e < E; ++e) {
-            const double r = small_to_double(mod_u32(u[e], p, bm));
+            const double r = small_to_double(mod_u32(u[e] + a.red_off[l], p, bm));
 #pragma unroll
             for (int c = 0; c < NCH; ++c) S[e][c] = fma(r, a.w[l][c], S[e][c]);
           }
@@ -1044,7 +1189,7 @@ __global__ void __launch_bounds__(256, 3) k_crt_pipe(const CrtArgs a) {
 #pragma unroll
     for (int e = 0; e < 4; ++e)
 #pragma unroll
-      for (int c = 0; c < NCH; ++c) S[e][c] = 0.0;
+      for (int c = 0; c < NCH; ++c) S[e][c] = a.s0[c];
 #pragma unroll
     for (int l = 0; l < (LM ? LM : kOzakiMaxModuli); ++l) {
       if (LM || l < L) {
@@ -1122,9 +1267,10 @@ CUtensorMap make_map(const uint8_t* base, long long rows, long long k_pad, int b
   return m;
 }
 
-constexpr int kStages = 4 / kJHalves + (kJHalves - 1);  // 4 x 48 or 3 x 64 KiB of stages
-constexpr size_t kMmaSmem =
-    size_t(kStages) * (kBytesJ + kBytesI) + 1024 /*alignment*/ + 256 /*barriers*/;
+constexpr size_t mma_smem(bool pair) {
+  return size_t(stages_of(pair)) * (kBytesJ + bytes_i_of(pair)) + 1024 /*alignment*/ +
+         256 /*barriers*/;
+}
 
 long long round_up(long long x, long long m) { return (x + m - 1) / m * m; }
 
@@ -1160,6 +1306,24 @@ struct Timer {
   }
 };
 
+// Output tile of the int8 products: the pair's 256 columns j unless they would be
+// mostly padding (one CTA is 1.2 to 1.4 times slower per padded column), and the
+// rows i per tile, a multiple of 32, that pad m least (the wider one of two
+// that differ by less than a sixteenth).
+struct ProductTile {
+  bool pair;
+  int tile_j, tile_i;
+};
+ProductTile product_tile(long long m, long long n) {
+  ProductTile t;
+  t.pair = 4 * round_up(n, 2 * kLanes) <= 5 * round_up(n, kLanes);
+  t.tile_j = t.pair ? 2 * kLanes : kLanes;
+  t.tile_i = kMaxTileI;
+  for (int ti = kMaxTileI; ti >= 128; ti -= 32)
+    if (16 * round_up(m, ti) < 15 * round_up(m, t.tile_i)) t.tile_i = ti;
+  return t;
+}
+
 // Runs one GEMM whose temporaries fit.  d.nbo2 == 1 or both batch dims are
 // handled through the plane maps.
 void run_core(const GemmDesc& d, const Consts& cs, int beta, cudaStream_t s) {
@@ -1167,7 +1331,8 @@ void run_core(const GemmDesc& d, const Consts& cs, int beta, cudaStream_t s) {
   const long long nbo1 = d.nbo1, nbo2 = d.nbo2, nbatch = nbo1 * nbo2;
   const long long k_total = d.k * d.nbr1 * d.nbr2;
   const long long k_pad = round_up(k_total, kTileK);
-  const long long m_pad = round_up(d.m, kTileI), n_pad = round_up(d.n, kItemJ);
+  const ProductTile pt = product_tile(d.m, d.n);
+  const long long m_pad = round_up(d.m, pt.tile_i), n_pad = round_up(d.n, pt.tile_j);
   const int a_var1 = d.sAo1 != 0 && nbo1 > 1, a_var2 = d.sAo2 != 0 && nbo2 > 1;
   const int b_var1 = d.sBo1 != 0 && nbo1 > 1, b_var2 = d.sBo2 != 0 && nbo2 > 1;
   const int pa1 = a_var1 ? int(nbo1) : 1, pa2 = a_var2 ? int(nbo2) : 1;
@@ -1177,12 +1342,14 @@ void run_core(const GemmDesc& d, const Consts& cs, int beta, cudaStream_t s) {
   // K chunks: <= kMaxKChunk bytes each; more chunks when the tile grid alone
   // would leave SMs idle.
   const long long kb_total = k_pad / kTileK;
-  const long long tiles_j = n_pad / kItemJ, tiles_i = m_pad / kTileI;
-  const long long ctas = tiles_j * tiles_i * L * nbatch;
+  const long long tiles_j = n_pad / pt.tile_j, tiles_i = m_pad / pt.tile_i;
+  const long long items = tiles_j * tiles_i * L * nbatch;
+  const long long groups = num_sms() / (pt.pair ? 2 : 1);
   long long splits = (k_pad + kMaxKChunk - 1) / kMaxKChunk;
-  const long long want = (2 * num_sms() + ctas - 1) / ctas;
+  const long long want = (2 * groups + items - 1) / items;
   splits = std::max(splits, std::min(want, std::max<long long>(1, kb_total / 8)));
   splits = std::min(splits, std::max<long long>(1, 65535 / nbatch));
+  splits = std::min<long long>(splits, 256);  // byte sums of the chunks fit 16 bits
   long long kb_per = (kb_total + splits - 1) / splits;
   kb_per = std::min<long long>(kb_per, kMaxKChunk / kTileK);
   splits = (kb_total + kb_per - 1) / kb_per;
@@ -1234,21 +1401,20 @@ void run_core(const GemmDesc& d, const Consts& cs, int beta, cudaStream_t s) {
       k_exponent_to_shift<<<static_cast<unsigned>((nsh + 255) / 256), 256, 0, s>>>(ep, nsh, beta,
                                                                                   sh);
       UW12_LAUNCHED();
-      const int tlog = tile_rows == 256 ? 8 : 7;
       const long long tiles = rows_pad / tile_rows;
       // the default modulus count runs a fully unrolled, unguarded moduli loop
       if (v.ks == 1 && L == kOzakiDefaultModuli)
-        k_residues<true, kOzakiDefaultModuli><<<g, 256, 0, s>>>(v, sh, mods, tlog, tiles, k_pad, out);
+        k_residues<true, kOzakiDefaultModuli><<<g, 256, 0, s>>>(v, sh, mods, tile_rows, tiles, k_pad, out);
       else if (v.ks == 1)
-        k_residues<true, 0><<<g, 256, 0, s>>>(v, sh, mods, tlog, tiles, k_pad, out);
+        k_residues<true, 0><<<g, 256, 0, s>>>(v, sh, mods, tile_rows, tiles, k_pad, out);
       else if (L == kOzakiDefaultModuli)
-        k_residues<false, kOzakiDefaultModuli><<<g, 256, 0, s>>>(v, sh, mods, tlog, tiles, k_pad, out);
+        k_residues<false, kOzakiDefaultModuli><<<g, 256, 0, s>>>(v, sh, mods, tile_rows, tiles, k_pad, out);
       else
-        k_residues<false, 0><<<g, 256, 0, s>>>(v, sh, mods, tlog, tiles, k_pad, out);
+        k_residues<false, 0><<<g, 256, 0, s>>>(v, sh, mods, tile_rows, tiles, k_pad, out);
       UW12_LAUNCHED();
     };
-    prep(va, planes_a, m_pad, kTileI, sa, ea, ra);
-    prep(vb, planes_b, n_pad, kItemJ, sb, eb, rb);
+    prep(va, planes_a, m_pad, pt.tile_i, sa, ea, ra);
+    prep(vb, planes_b, n_pad, pt.tile_j, sb, eb, rb);
     tm.stop();
   }
 
@@ -1261,18 +1427,28 @@ void run_core(const GemmDesc& d, const Consts& cs, int beta, cudaStream_t s) {
       UW12_CUDA(cudaGetDevice(&dev));
       std::lock_guard<std::mutex> lk(attr_mu);
       if (!attr_set[dev]) {
-        UW12_CUDA(cudaFuncSetAttribute(k_i8_mma<kStages>,
+        UW12_CUDA(cudaFuncSetAttribute(k_i8_mma<false>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(kMmaSmem)));
+                                       static_cast<int>(mma_smem(false))));
+        UW12_CUDA(cudaFuncSetAttribute(k_i8_mma<true>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       static_cast<int>(mma_smem(true))));
         attr_set[dev] = true;
       }
     }
-    const CUtensorMap tmj = make_map(rb, L * planes_b * n_pad, k_pad, kItemJ);
-    const CUtensorMap tmi = make_map(ra, L * planes_a * m_pad, k_pad, kTileI);
+    const CUtensorMap tmj = make_map(rb, L * planes_b * n_pad, k_pad, kLanes);
+    const CUtensorMap tmi = make_map(ra, L * planes_a * m_pad, k_pad,
+                                     pt.tile_i / (pt.pair ? 2 : 1));
     MmaArgs ma{};
     ma.tiles_j = static_cast<int>(tiles_j);
     ma.tiles_i = static_cast<int>(tiles_i);
-    ma.n_items = tiles_j * tiles_i * L * splits * nbatch;
+    ma.tile_j = pt.tile_j;
+    ma.tile_i = pt.tile_i;
+    const long long n_items = tiles_j * tiles_i * L * splits * nbatch;
+    if (n_items >= (1LL << 31) || L * planes_a * m_pad >= (1LL << 31) ||
+        L * planes_b * n_pad >= (1LL << 31))
+      throw Error(kErrInvalid, "split-precision GEMM: too many output tiles");
+    ma.n_items = static_cast<unsigned>(n_items);
     ma.L = L;
     ma.splits = static_cast<int>(splits);
     ma.nbatch = static_cast<int>(nbatch);
@@ -1285,9 +1461,12 @@ void run_core(const GemmDesc& d, const Consts& cs, int beta, cudaStream_t s) {
     ma.kb_per_split = static_cast<int>(kb_per);
     ma.kb_total = static_cast<int>(kb_total);
     for (int l = 0; l < L; ++l) {
-      ma.p[l] = cs.p[l];
-      ma.barrett[l] = cs.barrett[l];
-      ma.off[l] = cs.off[l];
+      const int p = static_cast<int>(cs.p[l]);
+      const double vmax = double(std::min(k_total, kb_per * kTileK)) * double(p / 2) * (p / 2);
+      ma.p[l] = p;
+      ma.inv_p[l] = 1.0f / float(p);
+      ma.c16[l] = 65536 % p > p / 2 ? 65536 % p - p : 65536 % p;
+      ma.mode[l] = p == 256 ? kMask : 0.5 * p + vmax * 0x1p-23 < 127.99 ? kFast : kFold;
     }
     ma.R = reinterpret_cast<uint8_t*>(R.get());
     ma.err = err_flag();
@@ -1296,8 +1475,32 @@ void run_core(const GemmDesc& d, const Consts& cs, int beta, cudaStream_t s) {
     std::snprintf(shape, sizeof(shape), "i8 %lld %lld %lld %lld L%d s%lld", d.m, d.n, k_total,
                   nbatch, L, splits);
     Timer tm(kProfI8Mma, ops, shape, s);
-    const unsigned grid = static_cast<unsigned>(std::min<long long>(ma.n_items, num_sms()));
-    k_i8_mma<kStages><<<grid, kThreads, kMmaSmem, s>>>(tmj, tmi, ma);
+    const unsigned n_groups = static_cast<unsigned>(std::min<long long>(n_items, groups));
+    {
+      const int radix[5] = {ma.tiles_j, ma.tiles_i, ma.L, ma.splits, ma.nbo1};
+      unsigned rest = n_groups;
+      for (int q = 0; q < 5; ++q) {
+        ma.step[q] = static_cast<int>(rest % radix[q]);
+        rest /= radix[q];
+      }
+      ma.step[5] = static_cast<int>(rest);
+    }
+    if (pt.pair) {
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(2 * n_groups);
+      cfg.blockDim = dim3(kThreads);
+      cfg.dynamicSmemBytes = mma_smem(true);
+      cfg.stream = s;
+      cudaLaunchAttribute attr{};
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = 2;
+      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      UW12_CUDA(cudaLaunchKernelEx(&cfg, k_i8_mma<true>, tmj, tmi, ma));
+    } else {
+      k_i8_mma<false><<<n_groups, kThreads, mma_smem(false), s>>>(tmj, tmi, ma);
+    }
     UW12_LAUNCHED();
     tm.stop();
   }
@@ -1320,7 +1523,11 @@ void run_core(const GemmDesc& d, const Consts& cs, int beta, cudaStream_t s) {
     for (int l = 0; l < L; ++l) {
       ca.p[l] = cs.p[l];
       ca.barrett[l] = cs.barrett[l];
-      for (int c = 0; c < kMaxChunks; ++c) ca.w[l][c] = cs.w[l][c];
+      ca.red_off[l] = cs.p[l] - static_cast<uint32_t>(128 * splits % cs.p[l]);
+      for (int c = 0; c < kMaxChunks; ++c) {
+        ca.w[l][c] = cs.w[l][c];
+        ca.s0[c] -= 128.0 * cs.w[l][c];
+      }
     }
     for (int c = 0; c < kMaxChunks; ++c) ca.mc[c] = cs.mc[c];
     ca.inv_m = cs.inv_m;
@@ -1376,7 +1583,8 @@ void run_core(const GemmDesc& d, const Consts& cs, int beta, cudaStream_t s) {
 long long slab_bytes(long long L, long long m, long long n, long long k_total, long long nbatch,
                      long long planes_a, long long planes_b) {
   const long long k_pad = round_up(k_total, kTileK);
-  const long long m_pad = round_up(m, kTileI), n_pad = round_up(n, kItemJ);
+  const ProductTile pt = product_tile(m, n);
+  const long long m_pad = round_up(m, pt.tile_i), n_pad = round_up(n, pt.tile_j);
   const long long splits = std::max<long long>(1, (k_pad + kMaxKChunk - 1) / kMaxKChunk);
   return L * (planes_a * m_pad + planes_b * n_pad) * k_pad +
          std::max<long long>(splits, 4) * L * nbatch * m_pad * n_pad;
@@ -1429,7 +1637,8 @@ void run_slabs(const GemmDesc& d, const Consts& cs, int beta, cudaStream_t s) {
   // first); row / column slabs would prepare each operand once per slab of
   // the other.  A large output is cut into row / column slabs instead (each
   // K range would reconstruct all of it).
-  const long long m_pad = round_up(d.m, kTileI), n_pad = round_up(d.n, kItemJ);
+  const ProductTile pt = product_tile(d.m, d.n);
+  const long long m_pad = round_up(d.m, pt.tile_i), n_pad = round_up(d.n, pt.tile_j);
   const long long op_bytes = L * (pa * m_pad + pb * n_pad) * round_up(k_total, kTileK);
   const long long out_bytes = 4 * L * nbatch * m_pad * n_pad;
   if (op_bytes > kSlabBudget / 2 && out_bytes <= kSlabBudget / 2 && k_total > kTileK) {
@@ -1474,10 +1683,10 @@ void run_slabs(const GemmDesc& d, const Consts& cs, int beta, cudaStream_t s) {
   // 3. rows i / columns j
   long long ms = m_pad, ns = n_pad;
   while (slab_bytes(L, ms, ns, k_total, nbatch, pa, pb) > kSlabBudget) {
-    if (ms >= ns && ms > kTileI)
-      ms = round_up(ms / 2, kTileI);
-    else if (ns > kItemJ)
-      ns = round_up(ns / 2, kItemJ);
+    if (ms >= ns && ms > kMaxTileI)
+      ms = round_up(ms / 2, kMaxTileI);
+    else if (ns > 2 * kLanes)
+      ns = round_up(ns / 2, 2 * kLanes);
     else
       break;
   }
