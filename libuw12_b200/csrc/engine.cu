@@ -737,7 +737,7 @@ size_t budget_need(const FockRequest& rq, bool adjoint, bool streamed) {
   const size_t blocks = stored && !streamed ? 0 : 16 * (np + R * N) * M;
   size_t need = blocks + 2 * (N * N + np) * M;                           // unpacked AO blocks
   need = std::max(need, (2 * (N + o1) + 3 * Rp) * o * M);                // whole transforms
-  if (rq.calc_fock) need = std::max(need, blocks + (4 * N * N + Rp * N + 2 * R * N + np) * M);
+  if (rq.calc_fock) need = std::max(need, blocks + (4 * Rp * N + np + R * N) * M);
   if (rq.indirect) {
     need = std::max(need, (3 * Rp * o1 + M) * o1 * o1);                  // pair products of energies
   }
@@ -803,11 +803,9 @@ void form_fock(const FockRequest& rq) {
 
   DevBuf acc(kAccDoubles);
   acc.zero();
-  std::vector<DevBuf> Fp(ns);
-  for (int s = 0; s < ns; ++s) {
-    Fp[s].alloc(N * N);
-    Fp[s].zero();
-  }
+  DevBuf Fall(N * N * ns);  // the spins' Fock matrices side by side
+  Fall.zero();
+  double* Fp[2] = {Fall.get(), Fall.get() + N * N};
 
   // =====================================================================
   // two-electron term (two_electron.cpp:11-153), WV integrals, active orbitals
@@ -851,7 +849,7 @@ void form_fock(const FockRequest& rq) {
         }
       }
       for (int s = 0; s < ns; ++s)
-        unpack_sym(gv.get() + np * s, LL(np), LL(N), 1, Fp[s].get(), LL(N), 0, 1.0, 1.0);
+        unpack_sym(gv.get() + np * s, LL(np), LL(N), 1, Fp[s], LL(N), 0, 1.0, 1.0);
     }
     if (do_ind && a_tot > 0) {
       // B1 of the active orbitals: the shard's aux range of sq(J3_0) Ca times
@@ -877,7 +875,7 @@ void form_fock(const FockRequest& rq) {
           scale_rc(B1.get(), LL(N * a), LL(N * a), LL(MX), nullptr, WV.lam.get(), 1.0, B1l.get(),
                    LL(N * a));
           GemmDesc gf = gemm_nn(LL(N), LL(N), LL(a * MX), -s_ss, B1.get(), LL(N), B1l.get(),
-                                LL(N), 1.0, Fp[s].get(), LL(N));
+                                LL(N), 1.0, Fp[s], LL(N));
           gf.b_ncontig = true;
           gemm(gf);
         }
@@ -1169,7 +1167,7 @@ void form_fock(const FockRequest& rq) {
           copy3d(Z.get() + N * (a0 - k0), LL(N * nk), 0, Z.get() + N * (a0 - k0), LL(N * nk), 0,
                  LL(N * (a1 - a0)), LL(MV), 1, 2.0);
         GemmDesc gf = gemm_nn(LL(N), LL(N), LL(nk * MV), 1.0, Z.get(), LL(N), bv, LL(N), 1.0,
-                              Fp[s].get(), LL(N));
+                              Fp[s], LL(N));
         gf.b_ncontig = true;
         if (ldb1 != N * nk) {
           // part of the whole B1: K = (k, A) as MV reduction batches of nk
@@ -1228,75 +1226,68 @@ void form_fock(const FockRequest& rq) {
       budget = budgets.doubles(0.7);
       const size_t vstep = aux_step(V, false, budget / 4), vrstep = aux_step(V, true, budget);
       const size_t vscr = (V.J3_0.get() ? 0 : np * vstep) + (V.J3_ri_0.get() ? 0 : R * N * vrstep);
-      const size_t per_a = 2 * N * N + Rp * N + R * N + (W.J3_0.get() ? 0 : np);
+      const size_t nq = tdx_spins.size(), gsz = Rp * N;
+      const size_t per_a = (2 + nq) * gsz + (W.J3_0.get() ? 0 : np) + (W.J3_ri_0.get() ? 0 : R * N);
       const size_t avail = budget > vscr ? budget - vscr : 0;
       const auto [alo, ahi] = part(MW);
       const size_t ac = tile_chunk(ahi - alo, 1,
                                    std::max<size_t>(1, std::min(ahi - alo, avail / per_a)));
-      // Per chunk of W's aux functions a: Ga = sq(J3_0^W[:, a]) (N x N per a;
-      // afterwards the packed s columns of each spin), L = S^-1 G_W (R' x N
-      // per a), Hao = sq(s_a) (N x N per a) and Hr = p_a (R x N per a, RI rows
-      // nu + R mu).  When W's RI tensor is produced, its block and Hr share
-      // one buffer: the block is consumed by L before p overwrites it.
-      DevBuf Ga(N * N * ac), Lb(Rp * N * ac), Hao(N * N * ac);
-      DevBuf scrW, scrWr, scrV, scrVr, HrBuf;
-      double* sbuf = Ga.get();
-      double* Hr = nullptr;
-      if (W.J3_ri_0.get()) {
-        HrBuf.alloc(R * N * ac);
-        Hr = HrBuf.get();
-      } else {
-        scrWr.alloc(R * N * ac);
-        Hr = scrWr.get();
+      // T2 of the spins interleaved: row q + nq a, so that H[a] of all spins comes
+      // out of one product and is one operand of the last
+      DevBuf T2i;
+      const double* T2 = T2s[0].get();
+      if (nq > 1) {
+        T2i.alloc(nq * MW * MV);
+        for (size_t q = 0; q < nq; ++q)
+          copy3d(T2s[q].get(), 1, LL(MW), T2i.get() + q, LL(nq), LL(nq * MW), 1, LL(MW), LL(MV));
+        T2 = T2i.get();
       }
+      // Per chunk of W's aux functions a: G = [sq(J3_0^W[:, a]); J3ri_0^W[:, a]]
+      // (R' x N per a; afterwards the packed s columns), L = S^-1 G and H (R' x N
+      // per a and spin).  Stacked AO + RI operands and stacked spins prepare (in
+      // split precision) and read every operand once per chunk, and each product
+      // is written once: the opposite-spin Fock at N = 500, M = 1500, R = 2000, open
+      // shell, 14 moduli 369 -> 332 ms.
+      DevBuf G(gsz * ac), Lb(gsz * ac), H(gsz * ac * nq), scrW, scrWr, scrV, scrVr;
       for (size_t a0 = alo; a0 < ahi; a0 += ac) {
         const size_t na = std::min(ac, ahi - a0);
-        // L[a] = S^-1[:, AO] sq(J3_0^W[:, a]) + S^-1[:, RI] J3ri_0^W[:, a], the RI
-        // block read where it lies (R x N per a, leading dimension R)
-        unpack_sym(aux_block(W, false, a0, na, scrW), LL(np), LL(N), LL(na), Ga.get(), LL(N),
-                   LL(N * N));
-        gemm(gemm_nn(LL(Rp), LL(N * na), LL(N), 1.0, AB.Sinv.get(), LL(Rp), Ga.get(), LL(N), 0.0,
+        unpack_sym(aux_block(W, false, a0, na, scrW), LL(np), LL(N), LL(na), G.get(), LL(Rp),
+                   LL(gsz));
+        copy3d(aux_block(W, true, a0, na, scrWr), LL(R), LL(R * N), G.get() + N, LL(Rp), LL(gsz),
+               LL(R), LL(N), LL(na));
+        gemm(gemm_nn(LL(Rp), LL(N * na), LL(Rp), 1.0, AB.Sinv.get(), LL(Rp), G.get(), LL(Rp), 0.0,
                      Lb.get(), LL(Rp)));
-        gemm(gemm_nn(LL(Rp), LL(N * na), LL(R), 1.0, AB.Sinv.get() + Rp * N, LL(Rp),
-                     aux_block(W, true, a0, na, scrWr), LL(R), 1.0, Lb.get(), LL(Rp)));
-        for (size_t q = 0; q < tdx_spins.size(); ++q) {
-          const double* T2 = T2s[q].get();
-          // s = J3_0^V T2^T and p = J3_ri_0^V T2^T, accumulated over V's aux
-          // blocks; p for all AO indices mu at once (rows nu + R mu)
-          for (size_t b0 = 0; b0 < MV; b0 += vstep) {
-            const size_t nb = std::min(vstep, MV - b0);
-            GemmDesc gs = gemm_nn(LL(np), LL(na), LL(nb), 1.0, aux_block(V, false, b0, nb, scrV),
-                                  LL(np), T2 + a0 + MW * b0, LL(MW), b0 ? 1.0 : 0.0, sbuf,
-                                  LL(np));
-            gs.b_ncontig = true;
-            gemm(gs);
-          }
-          unpack_sym(sbuf, LL(np), LL(N), LL(na), Hao.get(), LL(N), LL(N * N));
-          for (size_t b0 = 0; b0 < MV; b0 += vrstep) {
-            const size_t nb = std::min(vrstep, MV - b0);
-            GemmDesc gp = gemm_nn(LL(R * N), LL(na), LL(nb), 1.0,
-                                  aux_block(V, true, b0, nb, scrVr), LL(R * N),
-                                  T2 + a0 + MW * b0, LL(MW), b0 ? 1.0 : 0.0, Hr, LL(R * N));
-            gp.b_ncontig = true;
-            gemm(gp);
-          }
-          // F[sigma'] -= sum_a L[a]^T [Hao[a]; Hr[a]], AO rows then RI rows of L
-          double* F = Fp[tdx_spins[q]].get();
-          GemmDesc fa = gemm_nn(LL(N), LL(N), LL(N), -1.0, Lb.get(), LL(Rp), Hao.get(), LL(N),
-                                1.0, F, LL(N));
-          fa.a_kcontig = true;
-          fa.nbr1 = LL(na);
-          fa.sAr1 = LL(Rp * N);
-          fa.sBr1 = LL(N * N);
-          gemm(fa);
-          GemmDesc fr = gemm_nn(LL(N), LL(N), LL(R), -1.0, Lb.get() + N, LL(Rp), Hr, LL(R), 1.0,
-                                F, LL(N));
-          fr.a_kcontig = true;
-          fr.nbr1 = LL(na);
-          fr.sAr1 = LL(Rp * N);
-          fr.sBr1 = LL(R * N);
-          gemm(fr);
+        // s = J3_0^V T2^T and p = J3_ri_0^V T2^T, accumulated over V's aux blocks
+        double* sbuf = G.get();
+        const double* t2 = T2 + nq * a0;
+        for (size_t b0 = 0; b0 < MV; b0 += vstep) {
+          const size_t nb = std::min(vstep, MV - b0);
+          GemmDesc gs = gemm_nn(LL(np), LL(na * nq), LL(nb), 1.0,
+                                aux_block(V, false, b0, nb, scrV), LL(np), t2 + nq * MW * b0,
+                                LL(nq * MW), b0 ? 1.0 : 0.0, sbuf, LL(np));
+          gs.b_ncontig = true;
+          gemm(gs);
         }
+        unpack_sym(sbuf, LL(np), LL(N), LL(na * nq), H.get(), LL(Rp), LL(gsz));
+        for (size_t b0 = 0; b0 < MV; b0 += vrstep) {
+          const size_t nb = std::min(vrstep, MV - b0);
+          GemmDesc gp = gemm_nn(LL(R), LL(na * nq), LL(nb), 1.0,
+                                aux_block(V, true, b0, nb, scrVr), LL(R * N), t2 + nq * MW * b0,
+                                LL(nq * MW), b0 ? 1.0 : 0.0, H.get() + N, LL(gsz));
+          gp.b_ncontig = true;
+          gp.nbo1 = LL(N);
+          gp.sAo1 = LL(R);
+          gp.sCo1 = LL(Rp);
+          gemm(gp);
+        }
+        // F[sigma'] -= sum_a L[a]^T H[a], the spins' Fock matrices side by side
+        GemmDesc gf = gemm_nn(LL(N), LL(N * nq), LL(Rp), -1.0, Lb.get(), LL(Rp), H.get(), LL(Rp),
+                              1.0, Fp[tdx_spins[0]], LL(N));
+        gf.a_kcontig = true;
+        gf.nbr1 = LL(na);
+        gf.sAr1 = LL(gsz);
+        gf.sBr1 = LL(gsz * nq);
+        gemm(gf);
       }
     }
   }
@@ -1369,7 +1360,7 @@ void form_fock(const FockRequest& rq) {
         gemm(g);
         GemmDesc gi = gemm_nn(LL(N), LL(N), LL(a), s_ss * (c > 0 ? -1.0 : -2.0),
                               W43.get() + N * c, LL(No), V43.get() + N * c, LL(N), 1.0,
-                              Fp[s].get(), LL(N));
+                              Fp[s], LL(N));
         gi.b_ncontig = true;
         gi.nbr1 = LL(a);
         gi.nbr2 = LL(o);
@@ -1380,7 +1371,7 @@ void form_fock(const FockRequest& rq) {
         gemm(gi);
         if (c > 0) {
           GemmDesc gf = gemm_nn(LL(N), LL(N), LL(a), -s_ss, W43.get(), LL(No), V43.get(), LL(No),
-                                1.0, Fp[s].get(), LL(N));
+                                1.0, Fp[s], LL(N));
           gf.b_ncontig = true;
           gf.nbr1 = LL(o);
           gf.nbr2 = LL(o);
@@ -1438,8 +1429,8 @@ void form_fock(const FockRequest& rq) {
       const bool whole_k = kc == o;
       // pair (j, k) of a chunk of nk orbitals is matrix (k - k0) + nk j of a buffer
       const size_t nbuf = pair * a * kc;
-      DevBuf gpk(np * a * kc), xk(std::max(MW, MV) * a * kc), bufG(nbuf), bufS(nbuf),
-          bufY(do_ind ? nbuf : 0), bufZ(do_ind && fold ? nbuf : 0), scrX, scrXr;
+      DevBuf gpk(np * a * kc), xk(std::max(MW, MV) * a * kc), bufG(nbuf),
+          bufS(nbuf * (do_ind && fold ? 2 : 1)), bufY(do_ind ? nbuf : 0), scrX, scrXr;
       // dst = G_X of the chunk, over X's aux blocks
       auto form_g = [&](const IntegralsHandle& X, const double* xh, size_t k0, size_t nk,
                         double* dst) {
@@ -1496,18 +1487,18 @@ void form_fock(const FockRequest& rq) {
                        LL(Rp), 0.0, bufS.get(), LL(Rp)));
           if (do_ind) {
             form_y(XW.Wst[s].get(), b1wl.get(), MW, k0, nk, bufY.get());
-            add_pairs(s_ss, bufS.get(), bufY.get(), n_pairs, 1.0, Fp[s].get());
+            add_pairs(s_ss, bufS.get(), bufY.get(), n_pairs, 1.0, Fp[s]);
             if (whole_k) yw = bufY.get();
           }
           form_g(W, xhW.get(), k0, nk, bufG.get());
         } else {
           form_g(V, xhV.get(), k0, nk, bufG.get());
           form_y(XW.SV[s].get(), b1wl.get(), MW, k0, nk, bufY.get());
-          add_pairs(s_ss, bufG.get(), bufY.get(), n_pairs, 1.0, Fp[s].get());
+          add_pairs(s_ss, bufG.get(), bufY.get(), n_pairs, 1.0, Fp[s]);
           form_g(W, xhW.get(), k0, nk, bufG.get());
         }
         if (do_ind) {
-          double* zbuf = fold ? bufZ.get() : bufS.get();
+          double* zbuf = bufS.get() + (fold ? nbuf : 0);
           form_y(XV.SV[s].get(), b1vl.get(), MV, k0, nk, zbuf);
           z = zbuf;
           // k-term (fock_k) for active orbitals c + i inside this chunk
@@ -1515,7 +1506,7 @@ void form_fock(const FockRequest& rq) {
           if (i1 > i0) {
             const size_t ni = i1 - i0;
             GemmDesc fk = gemm_nn(LL(N), LL(N), LL(Rp), s_ss, yw, LL(Rp),
-                                  z + pair * (c + i0 - k0), LL(Rp), 1.0, Fp[s].get(), LL(N));
+                                  z + pair * (c + i0 - k0), LL(Rp), 1.0, Fp[s], LL(N));
             fk.a_kcontig = true;
             fk.nbr1 = LL(ni);
             fk.nbr2 = LL(a);
@@ -1541,7 +1532,7 @@ void form_fock(const FockRequest& rq) {
           }
         }
         if (!fold) {
-          add_pairs(s_ss, bufG.get(), z, n_pairs, 1.0, Fp[s].get());
+          add_pairs(s_ss, bufG.get(), z, n_pairs, 1.0, Fp[s]);
         } else if (ns == 1) {
           // one product for t~ dX and the same-spin term: G_W^T (s_ss S^-1 Y_V - cD S^-1 G_V)
           if (do_ind) {
@@ -1549,14 +1540,25 @@ void form_fock(const FockRequest& rq) {
             const double coefs[2] = {s_ss, -cD[0]};
             lincomb(bufS.get(), LL(pair), LL(n_pairs), 2, mats, coefs, nullptr, nullptr, nullptr);
           }
-          add_pairs(do_ind ? 1.0 : -cD[0], bufG.get(), bufS.get(), n_pairs, 1.0, Fp[s].get());
+          add_pairs(do_ind ? 1.0 : -cD[0], bufG.get(), bufS.get(), n_pairs, 1.0, Fp[s]);
         } else {
-          if (do_ind) add_pairs(s_ss, bufG.get(), z, n_pairs, 1.0, Fp[s].get());
-          DevBuf D(N * N);
-          add_pairs(1.0, bufG.get(), bufS.get(), n_pairs, 0.0, D.get());
+          // D and the same-spin term G_W^T S^-1 Y_V in one launch, G_W read once
+          DevBuf D(2 * N * N);
+          GemmDesc gd = gemm_nn(LL(N), LL(N), LL(Rp), 1.0, bufG.get(), LL(Rp), bufS.get(), LL(Rp),
+                                0.0, D.get(), LL(N));
+          gd.a_kcontig = true;
+          gd.nbr1 = LL(n_pairs);
+          gd.sAr1 = LL(pair);
+          gd.sBr1 = LL(pair);
+          gd.nbo1 = do_ind ? 2 : 1;
+          gd.sBo1 = LL(nbuf);
+          gd.sCo1 = LL(N * N);
+          gemm(gd);
+          if (do_ind)
+            copy3d(D.get() + N * N, LL(N), 0, Fp[s], LL(N), 0, LL(N), LL(N), 1, s_ss, 1.0);
           for (int sp = 0; sp < ns; ++sp)
             if (cD[sp] != 0.0)
-              copy3d(D.get(), LL(N), 0, Fp[sp].get(), LL(N), 0, LL(N), LL(N), 1, -cD[sp], 1.0);
+              copy3d(D.get(), LL(N), 0, Fp[sp], LL(N), 0, LL(N), LL(N), 1, -cD[sp], 1.0);
         }
       }
     }
@@ -1575,7 +1577,7 @@ void form_fock(const FockRequest& rq) {
       out.alloc(N * N * ns);
       dst = out.get();
     }
-    for (int s = 0; s < ns; ++s) symmetrise(Fp[s].get(), LL(N), LL(N), dst + N * N * s, LL(N));
+    for (int s = 0; s < ns; ++s) symmetrise(Fp[s], LL(N), LL(N), dst + N * N * s, LL(N));
     if (!rq.fock_device)
       UW12_CUDA(cudaMemcpyAsync(rq.fock, dst, N * N * ns * sizeof(double), cudaMemcpyDeviceToHost,
                                 st));
