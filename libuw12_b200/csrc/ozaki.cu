@@ -56,6 +56,11 @@ struct Consts {
   double mc[kMaxChunks];                  // chunks of M
   double inv_m;
   double log2_m;
+  // the same weights for k_crt_pipe: byte b of w_l for the moduli 4t .. 4t + 3 as
+  // the bytes of w8[b][t]; 32-bit digits m of M; 2^(32 m) / M; and 2^52 plus what
+  // the 128 added to every residue adds to digit m
+  uint32_t w8[16][4];
+  double m32[4], per_m[4], bias[4];
 };
 
 using u128 = unsigned __int128;
@@ -102,6 +107,19 @@ Consts make_consts(int L) {
   for (int ch = 0; ch < kMaxChunks; ++ch)
     c.mc[ch] = ch < c.nch ? double(static_cast<uint64_t>((M >> (kChunkBits * ch)) & mask)) : 0.0;
   c.inv_m = 1.0 / static_cast<double>(M);
+  for (auto& row : c.w8)
+    for (uint32_t& v : row) v = 0;
+  for (int m = 0; m < 4; ++m) {
+    c.m32[m] = double(static_cast<uint32_t>(M >> (32 * m)));
+    c.per_m[m] = std::ldexp(1.0, 32 * m) / static_cast<double>(M);
+    c.bias[m] = 0x1p52;
+  }
+  for (int l = 0; l < L; ++l) {
+    const u128 Ml = M / kModuli[l];
+    const u128 w = Ml * u128(inv_mod(static_cast<long long>(Ml % kModuli[l]), kModuli[l]));
+    for (int b = 0; b < 16; ++b) c.w8[b][l / 4] |= static_cast<uint32_t>((w >> (8 * b)) & 255) << (8 * (l % 4));
+    for (int m = 0; m < 4; ++m) c.bias[m] += 128.0 * double(static_cast<uint32_t>(w >> (32 * m)));
+  }
   return c;
 }
 
@@ -904,20 +922,20 @@ struct CrtArgs {
   uint32_t p[kOzakiMaxModuli], barrett[kOzakiMaxModuli];
   uint32_t red_off[kOzakiMaxModuli];  // REDUCE: undoes the 128 added to each K chunk's residue
   double w[kOzakiMaxModuli][kMaxChunks];
-  double s0[kMaxChunks];  // -128 sum_l w: undoes the 128 added to each residue (exact)
   double mc[kMaxChunks];
   double inv_m;
   int cw;          // CRT chunk width in bits
+  uint32_t w8[16][4];                  // k_crt_pipe (Consts)
+  double m32[4], per_m[4], bias[4];
   int c_aligned;   // C, ldc and the batch strides allow 16-byte accesses
 };
 
-// One thread = E (kCrtElems) consecutive rows i of a column j of one batch;
-// grid (row blocks of 256 E, columns strided by gridDim.y, batches).  The L
-// residue words of a column (and the E elements of C when beta != 0) are
-// loaded before any is used (one load per modulus and K chunk in flight per
-// thread), the K-chunk sums of the E bytes are kept as pairs of 16-bit lanes,
-// the CRT runs on NCH chunks of cw bits, and C is read and written 16 bytes at
-// a time when aligned.
+// Several K chunks (small outputs): one thread = four consecutive rows i of a
+// column j of one batch; grid (row blocks of 1024, columns strided by gridDim.y,
+// batches).  The L residue words of a column (and the elements of C when beta != 0)
+// are loaded before any is used, the K-chunk sums of the four bytes are kept as
+// pairs of 16-bit lanes, the CRT runs on NCH chunks of cw bits, and C is read and
+// written 16 bytes at a time when aligned.
 // x 2^e: one multiply by an exactly representable power of two when 2^e is a
 // normal double, ldexp otherwise.
 __device__ __forceinline__ double scale_pow2(double x, int e) {
@@ -957,39 +975,17 @@ __device__ __forceinline__ double join_chunks(const double (&d)[NCH], double chu
   return sum + err;
 }
 
-// Byte b (0..3) of w as a double: the byte placed in the low word under the
-// exponent of 2^52, minus 2^52.
-__device__ __forceinline__ double byte_to_double(uint32_t w, int b) {
-  return __dsub_rn(__hiloint2double(0x43300000, static_cast<int>(__byte_perm(w, 0, 0x4440 + b))),
-                   4503599627370496.0);
-}
-
 // Residue (< 2^16) to double without the conversion unit.
 __device__ __forceinline__ double small_to_double(uint32_t r) {
   return __dsub_rn(__hiloint2double(0x43300000, static_cast<int>(r)), 4503599627370496.0);
 }
 
-// Rows i per CRT thread: 4 (one 32-bit residue word per modulus) or 2 (one
-// 16-bit word; fewer registers, more resident warps).
-#ifndef UW12_CRT_ELEMS
-#define UW12_CRT_ELEMS 4
-#endif
-constexpr int kCrtElems = UW12_CRT_ELEMS;
-static_assert(kCrtElems == 2 || kCrtElems == 4, "2 or 4 rows per CRT thread");
-constexpr int kCrtMinBlocks = kCrtElems == 4 ? 3 : 4;
-
-template <int E>
-__device__ __forceinline__ uint32_t load_residues(const uint8_t* p) {
-  if (E == 4) return __ldg(reinterpret_cast<const uint32_t*>(p));
-  return __ldg(reinterpret_cast<const unsigned short*>(p));
-}
-
-// Stored residues are bytes in [0, 255], 128 more than a residue in [-128, 127].
-// REDUCE: several K chunks (at most 257), whose byte sums are reduced mod p; with
-// one K chunk the bytes enter the CRT sum directly, which starts at s0.
-template <int NCH, bool REDUCE>
-__global__ void __launch_bounds__(256, REDUCE ? 2 : kCrtMinBlocks) k_crt(const CrtArgs a) {
-  constexpr int E = kCrtElems;
+// Stored residues are bytes in [0, 255], 128 more than a residue in [-128, 127]; the
+// sums of the (at most 256) K chunks' bytes are reduced mod p, red_off undoing the
+// 128 of each.
+template <int NCH>
+__global__ void __launch_bounds__(256, 2) k_crt(const CrtArgs a) {
+  constexpr int E = 4;
   const long long i0 = (static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) * E;
   if (i0 >= a.m) return;
   const int b = blockIdx.z;
@@ -1009,12 +1005,10 @@ __global__ void __launch_bounds__(256, REDUCE ? 2 : kCrtMinBlocks) k_crt(const C
   for (long long j = blockIdx.y; j < a.n; j += gridDim.y) {
     const uint8_t* base = a.R + (static_cast<long long>(b) * a.n_pad + j) * a.L * a.m_pad + i0;
     double* Cb = a.C + b1 * a.sCo1 + b2 * a.sCo2 + j * a.ldc;
-    // one residue word (E rows) per modulus and K chunk, and the E elements of
-    // C when they are accumulated into: all loads issued first
     uint32_t w0[kOzakiMaxModuli];
 #pragma unroll
     for (int l = 0; l < kOzakiMaxModuli; ++l)
-      if (l < a.L) w0[l] = load_residues<E>(base + l * lstride);
+      if (l < a.L) w0[l] = __ldg(reinterpret_cast<const uint32_t*>(base + l * lstride));
     double cold[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) cold[e] = 0.0;
@@ -1036,51 +1030,36 @@ __global__ void __launch_bounds__(256, REDUCE ? 2 : kCrtMinBlocks) k_crt(const C
 #pragma unroll
     for (int e = 0; e < E; ++e)
 #pragma unroll
-      for (int c = 0; c < NCH; ++c) S[e][c] = REDUCE ? 0.0 : a.s0[c];
-    if (!REDUCE) {
-      // one K chunk: the stored residues enter the CRT sum directly
+      for (int c = 0; c < NCH; ++c) S[e][c] = 0.0;
+    // byte sums in 16-bit lanes (bytes 0, 2 and 1, 3), reduced mod p
+    uint32_t s02[kOzakiMaxModuli], s13[kOzakiMaxModuli];
+#pragma unroll
+    for (int l = 0; l < kOzakiMaxModuli; ++l) {
+      if (l < a.L) {
+        s02[l] = w0[l] & 0x00ff00ffu;
+        s13[l] = (w0[l] >> 8) & 0x00ff00ffu;
+      }
+    }
+    for (int sp = 1; sp < a.splits; ++sp) {
 #pragma unroll
       for (int l = 0; l < kOzakiMaxModuli; ++l) {
         if (l < a.L) {
-#pragma unroll
-          for (int e = 0; e < E; ++e) {
-            const double r = byte_to_double(w0[l], e);
-#pragma unroll
-            for (int c = 0; c < NCH; ++c) S[e][c] = fma(r, a.w[l][c], S[e][c]);
-          }
+          const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(base + sp * sstride + l * lstride));
+          s02[l] += w & 0x00ff00ffu;
+          s13[l] += (w >> 8) & 0x00ff00ffu;
         }
       }
-    } else {
-      // K chunks: byte sums in 16-bit lanes (bytes 0, 2 and 1, 3), reduced mod p
-      uint32_t s02[kOzakiMaxModuli], s13[kOzakiMaxModuli];
+    }
 #pragma unroll
-      for (int l = 0; l < kOzakiMaxModuli; ++l) {
-        if (l < a.L) {
-          s02[l] = w0[l] & 0x00ff00ffu;
-          s13[l] = (w0[l] >> 8) & 0x00ff00ffu;
-        }
-      }
-      for (int sp = 1; sp < a.splits; ++sp) {
+    for (int l = 0; l < kOzakiMaxModuli; ++l) {
+      if (l < a.L) {
+        const uint32_t p = a.p[l], bm = a.barrett[l];
+        const uint32_t u[4] = {s02[l] & 0xffffu, s13[l] & 0xffffu, s02[l] >> 16, s13[l] >> 16};
 #pragma unroll
-        for (int l = 0; l < kOzakiMaxModuli; ++l) {
-          if (l < a.L) {
-            const uint32_t w = load_residues<E>(base + sp * sstride + l * lstride);
-            s02[l] += w & 0x00ff00ffu;
-            s13[l] += (w >> 8) & 0x00ff00ffu;
-          }
-        }
-      }
+        for (int e = 0; e < E; ++e) {
+          const double r = small_to_double(mod_u32(u[e] + a.red_off[l], p, bm));
 #pragma unroll
-      for (int l = 0; l < kOzakiMaxModuli; ++l) {
-        if (l < a.L) {
-          const uint32_t p = a.p[l], bm = a.barrett[l];
-          const uint32_t u[4] = {s02[l] & 0xffffu, s13[l] & 0xffffu, s02[l] >> 16, s13[l] >> 16};
-#pragma unroll
-          for (int e = 0; e < E; ++e) {
-            const double r = small_to_double(mod_u32(u[e] + a.red_off[l], p, bm));
-#pragma unroll
-            for (int c = 0; c < NCH; ++c) S[e][c] = fma(r, a.w[l][c], S[e][c]);
-          }
+          for (int c = 0; c < NCH; ++c) S[e][c] = fma(r, a.w[l][c], S[e][c]);
         }
       }
     }
@@ -1110,49 +1089,92 @@ __global__ void __launch_bounds__(256, REDUCE ? 2 : kCrtMinBlocks) k_crt(const C
   }
 }
 
-// One K chunk, pipelined: a block owns 1024 rows i of a batch and walks its
+// One K chunk, pipelined: a block owns 512 rows i of a batch and walks its
 // columns j = blockIdx.y, + gridDim.y, ...; the L residue rows of the next
-// kCrtStages - 1 columns are copied into shared memory (16-byte cp.async.cg,
-// L x 1024 bytes per column) while the current one is reconstructed, so the
-// copies of a block stay in flight during its FP64 work.  Thread = 4 rows, as
-// in k_crt; the same arithmetic.
+// kCrtStages - 1 columns are copied into shared memory (16-byte cp.async.cg) while
+// the current one is reconstructed.
+//
+// The weighted sum sum_l r_l w_l of an element is a small matrix product of bytes:
+// 16 residues by the 16 bytes of every weight.  On the FP64 pipe it took 42 FMAs
+// and 14 conversions per element, the larger part of the 224 instructions that
+// bounded this kernel; mma.sync m16n8k32 (u8) forms it instead.  The A operand's row
+// holds four elements 16 apart (four groups of 16 moduli along K, two k steps),
+// read by ldmatrix.trans out of the modulus-major rows; column n of B carries one
+// byte of the weights in the K group n / 2 only, so that the two columns a thread
+// holds of every product are bytes 2 j and 2 j + 1 of one element: each thread ends
+// up with all 16 byte sums (exact, below 2^20) of two elements, with no exchange
+// between lanes.  Half of the products are with zeros: 16 MMAs per 64 elements, 68
+// cycles of the tensor pipe per 32, beside 64 of the FP64 pipe.
+//
+// Byte sums join to four digits of 32 bits (below 2^44) in integers, become doubles
+// (minus the bias of the 128 in every stored residue), lose q M, q the rounded
+// quotient by M (|C'| <= M / 4), and join error-free: exactly when the product is a
+// double, within one unit in the last place otherwise.  20000 x 6000 at 14 moduli 0.95
+// -> 0.77 ms; now 60 % of the pipe that FP64 and these MMAs share, half each.
 constexpr int kCrtStages = 3;
-constexpr int kCrtRows = 1024;  // rows i per block
+constexpr int kCrtRows = 512;             // rows i per block, 128 per warp
+constexpr int kCrtThreads = 128;
+constexpr int kCrtPitch = kCrtRows + 16;  // bytes of a modulus row: ldmatrix rows in distinct banks
 
-template <int NCH, int LM>
-__global__ void __launch_bounds__(256, 3) k_crt_pipe(const CrtArgs a) {
-  extern __shared__ __align__(16) uint8_t crt_smem[];  // kCrtStages x L x kCrtRows bytes
-  const int L = a.L;
+__device__ __forceinline__ void mma_u8(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%0, %1, %2, %3};"
+      : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+template <int LM>
+__global__ void __launch_bounds__(kCrtThreads, 4) k_crt_pipe(const CrtArgs a) {
+  extern __shared__ __align__(16) uint8_t crt_smem[];  // kCrtStages x L x kCrtPitch bytes
+  const int L = LM ? LM : a.L;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
   const long long iblk = static_cast<long long>(blockIdx.x) * kCrtRows;
-  const long long i0 = iblk + threadIdx.x * 4;
+  const long long iw = iblk + warp * 128;  // first row of this warp
   const int b = blockIdx.z;
   const int b1 = b % a.nbo1, b2 = b / a.nbo1;
   const int pa = (a.a_var1 ? b1 : 0) + (a.a_var1 ? a.nbo1 : 1) * (a.a_var2 ? b2 : 0);
   const int pb = (a.b_var1 ? b1 : 0) + (a.b_var1 ? a.nbo1 : 1) * (a.b_var2 ? b2 : 0);
-  // bytes of this block's rows inside one residue row (a multiple of 256)
-  const long long row_bytes = min(static_cast<long long>(kCrtRows), a.m_pad - iblk);
+  // bytes of this block's rows inside one residue row (a multiple of 32)
+  const int row_bytes = static_cast<int>(min(static_cast<long long>(kCrtRows), a.m_pad - iblk));
   const long long nj = (a.n - blockIdx.y + gridDim.y - 1) / gridDim.y;
-  const bool active = i0 < a.m;
-  int sa[4];
+  const bool active = iw < a.m;
+  // this thread's elements: rows iw + 64 z + 16 t + g + 8 h
+  int sa[2][2];
 #pragma unroll
-  for (int e = 0; e < 4; ++e)
-    sa[e] = i0 + e < a.m ? a.shift_a[pa * a.rows_a + i0 + e] : 0;
-  const double chunk = __longlong_as_double(static_cast<long long>(a.cw + 1023) << 52);  // 2^cw
-  const bool vec = i0 + 3 < a.m && a.c_aligned;
+  for (int z = 0; z < 2; ++z)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const long long i = iw + 64 * z + 16 * t + g + 8 * h;
+      sa[z][h] = i < a.m ? a.shift_a[pa * a.rows_a + i] : 0;
+    }
+  uint32_t w[8], in_group[4];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) w[q] = a.w8[2 * q + (g & 1)][t];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) in_group[u] = (g >> 1) == u ? 0xffffffffu : 0u;
+  // ldmatrix row of this lane: modulus lane % 16 of the first or second matrix
+  const unsigned ld_row = static_cast<unsigned>(__cvta_generic_to_shared(crt_smem)) +
+                          min(lane & 15, L - 1) * kCrtPitch + warp * 128 + 16 * (lane >> 4);
 
+  // copy lane: 16 bytes at (threadIdx.x % 32) of every fourth modulus row
+  const int cp_off = (threadIdx.x & 31) * 16;
+  const bool cp_in = cp_off < row_bytes;
   auto issue = [&](long long q, int slot) {
     const long long j = blockIdx.y + q * gridDim.y;
-    const uint8_t* src0 = a.R + (static_cast<long long>(b) * a.n_pad + j) * L * a.m_pad + iblk;
-    uint8_t* dst0 = crt_smem + slot * L * kCrtRows;
-    for (int c = threadIdx.x; c < L * (kCrtRows / 16); c += 256) {
-      const int l = c / (kCrtRows / 16);
-      const int off = (c % (kCrtRows / 16)) * 16;
-      const bool in = off < row_bytes;
-      const uint8_t* src = in ? src0 + l * a.m_pad + off : src0;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
-                       static_cast<unsigned>(__cvta_generic_to_shared(dst0 + l * kCrtRows + off))),
-                   "l"(src), "r"(in ? 16 : 0)
-                   : "memory");
+    const uint8_t* src = a.R + ((static_cast<long long>(b) * a.n_pad + j) * L + warp) * a.m_pad +
+                         iblk + (cp_in ? cp_off : 0);
+    unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(crt_smem)) +
+                   (slot * L + warp) * kCrtPitch + cp_off;
+#pragma unroll
+    for (int l0 = 0; l0 < (LM ? LM : kOzakiMaxModuli); l0 += 4) {
+      if (l0 + warp < L)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src),
+                     "r"(cp_in ? 16 : 0)
+                     : "memory");
+      src += 4 * a.m_pad;
+      dst += 4 * kCrtPitch;
     }
   };
 
@@ -1161,68 +1183,86 @@ __global__ void __launch_bounds__(256, 3) k_crt_pipe(const CrtArgs a) {
     if (q < nj) issue(q, q);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   }
+  int slot = 0;
   for (long long q = 0; q < nj; ++q) {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(kCrtStages - 2) : "memory");
     __syncthreads();  // column q landed; the slot refilled below is no longer read
     {
       const long long qn = q + kCrtStages - 1;
-      if (qn < nj) issue(qn, static_cast<int>(qn % kCrtStages));
+      const int to = slot == 0 ? kCrtStages - 1 : slot - 1;  // (slot + kCrtStages - 1) % kCrtStages
+      if (qn < nj) issue(qn, to);
       asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
+    const unsigned ld = ld_row + slot * L * kCrtPitch;
+    slot = slot + 1 == kCrtStages ? 0 : slot + 1;
     if (!active) continue;
     const long long j = blockIdx.y + q * gridDim.y;
-    const uint8_t* rs = crt_smem + static_cast<int>(q % kCrtStages) * L * kCrtRows + threadIdx.x * 4;
-    double* Cb = a.C + b1 * a.sCo1 + b2 * a.sCo2 + j * a.ldc;
-    double cold[4] = {0.0, 0.0, 0.0, 0.0};
-    if (a.beta != 0.0) {
-      if (vec) {
-        const double2 c01 = *reinterpret_cast<const double2*>(Cb + i0);
-        const double2 c23 = *reinterpret_cast<const double2*>(Cb + i0 + 2);
-        cold[0] = c01.x; cold[1] = c01.y; cold[2] = c23.x; cold[3] = c23.y;
-      } else {
+    double* Cb = a.C + b1 * a.sCo1 + b2 * a.sCo2 + j * a.ldc + iw + 16 * t + g;
+    const int sb = a.shift_b[pb * a.rows_b + j];
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (i0 + e < a.m) cold[e] = Cb[i0 + e];
+    for (int z = 0; z < 2; ++z) {
+      double* dst = Cb + 64 * z;
+      bool in[2];
+      double cold[2];  // read ahead of the products
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        in[h] = iw + 64 * z + 16 * t + g + 8 * h < a.m;
+        cold[h] = a.beta != 0.0 && in[h] ? dst[8 * h] : 0.0;
       }
-    }
-    double S[4][NCH];
+      int acc[8][4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
+      for (int n = 0; n < 8; ++n)
 #pragma unroll
-      for (int c = 0; c < NCH; ++c) S[e][c] = a.s0[c];
+        for (int c = 0; c < 4; ++c) acc[n][c] = 0;
 #pragma unroll
-    for (int l = 0; l < (LM ? LM : kOzakiMaxModuli); ++l) {
-      if (LM || l < L) {
-        const uint32_t w = *reinterpret_cast<const uint32_t*>(rs + l * kCrtRows);
+      for (int ks = 0; ks < 2; ++ks) {
+        uint32_t r[4];
+        asm volatile("ldmatrix.sync.aligned.m16n16.x2.trans.shared.b8 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(ld + 64 * z + 32 * ks)
+                     : "memory");
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const double r = byte_to_double(w, e);
+        for (int n = 0; n < 8; ++n)
+          mma_u8(acc[n], r, w[n] & in_group[2 * ks], w[n] & in_group[2 * ks + 1]);
+      }
+      double x[2][4], v[2];
 #pragma unroll
-          for (int c = 0; c < NCH; ++c) S[e][c] = fma(r, a.w[l][c], S[e][c]);
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t lo = static_cast<uint32_t>(acc[2 * m][2 * h] + (acc[2 * m][2 * h + 1] << 8));
+          const uint32_t hi =
+              static_cast<uint32_t>(acc[2 * m + 1][2 * h] + (acc[2 * m + 1][2 * h + 1] << 8));
+          const unsigned long long d = lo + (static_cast<unsigned long long>(hi) << 16);
+          x[h][m] = __dsub_rn(__longlong_as_double(static_cast<long long>(d | 0x4330000000000000ULL)),
+                              a.bias[m]);
+        }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        // the low digits are below 2^-31 of M at the default modulus count
+        double approx = fma(x[h][3], a.per_m[3], x[h][2] * a.per_m[2]);
+        if (!LM) approx = fma(x[h][1], a.per_m[1], fma(x[h][0], a.per_m[0], approx));
+        const double quo = round_int(approx);  // |q| < 2^13
+#pragma unroll
+        for (int m = 0; m < 4; ++m) x[h][m] = fma(-quo, a.m32[m], x[h][m]);  // exact
+        if (LM) {
+          const double d[3] = {x[h][0], x[h][1], fma(x[h][3], 4294967296.0, x[h][2])};  // exact: < 2^47
+          v[h] = join_chunks<3>(d, 4294967296.0);
+        } else {
+          v[h] = join_chunks<4>(x[h], 4294967296.0);
         }
       }
-    }
-    const int sb = a.shift_b[pb * a.rows_b + j];
-    double out[4];
+      const int e0 = -(sa[z][0] + sb), e1 = -(sa[z][1] + sb);
+      if (min(e0, e1) >= -1022 && max(e0, e1) <= 1023) {
+        v[0] *= pow2(e0);
+        v[1] *= pow2(e1);
+      } else {
+        v[0] = scale_pow2(v[0], e0);
+        v[1] = scale_pow2(v[1], e1);
+      }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      double approx = 0.0;
-#pragma unroll
-      for (int c = NCH - 1; c >= 0; --c) approx = fma(approx, chunk, S[e][c]);
-      const double qq = round_int(approx * a.inv_m);  // |q| < 2^13
-      double dig[NCH];
-#pragma unroll
-      for (int c = 0; c < NCH; ++c) dig[c] = fma(-qq, a.mc[c], S[e][c]);  // exact
-      out[e] = a.alpha * scale_pow2(join_chunks<NCH>(dig, chunk), -(sa[e] + sb));
-      if (a.beta != 0.0) out[e] = fma(a.beta, cold[e], out[e]);
-    }
-    if (vec) {
-      *reinterpret_cast<double2*>(Cb + i0) = make_double2(out[0], out[1]);
-      *reinterpret_cast<double2*>(Cb + i0 + 2) = make_double2(out[2], out[3]);
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (i0 + e < a.m) Cb[i0 + e] = out[e];
+      for (int h = 0; h < 2; ++h)
+        if (in[h]) dst[8 * h] = a.beta != 0.0 ? fma(a.beta, cold[h], a.alpha * v[h]) : a.alpha * v[h];
     }
   }
   asm volatile("cp.async.wait_all;\n" ::: "memory");
@@ -1524,10 +1564,14 @@ void run_core(const GemmDesc& d, const Consts& cs, int beta, cudaStream_t s) {
       ca.p[l] = cs.p[l];
       ca.barrett[l] = cs.barrett[l];
       ca.red_off[l] = cs.p[l] - static_cast<uint32_t>(128 * splits % cs.p[l]);
-      for (int c = 0; c < kMaxChunks; ++c) {
-        ca.w[l][c] = cs.w[l][c];
-        ca.s0[c] -= 128.0 * cs.w[l][c];
-      }
+      for (int c = 0; c < kMaxChunks; ++c) ca.w[l][c] = cs.w[l][c];
+    }
+    for (int q = 0; q < 16; ++q)
+      for (int t = 0; t < 4; ++t) ca.w8[q][t] = cs.w8[q][t];
+    for (int m = 0; m < 4; ++m) {
+      ca.m32[m] = cs.m32[m];
+      ca.per_m[m] = cs.per_m[m];
+      ca.bias[m] = cs.bias[m];
     }
     for (int c = 0; c < kMaxChunks; ++c) ca.mc[c] = cs.mc[c];
     ca.inv_m = cs.inv_m;
@@ -1537,43 +1581,31 @@ void run_core(const GemmDesc& d, const Consts& cs, int beta, cudaStream_t s) {
     const double bytes = double(splits * L) * double(d.m * d.n * nbatch) +
                          8.0 * double(d.m * d.n * nbatch) * (d.beta != 0.0 ? 2.0 : 1.0);
     Timer tm(kProfSplitCrt, bytes, "crt", s);
-    const dim3 g(static_cast<unsigned>((d.m + 256 * kCrtElems - 1) / (256 * kCrtElems)),
-                 static_cast<unsigned>(std::min<long long>(d.n, 65535)),
-                 static_cast<unsigned>(nbatch));
-    const bool reduce = splits > 1;
-    if (!reduce) {
-      // pipelined: about eight waves of 3 blocks per SM (a short tail), each
-      // block walking its share of the columns
+    if (splits == 1) {
+      // about eight waves of 4 blocks per SM (a short tail), each block walking its
+      // share of the columns
       const long long gx = (d.m + kCrtRows - 1) / kCrtRows;
       const long long per_col = gx * nbatch;
       const long long gy = std::min<long long>(
           std::min<long long>(d.n, 65535),
-          std::max<long long>(1, (24LL * num_sms() + per_col - 1) / per_col));
-      const dim3 gp(static_cast<unsigned>(gx), static_cast<unsigned>(gy), g.z);
-      const size_t smem = size_t(kCrtStages) * L * kCrtRows;
-      if (L == kOzakiDefaultModuli && cs.nch == 3) {
-        k_crt_pipe<3, kOzakiDefaultModuli><<<gp, 256, smem, s>>>(ca);
-      } else {
-        switch (cs.nch) {
-          case 1: k_crt_pipe<1, 0><<<gp, 256, smem, s>>>(ca); break;
-          case 2: k_crt_pipe<2, 0><<<gp, 256, smem, s>>>(ca); break;
-          case 3: k_crt_pipe<3, 0><<<gp, 256, smem, s>>>(ca); break;
-          default: k_crt_pipe<4, 0><<<gp, 256, smem, s>>>(ca); break;
-        }
+          std::max<long long>(1, (32LL * num_sms() + per_col - 1) / per_col));
+      const dim3 g(static_cast<unsigned>(gx), static_cast<unsigned>(gy),
+                   static_cast<unsigned>(nbatch));
+      const size_t smem = size_t(kCrtStages) * L * kCrtPitch;
+      if (L == kOzakiDefaultModuli)
+        k_crt_pipe<kOzakiDefaultModuli><<<g, kCrtThreads, smem, s>>>(ca);
+      else
+        k_crt_pipe<0><<<g, kCrtThreads, smem, s>>>(ca);
+    } else {
+      const dim3 g(static_cast<unsigned>((d.m + 1023) / 1024),
+                   static_cast<unsigned>(std::min<long long>(d.n, 65535)),
+                   static_cast<unsigned>(nbatch));
+      switch (cs.nch) {
+        case 1: k_crt<1><<<g, 256, 0, s>>>(ca); break;
+        case 2: k_crt<2><<<g, 256, 0, s>>>(ca); break;
+        case 3: k_crt<3><<<g, 256, 0, s>>>(ca); break;
+        default: k_crt<4><<<g, 256, 0, s>>>(ca); break;
       }
-      UW12_LAUNCHED();
-      tm.stop();
-      return;
-    }
-    switch (cs.nch * 2 + (reduce ? 1 : 0)) {
-      case 2: k_crt<1, false><<<g, 256, 0, s>>>(ca); break;
-      case 3: k_crt<1, true><<<g, 256, 0, s>>>(ca); break;
-      case 4: k_crt<2, false><<<g, 256, 0, s>>>(ca); break;
-      case 5: k_crt<2, true><<<g, 256, 0, s>>>(ca); break;
-      case 6: k_crt<3, false><<<g, 256, 0, s>>>(ca); break;
-      case 7: k_crt<3, true><<<g, 256, 0, s>>>(ca); break;
-      case 8: k_crt<4, false><<<g, 256, 0, s>>>(ca); break;
-      default: k_crt<4, true><<<g, 256, 0, s>>>(ca); break;
     }
     UW12_LAUNCHED();
     tm.stop();
