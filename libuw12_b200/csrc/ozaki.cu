@@ -222,14 +222,24 @@ __device__ __forceinline__ void load_tile(const OperandView& v, int plane, long 
 }
 
 // Per row: exponent e of its largest element (2^(e-1) <= max|x| < 2^e),
-// stored as e + 2048 through atomicMax (0 = all zeros).  One block covers 32
-// rows x kExpTileK k of one plane (grid: row tiles, k tiles, planes) and reads
-// straight into registers, 64 independent loads per thread: KCONTIG (rows
-// contiguous along k) lets each warp sweep 4 rows along k, otherwise each warp
-// takes every 8th k of all 32 rows (consecutive rows per warp load).
+// stored as e + 2048 through atomicMax (0 = all zeros).  Bound by HBM (8 bytes per
+// element, once).  One block covers 32 rows x kExpTileK k of one plane (grid: row
+// tiles, k tiles, planes) and reads straight into registers, eight or more loads in
+// flight per thread: KCONTIG (rows contiguous along k) lets each warp sweep 4 rows
+// along k, a pair of elements per load where the view allows it (PAIRS, as in
+// k_residues: 2 % of the preparation), otherwise each warp takes every 8th k of all
+// 32 rows (consecutive rows per warp load; pairs of rows by half warps were slower).
 constexpr int kExpTileK = 512;
 
-template <bool KCONTIG>
+__device__ __forceinline__ void note_exponent(unsigned* eplus, double mx) {
+  if (mx > 0.0) {
+    int e = 0;
+    frexp(mx, &e);
+    atomicMax(eplus, static_cast<unsigned>(e + 2048));
+  }
+}
+
+template <bool KCONTIG, bool PAIRS>
 __global__ void __launch_bounds__(256) k_row_exponent(OperandView v,
                                                       unsigned* __restrict__ eplus) {
   __shared__ long long koff[kExpTileK];
@@ -256,18 +266,25 @@ __global__ void __launch_bounds__(256) k_row_exponent(OperandView v,
       double mx = 0.0;
       if (row < v.rows) {
         const double* rp = pb + row * v.rs;
+        if (PAIRS) {
 #pragma unroll
-        for (int t = 0; t < kExpTileK / 32; ++t) {
-          const long long ko = koff[lane + 32 * t];
-          if (ko >= 0) mx = fmax(mx, fabs(rp[ko]));
+          for (int t = 0; t < kExpTileK / 64; ++t) {
+            const long long ko = koff[2 * lane + 64 * t];
+            if (ko >= 0) {
+              const double2 d = __ldg(reinterpret_cast<const double2*>(rp + ko));
+              mx = fmax(mx, fmax(fabs(d.x), fabs(d.y)));
+            }
+          }
+        } else {
+#pragma unroll
+          for (int t = 0; t < kExpTileK / 32; ++t) {
+            const long long ko = koff[lane + 32 * t];
+            if (ko >= 0) mx = fmax(mx, fabs(rp[ko]));
+          }
         }
       }
       for (int o = 16; o; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      if (lane == 0 && row < v.rows && mx > 0.0) {
-        int e = 0;
-        frexp(mx, &e);
-        atomicMax(&eplus[plane * v.rows + row], static_cast<unsigned>(e + 2048));
-      }
+      if (lane == 0 && row < v.rows) note_exponent(&eplus[plane * v.rows + row], mx);
     }
   } else {
     const long long row = row0 + lane;
@@ -284,11 +301,7 @@ __global__ void __launch_bounds__(256) k_row_exponent(OperandView v,
     __syncthreads();
     if (warp == 0) {
       for (int w = 1; w < 8; ++w) mx = fmax(mx, part[w][lane]);
-      if (row < v.rows && mx > 0.0) {
-        int e = 0;
-        frexp(mx, &e);
-        atomicMax(&eplus[plane * v.rows + row], static_cast<unsigned>(e + 2048));
-      }
+      if (row < v.rows) note_exponent(&eplus[plane * v.rows + row], mx);
     }
   }
 }
@@ -338,6 +351,19 @@ __device__ __forceinline__ uint32_t residue_low(int vl, double v, double inv_p, 
   return static_cast<uint32_t>(vl - q * p);  // low byte = residue
 }
 
+// How k_residues reads its operand (residue_load picks it): 16 bytes at a time along
+// k straight into registers, 16 bytes at a time along the rows through shared
+// memory, or 8 bytes at a time through shared memory where alignment, an odd k or
+// strides forbid pairs.
+enum ResidueLoad { kPairsK = 0, kPairsRows = 1, kSingleK = 2, kSingleRows = 3 };
+
+// Shared tile of kPairsRows, element (r, c) at c * 32 + 2 * ((r / 2) ^ (c / 8)) + r % 2:
+// a copy's pair of rows stays together, and the compute reads (16 lanes per row,
+// lane t at k = 8 t + q, two rows of a pair per warp) touch every bank once.
+__device__ __forceinline__ int pair_at(int r, int c) {
+  return c * 32 + 2 * ((r >> 1) ^ ((c >> 3) & 15)) + (r & 1);
+}
+
 // Tile of 32 rows x 128 k of one plane -> L residue rows per row: row r of
 // modulus l of a plane is out row ((plane * tiles + r / T) * L + l) * T + r % T
 // (T = tile_rows, the MMA tile height of this operand; tiles = rows_pad / T),
@@ -347,40 +373,93 @@ __device__ __forceinline__ uint32_t residue_low(int vl, double v, double inv_p, 
 // per modulus (16 lanes: 128 contiguous bytes per row and modulus).  The
 // moduli loop is unrolled to kOzakiMaxModuli, so that p and 1/p are
 // immediate constant-bank operands.  Grid: (row tiles, k tiles, planes).
-template <bool KCONTIG, int LM>
-__global__ void __launch_bounds__(256) k_residues(OperandView v, const int* __restrict__ shift,
+//
+// Bound by instruction issue, 75 % busy at 41 % of DRAM with 125 instructions per
+// element, of which the 14 residues need 40 (a DFMA, a multiply-add and packing
+// each): so a pair of elements is loaded at once, addresses advance by constants,
+// one FMA scales an element, rounds it and leaves its low word (the scaling is
+// by a power of two, so x 2^sh + 1.5 2^52 rounds once, to the same integer), and
+// modulus 256, always the first, is the low byte itself.  Preparation of both operands
+// (with the exponent pass): 500 x 500 x 2000 in 300 reduction batches 3.65 -> 3.13
+// ms (5.8 TB/s of 16 + L bytes per element), 1200 x 900 x 900 in 64 batches 0.50 ->
+// 0.45, 20000 x 6000 x 1500 0.305 -> 0.275.
+template <int LOAD, int LM>
+__global__ void __launch_bounds__(256, 4) k_residues(OperandView v, const int* __restrict__ shift,
                                                   ResidueMods mods, int tile_rows,
                                                   long long tiles, long long k_pad,
                                                   uint8_t* __restrict__ out) {
-  __shared__ __align__(16) double tile[32 * 128];
+  __shared__ __align__(16) double tile[LOAD == kPairsK ? 2 : 32 * 128];
   __shared__ long long koff[128];
   const int plane = blockIdx.z;
   const long long row0 = static_cast<long long>(blockIdx.x) * 32;
   const long long k0 = static_cast<long long>(blockIdx.y) * 128;
+  const double* pb = v.base + (plane % v.np1) * v.po1 + (plane / v.np1) * v.po2;
   tile_k_offsets(v, k0, koff);
   __syncthreads();
-  load_tile<KCONTIG>(v, plane, row0, koff, tile);
-  __syncthreads();
   const int t = threadIdx.x & 15;
+  double x[2][8];
+  if (LOAD == kPairsK) {
+#pragma unroll
+    for (int it = 0; it < 2; ++it) {
+      const long long row = row0 + (threadIdx.x >> 4) + 16 * it;
+      const double* rp = pb + row * v.rs;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const long long ko = koff[8 * t + 2 * q];
+        double2 d = make_double2(0.0, 0.0);
+        if (row < v.rows && ko >= 0) d = __ldg(reinterpret_cast<const double2*>(rp + ko));
+        x[it][2 * q] = d.x;
+        x[it][2 * q + 1] = d.y;
+      }
+    }
+  } else if (LOAD == kPairsRows) {
+    const long long row = row0 + 2 * t;
+    const long long left = v.rows - row;
+    const int full = left >= 2 ? 16 : left == 1 ? 8 : 0;
+    const double* rp = pb + (full ? row : 0);
+#pragma unroll
+    for (int it = 0; it < 8; ++it) {
+      const int c = (threadIdx.x >> 4) + 16 * it;
+      const long long ko = koff[c];
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
+                       static_cast<unsigned>(__cvta_generic_to_shared(&tile[pair_at(2 * t, c)]))),
+                   "l"(ko >= 0 ? rp + ko : pb), "r"(ko >= 0 ? full : 0)
+                   : "memory");
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+  } else {
+    load_tile<LOAD == kSingleK>(v, plane, row0, koff, tile);
+    __syncthreads();
+  }
   const long long lstep = k_pad * tile_rows;  // next modulus of the same row
-#pragma unroll 1
+#pragma unroll
   for (int it = 0; it < 2; ++it) {
     const int r = (threadIdx.x >> 4) + 16 * it;
     const long long row = row0 + r;
     const int sh = row < v.rows ? shift[plane * v.rows + row] : 0;
-    double x[8];
+    double xr[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) x[q] = tile[tile_at(r, 8 * t + q)];
-    if (sh > -1000 && sh < 1000) {  // 2^sh is a normal double: scale by one multiply
+    for (int q = 0; q < 8; ++q)
+      xr[q] = LOAD == kPairsK      ? x[it][q]
+              : LOAD == kPairsRows ? tile[pair_at(r, 8 * t + q)]
+                                   : tile[tile_at(r, 8 * t + q)];
+    int vl[8];
+    if (sh > -1000 && sh < 1000) {  // 2^sh is a normal double: scale and round in one FMA
       const double sc = pow2(sh);
 #pragma unroll
-      for (int q = 0; q < 8; ++q) x[q] = round_int(x[q] * sc);
+      for (int q = 0; q < 8; ++q) {
+        const double y = fma(xr[q], sc, kRound);
+        vl[q] = __double2loint(y);
+        xr[q] = __dadd_rn(y, -kRound);
+      }
     } else {
-      for (int q = 0; q < 8; ++q) x[q] = round_int(ldexp_slow(x[q], sh));
+      for (int q = 0; q < 8; ++q) {
+        xr[q] = round_int(ldexp_slow(xr[q], sh));
+        vl[q] = int_of(xr[q]);
+      }
     }
-    int vl[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) vl[q] = int_of(x[q]);
     // row of modulus 0 in the residue layout
     const unsigned ti = static_cast<unsigned>(row) / static_cast<unsigned>(tile_rows);
     const long long base_row =
@@ -391,18 +470,40 @@ __global__ void __launch_bounds__(256) k_residues(OperandView v, const int* __re
       if (LM || l < mods.L) {
         const double ip = mods.inv_p[l];
         const int p = mods.pi[l];
-        const uint32_t b01 =
-            __byte_perm(residue_low(vl[0], x[0], ip, p), residue_low(vl[1], x[1], ip, p), 0x0040);
-        const uint32_t b23 =
-            __byte_perm(residue_low(vl[2], x[2], ip, p), residue_low(vl[3], x[3], ip, p), 0x0040);
-        const uint32_t b45 =
-            __byte_perm(residue_low(vl[4], x[4], ip, p), residue_low(vl[5], x[5], ip, p), 0x0040);
-        const uint32_t b67 =
-            __byte_perm(residue_low(vl[6], x[6], ip, p), residue_low(vl[7], x[7], ip, p), 0x0040);
-        *reinterpret_cast<uint2*>(dst + l * lstep) =
-            make_uint2(__byte_perm(b01, b23, 0x5410), __byte_perm(b45, b67, 0x5410));
+        uint32_t low[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          low[q] = l == 0 ? static_cast<uint32_t>(vl[q]) : residue_low(vl[q], xr[q], ip, p);
+        *reinterpret_cast<uint2*>(dst) =
+            make_uint2(__byte_perm(__byte_perm(low[0], low[1], 0x0040),
+                                   __byte_perm(low[2], low[3], 0x0040), 0x5410),
+                       __byte_perm(__byte_perm(low[4], low[5], 0x0040),
+                                   __byte_perm(low[6], low[7], 0x0040), 0x5410));
+        dst += lstep;
       }
     }
+  }
+}
+
+// Pairs need 16-byte aligned addresses: even strides and base (in doubles), and along
+// k an even k, so that no pair spans two reduction batches.
+ResidueLoad residue_load(const OperandView& v) {
+  const bool even = reinterpret_cast<std::uintptr_t>(v.base) % 16 == 0 && v.sr1 % 2 == 0 &&
+                    v.sr2 % 2 == 0 && (v.np1 == 1 || v.po1 % 2 == 0) &&
+                    (v.np2 == 1 || v.po2 % 2 == 0);
+  if (v.ks == 1) return even && v.rs % 2 == 0 && v.k % 2 == 0 ? kPairsK : kSingleK;
+  return even && v.ks % 2 == 0 ? kPairsRows : kSingleRows;
+}
+
+template <int LM>
+void launch_residues(const OperandView& v, const int* shift, const ResidueMods& mods,
+                     int tile_rows, long long tiles, long long k_pad, uint8_t* out, dim3 g,
+                     cudaStream_t s) {
+  switch (residue_load(v)) {
+    case kPairsK: k_residues<kPairsK, LM><<<g, 256, 0, s>>>(v, shift, mods, tile_rows, tiles, k_pad, out); break;
+    case kPairsRows: k_residues<kPairsRows, LM><<<g, 256, 0, s>>>(v, shift, mods, tile_rows, tiles, k_pad, out); break;
+    case kSingleK: k_residues<kSingleK, LM><<<g, 256, 0, s>>>(v, shift, mods, tile_rows, tiles, k_pad, out); break;
+    default: k_residues<kSingleRows, LM><<<g, 256, 0, s>>>(v, shift, mods, tile_rows, tiles, k_pad, out); break;
   }
 }
 
@@ -1430,10 +1531,11 @@ void run_core(const GemmDesc& d, const Consts& cs, int beta, cudaStream_t s) {
       dim3 ge(static_cast<unsigned>(rows_pad / 32),
               static_cast<unsigned>((k_pad + kExpTileK - 1) / kExpTileK),
               static_cast<unsigned>(planes));
-      if (v.ks == 1)
-        k_row_exponent<true><<<ge, 256, 0, s>>>(v, ep);
-      else
-        k_row_exponent<false><<<ge, 256, 0, s>>>(v, ep);
+      switch (residue_load(v)) {
+        case kPairsK: k_row_exponent<true, true><<<ge, 256, 0, s>>>(v, ep); break;
+        case kSingleK: k_row_exponent<true, false><<<ge, 256, 0, s>>>(v, ep); break;
+        default: k_row_exponent<false, false><<<ge, 256, 0, s>>>(v, ep); break;
+      }
       dim3 g(static_cast<unsigned>(rows_pad / 32), static_cast<unsigned>(k_pad / 128),
              static_cast<unsigned>(planes));
       UW12_LAUNCHED();
@@ -1443,14 +1545,10 @@ void run_core(const GemmDesc& d, const Consts& cs, int beta, cudaStream_t s) {
       UW12_LAUNCHED();
       const long long tiles = rows_pad / tile_rows;
       // the default modulus count runs a fully unrolled, unguarded moduli loop
-      if (v.ks == 1 && L == kOzakiDefaultModuli)
-        k_residues<true, kOzakiDefaultModuli><<<g, 256, 0, s>>>(v, sh, mods, tile_rows, tiles, k_pad, out);
-      else if (v.ks == 1)
-        k_residues<true, 0><<<g, 256, 0, s>>>(v, sh, mods, tile_rows, tiles, k_pad, out);
-      else if (L == kOzakiDefaultModuli)
-        k_residues<false, kOzakiDefaultModuli><<<g, 256, 0, s>>>(v, sh, mods, tile_rows, tiles, k_pad, out);
+      if (L == kOzakiDefaultModuli)
+        launch_residues<kOzakiDefaultModuli>(v, sh, mods, tile_rows, tiles, k_pad, out, g, s);
       else
-        k_residues<false, 0><<<g, 256, 0, s>>>(v, sh, mods, tile_rows, tiles, k_pad, out);
+        launch_residues<0>(v, sh, mods, tile_rows, tiles, k_pad, out, g, s);
       UW12_LAUNCHED();
     };
     prep(va, planes_a, m_pad, pt.tile_i, sa, ea, ra);

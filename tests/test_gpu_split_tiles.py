@@ -41,3 +41,30 @@ def test_long_contraction(uw12lib, cuda_device):
                             dC.data_ptr(), m)
         torch.cuda.synchronize()
         assert np.array_equal(dC.cpu().numpy(), B @ A)
+
+
+@pytest.mark.parametrize("a_k", [False, True])
+@pytest.mark.parametrize("b_n", [False, True])
+@pytest.mark.parametrize("m,n,k,nbr,pad,off", [(33, 65, 20, 3, 0, 0), (32, 64, 21, 3, 0, 0),
+                                               (34, 66, 20, 3, 1, 0), (34, 66, 20, 3, 0, 1),
+                                               (1, 1, 130, 1, 0, 0), (515, 131, 258, 2, 2, 0)])
+def test_operand_loads(uw12lib, cuda_device, a_k, b_n, m, n, k, nbr, pad, off):
+    """Operands read in pairs and singly: odd and even extents, leading dimensions and
+    base addresses, both orders, several reduction batches."""
+    import torch
+    rng = np.random.default_rng(m + n + k)
+    lda, ldb = (k if a_k else m) + pad, (n if b_n else k) + pad
+    A = rng.integers(-9, 10, off + nbr * (m if a_k else k) * lda).astype(np.float64)
+    B = rng.integers(-9, 10, off + nbr * (k if b_n else n) * ldb).astype(np.float64)
+    Av = A[off:].reshape(nbr, m if a_k else k, lda)
+    Bv = B[off:].reshape(nbr, k if b_n else n, ldb)
+    ref = sum((x[:, :k] if a_k else x[:, :m].T) @ (y[:, :n] if b_n else y[:, :k].T)
+              for x, y in zip(Av, Bv))
+    dA, dB = torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda()
+    for moduli in (7, 14, 16):
+        dC = torch.full((n, m), float("nan"), dtype=torch.float64, device="cuda")
+        uw12lib.dgemm_split(m, n, k, 1.0, dA.data_ptr() + 8 * off, lda, a_k,
+                            dB.data_ptr() + 8 * off, ldb, b_n, 0.0, dC.data_ptr(), m, nbr1=nbr,
+                            sr=(Av[0].size, 0, Bv[0].size, 0), n_moduli=moduli)
+        torch.cuda.synchronize()
+        assert np.array_equal(dC.cpu().numpy().T, ref)
