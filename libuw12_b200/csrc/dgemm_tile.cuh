@@ -263,6 +263,7 @@ __global__ void __launch_bounds__(32 * WM * WN, CTAS) dgemm_dmma(const KParams p
     for (int ni = 0; ni < NI; ++ni) bf[buf][ni] = bs[LB::at(wn + ni * 8 + g, kk)];
   };
 
+  chain_wait();
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
     if (kt_begin + s < kt_end) load_stage(s);
@@ -299,6 +300,7 @@ __global__ void __launch_bounds__(32 * WM * WN, CTAS) dgemm_dmma(const KParams p
           dmma(acc[mi][ni], af[kq & 1][mi][0], af[kq & 1][mi][1], bf[kq & 1][ni]);
     }
   }
+  chain_release();  // the epilogue is left
   cp_async_wait<0>();
 
   // Epilogue: C = alpha acc + beta C, or the raw partial tile for split-K.
@@ -369,7 +371,7 @@ struct Ops {
   }
   static void launch(const KParams& p, int layout, long long grid, cudaStream_t s) {
     dispatch(layout, [&](auto kernel, size_t smem) {
-      kernel<<<static_cast<unsigned>(grid), THREADS, smem, s>>>(p);
+      launch_chained(kernel, dim3(static_cast<unsigned>(grid)), THREADS, smem, s, p);
     });
     UW12_LAUNCHED();
   }

@@ -26,9 +26,10 @@ constexpr long long kSMs = 148;
 // latency of the partials' loads at the small outputs that split: eight are in
 // flight per thread.  I: index type (32-bit divisions where the output allows).
 template <typename I>
-__global__ void splitk_reduce(const double* __restrict__ work, int split, I m, I mn, I total,
+__global__ void splitk_reduce(const double* work, int split, I m, I mn, I total,
                               I nbo1, double alpha, double beta, double* C, long long ldc,
                               long long sCo1, long long sCo2) {
+  chain_wait();
   const I step = static_cast<I>(gridDim.x) * blockDim.x;
   for (I idx = static_cast<I>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total; idx += step) {
     const I bo = idx / mn;
@@ -48,6 +49,7 @@ __global__ void splitk_reduce(const double* __restrict__ work, int split, I m, I
 // C = beta * C for an empty contraction.
 __global__ void scale_only(long long m, long long n, long long nbo, long long nbo1, double beta,
                            double* C, long long ldc, long long sCo1, long long sCo2) {
+  chain_wait();
   const long long total = m * n * nbo;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -188,7 +190,8 @@ void launch_scale_only(const GemmDesc& d, cudaStream_t s) {
   const long long nbo = d.nbo1 * d.nbo2;
   const long long total = d.m * d.n * nbo;
   const int blocks = static_cast<int>(std::min<long long>((total + 255) / 256, kSMs * 16));
-  scale_only<<<blocks, 256, 0, s>>>(d.m, d.n, nbo, d.nbo1, d.beta, d.C, d.ldc, d.sCo1, d.sCo2);
+  launch_chained(scale_only, blocks, 256, 0, s, d.m, d.n, nbo, d.nbo1, d.beta, d.C, d.ldc, d.sCo1,
+                 d.sCo2);
   UW12_LAUNCHED();
 }
 
@@ -221,14 +224,13 @@ void launch(const GemmDesc& d, KParams p, const Plan& plan, cudaStream_t s) {
     const long long total = d.m * d.n * p.nbo;
     const int blocks = static_cast<int>(std::min<long long>((total + 255) / 256, kSMs * 16));
     if (total < (1LL << 31))
-      splitk_reduce<unsigned><<<blocks, 256, 0, s>>>(
-          p.work, p.split, static_cast<unsigned>(d.m), static_cast<unsigned>(d.m * d.n),
-          static_cast<unsigned>(total), static_cast<unsigned>(d.nbo1), d.alpha, d.beta, d.C,
-          d.ldc, d.sCo1, d.sCo2);
+      launch_chained(splitk_reduce<unsigned>, blocks, 256, 0, s, p.work, p.split,
+                     static_cast<unsigned>(d.m), static_cast<unsigned>(d.m * d.n),
+                     static_cast<unsigned>(total), static_cast<unsigned>(d.nbo1), d.alpha, d.beta,
+                     d.C, d.ldc, d.sCo1, d.sCo2);
     else
-      splitk_reduce<long long><<<blocks, 256, 0, s>>>(p.work, p.split, d.m, d.m * d.n, total,
-                                                      d.nbo1, d.alpha, d.beta, d.C, d.ldc, d.sCo1,
-                                                      d.sCo2);
+      launch_chained(splitk_reduce<long long>, blocks, 256, 0, s, p.work, p.split, d.m, d.m * d.n,
+                     total, d.nbo1, d.alpha, d.beta, d.C, d.ldc, d.sCo1, d.sCo2);
     UW12_LAUNCHED();
   }
 }

@@ -31,10 +31,11 @@ __device__ __forceinline__ void lower_tile(int t, int& ti, int& tj) {
 // coalesced (an element per thread instead reads the packed rows of half of the
 // output at a stride, and divides twice in 64 bits per element: 300 x 300 x 900
 // 0.34 -> 0.19 ms, 5.1 TB/s).
-__global__ void __launch_bounds__(256) k_unpack_sym(const double* __restrict__ P, long long ldp,
+__global__ void __launch_bounds__(256) k_unpack_sym(const double* P, long long ldp,
                                                     int n, long long ncols, double* out,
                                                     long long ldo, long long so, double alpha,
                                                     double beta) {
+  chain_wait();
   __shared__ double tile[32][33];
   int ti, tj;
   lower_tile(blockIdx.x, ti, tj);
@@ -72,8 +73,9 @@ __global__ void __launch_bounds__(256) k_unpack_sym(const double* __restrict__ P
   }
 }
 
-__global__ void k_pack_density(const double* __restrict__ C, long long ldc, long long n,
+__global__ void k_pack_density(const double* C, long long ldc, long long n,
                                long long nc, double scale, double* d) {
+  chain_wait();
   const long long total = tri(n);
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -89,9 +91,10 @@ __global__ void k_pack_density(const double* __restrict__ C, long long ldc, long
 }
 
 template <typename I>
-__global__ void k_scale_rc(const double* __restrict__ X, long long ldx, long long rows,
-                           long long cols, const double* __restrict__ r,
-                           const double* __restrict__ c, double alpha, double* Y, long long ldy) {
+__global__ void k_scale_rc(const double* X, long long ldx, long long rows,
+                           long long cols, const double* r,
+                           const double* c, double alpha, double* Y, long long ldy) {
+  chain_wait();
   const I nr = static_cast<I>(rows), total = nr * static_cast<I>(cols);
   for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
        idx += static_cast<I>(gridDim.x) * blockDim.x) {
@@ -104,9 +107,10 @@ __global__ void k_scale_rc(const double* __restrict__ X, long long ldx, long lon
 }
 
 template <typename I>
-__global__ void k_copy3d(const double* __restrict__ src, long long s1, long long s2, double* dst,
+__global__ void k_copy3d(const double* src, long long s1, long long s2, double* dst,
                          long long d1, long long d2, long long n0, long long n1, long long n2,
                          double alpha, double beta) {
+  chain_wait();
   const I m0 = static_cast<I>(n0), m1 = static_cast<I>(n1);
   const I total = m0 * m1 * static_cast<I>(n2);
   for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
@@ -162,10 +166,11 @@ __device__ __forceinline__ void finish_reduction(double s, double* partials, dou
 }
 
 template <typename I>
-__global__ void k_wdot(const double* __restrict__ x, long long ldx, const double* __restrict__ y,
-                       long long ldy, long long rows, long long cols, const double* __restrict__ rw,
-                       const double* __restrict__ cw, double* partials, double coef, double* acc,
+__global__ void k_wdot(const double* x, long long ldx, const double* y,
+                       long long ldy, long long rows, long long cols, const double* rw,
+                       const double* cw, double* partials, double coef, double* acc,
                        int slot) {
+  chain_wait();
   const I nr = static_cast<I>(rows), total = nr * static_cast<I>(cols);
   double s = 0.0;
   for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
@@ -180,9 +185,10 @@ __global__ void k_wdot(const double* __restrict__ x, long long ldx, const double
 }
 
 template <typename I>
-__global__ void k_permdot_4el(const double* __restrict__ X, const double* __restrict__ Y,
+__global__ void k_permdot_4el(const double* X, const double* Y,
                               long long a, long long o, double* partials, double coef,
                               double* acc, int slot) {
+  chain_wait();
   const I na = static_cast<I>(a), nao = na * static_cast<I>(o);
   const I total = nao * nao;  // (i, l, j, k)
   const long long ao = a * o;
@@ -197,9 +203,10 @@ __global__ void k_permdot_4el(const double* __restrict__ X, const double* __rest
 }
 
 // One warp per (i, j, k) triple, summing the contiguous p index.
-__global__ void k_permdot_3el(const double* __restrict__ Yw, const double* __restrict__ Zv,
+__global__ void k_permdot_3el(const double* Yw, const double* Zv,
                               long long rp, long long a, long long kc, double* partials,
                               double coef, double* acc, int slot) {
+  chain_wait();
   const long long triples = a * a * kc;
   const int lane = threadIdx.x & 31;
   const long long warp_global = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
@@ -217,8 +224,9 @@ __global__ void k_permdot_3el(const double* __restrict__ Yw, const double* __res
   finish_reduction(s, partials, coef, acc, slot);
 }
 
-__global__ void k_symmetrise(const double* __restrict__ G, long long ldg, long long n, double* F,
+__global__ void k_symmetrise(const double* G, long long ldg, long long n, double* F,
                              long long ldf) {
+  chain_wait();
   const long long total = n * n;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -227,8 +235,9 @@ __global__ void k_symmetrise(const double* __restrict__ G, long long ldg, long l
   }
 }
 
-__global__ void k_symmetry_stats(const double* __restrict__ A, long long lda, long long n,
+__global__ void k_symmetry_stats(const double* A, long long lda, long long n,
                                  double* partials) {
+  chain_wait();
   const long long total = n * n;
   double dmax = 0.0, amax = 0.0;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
@@ -256,6 +265,7 @@ __global__ void k_symmetry_stats(const double* __restrict__ A, long long lda, lo
 }
 
 __global__ void k_max_pairs(const double* partials, int n, double* out) {
+  chain_wait();
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     double d = 0.0, a = 0.0;
     for (int q = 0; q < n; ++q) { d = fmax(d, partials[2 * q]); a = fmax(a, partials[2 * q + 1]); }
@@ -273,7 +283,8 @@ struct CombineArgs {
 
 template <typename I>
 __global__ void k_combine_y(double* Y, long long m, CombineArgs a, int nq,
-                            const double* __restrict__ r, const double* __restrict__ c) {
+                            const double* r, const double* c) {
+  chain_wait();
   const I nr = static_cast<I>(m), total = nr * nr;
   for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
        idx += static_cast<I>(gridDim.x) * blockDim.x) {
@@ -291,8 +302,9 @@ struct VecArgs {
   double coef[4];
 };
 
-__global__ void k_combine_vecs(const double* __restrict__ U, long long m, int ns, VecArgs a,
-                               const double* __restrict__ w, double* V) {
+__global__ void k_combine_vecs(const double* U, long long m, int ns, VecArgs a,
+                               const double* w, double* V) {
+  chain_wait();
   const long long total = m * ns;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -312,7 +324,8 @@ struct LincombArgs {
 
 template <typename I>
 __global__ void k_lincomb(double* Y, long long m, long long n, int nt, LincombArgs a,
-                          const double* __restrict__ r, const double* __restrict__ c) {
+                          const double* r, const double* c) {
+  chain_wait();
   const I nr = static_cast<I>(m), total = nr * static_cast<I>(n);
   for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
        idx += static_cast<I>(gridDim.x) * blockDim.x) {
@@ -338,8 +351,9 @@ __global__ void k_lincomb(double* Y, long long m, long long n, int nt, LincombAr
 // through shared memory as in k_unpack_sym took 0.36 ms, two dependent phases
 // for no fewer bytes.
 template <typename I>
-__global__ void k_pack_sym_sum(const double* __restrict__ G, I n, I np, I total, double* out,
+__global__ void k_pack_sym_sum(const double* G, I n, I np, I total, double* out,
                                long long ldo, double beta) {
+  chain_wait();
   for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
        idx += static_cast<I>(gridDim.x) * blockDim.x) {
     const I a = idx / np, p = idx - a * np;
@@ -359,8 +373,9 @@ __global__ void k_pack_sym_sum(const double* __restrict__ G, I n, I np, I total,
 // the two active-orbital indices of the same-spin three-electron products
 // exchanged (the permutation under which YW and ZV are contracted).
 template <typename I>
-__global__ void k_perm_3el(const double* __restrict__ Z, double* __restrict__ out,
+__global__ void k_perm_3el(const double* Z, double* out,
                            long long rp, long long a, long long kc, double alpha) {
+  chain_wait();
   const I nr = static_cast<I>(rp), na = static_cast<I>(a);
   const I total = nr * na * na * static_cast<I>(kc);
   for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
@@ -376,8 +391,9 @@ __global__ void k_perm_3el(const double* __restrict__ Z, double* __restrict__ ou
 // out[i + a*l + ao*(j + a*k)] = alpha * V[i + a*k + ao*(j + a*l)], ao = a*o:
 // the occupied indices of rows and columns of (ik|jl) exchanged.
 template <typename I>
-__global__ void k_perm_4el(const double* __restrict__ V, double* __restrict__ out,
+__global__ void k_perm_4el(const double* V, double* out,
                            long long a, long long o, double alpha) {
+  chain_wait();
   const I na = static_cast<I>(a), no = static_cast<I>(o), total = na * no * na * no;
   const long long ao = a * o;
   for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
@@ -389,8 +405,9 @@ __global__ void k_perm_4el(const double* __restrict__ V, double* __restrict__ ou
   }
 }
 
-__global__ void k_scale_pinv_cols(double* Q, long long n, const double* __restrict__ lam,
+__global__ void k_scale_pinv_cols(double* Q, long long n, const double* lam,
                                   double tol) {
+  chain_wait();
   const long long total = n * n;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -401,15 +418,17 @@ __global__ void k_scale_pinv_cols(double* Q, long long n, const double* __restri
 }
 
 __global__ void k_set_identity(double* A, long long n) {
+  chain_wait();
   const long long total = n * n;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x)
     A[idx] = (idx % n == idx / n) ? 1.0 : 0.0;
 }
 
-__global__ void k_gather_scale_cols(const double* __restrict__ src, long long rows,
-                                    const int* __restrict__ idxv, const double* __restrict__ s,
+__global__ void k_gather_scale_cols(const double* src, long long rows,
+                                    const int* idxv, const double* s,
                                     long long nq, double* dst) {
+  chain_wait();
   const long long total = rows * nq;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -436,8 +455,8 @@ void unpack_sym(const double* P, long long ldp, long long n, long long ncols, do
                 long long ldo, long long so, double alpha, double beta) {
   const long long total = n * n * ncols;
   if (total <= 0) return;
-  k_unpack_sym<<<tile_grid(n, ncols), kT, 0, current_stream()>>>(
-      P, ldp, static_cast<int>(n), ncols, out, ldo, so, alpha, beta);
+  launch_chained(k_unpack_sym, tile_grid(n, ncols), kT, 0, current_stream(), P, ldp,
+                 static_cast<int>(n), ncols, out, ldo, so, alpha, beta);
   UW12_LAUNCHED();
 }
 
@@ -445,7 +464,7 @@ void pack_density(const double* C, long long ldc, long long n, long long nc, dou
                   double* d) {
   const long long total = n * (n + 1) / 2;
   if (total <= 0) return;
-  k_pack_density<<<grid_for(total), kT, 0, current_stream()>>>(C, ldc, n, nc, scale, d);
+  launch_chained(k_pack_density, grid_for(total), kT, 0, current_stream(), C, ldc, n, nc, scale, d);
   UW12_LAUNCHED();
 }
 
@@ -454,11 +473,11 @@ void scale_rc(const double* X, long long ldx, long long rows, long long cols, co
   const long long total = rows * cols;
   if (total <= 0) return;
   if (small_index(total))
-    k_scale_rc<unsigned><<<grid_for(total), kT, 0, current_stream()>>>(X, ldx, rows, cols, r, c, alpha, Y,
-                                                            ldy);
+    launch_chained(k_scale_rc<unsigned>, grid_for(total), kT, 0, current_stream(), X, ldx, rows,
+                   cols, r, c, alpha, Y, ldy);
   else
-    k_scale_rc<long long><<<grid_for(total), kT, 0, current_stream()>>>(X, ldx, rows, cols, r, c, alpha, Y,
-                                                            ldy);
+    launch_chained(k_scale_rc<long long>, grid_for(total), kT, 0, current_stream(), X, ldx, rows,
+                   cols, r, c, alpha, Y, ldy);
   UW12_LAUNCHED();
 }
 
@@ -467,11 +486,11 @@ void copy3d(const double* src, long long s1, long long s2, double* dst, long lon
   const long long total = n0 * n1 * n2;
   if (total <= 0) return;
   if (small_index(total))
-    k_copy3d<unsigned><<<grid_for(total), kT, 0, current_stream()>>>(src, s1, s2, dst, d1, d2, n0, n1, n2,
-                                                          alpha, beta);
+    launch_chained(k_copy3d<unsigned>, grid_for(total), kT, 0, current_stream(), src, s1, s2, dst,
+                   d1, d2, n0, n1, n2, alpha, beta);
   else
-    k_copy3d<long long><<<grid_for(total), kT, 0, current_stream()>>>(src, s1, s2, dst, d1, d2, n0, n1, n2,
-                                                          alpha, beta);
+    launch_chained(k_copy3d<long long>, grid_for(total), kT, 0, current_stream(), src, s1, s2, dst,
+                   d1, d2, n0, n1, n2, alpha, beta);
   UW12_LAUNCHED();
 }
 
@@ -484,11 +503,11 @@ void wdot(const double* x, long long ldx, const double* y, long long ldy, long l
   const int blocks = grid_for(total, 4);
   DevBuf part(blocks, s);
   if (small_index(total))
-    k_wdot<unsigned><<<blocks, kT, 0, s>>>(x, ldx, y, ldy, rows, cols, rw, cw, part.get(), coef,
-                                           acc, slot);
+    launch_chained(k_wdot<unsigned>, blocks, kT, 0, s, x, ldx, y, ldy, rows, cols, rw, cw,
+                   part.get(), coef, acc, slot);
   else
-    k_wdot<long long><<<blocks, kT, 0, s>>>(x, ldx, y, ldy, rows, cols, rw, cw, part.get(), coef,
-                                            acc, slot);
+    launch_chained(k_wdot<long long>, blocks, kT, 0, s, x, ldx, y, ldy, rows, cols, rw, cw,
+                   part.get(), coef, acc, slot);
   UW12_LAUNCHED();
 }
 
@@ -500,9 +519,11 @@ void permdot_4el(const double* X, const double* Y, long long a, long long o, dou
   const int blocks = grid_for(total, 4);
   DevBuf part(blocks, s);
   if (small_index(total))
-    k_permdot_4el<unsigned><<<blocks, kT, 0, s>>>(X, Y, a, o, part.get(), coef, acc, slot);
+    launch_chained(k_permdot_4el<unsigned>, blocks, kT, 0, s, X, Y, a, o, part.get(), coef, acc,
+                   slot);
   else
-    k_permdot_4el<long long><<<blocks, kT, 0, s>>>(X, Y, a, o, part.get(), coef, acc, slot);
+    launch_chained(k_permdot_4el<long long>, blocks, kT, 0, s, X, Y, a, o, part.get(), coef, acc,
+                   slot);
   UW12_LAUNCHED();
 }
 
@@ -513,14 +534,14 @@ void permdot_3el(const double* Y, const double* Z, long long rp, long long a, lo
   cudaStream_t s = current_stream();
   const int blocks = grid_for(triples * 32, 8);
   DevBuf part(blocks, s);
-  k_permdot_3el<<<blocks, kT, 0, s>>>(Y, Z, rp, a, kc, part.get(), coef, acc, slot);
+  launch_chained(k_permdot_3el, blocks, kT, 0, s, Y, Z, rp, a, kc, part.get(), coef, acc, slot);
   UW12_LAUNCHED();
 }
 
 void symmetrise(const double* G, long long ldg, long long n, double* F, long long ldf) {
   const long long total = n * n;
   if (total <= 0) return;
-  k_symmetrise<<<grid_for(total), kT, 0, current_stream()>>>(G, ldg, n, F, ldf);
+  launch_chained(k_symmetrise, grid_for(total), kT, 0, current_stream(), G, ldg, n, F, ldf);
   UW12_LAUNCHED();
 }
 
@@ -529,9 +550,9 @@ void symmetry_stats(const double* A, long long lda, long long n, double* out) {
   const long long total = n * n;
   const int blocks = grid_for(std::max<long long>(total, 1), 4);
   DevBuf part(2 * blocks, s);
-  k_symmetry_stats<<<blocks, kT, 0, s>>>(A, lda, n, part.get());
+  launch_chained(k_symmetry_stats, blocks, kT, 0, s, A, lda, n, part.get());
   UW12_LAUNCHED();
-  k_max_pairs<<<1, 32, 0, s>>>(part.get(), blocks, out);
+  launch_chained(k_max_pairs, 1, 32, 0, s, part.get(), blocks, out);
   UW12_LAUNCHED();
 }
 
@@ -545,9 +566,11 @@ void combine_y(double* Y, long long m, const double* const* T, const double* coe
     a.T[q] = T[q]; a.X[q] = X[q]; a.cT[q] = coefT[q]; a.cX[q] = coefX[q];
   }
   if (small_index(total))
-    k_combine_y<unsigned><<<grid_for(total), kT, 0, current_stream()>>>(Y, m, a, nq, r, c);
+    launch_chained(k_combine_y<unsigned>, grid_for(total), kT, 0, current_stream(), Y, m, a, nq, r,
+                   c);
   else
-    k_combine_y<long long><<<grid_for(total), kT, 0, current_stream()>>>(Y, m, a, nq, r, c);
+    launch_chained(k_combine_y<long long>, grid_for(total), kT, 0, current_stream(), Y, m, a, nq, r,
+                   c);
   UW12_LAUNCHED();
 }
 
@@ -556,7 +579,7 @@ void combine_vecs(const double* U, long long m, int ns, const double* coef, cons
   if (m <= 0) return;
   VecArgs a{};
   for (int q = 0; q < ns * ns; ++q) a.coef[q] = coef[q];
-  k_combine_vecs<<<grid_for(m * ns), kT, 0, current_stream()>>>(U, m, ns, a, w, V);
+  launch_chained(k_combine_vecs, grid_for(m * ns), kT, 0, current_stream(), U, m, ns, a, w, V);
   UW12_LAUNCHED();
 }
 
@@ -572,9 +595,11 @@ void lincomb(double* Y, long long m, long long n, int nt, const double* const* m
     a.scaled[q] = scaled ? scaled[q] : 0;
   }
   if (small_index(total))
-    k_lincomb<unsigned><<<grid_for(total), kT, 0, current_stream()>>>(Y, m, n, nt, a, r, c);
+    launch_chained(k_lincomb<unsigned>, grid_for(total), kT, 0, current_stream(), Y, m, n, nt, a, r,
+                   c);
   else
-    k_lincomb<long long><<<grid_for(total), kT, 0, current_stream()>>>(Y, m, n, nt, a, r, c);
+    launch_chained(k_lincomb<long long>, grid_for(total), kT, 0, current_stream(), Y, m, n, nt, a,
+                   r, c);
   UW12_LAUNCHED();
 }
 
@@ -584,12 +609,12 @@ void pack_sym_sum(const double* G, long long n, long long na, double* out, long 
   if (total <= 0) return;
   const long long np = n * (n + 1) / 2;
   if (small_index(std::max(total, n * n)))
-    k_pack_sym_sum<unsigned><<<grid_for(total), kT, 0, current_stream()>>>(
-        G, static_cast<unsigned>(n), static_cast<unsigned>(np), static_cast<unsigned>(total), out,
-        ldo, beta);
+    launch_chained(k_pack_sym_sum<unsigned>, grid_for(total), kT, 0, current_stream(), G,
+                   static_cast<unsigned>(n), static_cast<unsigned>(np),
+                   static_cast<unsigned>(total), out, ldo, beta);
   else
-    k_pack_sym_sum<long long><<<grid_for(total), kT, 0, current_stream()>>>(G, n, np, total, out,
-                                                                            ldo, beta);
+    launch_chained(k_pack_sym_sum<long long>, grid_for(total), kT, 0, current_stream(), G, n, np,
+                   total, out, ldo, beta);
   UW12_LAUNCHED();
 }
 
@@ -598,9 +623,11 @@ void perm_3el(const double* Z, double* out, long long rp, long long a, long long
   const long long total = rp * a * a * kc;
   if (total <= 0) return;
   if (small_index(total))
-    k_perm_3el<unsigned><<<grid_for(total), kT, 0, current_stream()>>>(Z, out, rp, a, kc, alpha);
+    launch_chained(k_perm_3el<unsigned>, grid_for(total), kT, 0, current_stream(), Z, out, rp, a,
+                   kc, alpha);
   else
-    k_perm_3el<long long><<<grid_for(total), kT, 0, current_stream()>>>(Z, out, rp, a, kc, alpha);
+    launch_chained(k_perm_3el<long long>, grid_for(total), kT, 0, current_stream(), Z, out, rp, a,
+                   kc, alpha);
   UW12_LAUNCHED();
 }
 
@@ -608,37 +635,40 @@ void perm_4el(const double* V, double* out, long long a, long long o, double alp
   const long long total = a * o * a * o;
   if (total <= 0) return;
   if (small_index(total))
-    k_perm_4el<unsigned><<<grid_for(total), kT, 0, current_stream()>>>(V, out, a, o, alpha);
+    launch_chained(k_perm_4el<unsigned>, grid_for(total), kT, 0, current_stream(), V, out, a, o,
+                   alpha);
   else
-    k_perm_4el<long long><<<grid_for(total), kT, 0, current_stream()>>>(V, out, a, o, alpha);
+    launch_chained(k_perm_4el<long long>, grid_for(total), kT, 0, current_stream(), V, out, a, o,
+                   alpha);
   UW12_LAUNCHED();
 }
 
 void scale_pinv_cols(double* Q, long long n, const double* lambda, double tol) {
   if (n <= 0) return;
-  k_scale_pinv_cols<<<grid_for(n * n), kT, 0, current_stream()>>>(Q, n, lambda, tol);
+  launch_chained(k_scale_pinv_cols, grid_for(n * n), kT, 0, current_stream(), Q, n, lambda, tol);
   UW12_LAUNCHED();
 }
 
 void set_identity(double* A, long long n) {
   if (n <= 0) return;
-  k_set_identity<<<grid_for(n * n), kT, 0, current_stream()>>>(A, n);
+  launch_chained(k_set_identity, grid_for(n * n), kT, 0, current_stream(), A, n);
   UW12_LAUNCHED();
 }
 
 void gather_scale_cols(const double* src, long long rows, const int* idx, const double* s,
                        long long nq, double* dst) {
   if (rows * nq <= 0) return;
-  k_gather_scale_cols<<<grid_for(rows * nq), kT, 0, current_stream()>>>(src, rows, idx, s, nq,
-                                                                        dst);
+  launch_chained(k_gather_scale_cols, grid_for(rows * nq), kT, 0, current_stream(), src, rows, idx,
+                 s, nq, dst);
   UW12_LAUNCHED();
 }
 
 // out += sum of squares of the rows x cols block A (leading dimension lda):
 // grid-stride partial sums, a warp-shuffle and shared-memory block reduction,
 // one atomic add per block (summation order not fixed).
-__global__ void k_sumsq_add(const double* __restrict__ A, long long lda, long long rows,
+__global__ void k_sumsq_add(const double* A, long long lda, long long rows,
                             long long cols, double* out) {
+  chain_wait();
   __shared__ double part[32];
   const long long total = rows * cols;
   double acc = 0.0;
@@ -663,7 +693,7 @@ void sumsq_add(const double* A, long long lda, long long rows, long long cols, d
                cudaStream_t s) {
   const long long total = rows * cols;
   if (total <= 0) return;
-  k_sumsq_add<<<grid_for(total, 4), kT, 0, s>>>(A, lda, rows, cols, out);
+  launch_chained(k_sumsq_add, grid_for(total, 4), kT, 0, s, A, lda, rows, cols, out);
   UW12_LAUNCHED();
 }
 
