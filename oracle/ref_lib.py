@@ -39,7 +39,7 @@ class RefLogicError(ValueError):
 def build(quiet: bool = True) -> bool:
     """Compile the reference when its source tree is present; True if the
     library exists afterwards."""
-    if os.path.isdir(REFERENCE_TREE):
+    if os.path.isfile(os.path.join(REFERENCE_TREE, "libuw12.cpp")):
         out = subprocess.run(
             ["make", "-f", os.path.join(HERE, "ref.mk"), f"REF={REFERENCE_TREE}", "-j8", "all"],
             capture_output=True, text=True)
