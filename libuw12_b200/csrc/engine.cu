@@ -648,6 +648,14 @@ struct SpinDims {
   size_t o = 0, a = 0, c = 0, ooff = 0, aoff = 0;
 };
 
+// Pairs (j, k) of active orbitals j and occupied orbitals k < k_end in pair order: k
+// ascending and j ascending within it, every j for a core orbital, j <= k - c for
+// an active one.
+size_t pair_count(size_t a, size_t c, size_t k_end) {
+  const size_t i = k_end > c ? k_end - c : 0;
+  return a * std::min(k_end, c) + i * (i + 1) / 2;
+}
+
 // Occupation-weighted occupied orbitals Co (utils.hpp:289-310) of both spins side
 // by side (N x o_tot) and their active (last n_active) columns Ca (freeze_core,
 // utils.hpp:235-253; N x a_tot), one after the other on the device.
@@ -712,12 +720,12 @@ bool pair_form_cheaper(const FockRequest& rq, const std::vector<SpinDims>& sd, b
   if (aux == 0.0) return false;
   aux += Rp * Rp * N * MW;
   for (int s = 0; s < ns; ++s) {
-    const double a = double(sd[s].a), ao = a * double(sd[s].o);
-    pairs += ao * (Rp * Rp * N + (same_spin && ns == 1 ? 0.0 : N * N * Rp));
+    const double a = double(sd[s].a), ap = double(pair_count(sd[s].a, sd[s].c, sd[s].o));
+    pairs += ap * (Rp * Rp * N + (same_spin && ns == 1 ? 0.0 : N * N * Rp));
     if (same_spin)
       aux += a * a * N * Rp * MW + Rp * Rp * a * MW;
     else
-      pairs += ao * (J * (MW + MV) + MW * MW + MV * MV);
+      pairs += ap * (J * (MW + MV) + MW * MW + MV * MV);
   }
   return pairs <= aux;
 }
@@ -741,7 +749,7 @@ size_t budget_need(const FockRequest& rq, bool adjoint, bool streamed) {
   if (rq.indirect) {
     need = std::max(need, (3 * Rp * o1 + M) * o1 * o1);                  // pair products of energies
   }
-  if (rq.calc_fock) need = std::max(need, blocks + o1 * o1 * (4 * Rp * N + np));  // pair products
+  if (rq.calc_fock) need = std::max(need, blocks + o1 * o1 * (5 * Rp * N + np));  // pair products
   if (adjoint)
     need = std::max({need, 2 * (N + R + 2 * (o1 + 2 * Rp)) * o * M, (4 * N * N + N * o) * M});
   return need;
@@ -1301,10 +1309,12 @@ void form_fock(const FockRequest& rq) {
       const size_t o = sd[s].o, a = sd[s].a, c = sd[s].c;
       if (a == 0 || o == 0) continue;
       const size_t ao = a * o, No = N * o;
-      DevBuf b2wl(ao * MW), b2vl(ao * MV), b1wl, b1vl;
+      DevBuf b2wl, b2vl, b1wl, b1vl;
+      if (do_ind) {
+      b2wl.alloc(ao * MW);
+      b2vl.alloc(ao * MV);
       scale_rc(XW.B2[s].get(), LL(ao), LL(ao), LL(MW), nullptr, W.lam.get(), 1.0, b2wl.get(), LL(ao));
       scale_rc(XV.B2[s].get(), LL(ao), LL(ao), LL(MV), nullptr, V.lam.get(), 1.0, b2vl.get(), LL(ao));
-      if (do_ind) {
       clock.mark("ss_4el_energy");
       // ---- 4-el indirect energy (four_electron.cpp:143-179)
       if (lead) {
@@ -1398,21 +1408,33 @@ void form_fock(const FockRequest& rq) {
       // the same-spin terms G_W and G_V are there already, S^-1 G_V also
       // replaces S^-1 Y_W (Y_W then serves the k-term as it is), and no
       // product has an aux x aux operand.  pair_form_cheaper counts both forms.
-      // One B200, against the form over aux functions and k-chunked Y_W (same GEMM
-      // kernels): closed shell N=300, M=900, R=1200, o=30 in FP64 229 -> 176 ms; open
-      // shell N=200, M=600, R=800, o=16/15 53.3 -> 35.3 ms.
+      // The integrals are symmetric, so x^ and G of the active pairs (j, c + i)
+      // and (i, c + j) are the same: G, S^-1 G and the sums with them run over
+      // the a c pairs with a core orbital and the a (a + 1) / 2 pairs j <= i, with
+      // Y[j, c+i] + Y[i, c+j] beside G.  Only Y, which the k-term pairs with its
+      // mirror image, is formed for both orders.
+      // One B200, against the same sums over all a o pairs: closed shell N=300, M=900,
+      // R=1200, o=30 in FP64 176 -> 130 ms, o=30/29 in split precision 186 -> 141; open
+      // shell N=200, M=600, R=800, o=16/15 35.1 -> 26.7 ms.
       double cD[2] = {0.0, 0.0};
       for (int sp = 0; sp < ns && fold; ++sp) cD[sp] = half * spin_factor(ns, s, sp, s_os, s_ss);
       if (!do_ind && cD[0] == 0.0 && cD[1] == 0.0) continue;
-      DevBuf xhW(MW * ao), xhV(MV * ao);
-      GemmDesc g = gemm_nn(LL(MW), LL(ao), LL(MW), 1.0, W.P2.get(), LL(MW), b2wl.get(), LL(ao),
-                           0.0, xhW.get(), LL(MW));
-      g.b_ncontig = true;
-      gemm(g);
-      g = gemm_nn(LL(MV), LL(ao), LL(MV), 1.0, V.P2.get(), LL(MV), b2vl.get(), LL(ao), 0.0,
-                  xhV.get(), LL(MV));
-      g.b_ncontig = true;
-      gemm(g);
+      // x^ of the pairs, in pair order; twice the mean of the two orders for V, so that
+      // S^-1 G_V carries the weight of a pair, the mean for W
+      const size_t n_all = pair_count(a, c, o);
+      DevBuf xhW(MW * n_all), xhV(MV * n_all);
+      {
+        DevBuf b2p(n_all * std::max(MW, MV));
+        for (const bool is_w : {true, false}) {
+          const IntegralsHandle& X = is_w ? W : V;
+          pack_pairs((is_w ? XW : XV).B2[s].get(), LL(a), LL(c), LL(o), LL(X.n_df), X.lam.get(),
+                     is_w ? 0.5 : 1.0, b2p.get());
+          GemmDesc g = gemm_nn(LL(X.n_df), LL(n_all), LL(X.n_df), 1.0, X.P2.get(), LL(X.n_df),
+                               b2p.get(), LL(n_all), 0.0, (is_w ? xhW : xhV).get(), LL(X.n_df));
+          g.b_ncontig = true;
+          gemm(g);
+        }
+      }
       budget = budgets.doubles();
       // unstored W / V blocks (accumulated over, for every k chunk) take at
       // most an eighth of the budget each
@@ -1421,133 +1443,165 @@ void form_fock(const FockRequest& rq) {
         xscr = std::max(xscr, (Xi->J3_0.get() ? 0 : np * aux_step(*Xi, false, budget / 2)) +
                                   (Xi->J3_ri_0.get() ? 0 : R * N * aux_step(*Xi, true, budget / 2)));
       const size_t pair = Rp * N;  // doubles of one pair's matrix
-      const size_t per_k = a * (pair * (do_ind ? (fold ? 4 : 3) : 2) + np + std::max(MW, MV));
       const auto [klo, khi] = part(o);
       const size_t kavail = budget > xscr ? budget - xscr : 0;
-      const size_t kc = tile_chunk(khi - klo, a,
-                                   std::max<size_t>(1, std::min(khi - klo, kavail / per_k)));
-      const bool whole_k = kc == o;
-      // pair (j, k) of a chunk of nk orbitals is matrix (k - k0) + nk j of a buffer
-      const size_t nbuf = pair * a * kc;
-      DevBuf gpk(np * a * kc), xk(std::max(MW, MV) * a * kc), bufG(nbuf),
-          bufS(nbuf * (do_ind && fold ? 2 : 1)), bufY(do_ind ? nbuf : 0), scrX, scrXr;
-      // dst = G_X of the chunk, over X's aux blocks
-      auto form_g = [&](const IntegralsHandle& X, const double* xh, size_t k0, size_t nk,
+      // A chunk of occupied orbitals [k0, k0 + nk): its pairs are [p0, p0 + np_) in
+      // pair order.  Y of its pairs lies in two blocks: Y[j, k], j < nj, is matrix
+      // (k - k0) + nk j; where the chunk's active orbitals are [i0, i1), the mirror
+      // images Y[i, c + j], j < i0, are matrices j + i0 (i - i0) behind them.
+      // Unless it takes every orbital, a chunk has core or active orbitals only.
+      struct PairChunk {
+        size_t k0, nk, p0, n_pairs, nj, i0, i1, n_y;
+      };
+      const size_t n_s = do_ind && fold && ns == 2 ? 2 : 1;
+      auto pair_chunk = [&](size_t k0, size_t nk) {
+        PairChunk q{};
+        q.k0 = k0;
+        q.nk = nk;
+        q.p0 = pair_count(a, c, k0);
+        q.n_pairs = pair_count(a, c, k0 + nk) - q.p0;
+        q.i0 = std::max(k0, c) - c;
+        q.i1 = std::max(k0 + nk, c) - c;
+        q.nj = k0 < c ? a : q.i1;
+        q.n_y = do_ind ? nk * q.nj + q.i0 * (q.i1 - q.i0) : 0;
+        return q;
+      };
+      std::vector<PairChunk> chunks;
+      size_t max_pairs = 0, max_y = 0;
+      for (size_t k0 = klo; k0 < khi;) {
+        PairChunk q = pair_chunk(k0, khi - k0);
+        auto need = [&] { return pair * (q.n_pairs * (1 + n_s) + 2 * q.n_y) + np * q.n_pairs; };
+        if (q.nk < o || need() > kavail) {
+          const size_t end = k0 < c ? std::min(c, khi) : khi;
+          q = pair_chunk(k0, end - k0);
+          while (q.nk > 1 && need() > kavail) q = pair_chunk(k0, q.nk - 1);
+        }
+        chunks.push_back(q);
+        max_pairs = std::max(max_pairs, q.n_pairs);
+        max_y = std::max(max_y, q.n_y);
+        k0 += q.nk;
+      }
+      const size_t nbuf = pair * max_pairs;
+      DevBuf gpk(np * max_pairs), bufG(nbuf), bufS(nbuf * n_s), bufY(pair * max_y),
+          bufZ(pair * max_y), scrX, scrXr;
+      // dst = G_X of the chunk's pairs, over X's aux blocks
+      auto form_g = [&](const IntegralsHandle& X, const double* xh, const PairChunk& q,
                         double* dst) {
         const size_t M = X.n_df;
-        copy3d(xh + M * a * k0, LL(M), LL(M * a), xk.get(), LL(M * nk), LL(M), LL(M), LL(a),
-               LL(nk));
+        const double* x = xh + M * q.p0;
         const size_t st_ao = aux_step(X, false, budget / 2);
         const size_t st_ri = aux_step(X, true, budget / 2);
         for (size_t b0 = 0; b0 < M; b0 += st_ao) {
           const size_t nb = std::min(st_ao, M - b0);
-          gemm(gemm_nn(LL(np), LL(a * nk), LL(nb), 1.0, aux_block(X, false, b0, nb, scrX), LL(np),
-                       xk.get() + b0, LL(M), b0 ? 1.0 : 0.0, gpk.get(), LL(np)));
+          gemm(gemm_nn(LL(np), LL(q.n_pairs), LL(nb), 1.0, aux_block(X, false, b0, nb, scrX),
+                       LL(np), x + b0, LL(M), b0 ? 1.0 : 0.0, gpk.get(), LL(np)));
         }
-        unpack_sym(gpk.get(), LL(np), LL(N), LL(a * nk), dst, LL(Rp), LL(pair));
+        unpack_sym(gpk.get(), LL(np), LL(N), LL(q.n_pairs), dst, LL(Rp), LL(pair));
         for (size_t b0 = 0; b0 < M; b0 += st_ri) {
           const size_t nb = std::min(st_ri, M - b0);
-          GemmDesc gr = gemm_nn(LL(R), LL(a * nk), LL(nb), 1.0, aux_block(X, true, b0, nb, scrXr),
-                                LL(R * N), xk.get() + b0, LL(M), b0 ? 1.0 : 0.0, dst + N,
-                                LL(pair));
+          GemmDesc gr = gemm_nn(LL(R), LL(q.n_pairs), LL(nb), 1.0,
+                                aux_block(X, true, b0, nb, scrXr), LL(R * N), x + b0, LL(M),
+                                b0 ? 1.0 : 0.0, dst + N, LL(pair));
           gr.nbo1 = LL(N);
           gr.sAo1 = LL(R);
           gr.sCo1 = LL(Rp);
           gemm(gr);
         }
       };
-      // dst = St[j] L B1[k]^T of the chunk (St: R' a x M)
-      auto form_y = [&](const double* St, const double* b1l, size_t M, size_t k0, size_t nk,
+      // dst = St[j] L B1[k]^T of the chunk, both blocks (St: R' a x M)
+      auto form_y = [&](const double* St, const double* b1l, size_t M, const PairChunk& q,
                         double* dst) {
-        GemmDesc gy = gemm_nn(LL(Rp), LL(N * nk), LL(M), 1.0, St, LL(Rp * a), b1l + N * k0,
-                              LL(No), 0.0, dst, LL(Rp));
-        gy.b_ncontig = true;
-        gy.nbo1 = LL(a);
-        gy.sAo1 = LL(Rp);
-        gy.sCo1 = LL(pair * nk);
-        gemm(gy);
+        auto block = [&](size_t j0, size_t nj, size_t k0, size_t nk, double* to) {
+          if (nj == 0 || nk == 0) return;
+          GemmDesc gy = gemm_nn(LL(Rp), LL(N * nk), LL(M), 1.0, St + Rp * j0, LL(Rp * a),
+                                b1l + N * k0, LL(No), 0.0, to, LL(Rp));
+          gy.b_ncontig = true;
+          gy.nbo1 = LL(nj);
+          gy.sAo1 = LL(Rp);
+          gy.sCo1 = LL(pair * nk);
+          gemm(gy);
+        };
+        block(0, q.nj, q.k0, q.nk, dst);
+        block(q.i0, q.i1 - q.i0, c, q.i0, dst + pair * q.nk * q.nj);
+      };
+      // out = coef (Y[j, k] + Y[i, c + j]) + coef_s S per pair; the sum is scaled by
+      // mirror where it has two terms
+      auto sum_y = [&](const PairChunk& q, const double* Y, double coef, double mirror,
+                       const double* S, double coef_s, double* dst) {
+        sum_pairs(Y, Y + pair * q.nk * q.nj, LL(pair), LL(a), LL(c), LL(q.k0), LL(q.nk),
+                  LL(q.n_pairs), coef, mirror, S, coef_s, dst);
       };
       // F += coef sum_pairs A[pair]^T B[pair]
-      auto add_pairs = [&](double coef, const double* A, const double* B, size_t n_pairs, double beta,
+      auto add_pairs = [&](double coef, const double* A, const double* B, size_t n_pairs,
                            double* F) {
-        GemmDesc gf = gemm_nn(LL(N), LL(N), LL(Rp), coef, A, LL(Rp), B, LL(Rp), beta, F, LL(N));
+        GemmDesc gf = gemm_nn(LL(N), LL(N), LL(Rp), coef, A, LL(Rp), B, LL(Rp), 1.0, F, LL(N));
         gf.a_kcontig = true;
         gf.nbr1 = LL(n_pairs);
         gf.sAr1 = LL(pair);
         gf.sBr1 = LL(pair);
         gemm(gf);
       };
-      for (size_t k0 = klo; k0 < khi; k0 += kc) {
-        const size_t nk = std::min(kc, khi - k0), n_pairs = a * nk;
-        const double* z = nullptr;   // S^-1 Y_V
-        const double* yw = nullptr;  // Y_W, when the whole of it is held
+      // k-term (fock_k): F += s_ss sum Y_W[i, c + j]^T Z[j, c + i] over the chunk's
+      // active pairs, both orders
+      auto k_term = [&](const PairChunk& q, const double* Yw, const double* Z) {
+        const size_t ni = q.i1 - q.i0, i0 = q.i0, nk = q.nk;
+        if (ni == 0) return;
+        auto add = [&](size_t nj, const double* A, size_t sAi, size_t sAj, const double* B,
+                       size_t sBi, size_t sBj) {
+          if (nj == 0) return;
+          GemmDesc fk = gemm_nn(LL(N), LL(N), LL(Rp), s_ss, A, LL(Rp), B, LL(Rp), 1.0, Fp[s],
+                                LL(N));
+          fk.a_kcontig = true;
+          fk.nbr1 = LL(ni);
+          fk.nbr2 = LL(nj);
+          fk.sAr1 = LL(pair * sAi);
+          fk.sAr2 = LL(pair * sAj);
+          fk.sBr1 = LL(pair * sBi);
+          fk.sBr2 = LL(pair * sBj);
+          gemm(fk);
+        };
+        const size_t first = c + i0 - q.k0;  // orbital c + i0 in the chunk
+        const size_t blk = pair * (first + nk * i0), back = pair * nk * q.nj;
+        add(ni, Yw + blk, nk, 1, Z + blk, 1, nk);
+        add(i0, Yw + back, i0, 1, Z + pair * first, 1, nk);
+        add(i0, Yw + pair * first, 1, nk, Z + back, i0, 1);
+      };
+      for (const PairChunk& q : chunks) {
+        form_g(V, xhV.get(), q, bufG.get());
         if (fold) {
-          form_g(V, xhV.get(), k0, nk, bufG.get());
-          gemm(gemm_nn(LL(Rp), LL(N * n_pairs), LL(Rp), 1.0, AB.Sinv.get(), LL(Rp), bufG.get(),
+          gemm(gemm_nn(LL(Rp), LL(N * q.n_pairs), LL(Rp), 1.0, AB.Sinv.get(), LL(Rp), bufG.get(),
                        LL(Rp), 0.0, bufS.get(), LL(Rp)));
           if (do_ind) {
-            form_y(XW.Wst[s].get(), b1wl.get(), MW, k0, nk, bufY.get());
-            add_pairs(s_ss, bufS.get(), bufY.get(), n_pairs, 1.0, Fp[s]);
-            if (whole_k) yw = bufY.get();
+            form_y(XW.Wst[s].get(), b1wl.get(), MW, q, bufY.get());
+            sum_y(q, bufY.get(), 1.0, 0.5, nullptr, 0.0, bufG.get());
+            add_pairs(s_ss, bufS.get(), bufG.get(), q.n_pairs, Fp[s]);
           }
-          form_g(W, xhW.get(), k0, nk, bufG.get());
         } else {
-          form_g(V, xhV.get(), k0, nk, bufG.get());
-          form_y(XW.SV[s].get(), b1wl.get(), MW, k0, nk, bufY.get());
-          add_pairs(s_ss, bufG.get(), bufY.get(), n_pairs, 1.0, Fp[s]);
-          form_g(W, xhW.get(), k0, nk, bufG.get());
+          form_y(XW.SV[s].get(), b1wl.get(), MW, q, bufY.get());
+          sum_y(q, bufY.get(), 1.0, 0.5, nullptr, 0.0, bufS.get());
+          add_pairs(s_ss, bufG.get(), bufS.get(), q.n_pairs, Fp[s]);
+          if (q.i1 > q.i0) form_y(XW.Wst[s].get(), b1wl.get(), MW, q, bufY.get());
         }
+        form_g(W, xhW.get(), q, bufG.get());
         if (do_ind) {
-          double* zbuf = bufS.get() + (fold ? nbuf : 0);
-          form_y(XV.SV[s].get(), b1vl.get(), MV, k0, nk, zbuf);
-          z = zbuf;
-          // k-term (fock_k) for active orbitals c + i inside this chunk
-          const size_t i0 = std::max(k0, c) - c, i1 = std::max(k0 + nk, c) - c;
-          if (i1 > i0) {
-            const size_t ni = i1 - i0;
-            GemmDesc fk = gemm_nn(LL(N), LL(N), LL(Rp), s_ss, yw, LL(Rp),
-                                  z + pair * (c + i0 - k0), LL(Rp), 1.0, Fp[s], LL(N));
-            fk.a_kcontig = true;
-            fk.nbr1 = LL(ni);
-            fk.nbr2 = LL(a);
-            fk.sBr1 = LL(pair);
-            fk.sBr2 = LL(pair * nk);
-            if (yw) {
-              fk.A = yw + pair * c;
-              fk.sAr1 = LL(pair * nk);
-              fk.sAr2 = LL(pair);
-            } else {
-              // Y_W[i, c + j] of the chunk's i and all j
-              GemmDesc gw = gemm_nn(LL(Rp * ni), LL(N * a), LL(MW), 1.0,
-                                    XW.Wst[s].get() + Rp * i0, LL(Rp * a), b1wl.get() + N * c,
-                                    LL(No), 0.0, bufY.get(), LL(Rp * ni));
-              gw.b_ncontig = true;
-              gemm(gw);
-              fk.A = bufY.get();
-              fk.lda = LL(Rp * ni);
-              fk.sAr1 = LL(Rp);
-              fk.sAr2 = LL(Rp * ni * N);
-            }
-            gemm(fk);
-          }
+          form_y(XV.SV[s].get(), b1vl.get(), MV, q, bufZ.get());
+          k_term(q, bufY.get(), bufZ.get());
         }
         if (!fold) {
-          add_pairs(s_ss, bufG.get(), z, n_pairs, 1.0, Fp[s]);
+          sum_y(q, bufZ.get(), s_ss, 1.0, nullptr, 0.0, bufS.get());
+          add_pairs(1.0, bufG.get(), bufS.get(), q.n_pairs, Fp[s]);
         } else if (ns == 1) {
           // one product for t~ dX and the same-spin term: G_W^T (s_ss S^-1 Y_V - cD S^-1 G_V)
-          if (do_ind) {
-            const double* mats[2] = {z, bufS.get()};
-            const double coefs[2] = {s_ss, -cD[0]};
-            lincomb(bufS.get(), LL(pair), LL(n_pairs), 2, mats, coefs, nullptr, nullptr, nullptr);
-          }
-          add_pairs(do_ind ? 1.0 : -cD[0], bufG.get(), bufS.get(), n_pairs, 1.0, Fp[s]);
+          if (do_ind) sum_y(q, bufZ.get(), s_ss, 1.0, bufS.get(), -cD[0], bufS.get());
+          add_pairs(do_ind ? 1.0 : -cD[0], bufG.get(), bufS.get(), q.n_pairs, Fp[s]);
         } else {
           // D and the same-spin term G_W^T S^-1 Y_V in one launch, G_W read once
+          if (do_ind) sum_y(q, bufZ.get(), 1.0, 1.0, nullptr, 0.0, bufS.get() + nbuf);
           DevBuf D(2 * N * N);
           GemmDesc gd = gemm_nn(LL(N), LL(N), LL(Rp), 1.0, bufG.get(), LL(Rp), bufS.get(), LL(Rp),
                                 0.0, D.get(), LL(N));
           gd.a_kcontig = true;
-          gd.nbr1 = LL(n_pairs);
+          gd.nbr1 = LL(q.n_pairs);
           gd.sAr1 = LL(pair);
           gd.sBr1 = LL(pair);
           gd.nbo1 = do_ind ? 2 : 1;

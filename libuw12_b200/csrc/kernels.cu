@@ -343,6 +343,97 @@ __global__ void k_lincomb(double* Y, long long m, long long n, int nt, LincombAr
   }
 }
 
+// Row i and column j <= i of element q of a packed lower triangle.
+__device__ __forceinline__ void triangle_index(long long q, long long& i, long long& j) {
+  i = static_cast<long long>((sqrt(8.0 * static_cast<double>(q) + 1.0) - 1.0) * 0.5);
+  while (i * (i + 1) / 2 > q) --i;
+  while ((i + 1) * (i + 2) / 2 <= q) ++i;
+  j = q - i * (i + 1) / 2;
+}
+
+// x^ of orbital pairs before the metric: a few MB at most, one block per pair so
+// that the pair is found once; its strided reads of B2 are shared in L2 by the
+// neighbouring pairs' blocks.
+__global__ void k_pack_pairs(const double* B2, long long a, long long c, long long o, long long m,
+                             const double* r, double h, double* out) {
+  chain_wait();
+  const long long p = blockIdx.x, n = gridDim.x, ao = a * o;
+  long long j, k, mirror = -1;
+  if (p < a * c) {
+    k = p / a;
+    j = p - a * k;
+  } else {
+    long long i;
+    triangle_index(p - a * c, i, j);
+    k = c + i;
+    if (j != i) mirror = i + a * (c + j);
+  }
+  for (long long A = threadIdx.x; A < m; A += blockDim.x) {
+    double v = B2[j + a * k + ao * A];
+    if (mirror >= 0) v = h * (v + B2[mirror + ao * A]);
+    out[p + n * A] = r[A] * v;
+  }
+}
+
+struct PairRange {
+  long long a, c, k0, nk, i0, core_pairs, size;  // core_pairs: those of the range's core orbitals
+};
+
+// Bound by HBM: two or three matrices read and one written per pair.  A block
+// finds its pair once and takes a run of its elements, 16 bytes per load where
+// every matrix starts on 16 bytes (VEC 2).
+template <int VEC>
+__global__ void __launch_bounds__(kT) k_sum_pairs(const double* Y, const double* Y2, PairRange g,
+                                                  long long run, long long runs, double coef,
+                                                  double h, const double* S, double coef_s,
+                                                  double* out) {
+  chain_wait();
+  const long long p = blockIdx.x / runs, part = blockIdx.x - p * runs;
+  long long j, k;
+  const double* mirror = nullptr;
+  if (p < g.core_pairs) {
+    k = g.k0 + p / g.a;
+    j = p % g.a;
+  } else {
+    long long i;
+    triangle_index(p - g.core_pairs + g.i0 * (g.i0 + 1) / 2, i, j);
+    k = g.c + i;
+    if (j < g.i0)
+      mirror = Y2 + g.size * (j + g.i0 * (i - g.i0));
+    else if (j < i)
+      mirror = Y + g.size * ((g.c + j - g.k0) + g.nk * i);
+  }
+  const double* y = Y + g.size * ((k - g.k0) + g.nk * j);
+  const double f = mirror ? coef * h : coef;
+  const long long end = (part + 1) * run < g.size ? (part + 1) * run : g.size;
+  const double* s = S ? S + g.size * p : nullptr;
+  double* d = out + g.size * p;
+  for (long long e = part * run + VEC * threadIdx.x; e < end; e += VEC * kT) {
+    if constexpr (VEC == 2) {
+      double2 v = *reinterpret_cast<const double2*>(y + e);
+      if (mirror) {
+        const double2 w = *reinterpret_cast<const double2*>(mirror + e);
+        v.x += w.x;
+        v.y += w.y;
+      }
+      v.x *= f;
+      v.y *= f;
+      if (s) {
+        const double2 w = *reinterpret_cast<const double2*>(s + e);
+        v.x += coef_s * w.x;
+        v.y += coef_s * w.y;
+      }
+      *reinterpret_cast<double2*>(d + e) = v;
+    } else {
+      double v = y[e];
+      if (mirror) v += mirror[e];
+      v *= f;
+      if (s) v += coef_s * s[e];
+      d[e] = v;
+    }
+  }
+}
+
 // out[i(i+1)/2 + j, a] = G[i, j, a] + G[j, i, a] (j < i), G[i, i, a] (j = i):
 // the gradient of a function of sq(x) with respect to the packed x.  Bound by
 // HBM and L2 (G[i, j] is read at a stride; its lines serve the neighbouring rows
@@ -600,6 +691,42 @@ void lincomb(double* Y, long long m, long long n, int nt, const double* const* m
   else
     launch_chained(k_lincomb<long long>, grid_for(total), kT, 0, current_stream(), Y, m, n, nt, a,
                    r, c);
+  UW12_LAUNCHED();
+}
+
+void pack_pairs(const double* B2, long long a, long long c, long long o, long long m,
+                const double* r, double h, double* out) {
+  const long long n = a * c + (o - c) * (o - c + 1) / 2;
+  if (n <= 0 || m <= 0) return;
+  launch_chained(k_pack_pairs, static_cast<unsigned>(n), kT, 0, current_stream(), B2, a, c, o, m, r,
+                 h, out);
+  UW12_LAUNCHED();
+}
+
+void sum_pairs(const double* Y, const double* Y2, long long size, long long a, long long c,
+               long long k0, long long nk, long long n_pairs, double coef, double h,
+               const double* S, double coef_s, double* out) {
+  if (n_pairs <= 0 || size <= 0) return;
+  PairRange g{};
+  g.a = a;
+  g.c = c;
+  g.k0 = k0;
+  g.nk = nk;
+  g.i0 = std::max(k0, c) - c;
+  g.core_pairs = a * std::max(0LL, std::min(k0 + nk, c) - k0);
+  g.size = size;
+  // four loads per thread and matrix, more only to keep the block count in 31 bits
+  const bool vec = size % 2 == 0;  // every matrix of a 16-byte aligned buffer is aligned
+  long long run = 4LL * kT * (vec ? 2 : 1);
+  while (n_pairs * ((size + run - 1) / run) >= (1LL << 31)) run *= 2;
+  const long long runs = (size + run - 1) / run;
+  const dim3 grid(static_cast<unsigned>(n_pairs * runs));
+  if (vec)
+    launch_chained(k_sum_pairs<2>, grid, kT, 0, current_stream(), Y, Y2, g, run, runs, coef, h, S,
+                   coef_s, out);
+  else
+    launch_chained(k_sum_pairs<1>, grid, kT, 0, current_stream(), Y, Y2, g, run, runs, coef, h, S,
+                   coef_s, out);
   UW12_LAUNCHED();
 }
 

@@ -93,6 +93,23 @@ void perm_3el(const double* Z, double* out, long long rp, long long a, long long
 // and columns; out and V distinct.
 void perm_4el(const double* V, double* out, long long a, long long o, double alpha);
 
+// Pair order (a active, c core, o = a + c occupied orbitals): occupied k ascending, within
+// it active j ascending, every j for a core k and j <= i for the active k = c + i.
+// out[p, A] (contiguous, all pairs x m) = r_A B2[j + a k, A], and where the mirror image
+// (i, c + j) is another entry, r_A h (B2[j + a k, A] + B2[i + a (c + j), A]);
+// B2 is (a o) x m.
+void pack_pairs(const double* B2, long long a, long long c, long long o, long long m,
+                const double* r, double h, double* out);
+
+// out[p] = coef (Y[j, k] + mirror image) + coef_s S[p] for the pairs of the occupied
+// orbitals [k0, k0 + nk), matrices of `size` elements; where there is a mirror image the
+// sum of both is scaled by h.  Y[j, k] is matrix (k - k0) + nk j of Y, the mirror
+// image Y[i, c + j] too where c + j >= k0, matrix j + i0 (i - i0) of Y2 before it (c + i0 the
+// first active orbital of the range).  S may be null, or out itself.
+void sum_pairs(const double* Y, const double* Y2, long long size, long long a, long long c,
+               long long k0, long long nk, long long n_pairs, double coef, double h,
+               const double* S, double coef_s, double* out);
+
 // A = I (n x n, column-major).
 void set_identity(double* A, long long n);
 
