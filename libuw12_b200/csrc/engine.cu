@@ -36,6 +36,7 @@
 #include "engine.cuh"
 #include "gemm_f64.cuh"
 #include "kernels.cuh"
+#include "ozaki.cuh"
 
 namespace uw12b {
 
@@ -704,28 +705,40 @@ namespace {
 // over a.  Over pairs: S^-1 G_V and D, and without the same-spin terms (which
 // form them anyway) G_W and G_V; with them Y_W is used twice and S^-1 Wst_W is
 // not needed.  With 3 DF and 4 RI functions per AO and closed shell the pairs
-// win up to a o = 0.8 M without and 4 M with the same-spin terms.
+// win in FP64 up to a o = 1.6 M without and 8 M with the same-spin terms.
+// In split precision an operand element costs its preparation (8 bytes read twice and L
+// residue bytes written at 5.8 TB/s) and a result element its reconstruction (L + 8
+// bytes at 3.4 TB/s), in units of a multiply-add (L of them at 2.88 POPS): the forms'
+// operations are equal at N=500, M=1500, R=2000, o=40/38, opposite spin, but the pairs
+// prepare the three-index tensors once per spin: 339 ms, over aux functions 321.
 bool pair_form_cheaper(const FockRequest& rq, const std::vector<SpinDims>& sd, bool same_spin) {
   const int ns = rq.n_spin;
   const double N = double(rq.n_ao), R = double(rq.W->n_ri), Rp = N + R;
   const double MW = double(rq.W->n_df), MV = double(rq.V->n_df);
   const double J = 0.5 * N * (N + 1.0) + R * N;  // rows of a three-index tensor
-  double aux = 0.0, pairs = 0.0;
+  const double L = split_moduli();
+  const double prep = L > 0.0 ? 248.0 * (16.0 + L) / L : 0.0;
+  const double crt = L > 0.0 ? 424.0 * (8.0 + L) / L : 0.0;
+  auto product = [&](double m, double n, double k) {
+    return m * n * k + prep * (m + n) * k + crt * m * n;
+  };
+  double aux = 0.0, pairs = 0.0, nq = 0.0;
   for (int sp = 0; sp < ns; ++sp) {
     bool any = false;
     for (int s = 0; s < ns; ++s)
       any = any || (spin_factor(ns, s, sp, rq.s_os, rq.s_ss) != 0.0 && sd[s].a > 0);
-    if (any) aux += J * MW * MV + N * N * Rp * MW + MW * MV * (MW + MV);
+    if (any) nq += 1.0;
   }
-  if (aux == 0.0) return false;
-  aux += Rp * Rp * N * MW;
+  if (nq == 0.0) return false;
+  aux = product(J, nq * MW, MV) + product(N, nq * N, Rp * MW) + nq * MW * MV * (MW + MV) +
+        product(Rp, N * MW, Rp);
   for (int s = 0; s < ns; ++s) {
     const double a = double(sd[s].a), ap = double(pair_count(sd[s].a, sd[s].c, sd[s].o));
-    pairs += ap * (Rp * Rp * N + (same_spin && ns == 1 ? 0.0 : N * N * Rp));
+    pairs += product(Rp, N * ap, Rp) + (same_spin && ns == 1 ? 0.0 : product(N, N, Rp * ap));
     if (same_spin)
-      aux += a * a * N * Rp * MW + Rp * Rp * a * MW;
+      aux += product(Rp * a, N * a, MW) + product(Rp, a * MW, Rp);
     else
-      pairs += ap * (J * (MW + MV) + MW * MW + MV * MV);
+      pairs += product(J, ap, MW) + product(J, ap, MV) + ap * (MW * MW + MV * MV);
   }
   return pairs <= aux;
 }
