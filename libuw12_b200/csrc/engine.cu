@@ -581,6 +581,44 @@ void fitted_density_raw(const IntegralsHandle& X, const double* dmat, int ns, do
   }
 }
 
+// Largest product (operations) of W and V in one launch, and largest evaluation (doubles of
+// both potentials' transforms) that forms them side by side.
+constexpr double kJointFlops = 2e9;
+constexpr size_t kJointDoubles = size_t(1) << 24;
+
+// The same product for W and for V.  Small ones are bound by their launch and the
+// latency of a k tile, so equal shapes run as two output batches of one launch, the
+// batch strides being the distances between the operands (one B200, N=24 Fock 310 -> 270 us, open-shell energy at N=61 257 ->
+// 231 us, N=120 Fock 2.38 -> 2.33 ms); larger
+// ones fill the device by themselves, and split precision prepares its operands one by
+// one.
+void gemm_both(const GemmDesc& w, const GemmDesc& v) {
+  const double flops = 2.0 * double(w.m) * double(w.n) * double(w.k) * double(w.nbo1) *
+                       double(w.nbr1) * double(w.nbr2);
+  const bool same = w.m == v.m && w.n == v.n && w.k == v.k && w.lda == v.lda && w.ldb == v.ldb &&
+                    w.ldc == v.ldc && w.a_kcontig == v.a_kcontig && w.b_ncontig == v.b_ncontig &&
+                    w.alpha == v.alpha && w.beta == v.beta && w.nbo1 == v.nbo1 && w.nbo2 == 1 &&
+                    v.nbo2 == 1 && w.sAo1 == v.sAo1 && w.sBo1 == v.sBo1 && w.sCo1 == v.sCo1 &&
+                    w.nbr1 == v.nbr1 && w.nbr2 == v.nbr2 && w.sAr1 == v.sAr1 &&
+                    w.sAr2 == v.sAr2 && w.sBr1 == v.sBr1 && w.sBr2 == v.sBr2;
+  if (!same || split_moduli() > 0 || flops > kJointFlops) {
+    gemm(w);
+    gemm(v);
+    return;
+  }
+  auto distance = [](const double* from, const double* to) {
+    return static_cast<long long>(reinterpret_cast<std::intptr_t>(to) -
+                                  reinterpret_cast<std::intptr_t>(from)) /
+           static_cast<long long>(sizeof(double));
+  };
+  GemmDesc g = w;
+  g.nbo2 = 2;
+  g.sAo2 = distance(w.A, v.A);
+  g.sBo2 = distance(w.B, v.B);
+  g.sCo2 = distance(w.C, v.C);
+  gemm(g);
+}
+
 // H2 (R*na x (a_hi - a_lo)) = [J3_ri_0[:,A] (R x N) Cm] for A in [a_lo, a_hi)
 // (transform_second_index, transformations.hpp:130-158), over aux blocks.
 void ri_transform(const IntegralsHandle& X, const double* Cm, size_t na, double* H2,
@@ -937,60 +975,113 @@ void form_fock(const FockRequest& rq) {
     orbital_chunked = any > 0.0;
   }
   const bool fold = pairs_cheaper && !orbital_chunked;
-  for (int which = 0; which < 2 && !orbital_chunked; ++which) {
-    const IntegralsHandle& X = which == 0 ? W : V;
-    PerX& P = which == 0 ? XW : XV;
-    const size_t M = X.n_df;
+  // Small evaluations form W's and V's intermediates side by side, in joint launches.
+  const bool joint = !sharded && MW == MV && W.J3_0.get() && V.J3_0.get() && W.J3_ri_0.get() &&
+                     V.J3_ri_0.get() && split_moduli() == 0 &&
+                     2 * (N * N + N * o_tot + R * a_tot) * MW <= kJointDoubles;
+  for (int first = 0; first < 2 && !orbital_chunked; first += joint ? 2 : 1) {
+    const int n_x = joint ? 2 : 1;
+    const IntegralsHandle* Xs[2] = {first == 0 ? &W : &V, &V};
+    PerX* Ps[2] = {first == 0 ? &XW : &XV, &XV};
+    const size_t M = Xs[0]->n_df;
+    auto each = [&](auto desc) {  // desc(q): the product of the group's potential q
+      if (joint)
+        gemm_both(desc(0), desc(1));
+      else
+        gemm(desc(0));
+    };
     budget = budgets.doubles();
-    P.B1.resize(ns);
-    P.B2.resize(ns);
-    P.Wst.resize(ns);
-    P.SV.resize(ns);
     // this shard's aux functions [xlo, xhi): B1 and the stacked RI rows are
     // partial products H[:, xlo:xhi] P2[xlo:xhi, :], summed over the shards
-    const auto [xlo, xhi] = part(M);
+    const auto range = part(M);
+    const size_t xlo = range.first, xhi = range.second;
+    for (int q = 0; q < n_x; ++q) {
+      Ps[q]->B1.resize(ns);
+      Ps[q]->B2.resize(ns);
+      Ps[q]->Wst.resize(ns);
+      Ps[q]->SV.resize(ns);
+      for (int s = 0; s < ns; ++s) Ps[q]->B1[s].alloc(N * sd[s].o * M);
+    }
     {
-      DevBuf H(N * o_tot * (xhi - xlo));
-      transform_ao(X, Co, o_tot, H.get(), budget / 2, xlo, xhi);
+      const size_t nh = N * o_tot * (xhi - xlo);
+      DevBuf H(nh * n_x);
+      if (joint) {
+        DevBuf U(2 * N * N * M);
+        for (int q = 0; q < 2; ++q)
+          unpack_sym(Xs[q]->J3_0.get(), LL(np), LL(N), LL(M), U.get() + q * N * N * M, LL(N),
+                     LL(N * N));
+        GemmDesc g = gemm_nn(LL(N), LL(o_tot), LL(N), 1.0, U.get(), LL(N), Co, LL(N), 0.0, H.get(),
+                             LL(N));
+        g.nbo1 = LL(2 * M);
+        g.sAo1 = LL(N * N);
+        g.sCo1 = LL(N * o_tot);
+        gemm(g);
+      } else {
+        transform_ao(*Xs[0], Co, o_tot, H.get(), budget / 2, xlo, xhi);
+      }
       for (int s = 0; s < ns; ++s) {
         const size_t o = sd[s].o;
         if (!o) continue;
-        P.B1[s].alloc(N * o * M);
-        gemm(gemm_nn(LL(N * o), LL(M), LL(xhi - xlo), 1.0, H.get() + N * sd[s].ooff,
-                     LL(N * o_tot), X.P2.get() + xlo, LL(M), 0.0, P.B1[s].get(), LL(N * o)));
-        allreduce(P.B1[s].get(), N * o * M);
+        each([&](int q) {
+          return gemm_nn(LL(N * o), LL(M), LL(xhi - xlo), 1.0,
+                         H.get() + nh * q + N * sd[s].ooff, LL(N * o_tot),
+                         Xs[q]->P2.get() + xlo, LL(M), 0.0, Ps[q]->B1[s].get(), LL(N * o));
+        });
+        if (!joint) allreduce(Ps[0]->B1[s].get(), N * o * M);
       }
     }
-    DevBuf H2(R * a_tot * (xhi - xlo));
-    if (a_tot) ri_transform(X, Ca, a_tot, H2.get(), budget, xlo, xhi);
+    const size_t nh2 = R * a_tot * (xhi - xlo);
+    DevBuf H2(nh2 * n_x);
+    if (a_tot && joint) {
+      each([&](int q) {
+        GemmDesc g = gemm_nn(LL(R), LL(a_tot), LL(N), 1.0, Xs[q]->J3_ri_0.get(), LL(R), Ca, LL(N),
+                             0.0, H2.get() + nh2 * q, LL(R));
+        g.nbo1 = LL(M);
+        g.sAo1 = LL(R * N);
+        g.sCo1 = LL(R * a_tot);
+        return g;
+      });
+    } else if (a_tot) {
+      ri_transform(*Xs[0], Ca, a_tot, H2.get(), budget, xlo, xhi);
+    }
     for (int s = 0; s < ns; ++s) {
       const size_t o = sd[s].o, a = sd[s].a, c = sd[s].c;
       if (!a) continue;
-      P.B2[s].alloc(a * o * M);
-      GemmDesc g3 = gemm_nn(LL(a), LL(o * M), LL(N), 1.0, Ca_s(s), LL(N), P.B1[s].get(), LL(N),
-                            0.0, P.B2[s].get(), LL(a));
-      g3.a_kcontig = true;
-      gemm(g3);
-      P.Wst[s].alloc(Rp * a * M);
-      if (sharded) P.Wst[s].zero();  // AO rows stay zero through the sum
-      GemmDesc g2 = gemm_nn(LL(R), LL(M), LL(xhi - xlo), 1.0, H2.get() + R * sd[s].aoff,
-                            LL(R * a_tot), X.P2.get() + xlo, LL(M), 0.0, P.Wst[s].get() + N,
-                            LL(Rp * a));
-      g2.nbo1 = LL(a);
-      g2.sAo1 = LL(R);
-      g2.sCo1 = LL(Rp);
-      gemm(g2);
-      allreduce(P.Wst[s].get(), Rp * a * M);
-      copy3d(P.B1[s].get() + N * c, LL(N), LL(N * o), P.Wst[s].get(), LL(Rp), LL(Rp * a), LL(N),
-             LL(a), LL(M));
-      if (which == 1 || need_sv_w) {
-        // S^-1 Wst (R' x a M): this shard's aux columns, gathered by the sum
-        P.SV[s].alloc(Rp * a * M);
-        if (sharded) P.SV[s].zero();
-        gemm(gemm_nn(LL(Rp), LL(a * (xhi - xlo)), LL(Rp), 1.0, AB.Sinv.get(), LL(Rp),
-                     P.Wst[s].get() + Rp * a * xlo, LL(Rp), 0.0, P.SV[s].get() + Rp * a * xlo,
-                     LL(Rp)));
-        allreduce(P.SV[s].get(), Rp * a * M);
+      for (int q = 0; q < n_x; ++q) {
+        Ps[q]->B2[s].alloc(a * o * M);
+        Ps[q]->Wst[s].alloc(Rp * a * M);
+        if (sharded) Ps[q]->Wst[s].zero();  // AO rows stay zero through the sum
+      }
+      each([&](int q) {
+        GemmDesc g3 = gemm_nn(LL(a), LL(o * M), LL(N), 1.0, Ca_s(s), LL(N), Ps[q]->B1[s].get(),
+                              LL(N), 0.0, Ps[q]->B2[s].get(), LL(a));
+        g3.a_kcontig = true;
+        return g3;
+      });
+      each([&](int q) {
+        GemmDesc g2 = gemm_nn(LL(R), LL(M), LL(xhi - xlo), 1.0,
+                              H2.get() + nh2 * q + R * sd[s].aoff, LL(R * a_tot),
+                              Xs[q]->P2.get() + xlo, LL(M), 0.0, Ps[q]->Wst[s].get() + N,
+                              LL(Rp * a));
+        g2.nbo1 = LL(a);
+        g2.sAo1 = LL(R);
+        g2.sCo1 = LL(Rp);
+        return g2;
+      });
+      for (int q = 0; q < n_x; ++q) {
+        PerX& P = *Ps[q];
+        if (!joint) allreduce(P.Wst[s].get(), Rp * a * M);
+        copy3d(P.B1[s].get() + N * c, LL(N), LL(N * o), P.Wst[s].get(), LL(Rp), LL(Rp * a), LL(N),
+               LL(a), LL(M));
+        if (first + q == 1 || need_sv_w) {
+          // S^-1 Wst (R' x a M): this shard's aux columns, gathered by the sum
+          P.SV[s].alloc(Rp * a * M);
+          if (sharded) P.SV[s].zero();
+          gemm(gemm_nn(LL(Rp), LL(a * (xhi - xlo)), LL(Rp), 1.0, AB.Sinv.get(), LL(Rp),
+                       P.Wst[s].get() + Rp * a * xlo, LL(Rp), 0.0, P.SV[s].get() + Rp * a * xlo,
+                       LL(Rp)));
+          if (!joint) allreduce(P.SV[s].get(), Rp * a * M);
+        }
       }
     }
   }
@@ -1332,14 +1423,13 @@ void form_fock(const FockRequest& rq) {
       // ---- 4-el indirect energy (four_electron.cpp:143-179)
       if (lead) {
         DevBuf W4(ao * ao), V4(ao * ao);
-        GemmDesc g = gemm_nn(LL(ao), LL(ao), LL(MW), 1.0, b2wl.get(), LL(ao), XW.B2[s].get(),
-                             LL(ao), 0.0, W4.get(), LL(ao));
-        g.b_ncontig = true;
-        gemm(g);
-        g = gemm_nn(LL(ao), LL(ao), LL(MV), 1.0, b2vl.get(), LL(ao), XV.B2[s].get(), LL(ao), 0.0,
-                    V4.get(), LL(ao));
-        g.b_ncontig = true;
-        gemm(g);
+        GemmDesc gw = gemm_nn(LL(ao), LL(ao), LL(MW), 1.0, b2wl.get(), LL(ao), XW.B2[s].get(),
+                              LL(ao), 0.0, W4.get(), LL(ao));
+        gw.b_ncontig = true;
+        GemmDesc gv = gemm_nn(LL(ao), LL(ao), LL(MV), 1.0, b2vl.get(), LL(ao), XV.B2[s].get(),
+                              LL(ao), 0.0, V4.get(), LL(ao));
+        gv.b_ncontig = true;
+        gemm_both(gw, gv);
         permdot_4el(W4.get(), V4.get(), LL(a), LL(o), -0.5 * two, acc.get(), kE4i);
       }
       clock.mark("ss_3el_energy");
@@ -1353,14 +1443,13 @@ void form_fock(const FockRequest& rq) {
         DevBuf YW(Rp * a * a * kc), ZV(Rp * a * a * kc);
         for (size_t k0 = klo; k0 < khi; k0 += kc) {
           const size_t nk = std::min(kc, khi - k0);
-          GemmDesc g = gemm_nn(LL(Rp * a), LL(a * nk), LL(MW), 1.0, XW.Wst[s].get(), LL(Rp * a),
-                               b2wl.get() + a * k0, LL(ao), 0.0, YW.get(), LL(Rp * a));
-          g.b_ncontig = true;
-          gemm(g);
-          g = gemm_nn(LL(Rp * a), LL(a * nk), LL(MV), 1.0, XV.SV[s].get(), LL(Rp * a),
-                      b2vl.get() + a * k0, LL(ao), 0.0, ZV.get(), LL(Rp * a));
-          g.b_ncontig = true;
-          gemm(g);
+          GemmDesc gw = gemm_nn(LL(Rp * a), LL(a * nk), LL(MW), 1.0, XW.Wst[s].get(), LL(Rp * a),
+                                b2wl.get() + a * k0, LL(ao), 0.0, YW.get(), LL(Rp * a));
+          gw.b_ncontig = true;
+          GemmDesc gv = gemm_nn(LL(Rp * a), LL(a * nk), LL(MV), 1.0, XV.SV[s].get(), LL(Rp * a),
+                                b2vl.get() + a * k0, LL(ao), 0.0, ZV.get(), LL(Rp * a));
+          gv.b_ncontig = true;
+          gemm_both(gw, gv);
           permdot_3el(YW.get(), ZV.get(), LL(Rp), LL(a), LL(nk), two, acc.get(), kE3i);
         }
       }
@@ -1373,14 +1462,13 @@ void form_fock(const FockRequest& rq) {
       // ---- 4-el indirect Fock (four_electron.cpp:181-249)
       if (lead) {
         DevBuf W43(No * ao), V43(No * ao);
-        GemmDesc g = gemm_nn(LL(No), LL(ao), LL(MW), 1.0, b1wl.get(), LL(No), XW.B2[s].get(),
-                             LL(ao), 0.0, W43.get(), LL(No));
-        g.b_ncontig = true;
-        gemm(g);
-        g = gemm_nn(LL(No), LL(ao), LL(MV), 1.0, b1vl.get(), LL(No), XV.B2[s].get(), LL(ao), 0.0,
-                    V43.get(), LL(No));
-        g.b_ncontig = true;
-        gemm(g);
+        GemmDesc gw = gemm_nn(LL(No), LL(ao), LL(MW), 1.0, b1wl.get(), LL(No), XW.B2[s].get(),
+                              LL(ao), 0.0, W43.get(), LL(No));
+        gw.b_ncontig = true;
+        GemmDesc gv = gemm_nn(LL(No), LL(ao), LL(MV), 1.0, b1vl.get(), LL(No), XV.B2[s].get(),
+                              LL(ao), 0.0, V43.get(), LL(No));
+        gv.b_ncontig = true;
+        gemm_both(gw, gv);
         GemmDesc gi = gemm_nn(LL(N), LL(N), LL(a), s_ss * (c > 0 ? -1.0 : -2.0),
                               W43.get() + N * c, LL(No), V43.get() + N * c, LL(N), 1.0,
                               Fp[s], LL(N));
@@ -1437,16 +1525,17 @@ void form_fock(const FockRequest& rq) {
       const size_t n_all = pair_count(a, c, o);
       DevBuf xhW(MW * n_all), xhV(MV * n_all);
       {
-        DevBuf b2p(n_all * std::max(MW, MV));
-        for (const bool is_w : {true, false}) {
-          const IntegralsHandle& X = is_w ? W : V;
-          pack_pairs((is_w ? XW : XV).B2[s].get(), LL(a), LL(c), LL(o), LL(X.n_df), X.lam.get(),
-                     is_w ? 0.5 : 1.0, b2p.get());
-          GemmDesc g = gemm_nn(LL(X.n_df), LL(n_all), LL(X.n_df), 1.0, X.P2.get(), LL(X.n_df),
-                               b2p.get(), LL(n_all), 0.0, (is_w ? xhW : xhV).get(), LL(X.n_df));
-          g.b_ncontig = true;
-          gemm(g);
-        }
+        DevBuf b2p(n_all * (MW + MV));
+        double* b2v = b2p.get() + n_all * MW;
+        pack_pairs(XW.B2[s].get(), LL(a), LL(c), LL(o), LL(MW), W.lam.get(), 0.5, b2p.get());
+        pack_pairs(XV.B2[s].get(), LL(a), LL(c), LL(o), LL(MV), V.lam.get(), 1.0, b2v);
+        GemmDesc gw = gemm_nn(LL(MW), LL(n_all), LL(MW), 1.0, W.P2.get(), LL(MW), b2p.get(),
+                              LL(n_all), 0.0, xhW.get(), LL(MW));
+        gw.b_ncontig = true;
+        GemmDesc gv = gemm_nn(LL(MV), LL(n_all), LL(MV), 1.0, V.P2.get(), LL(MV), b2v, LL(n_all),
+                              0.0, xhV.get(), LL(MV));
+        gv.b_ncontig = true;
+        gemm_both(gw, gv);
       }
       budget = budgets.doubles();
       // unstored W / V blocks (accumulated over, for every k chunk) take at
@@ -1467,6 +1556,7 @@ void form_fock(const FockRequest& rq) {
         size_t k0, nk, p0, n_pairs, nj, i0, i1, n_y;
       };
       const size_t n_s = do_ind && fold && ns == 2 ? 2 : 1;
+      const size_t n_g = joint && fold ? 2 : 1;  // G_V alone, or G_V and G_W at once
       auto pair_chunk = [&](size_t k0, size_t nk) {
         PairChunk q{};
         q.k0 = k0;
@@ -1483,7 +1573,9 @@ void form_fock(const FockRequest& rq) {
       size_t max_pairs = 0, max_y = 0;
       for (size_t k0 = klo; k0 < khi;) {
         PairChunk q = pair_chunk(k0, khi - k0);
-        auto need = [&] { return pair * (q.n_pairs * (1 + n_s) + 2 * q.n_y) + np * q.n_pairs; };
+        auto need = [&] {
+          return pair * (q.n_pairs * (n_g + n_s) + 2 * q.n_y) + np * q.n_pairs * n_g;
+        };
         if (q.nk < o || need() > kavail) {
           const size_t end = k0 < c ? std::min(c, khi) : khi;
           q = pair_chunk(k0, end - k0);
@@ -1495,7 +1587,7 @@ void form_fock(const FockRequest& rq) {
         k0 += q.nk;
       }
       const size_t nbuf = pair * max_pairs;
-      DevBuf gpk(np * max_pairs), bufG(nbuf), bufS(nbuf * n_s), bufY(pair * max_y),
+      DevBuf gpk(np * max_pairs * n_g), bufG(nbuf * n_g), bufS(nbuf * n_s), bufY(pair * max_y),
           bufZ(pair * max_y), scrX, scrXr;
       // dst = G_X of the chunk's pairs, over X's aux blocks
       auto form_g = [&](const IntegralsHandle& X, const double* xh, const PairChunk& q,
@@ -1521,21 +1613,42 @@ void form_fock(const FockRequest& rq) {
           gemm(gr);
         }
       };
-      // dst = St[j] L B1[k]^T of the chunk, both blocks (St: R' a x M)
+      // G_V of the chunk's pairs and G_W behind it (stored integrals)
+      auto form_g_both = [&](const PairChunk& q, double* dst) {
+        auto ao_rows = [&](const IntegralsHandle& X, const double* xh, size_t at) {
+          return gemm_nn(LL(np), LL(q.n_pairs), LL(X.n_df), 1.0, X.J3_0.get(), LL(np),
+                         xh + X.n_df * q.p0, LL(X.n_df), 0.0, gpk.get() + np * at, LL(np));
+        };
+        auto ri_rows = [&](const IntegralsHandle& X, const double* xh, double* to) {
+          GemmDesc gr = gemm_nn(LL(R), LL(q.n_pairs), LL(X.n_df), 1.0, X.J3_ri_0.get(), LL(R * N),
+                                xh + X.n_df * q.p0, LL(X.n_df), 0.0, to + N, LL(pair));
+          gr.nbo1 = LL(N);
+          gr.sAo1 = LL(R);
+          gr.sCo1 = LL(Rp);
+          return gr;
+        };
+        gemm_both(ao_rows(V, xhV.get(), 0), ao_rows(W, xhW.get(), q.n_pairs));
+        unpack_sym(gpk.get(), LL(np), LL(N), LL(2 * q.n_pairs), dst, LL(Rp), LL(pair));
+        gemm_both(ri_rows(V, xhV.get(), dst), ri_rows(W, xhW.get(), dst + pair * q.n_pairs));
+      };
+      // block 0 (Y[j, k]) or 1 (the mirror images behind them) of dst = St[j] L B1[k]^T of
+      // the chunk (St: R' a x M)
+      auto y_block = [&](int b, const double* St, const double* b1l, size_t M,
+                         const PairChunk& q, double* dst) {
+        const size_t j0 = b ? q.i0 : 0, nj = b ? q.i1 - q.i0 : q.nj;
+        const size_t k0 = b ? c : q.k0, nk = b ? q.i0 : q.nk;
+        GemmDesc gy = gemm_nn(LL(Rp), LL(N * nk), LL(M), 1.0, St + Rp * j0, LL(Rp * a),
+                              b1l + N * k0, LL(No), 0.0, dst + (b ? pair * q.nk * q.nj : 0),
+                              LL(Rp));
+        gy.b_ncontig = true;
+        gy.nbo1 = LL(nj);
+        gy.sAo1 = LL(Rp);
+        gy.sCo1 = LL(pair * nk);
+        return gy;
+      };
       auto form_y = [&](const double* St, const double* b1l, size_t M, const PairChunk& q,
                         double* dst) {
-        auto block = [&](size_t j0, size_t nj, size_t k0, size_t nk, double* to) {
-          if (nj == 0 || nk == 0) return;
-          GemmDesc gy = gemm_nn(LL(Rp), LL(N * nk), LL(M), 1.0, St + Rp * j0, LL(Rp * a),
-                                b1l + N * k0, LL(No), 0.0, to, LL(Rp));
-          gy.b_ncontig = true;
-          gy.nbo1 = LL(nj);
-          gy.sAo1 = LL(Rp);
-          gy.sCo1 = LL(pair * nk);
-          gemm(gy);
-        };
-        block(0, q.nj, q.k0, q.nk, dst);
-        block(q.i0, q.i1 - q.i0, c, q.i0, dst + pair * q.nk * q.nj);
+        for (int b = 0; b < (q.i0 ? 2 : 1); ++b) gemm(y_block(b, St, b1l, M, q, dst));
       };
       // out = coef (Y[j, k] + Y[i, c + j]) + coef_s S per pair; the sum is scaled by
       // mirror where it has two terms
@@ -1580,12 +1693,21 @@ void form_fock(const FockRequest& rq) {
         add(i0, Yw + pair * first, 1, nk, Z + back, i0, 1);
       };
       for (const PairChunk& q : chunks) {
-        form_g(V, xhV.get(), q, bufG.get());
+        const bool both = n_g == 2;
+        const double* gw = bufG.get() + (both ? pair * q.n_pairs : 0);  // G_W
+        if (both)
+          form_g_both(q, bufG.get());
+        else
+          form_g(V, xhV.get(), q, bufG.get());
+        if (both && do_ind)
+          for (int b = 0; b < (q.i0 ? 2 : 1); ++b)
+            gemm_both(y_block(b, XW.Wst[s].get(), b1wl.get(), MW, q, bufY.get()),
+                      y_block(b, XV.SV[s].get(), b1vl.get(), MV, q, bufZ.get()));
         if (fold) {
           gemm(gemm_nn(LL(Rp), LL(N * q.n_pairs), LL(Rp), 1.0, AB.Sinv.get(), LL(Rp), bufG.get(),
                        LL(Rp), 0.0, bufS.get(), LL(Rp)));
           if (do_ind) {
-            form_y(XW.Wst[s].get(), b1wl.get(), MW, q, bufY.get());
+            if (!both) form_y(XW.Wst[s].get(), b1wl.get(), MW, q, bufY.get());
             sum_y(q, bufY.get(), 1.0, 0.5, nullptr, 0.0, bufG.get());
             add_pairs(s_ss, bufS.get(), bufG.get(), q.n_pairs, Fp[s]);
           }
@@ -1595,9 +1717,9 @@ void form_fock(const FockRequest& rq) {
           add_pairs(s_ss, bufG.get(), bufS.get(), q.n_pairs, Fp[s]);
           if (q.i1 > q.i0) form_y(XW.Wst[s].get(), b1wl.get(), MW, q, bufY.get());
         }
-        form_g(W, xhW.get(), q, bufG.get());
+        if (!both) form_g(W, xhW.get(), q, bufG.get());
         if (do_ind) {
-          form_y(XV.SV[s].get(), b1vl.get(), MV, q, bufZ.get());
+          if (!both) form_y(XV.SV[s].get(), b1vl.get(), MV, q, bufZ.get());
           k_term(q, bufY.get(), bufZ.get());
         }
         if (!fold) {
@@ -1606,13 +1728,13 @@ void form_fock(const FockRequest& rq) {
         } else if (ns == 1) {
           // one product for t~ dX and the same-spin term: G_W^T (s_ss S^-1 Y_V - cD S^-1 G_V)
           if (do_ind) sum_y(q, bufZ.get(), s_ss, 1.0, bufS.get(), -cD[0], bufS.get());
-          add_pairs(do_ind ? 1.0 : -cD[0], bufG.get(), bufS.get(), q.n_pairs, Fp[s]);
+          add_pairs(do_ind ? 1.0 : -cD[0], gw, bufS.get(), q.n_pairs, Fp[s]);
         } else {
           // D and the same-spin term G_W^T S^-1 Y_V in one launch, G_W read once
           if (do_ind) sum_y(q, bufZ.get(), 1.0, 1.0, nullptr, 0.0, bufS.get() + nbuf);
           DevBuf D(2 * N * N);
-          GemmDesc gd = gemm_nn(LL(N), LL(N), LL(Rp), 1.0, bufG.get(), LL(Rp), bufS.get(), LL(Rp),
-                                0.0, D.get(), LL(N));
+          GemmDesc gd = gemm_nn(LL(N), LL(N), LL(Rp), 1.0, gw, LL(Rp), bufS.get(), LL(Rp), 0.0,
+                                D.get(), LL(N));
           gd.a_kcontig = true;
           gd.nbr1 = LL(q.n_pairs);
           gd.sAr1 = LL(pair);
