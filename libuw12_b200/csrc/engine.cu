@@ -588,8 +588,8 @@ constexpr size_t kJointDoubles = size_t(1) << 24;
 
 // The same product for W and for V.  Small ones are bound by their launch and the
 // latency of a k tile, so equal shapes run as two output batches of one launch, the
-// batch strides being the distances between the operands (one B200, N=24 Fock 310 -> 270 us, open-shell energy at N=61 257 ->
-// 231 us, N=120 Fock 2.38 -> 2.33 ms); larger
+// batch strides being the distances between the operands (one B200, N=24 Fock 310 ->
+// 270 us, open-shell energy at N=61 257 -> 231 us, N=120 Fock 2.38 -> 2.33 ms); larger
 // ones fill the device by themselves, and split precision prepares its operands one by
 // one.
 void gemm_both(const GemmDesc& w, const GemmDesc& v) {
@@ -1433,24 +1433,35 @@ void form_fock(const FockRequest& rq) {
         permdot_4el(W4.get(), V4.get(), LL(a), LL(o), -0.5 * two, acc.get(), kE4i);
       }
       clock.mark("ss_3el_energy");
-      // ---- 3-el indirect energy (indirect_utils.cpp:101-133), chunked over k
+      // ---- 3-el indirect energy (indirect_utils.cpp:101-133), chunked over k, YW and ZV
+      // formed once per pair of a chunk (B2 is symmetric in the active pair): N=300 Fock
+      // 129.5 -> 125.9 ms
       {
         budget = budgets.doubles();
-        const size_t per_k = 2 * Rp * a * a;
+        const size_t per_k = 2 * Rp * a * a + a * (MW + MV);
         const auto [klo, khi] = part(o);
         const size_t kc = tile_chunk(khi - klo, a,
                                      std::max<size_t>(1, std::min(khi - klo, budget / per_k)));
-        DevBuf YW(Rp * a * a * kc), ZV(Rp * a * a * kc);
+        DevBuf YW, ZV, b2p;
         for (size_t k0 = klo; k0 < khi; k0 += kc) {
-          const size_t nk = std::min(kc, khi - k0);
-          GemmDesc gw = gemm_nn(LL(Rp * a), LL(a * nk), LL(MW), 1.0, XW.Wst[s].get(), LL(Rp * a),
-                                b2wl.get() + a * k0, LL(ao), 0.0, YW.get(), LL(Rp * a));
+          const PairColumns q = PairColumns::of(LL(a), LL(c), LL(k0), LL(std::min(kc, khi - k0)));
+          const size_t n = static_cast<size_t>(q.count());
+          if (YW.size() < Rp * a * n) {
+            YW.alloc(Rp * a * n);
+            ZV.alloc(Rp * a * n);
+            b2p.alloc(n * (MW + MV));
+          }
+          double* b2v = b2p.get() + n * MW;
+          pack_pairs(XW.B2[s].get(), q, LL(o), LL(MW), W.lam.get(), 0.5, b2p.get());
+          pack_pairs(XV.B2[s].get(), q, LL(o), LL(MV), V.lam.get(), 0.5, b2v);
+          GemmDesc gw = gemm_nn(LL(Rp * a), LL(n), LL(MW), 1.0, XW.Wst[s].get(), LL(Rp * a),
+                                b2p.get(), LL(n), 0.0, YW.get(), LL(Rp * a));
           gw.b_ncontig = true;
-          GemmDesc gv = gemm_nn(LL(Rp * a), LL(a * nk), LL(MV), 1.0, XV.SV[s].get(), LL(Rp * a),
-                                b2vl.get() + a * k0, LL(ao), 0.0, ZV.get(), LL(Rp * a));
+          GemmDesc gv = gemm_nn(LL(Rp * a), LL(n), LL(MV), 1.0, XV.SV[s].get(), LL(Rp * a), b2v,
+                                LL(n), 0.0, ZV.get(), LL(Rp * a));
           gv.b_ncontig = true;
           gemm_both(gw, gv);
-          permdot_3el(YW.get(), ZV.get(), LL(Rp), LL(a), LL(nk), two, acc.get(), kE3i);
+          permdot_3el(YW.get(), ZV.get(), LL(Rp), q, two, acc.get(), kE3i);
         }
       }
       if (!calc) continue;
@@ -1527,8 +1538,9 @@ void form_fock(const FockRequest& rq) {
       {
         DevBuf b2p(n_all * (MW + MV));
         double* b2v = b2p.get() + n_all * MW;
-        pack_pairs(XW.B2[s].get(), LL(a), LL(c), LL(o), LL(MW), W.lam.get(), 0.5, b2p.get());
-        pack_pairs(XV.B2[s].get(), LL(a), LL(c), LL(o), LL(MV), V.lam.get(), 1.0, b2v);
+        const PairColumns all = PairColumns::of(LL(a), LL(c), 0, LL(o));
+        pack_pairs(XW.B2[s].get(), all, LL(o), LL(MW), W.lam.get(), 0.5, b2p.get());
+        pack_pairs(XV.B2[s].get(), all, LL(o), LL(MV), V.lam.get(), 1.0, b2v);
         GemmDesc gw = gemm_nn(LL(MW), LL(n_all), LL(MW), 1.0, W.P2.get(), LL(MW), b2p.get(),
                               LL(n_all), 0.0, xhW.get(), LL(MW));
         gw.b_ncontig = true;
@@ -2120,39 +2132,51 @@ void form_fock_adjoint(const FockRequest& rq_in, const AdjointOutputs& out) {
       // three-electron, chunks of occupied orbitals k
       {
         budget = budgets.doubles();
-        const size_t per_k = 3 * Ra * a + a * std::max(MW, MV);
+        const size_t per_k = 3 * Ra * a + 2 * a * std::max(MW, MV);
         const size_t kc = tile_chunk(o, a, std::max<size_t>(1, std::min(o, budget / per_k)));
-        DevBuf TY(Ra * MW), TZ(Ra * MV), Tmp(Ra * a * kc), GY(Ra * a * kc), GZ(Ra * a * kc),
-            Bt(a * kc * std::max(MW, MV));
+        const size_t c = o - a;
+        // pairs of the largest chunk: fewer than a per orbital, and for whole sets half
+        size_t most = 0;
+        for (size_t k0 = 0; k0 < o; k0 += kc)
+          most = std::max(most, static_cast<size_t>(PairColumns::of(LL(a), LL(c), LL(k0),
+                                                                    LL(std::min(kc, o - k0)))
+                                                        .count()));
+        DevBuf TY(Ra * MW), TZ(Ra * MV), Tmp(Ra * most), GY(Ra * most), GZ(Ra * most),
+            Bt(most * std::max(MW, MV)), b2p(most * std::max(MW, MV));
+        // B2 is symmetric in the active pair, and so are the gradients that matter: a pair
+        // of a chunk is formed once, G_Y and G_Z sum its two orders, and B2-bar of both
+        // is half of the product (one B200, with the energy's: open shell N=200, M=600,
+        // R=800, o=16/15 44.1 -> 42.7 ms, N=300, M=900, R=1200, o=30 in split precision
+        // 103.0 -> 99.7)
         for (size_t k0 = 0; k0 < o; k0 += kc) {
-          const size_t nk = std::min(kc, o - k0);
           const double beta = k0 ? 1.0 : 0.0;
-          GemmDesc g = gemm_nn(LL(Ra), LL(a * nk), LL(MV), 1.0, XV.SW[s].get(), LL(Ra),
-                               b2vl.get() + a * k0, LL(ao), 0.0, Tmp.get(), LL(Ra));
-          g.b_ncontig = true;
-          gemm(g);
-          perm_3el(Tmp.get(), GY.get(), LL(Rp), LL(a), LL(nk), gs);
-          g = gemm_nn(LL(Ra), LL(a * nk), LL(MW), 1.0, XW.Wst[s].get(), LL(Ra),
-                      b2wl.get() + a * k0, LL(ao), 0.0, Tmp.get(), LL(Ra));
-          g.b_ncontig = true;
-          gemm(g);
-          perm_3el(Tmp.get(), GZ.get(), LL(Rp), LL(a), LL(nk), gs);
-          gemm(gemm_nn(LL(Ra), LL(MW), LL(a * nk), 1.0, GY.get(), LL(Ra),
-                       XW.B2[s].get() + a * k0, LL(ao), beta, TY.get(), LL(Ra)));
-          gemm(gemm_nn(LL(Ra), LL(MV), LL(a * nk), 1.0, GZ.get(), LL(Ra),
-                       XV.B2[s].get() + a * k0, LL(ao), beta, TZ.get(), LL(Ra)));
-          g = gemm_nn(LL(a * nk), LL(MW), LL(Ra), 1.0, GY.get(), LL(Ra), XW.Wst[s].get(),
-                      LL(Ra), 0.0, Bt.get(), LL(a * nk));
-          g.a_kcontig = true;
-          gemm(g);
-          scale_rc(Bt.get(), LL(a * nk), LL(a * nk), LL(MW), nullptr, W.lam.get(), 1.0,
-                   ssB2b[0][s].get() + a * k0, LL(ao));
-          g = gemm_nn(LL(a * nk), LL(MV), LL(Ra), 1.0, GZ.get(), LL(Ra), XV.SW[s].get(), LL(Ra),
-                      0.0, Bt.get(), LL(a * nk));
-          g.a_kcontig = true;
-          gemm(g);
-          scale_rc(Bt.get(), LL(a * nk), LL(a * nk), LL(MV), nullptr, V.lam.get(), 1.0,
-                   ssB2b[1][s].get() + a * k0, LL(ao));
+          const PairColumns q = PairColumns::of(LL(a), LL(c), LL(k0), LL(std::min(kc, o - k0)));
+          const long long n = q.count();
+          for (const bool is_w : {false, true}) {  // ZV and G_Y, then YW and G_Z
+            const IntegralsHandle& X = is_w ? W : V;
+            const double* St = is_w ? XW.Wst[s].get() : XV.SW[s].get();
+            pack_pairs((is_w ? XW : XV).B2[s].get(), q, LL(o), LL(X.n_df), X.lam.get(), 0.5,
+                       b2p.get());
+            GemmDesc g = gemm_nn(LL(Ra), n, LL(X.n_df), 1.0, St, LL(Ra), b2p.get(), n, 0.0,
+                                 Tmp.get(), LL(Ra));
+            g.b_ncontig = true;
+            gemm(g);
+            perm_3el(Tmp.get(), (is_w ? GZ : GY).get(), LL(Rp), q, gs);
+          }
+          for (const bool is_w : {true, false}) {
+            const IntegralsHandle& X = is_w ? W : V;
+            const double* St = is_w ? XW.Wst[s].get() : XV.SW[s].get();
+            const double* G = (is_w ? GY : GZ).get();
+            pack_pairs((is_w ? XW : XV).B2[s].get(), q, LL(o), LL(X.n_df), nullptr, 0.5, b2p.get());
+            gemm(gemm_nn(LL(Ra), LL(X.n_df), n, 1.0, G, LL(Ra), b2p.get(), n, beta,
+                         (is_w ? TY : TZ).get(), LL(Ra)));
+            GemmDesc g = gemm_nn(n, LL(X.n_df), LL(Ra), 1.0, G, LL(Ra), St, LL(Ra), 0.0, Bt.get(),
+                                 n);
+            g.a_kcontig = true;
+            gemm(g);
+            unpack_pairs(Bt.get(), q, LL(o), LL(X.n_df), X.lam.get(), 0.5,
+                         ssB2b[is_w ? 0 : 1][s].get());
+          }
         }
         Tmp = DevBuf();  // the chunk buffers are done: their memory goes to Wst-bar
         GY = DevBuf();

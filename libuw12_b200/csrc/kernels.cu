@@ -203,22 +203,21 @@ __global__ void k_permdot_4el(const double* X, const double* Y,
 }
 
 // One warp per (i, j, k) triple, summing the contiguous p index.
-__global__ void k_permdot_3el(const double* Yw, const double* Zv,
-                              long long rp, long long a, long long kc, double* partials,
-                              double coef, double* acc, int slot) {
+__global__ void k_permdot_3el(const double* Yw, const double* Zv, long long rp, PairColumns q,
+                              double* partials, double coef, double* acc, int slot) {
   chain_wait();
-  const long long triples = a * a * kc;
+  const long long triples = q.a * q.a * q.nk;
   const int lane = threadIdx.x & 31;
   const long long warp_global = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-  const long long ra = rp * a;
+  const long long ra = rp * q.a;
   double s = 0.0;
   for (long long tix = warp_global; tix < triples; tix += nwarps) {
-    const long long i = tix % a;
-    const long long rest = tix / a;
-    const long long j = rest % a, k = rest / a;
-    const double* y = Yw + rp * i + ra * (j + a * k);
-    const double* z = Zv + rp * j + ra * (i + a * k);
+    const long long i = tix % q.a;
+    const long long rest = tix / q.a;
+    const long long j = rest % q.a, k = q.k0 + rest / q.a;
+    const double* y = Yw + rp * i + ra * q.column(j, k);
+    const double* z = Zv + rp * j + ra * q.column(i, k);
     for (long long p = lane; p < rp; p += 32) s += y[p] * z[p];
   }
   finish_reduction(s, partials, coef, acc, slot);
@@ -354,25 +353,29 @@ __device__ __forceinline__ void triangle_index(long long q, long long& i, long l
 // x^ of orbital pairs before the metric: a few MB at most, one block per pair so
 // that the pair is found once; its strided reads of B2 are shared in L2 by the
 // neighbouring pairs' blocks.
-__global__ void k_pack_pairs(const double* B2, long long a, long long c, long long o, long long m,
+__global__ void k_pack_pairs(const double* B2, PairColumns q, long long o, long long m,
                              const double* r, double h, double* out) {
   chain_wait();
-  const long long p = blockIdx.x, n = gridDim.x, ao = a * o;
-  long long j, k, mirror = -1;
-  if (p < a * c) {
-    k = p / a;
-    j = p - a * k;
-  } else {
-    long long i;
-    triangle_index(p - a * c, i, j);
-    k = c + i;
-    if (j != i) mirror = i + a * (c + j);
-  }
+  const long long k = q.k0 + blockIdx.x / q.a, j = blockIdx.x % q.a, ao = q.a * o;
+  const bool both = q.mirrored(j, k);
+  if (both && j > k - q.c) return;  // the pair's other block writes it
+  const long long p = q.column(j, k), n = q.count();
+  const long long mirror = both ? k - q.c + q.a * (q.c + j) : 0;
   for (long long A = threadIdx.x; A < m; A += blockDim.x) {
-    double v = B2[j + a * k + ao * A];
-    if (mirror >= 0) v = h * (v + B2[mirror + ao * A]);
-    out[p + n * A] = r[A] * v;
+    double v = B2[j + q.a * k + ao * A];
+    if (both) v = h * (v + B2[mirror + ao * A]);
+    out[p + n * A] = r ? r[A] * v : v;
   }
+}
+
+__global__ void k_unpack_pairs(const double* X, PairColumns q, long long o, long long m,
+                               const double* r, double h, double* out) {
+  chain_wait();
+  const long long k = q.k0 + blockIdx.x / q.a, j = blockIdx.x % q.a, ao = q.a * o;
+  const double f = q.mirrored(j, k) ? h : 1.0;
+  const long long p = q.column(j, k), n = q.count();
+  for (long long A = threadIdx.x; A < m; A += blockDim.x)
+    out[j + q.a * k + ao * A] = f * (r ? r[A] : 1.0) * X[p + n * A];
 }
 
 struct PairRange {
@@ -460,23 +463,18 @@ __global__ void k_pack_sym_sum(const double* G, I n, I np, I total, double* out,
   }
 }
 
-// out[p + rp*i + rp*a*(j + a*kk)] = alpha * Z[p + rp*j + rp*a*(i + a*kk)]:
-// the two active-orbital indices of the same-spin three-electron products
-// exchanged (the permutation under which YW and ZV are contracted).
-template <typename I>
-__global__ void k_perm_3el(const double* Z, double* out,
-                           long long rp, long long a, long long kc, double alpha) {
+// Pairs and active orbitals i by block, so that no element divides; bound by HBM.
+__global__ void __launch_bounds__(kT) k_perm_3el(const double* Z, double* out, long long rp,
+                                                 PairColumns q, double alpha) {
   chain_wait();
-  const I nr = static_cast<I>(rp), na = static_cast<I>(a);
-  const I total = nr * na * na * static_cast<I>(kc);
-  for (I idx = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; idx < total;
-       idx += static_cast<I>(gridDim.x) * blockDim.x) {
-    I t = idx / nr;
-    const I p = idx - t * nr;
-    const I t1 = t / na, i = t - t1 * na;
-    const I kk = t1 / na, j = t1 - kk * na;
-    out[idx] = alpha * Z[p + rp * (j + a * (i + a * static_cast<long long>(kk)))];
-  }
+  const long long i = blockIdx.x % q.a, t = blockIdx.x / q.a;
+  const long long k = q.k0 + t / q.a, j = t % q.a, ra = rp * q.a;
+  const bool both = q.mirrored(j, k);
+  if (both && j > k - q.c) return;  // the pair's other blocks write it
+  const double* z = Z + rp * j + ra * q.column(i, k);
+  const double* w = both ? Z + rp * (k - q.c) + ra * q.column(i, q.c + j) : nullptr;
+  double* d = out + rp * i + ra * q.column(j, k);
+  for (long long p = threadIdx.x; p < rp; p += kT) d[p] = alpha * (w ? z[p] + w[p] : z[p]);
 }
 
 // out[i + a*l + ao*(j + a*k)] = alpha * V[i + a*k + ao*(j + a*l)], ao = a*o:
@@ -618,14 +616,14 @@ void permdot_4el(const double* X, const double* Y, long long a, long long o, dou
   UW12_LAUNCHED();
 }
 
-void permdot_3el(const double* Y, const double* Z, long long rp, long long a, long long kc,
+void permdot_3el(const double* Y, const double* Z, long long rp, const PairColumns& q,
                  double coef, double* acc, int slot) {
-  const long long triples = a * a * kc;
+  const long long triples = q.a * q.a * q.nk;
   if (triples <= 0 || rp <= 0 || coef == 0.0) return;
   cudaStream_t s = current_stream();
   const int blocks = grid_for(triples * 32, 8);
   DevBuf part(blocks, s);
-  launch_chained(k_permdot_3el, blocks, kT, 0, s, Y, Z, rp, a, kc, part.get(), coef, acc, slot);
+  launch_chained(k_permdot_3el, blocks, kT, 0, s, Y, Z, rp, q, part.get(), coef, acc, slot);
   UW12_LAUNCHED();
 }
 
@@ -694,12 +692,24 @@ void lincomb(double* Y, long long m, long long n, int nt, const double* const* m
   UW12_LAUNCHED();
 }
 
-void pack_pairs(const double* B2, long long a, long long c, long long o, long long m,
-                const double* r, double h, double* out) {
-  const long long n = a * c + (o - c) * (o - c + 1) / 2;
-  if (n <= 0 || m <= 0) return;
-  launch_chained(k_pack_pairs, static_cast<unsigned>(n), kT, 0, current_stream(), B2, a, c, o, m, r,
-                 h, out);
+// blocks of a kernel with one per (j, k) of the range, times `each`
+static unsigned pair_blocks(const PairColumns& q, long long each) {
+  const long long n = q.a * q.nk * each;
+  if (n >= (1LL << 31)) throw Error(kErrInvalid, "too many orbital pairs for one launch");
+  return static_cast<unsigned>(n);
+}
+
+void pack_pairs(const double* B2, const PairColumns& q, long long o, long long m, const double* r,
+                double h, double* out) {
+  if (q.a * q.nk <= 0 || m <= 0) return;
+  launch_chained(k_pack_pairs, pair_blocks(q, 1), kT, 0, current_stream(), B2, q, o, m, r, h, out);
+  UW12_LAUNCHED();
+}
+
+void unpack_pairs(const double* X, const PairColumns& q, long long o, long long m, const double* r,
+                  double h, double* out) {
+  if (q.a * q.nk <= 0 || m <= 0) return;
+  launch_chained(k_unpack_pairs, pair_blocks(q, 1), kT, 0, current_stream(), X, q, o, m, r, h, out);
   UW12_LAUNCHED();
 }
 
@@ -745,16 +755,9 @@ void pack_sym_sum(const double* G, long long n, long long na, double* out, long 
   UW12_LAUNCHED();
 }
 
-void perm_3el(const double* Z, double* out, long long rp, long long a, long long kc,
-              double alpha) {
-  const long long total = rp * a * a * kc;
-  if (total <= 0) return;
-  if (small_index(total))
-    launch_chained(k_perm_3el<unsigned>, grid_for(total), kT, 0, current_stream(), Z, out, rp, a,
-                   kc, alpha);
-  else
-    launch_chained(k_perm_3el<long long>, grid_for(total), kT, 0, current_stream(), Z, out, rp, a,
-                   kc, alpha);
+void perm_3el(const double* Z, double* out, long long rp, const PairColumns& q, double alpha) {
+  if (rp <= 0 || q.a * q.nk <= 0) return;
+  launch_chained(k_perm_3el, pair_blocks(q, q.a), kT, 0, current_stream(), Z, out, rp, q, alpha);
   UW12_LAUNCHED();
 }
 

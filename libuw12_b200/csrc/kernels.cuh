@@ -28,6 +28,45 @@ void copy3d(const double* src, long long s1, long long s2, double* dst, long lon
             long long d2, long long n0, long long n1, long long n2, double alpha = 1.0,
             double beta = 0.0);
 
+// The distinct pairs (j, k) of a active orbitals j and the occupied orbitals k of
+// [k0, k0 + nk), c of the occupied orbitals being core: (j, c + i) and (i, c + j) are one
+// pair.  In column order: the range's core orbitals k ascending, j ascending within them;
+// the range's active orbitals i0 + i with those up to themselves, triangle
+// i (i + 1) / 2 + j - i0; then those with the active orbitals outside the range.  For a range
+// from 0 to k this is the order of all pairs with j <= i.
+struct PairColumns {
+  long long a, c, k0, nk, nc, i0, ni;  // nc core, ni active orbitals of the range from i0
+
+  __host__ __device__ static PairColumns of(long long a, long long c, long long k0, long long nk) {
+    PairColumns q{};
+    const long long k1 = k0 + nk;
+    q.a = a;
+    q.c = c;
+    q.k0 = k0;
+    q.nk = nk;
+    q.nc = (k1 < c ? k1 : c) > k0 ? (k1 < c ? k1 : c) - k0 : 0;
+    q.i0 = k0 > c ? k0 - c : 0;
+    q.ni = (k1 > c ? k1 - c : 0) - q.i0;
+    return q;
+  }
+  __host__ __device__ long long count() const {
+    return a * nc + ni * (ni + 1) / 2 + (a - ni) * ni;
+  }
+  // whether (j, k) and its mirror image are two entries of the range
+  __host__ __device__ bool mirrored(long long j, long long k) const {
+    return k >= c && j >= i0 && j < i0 + ni && j != k - c;
+  }
+  __host__ __device__ long long column(long long j, long long k) const {
+    if (k < c) return j + a * (k - k0);
+    const long long i = k - c - i0, t = j - i0;
+    if (t >= 0 && t < ni) {
+      const long long hi = t > i ? t : i, lo = t > i ? i : t;
+      return a * nc + hi * (hi + 1) / 2 + lo;
+    }
+    return a * nc + ni * (ni + 1) / 2 + (t < 0 ? j : j - ni) + (a - ni) * i;
+  }
+};
+
 // Sums of wdot, permdot_4el and permdot_3el: acc is a device array of
 // kAccDoubles, zeroed before its first use; slots below kAccSlots hold sums, the
 // last double is the ticket of the reductions' last block.
@@ -44,10 +83,10 @@ void wdot(const double* x, long long ldx, const double* y, long long ldy, long l
 void permdot_4el(const double* X, const double* Y, long long a, long long o, double coef,
                  double* acc, int slot);
 
-// acc[slot] += coef * sum_{p<rp; i,j<a; k in [k0,k1)} Y[p + rp*i + rp*a*(j + a*(k-k0))]
-//                                                   * Z[p + rp*j + rp*a*(i + a*(k-k0))]
-// the same-spin three-electron energy.
-void permdot_3el(const double* Y, const double* Z, long long rp, long long a, long long kc,
+// acc[slot] += coef * sum_{p<rp; i,j<a; k of q} Y[p + rp*i + rp*a*col(j, k)]
+//                                             * Z[p + rp*j + rp*a*col(i, k)]
+// (Y, Z rp*a x q.count()): the same-spin three-electron energy.
+void permdot_3el(const double* Y, const double* Z, long long rp, const PairColumns& q,
                  double coef, double* acc, int slot);
 
 // F[i + ld*j] = 0.5 * (G[i + ldg*j] + G[j + ldg*i]) written into column-block
@@ -82,24 +121,26 @@ void lincomb(double* Y, long long m, long long n, int nt, const double* const* m
 void pack_sym_sum(const double* G, long long n, long long na, double* out, long long ldo,
                   double beta = 0.0);
 
-// out[p + rp*i + rp*a*(j + a*k)] = alpha * Z[p + rp*j + rp*a*(i + a*k)] for
-// p < rp, i, j < a, k < kc: the active-orbital pair of a same-spin
-// three-electron product (YW or ZV, rp*a x a*kc) exchanged; out and Z distinct.
-void perm_3el(const double* Z, double* out, long long rp, long long a, long long kc,
-              double alpha);
+// out[p + rp*i + rp*a*col(j, k)] = alpha * (Z[p + rp*j + rp*a*col(i, k)] + the mirror
+// image's) for p < rp, i < a and the pairs (j, k) of q: the active-orbital pair of a
+// same-spin three-electron product (YW or ZV, rp*a x q.count()) exchanged and summed over
+// both orders; out and Z distinct.
+void perm_3el(const double* Z, double* out, long long rp, const PairColumns& q, double alpha);
 
 // out[i + a*l + ao*(j + a*k)] = alpha * V[i + a*k + ao*(j + a*l)], ao = a*o:
 // the occupied indices of an (ik|jl) matrix (ao x ao) exchanged between rows
 // and columns; out and V distinct.
 void perm_4el(const double* V, double* out, long long a, long long o, double alpha);
 
-// Pair order (a active, c core, o = a + c occupied orbitals): occupied k ascending, within
-// it active j ascending, every j for a core k and j <= i for the active k = c + i.
-// out[p, A] (contiguous, all pairs x m) = r_A B2[j + a k, A], and where the mirror image
-// (i, c + j) is another entry, r_A h (B2[j + a k, A] + B2[i + a (c + j), A]);
-// B2 is (a o) x m.
-void pack_pairs(const double* B2, long long a, long long c, long long o, long long m,
-                const double* r, double h, double* out);
+// out[col, A] (contiguous, q.count() x m) = r_A B2[j + a k, A] and, for mirrored pairs,
+// r_A h (B2[j + a k, A] + B2[i + a (c + j), A]); B2 is (a o) x m, r may be null (ones).
+void pack_pairs(const double* B2, const PairColumns& q, long long o, long long m, const double* r,
+                double h, double* out);
+
+// out[j + a k, A] = r_A h X[col, A] for mirrored pairs, r_A X[col, A] for the others, for
+// every j and the range's k (out (a o) x m, X q.count() x m).
+void unpack_pairs(const double* X, const PairColumns& q, long long o, long long m, const double* r,
+                  double h, double* out);
 
 // out[p] = coef (Y[j, k] + mirror image) + coef_s S[p] for the pairs of the occupied
 // orbitals [k0, k0 + nk), matrices of `size` elements; where there is a mirror image the
