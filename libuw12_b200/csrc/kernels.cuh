@@ -142,9 +142,10 @@ void pack_pairs(const double* B2, const PairColumns& q, long long o, long long m
 void unpack_pairs(const double* X, const PairColumns& q, long long o, long long m, const double* r,
                   double h, double* out);
 
-// out[p] = coef (Y[j, k] + mirror image) + coef_s S[p] for the pairs of the occupied
-// orbitals [k0, k0 + nk), matrices of `size` elements; where there is a mirror image the
-// sum of both is scaled by h.  Y[j, k] is matrix (k - k0) + nk j of Y, the mirror
+// out[p] = coef (Y[j, k] + mirror image) + coef_s S[p], matrices of `size` elements, for the
+// n_pairs pairs of the occupied orbitals [k0, k0 + nk) in the order of all pairs (every j for a
+// core orbital k, j <= i for k = c + i); where there is a mirror image the sum of both is
+// scaled by h.  Y[j, k] is matrix (k - k0) + nk j of Y, the mirror
 // image Y[i, c + j] too where c + j >= k0, matrix j + i0 (i - i0) of Y2 before it (c + i0 the
 // first active orbital of the range).  S may be null, or out itself.
 void sum_pairs(const double* Y, const double* Y2, long long size, long long a, long long c,
