@@ -1218,15 +1218,23 @@ void form_fock(const FockRequest& rq) {
     scale_rc(tab[s].get(), LL(MW), LL(MW), LL(MV), W.lam.get(), V.lam.get(), 1.0, ttl[s].get(),
              LL(MW));
   }
-  for (int s = 0; s < ns && lead; ++s)
-    for (int sp = 0; sp < ns; ++sp) {
-      const double f = spin_factor(ns, s, sp, s_os, s_ss);
-      wdot(Xab[s].get(), LL(MW), ttl[sp].get(), LL(MW), LL(MW), LL(MV), nullptr, nullptr, -f,
-           acc.get(), kE3d);
-      if (f != 0.0)
-        wdot(ttl[sp].get(), LL(MW), tab[s].get(), LL(MW), LL(MW), LL(MV), nullptr, nullptr,
-             0.5 * f, acc.get(), kE4d);
+  if (lead) {
+    const double* X[2] = {};
+    const double* t[2] = {};
+    const double* T[2] = {};
+    double cx[4] = {}, ct[4] = {};
+    for (int s = 0; s < ns; ++s) {
+      X[s] = Xab[s].get();
+      t[s] = tab[s].get();
+      T[s] = ttl[s].get();
+      for (int sp = 0; sp < ns; ++sp) {
+        const double f = spin_factor(ns, s, sp, s_os, s_ss);
+        cx[s + 2 * sp] = -f;
+        ct[s + 2 * sp] = 0.5 * f;
+      }
     }
+    spin_dots(X, t, T, ns, LL(MW * MV), cx, ct, acc.get(), kE3d, kE4d);
+  }
   if (!do_ind && !orbital_chunked)  // the stacked transforms serve only X_AB and the same-spin terms
     for (int s = 0; s < ns; ++s) {
       XW.Wst[s].release();

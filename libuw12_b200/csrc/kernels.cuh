@@ -78,6 +78,12 @@ constexpr int kAccDoubles = kAccSlots + 1;
 void wdot(const double* x, long long ldx, const double* y, long long ldy, long long rows,
           long long cols, const double* rw, const double* cw, double coef, double* acc, int slot);
 
+// acc[slot_x] += sum_{s,q} cx[s + 2 q] <X[s], T[q]> and acc[slot_t] += sum_{s,q} ct[s + 2 q]
+// <T[q], t[s]> over n elements, s, q < ns <= 2; terms with coefficient zero are left out.
+void spin_dots(const double* const* X, const double* const* t, const double* const* T, int ns,
+               long long n, const double* cx, const double* ct, double* acc, int slot_x,
+               int slot_t);
+
 // acc[slot] += coef * sum_{i,l<a; j,k<o} X[i + a*l + lda*(j + a*k)] * Y[i + a*k + lda*(j + a*l)]
 // with lda = a*o: the same-spin four-electron energy over (ik|jl) blocks.
 void permdot_4el(const double* X, const double* Y, long long a, long long o, double coef,
