@@ -975,10 +975,13 @@ void form_fock(const FockRequest& rq) {
     orbital_chunked = any > 0.0;
   }
   const bool fold = pairs_cheaper && !orbital_chunked;
-  // Small evaluations form W's and V's intermediates side by side, in joint launches.
+  // Small evaluations form W's and V's intermediates side by side, in joint launches: the
+  // unpacked blocks and half transforms of both at once, so only within half of the chunk
+  // budget, the share that the unpacked blocks have one after the other.
+  const size_t side_by_side = 2 * (N * N + N * o_tot + R * a_tot) * MW;
   const bool joint = !sharded && MW == MV && W.J3_0.get() && V.J3_0.get() && W.J3_ri_0.get() &&
                      V.J3_ri_0.get() && split_moduli() == 0 &&
-                     2 * (N * N + N * o_tot + R * a_tot) * MW <= kJointDoubles;
+                     side_by_side <= std::min(kJointDoubles, budget / 2);
   for (int first = 0; first < 2 && !orbital_chunked; first += joint ? 2 : 1) {
     const int n_x = joint ? 2 : 1;
     const IntegralsHandle* Xs[2] = {first == 0 ? &W : &V, &V};
