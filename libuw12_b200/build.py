@@ -18,7 +18,7 @@ OUT_DIR = HERE / "_lib"
 LIB = OUT_DIR / "libuw12_b200.so"
 SOURCES = ["gemm_f64.cu", "dgemm_tile_64x64.cu", "dgemm_tile_64x32.cu", "dgemm_tile_32x32.cu",
            "dgemm_tile_128x16.cu", "dgemm_tile_128x8.cu", "ozaki.cu", "kernels.cu", "engine.cu",
-           "synth.cu", "capi.cu"]
+           "synth.cu", "arena.cu", "capi.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -77,30 +77,6 @@ cudaMemPool_t library_pool() {
   return g_pools[dev];
 }
 
-namespace {
-thread_local Arena* t_arena = nullptr;
-}  // namespace
-
-Arena::Arena() {
-  if (t_arena) return;
-  s_ = current_stream();
-  void* p = nullptr;
-  if (cudaMallocFromPoolAsync(&p, kDoubles * sizeof(double), library_pool(), s_) != cudaSuccess) {
-    cudaGetLastError();
-    return;
-  }
-  base_ = static_cast<double*>(p);
-  t_arena = this;
-}
-
-Arena::~Arena() {
-  if (t_arena != this) return;
-  t_arena = nullptr;
-  cudaFreeAsync(base_, s_);
-}
-
-Arena* Arena::current() { return t_arena; }
-
 void trim_pools() {
   std::lock_guard<std::mutex> lk(g_pool_mu);
   for (int d = 0; d < 64; ++d)

@@ -118,14 +118,10 @@ class Arena {
 
   // The calling thread's arena (null: none).
   static Arena* current();
-  // n doubles for stream s, or null when they do not fit.
-  double* take(size_t n_doubles, cudaStream_t s) {
-    const size_t n = (n_doubles + 31) / 32 * 32;  // 256-byte aligned
-    if (s != s_ || n > kDoubles - off_) return nullptr;
-    double* p = base_ + off_;
-    off_ += n;
-    return p;
-  }
+  // n doubles for stream s of the current device, or null when they do not fit or the
+  // block is another stream's or device's (a call made by a producer or a sink inside the
+  // evaluation may be on either; the default stream is the same handle on every device).
+  double* take(size_t n_doubles, cudaStream_t s);
   void give(const double* p, size_t n_doubles) {
     const size_t n = (n_doubles + 31) / 32 * 32;
     if (p + n == base_ + off_) off_ -= n;
@@ -136,6 +132,7 @@ class Arena {
   double* base_ = nullptr;
   size_t off_ = 0;
   cudaStream_t s_ = nullptr;
+  int dev_ = -1;
 };
 
 // Device memory from the calling thread's arena, when it fits there, or from the
