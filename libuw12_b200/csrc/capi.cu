@@ -228,7 +228,6 @@ void run_form_fock(const uw12c_integrals* W, const uw12c_integrals* V, const uw1
     evaluate();
   } catch (const Error& e) {
     if (e.code != UW12C_ERR_ALLOC || !rq.assume_memory || rq.mem_budget) throw;
-    cudaGetLastError();  // the failed allocation's, which the next launch check would see
     rq.assume_memory = false;
     evaluate();
   }

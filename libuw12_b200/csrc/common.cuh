@@ -33,6 +33,9 @@ struct Error : std::runtime_error {
 inline void cuda_check(cudaError_t e, const char* what, const char* file, int line) {
   if (e != cudaSuccess) {
     const int code = (e == cudaErrorMemoryAllocation) ? kErrAlloc : kErrCuda;
+    // a failed allocation is reported here: left behind as the thread's last error, it would
+    // fail the next launch check, the library's or its caller's
+    if (code == kErrAlloc) cudaGetLastError();
     throw Error(code, std::string(what) + ": " + cudaGetErrorString(e) + " (" + file + ":" +
                           std::to_string(line) + ")");
   }
