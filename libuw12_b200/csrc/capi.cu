@@ -7,6 +7,7 @@
 #include <exception>
 #include <memory>
 #include <mutex>
+#include <optional>
 #include <string>
 #include <thread>
 #include <vector>
@@ -211,25 +212,31 @@ void run_form_fock(const uw12c_integrals* W, const uw12c_integrals* V, const uw1
   rq.allreduce = uw12b::g_allreduce;
   rq.allreduce_user = uw12b::g_allreduce_user;
   DeviceGuard dg(w.device);
-  auto evaluate = [&] {
-    uw12b::Arena arena;
+  // An evaluation that hands out gradient blocks or joins collectives is not repeated, so
+  // it asks for the free memory and leaves every buffer to the pool.  Any other assumes
+  // memory first; when an allocation fails it runs again with neither the assumption nor
+  // the block of small buffers, whose unused part would be out of reach of a large one, on
+  // a trimmed pool: what the first attempt reserved was cut for its own buffers.
+  bool repeatable = rq.n_shards <= 1;
+  if (adjoint)
+    for (int i = 0; i < 3; ++i)
+      repeatable = repeatable && !adjoint->sink3[i] && (i == 2 || !adjoint->sink3_ri[i]);
+  auto evaluate = [&](bool first) {
+    rq.assume_memory = first;
+    std::optional<uw12b::Arena> arena;
+    if (first) arena.emplace();
     if (adjoint)
       uw12b::form_fock_adjoint(rq, *adjoint);
     else
       uw12b::form_fock(rq);
   };
-  // an evaluation that hands out gradient blocks or joins collectives is not repeated
-  bool streamed = false;
-  if (adjoint)
-    for (int i = 0; i < 3; ++i)
-      streamed = streamed || adjoint->sink3[i] || (i < 2 && adjoint->sink3_ri[i]);
-  rq.assume_memory = !streamed && rq.n_shards <= 1;
   try {
-    evaluate();
+    evaluate(repeatable);
   } catch (const Error& e) {
-    if (e.code != UW12C_ERR_ALLOC || !rq.assume_memory || rq.mem_budget) throw;
-    rq.assume_memory = false;
-    evaluate();
+    if (e.code != UW12C_ERR_ALLOC || !repeatable) throw;
+    UW12_CUDA(cudaStreamSynchronize(uw12b::current_stream()));
+    uw12b::trim_pools();
+    evaluate(false);
   }
   check_split_pipeline();
 }
