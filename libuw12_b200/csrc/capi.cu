@@ -33,6 +33,8 @@ thread_local cudaStream_t g_stream = nullptr;
 std::atomic<size_t> g_budget{0};
 // Per-thread budget of the worker threads of a batched evaluation (0 = none).
 thread_local size_t g_budget_override = 0;
+// Workers that evaluate beside the calling thread and share the free memory with it.
+thread_local size_t g_sharers = 1;
 thread_local size_t g_shard = 0, g_n_shards = 1;
 thread_local uw12c_allreduce_fn g_allreduce = nullptr;
 thread_local void* g_allreduce_user = nullptr;
@@ -207,6 +209,7 @@ void run_form_fock(const uw12c_integrals* W, const uw12c_integrals* V, const uw1
   rq.fock = fock;
   rq.fock_device = fock_mem == UW12C_MEM_DEVICE;
   rq.mem_budget = uw12b::g_budget_override ? uw12b::g_budget_override : uw12b::g_budget.load();
+  rq.sharers = uw12b::g_sharers;
   rq.shard = uw12b::g_shard;
   rq.n_shards = uw12b::g_n_shards;
   rq.allreduce = uw12b::g_allreduce;
@@ -797,7 +800,9 @@ int uw12c_fock_batched(const uw12c_molecule* mols, size_t n, int indirect_term,
     size_t total_budget = uw12b::g_budget.load();
     // small molecules: each worker's share of the memory that an evaluation may
     // assume holds any of them whole, without asking for the free memory
-    // (engine.cuh); a worker that then runs out of memory asks for itself
+    // (engine.cuh); a worker that then runs out of memory repeats its molecule within
+    // its share of the free memory, and a molecule that fails again, beside the others'
+    // buffers, is evaluated alone at the end
     const size_t assumed = uw12b::assumed_doubles() * sizeof(double) / workers;
     size_t largest = 0;
     for (size_t i = 0; i < n; ++i) {
@@ -824,6 +829,11 @@ int uw12c_fock_batched(const uw12c_molecule* mols, size_t n, int indirect_term,
     std::atomic<size_t> next{0};
     std::vector<int> st(n, UW12C_OK);
     std::vector<std::string> msg(n);
+    auto evaluate = [&](const uw12c_molecule& m) {
+      run_form_fock(m.W, m.V, m.WV, m.abs, m.n_ao, m.n_spin, m.C, m.ldc, m.n_orb, m.occ, m.n_occ,
+                    m.n_active, indirect_term, calculate_fock, scale_opp_spin, scale_same_spin, 0,
+                    m.energy, m.terms, m.fock, m.fock_mem_kind);
+    };
     auto work = [&](int slot) {
       const int prev_slot = uw12b::set_error_slot(slot);
       cudaStream_t stream = nullptr;
@@ -831,6 +841,7 @@ int uw12c_fock_batched(const uw12c_molecule* mols, size_t n, int indirect_term,
       uw12b::set_split_moduli(moduli);
       uw12b::set_split_min_flops(min_flops);
       uw12b::g_budget_override = assume ? 0 : worker_budget;
+      uw12b::g_sharers = workers;
       for (size_t q; (q = next.fetch_add(1)) < n;) {
         const size_t i = order[q];
         const uw12c_molecule& m = mols[i];
@@ -843,9 +854,7 @@ int uw12c_fock_batched(const uw12c_molecule* mols, size_t n, int indirect_term,
             UW12_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
             uw12b::g_stream = stream;
           }
-          run_form_fock(m.W, m.V, m.WV, m.abs, m.n_ao, m.n_spin, m.C, m.ldc, m.n_orb, m.occ,
-                        m.n_occ, m.n_active, indirect_term, calculate_fock, scale_opp_spin,
-                        scale_same_spin, 0, m.energy, m.terms, m.fock, m.fock_mem_kind);
+          evaluate(m);
         });
         if (st[i] != UW12C_OK) msg[i] = uw12b::g_last_msg;
       }
@@ -855,6 +864,7 @@ int uw12c_fock_batched(const uw12c_molecule* mols, size_t n, int indirect_term,
       }
       uw12b::g_stream = nullptr;
       uw12b::g_budget_override = 0;
+      uw12b::g_sharers = 1;
       uw12b::set_error_slot(prev_slot);
     };
     std::vector<std::thread> pool;
@@ -869,6 +879,12 @@ int uw12c_fock_batched(const uw12c_molecule* mols, size_t n, int indirect_term,
       cudaSetDevice(saved_dev);
     }
     for (auto& t : pool) t.join();
+    for (size_t i = 0; i < n; ++i)
+      if (st[i] == UW12C_ERR_ALLOC && assume && workers > 1) {
+        uw12b::trim_pools();
+        st[i] = guarded([&] { evaluate(mols[i]); });
+        if (st[i] != UW12C_OK) msg[i] = uw12b::g_last_msg;
+      }
     if (statuses)
       for (size_t i = 0; i < n; ++i) statuses[i] = st[i];
     for (size_t i = 0; i < n; ++i)

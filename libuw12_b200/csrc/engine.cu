@@ -181,9 +181,10 @@ void eigh(double* A, size_t n, double* w) {
 }
 
 // Chunk budget of one evaluation, in doubles: the caller's, or `fraction` (45% by
-// default, at least 64 MiB) of the device memory available now (free memory
-// plus what the library's pool holds unused).  Re-read at the start of each
-// chunked phase, after the phase's persistent intermediates are allocated.
+// default, at least 64 MiB) of its share of the device memory available now (free
+// memory plus what the library's pool holds unused, over the evaluations that share
+// it).  Re-read at the start of each chunked phase, after the phase's persistent
+// intermediates are allocated.
 //
 // Asking for the free memory (cudaMemGetInfo) enters the kernel driver: 90 us on
 // a quiet host, tens of milliseconds while other processes of the host are in
@@ -197,9 +198,9 @@ void eigh(double* A, size_t n, double* w) {
 //    latter fail, the caller runs it again without the assumption.
 class Budget {
  public:
-  Budget(size_t requested_bytes, size_t need, bool assume_memory)
-      : requested_(requested_bytes), need_(need) {
-    if (!requested_ && assume_memory) whole_ = std::max(whole_, assumed_doubles());
+  Budget(const FockRequest& rq, size_t need)
+      : requested_(rq.mem_budget), need_(need), sharers_(std::max<size_t>(1, rq.sharers)) {
+    if (!requested_ && rq.assume_memory) whole_ = std::max(whole_, assumed_doubles());
   }
 
   size_t doubles(double fraction = 0.45) {
@@ -217,12 +218,13 @@ class Budget {
     }
     const double free_now = std::max(0.0, free0_ - (double(reserved) - reserved0_));
     const double avail = free_now + (reserved > used ? double(reserved - used) : 0.0);
-    return std::max<size_t>(static_cast<size_t>(fraction * avail) / sizeof(double), kFloor);
+    return std::max<size_t>(static_cast<size_t>(fraction * avail / double(sharers_)) / sizeof(double),
+                            kFloor);
   }
 
  private:
   static constexpr size_t kFloor = (size_t(64) << 20) / sizeof(double);
-  size_t requested_, need_, whole_ = kFloor;
+  size_t requested_, need_, sharers_, whole_ = kFloor;
   double free0_ = -1.0, reserved0_ = 0.0;
 };
 
@@ -823,7 +825,7 @@ void form_fock(const FockRequest& rq) {
   const double two = (ns == 1) ? 2.0 : 1.0;
   const double kap4 = 2.0 * half;
   cudaStream_t st = current_stream();
-  Budget budgets(rq.mem_budget, budget_need(rq, false, false), rq.assume_memory);
+  Budget budgets(rq, budget_need(rq, false, false));
   size_t budget = budgets.doubles();
   // Sharding: aux functions and occupied orbitals are dealt out in
   // contiguous, balanced ranges (part).  The fitted densities, the MO
@@ -1885,7 +1887,7 @@ void form_fock_adjoint(const FockRequest& rq_in, const AdjointOutputs& out) {
   cudaStream_t st = current_stream();
   const bool streamed = out.sink3[0] || out.sink3[1] || out.sink3[2] || out.sink3_ri[0] ||
                         out.sink3_ri[1];
-  Budget budgets(rq.mem_budget, budget_need(rq, true, streamed), rq.assume_memory);
+  Budget budgets(rq, budget_need(rq, true, streamed));
   size_t budget = budgets.doubles();
   double F[2][2] = {{0, 0}, {0, 0}};
   for (int s = 0; s < ns; ++s)

@@ -102,6 +102,7 @@ struct FockRequest {
   // Chunks that fit assumed_doubles() whole are laid out without asking for the
   // free memory; on a failed allocation the caller evaluates again with false.
   bool assume_memory = false;
+  size_t sharers = 1;               // evaluations at once that share the free memory
   size_t shard = 0, n_shards = 1;   // partial evaluation: this shard's share only
   // Sum over the shards of a device buffer (in place, ordered on `stream`),
   // called at the same points, with the same counts, on every shard; needed
