@@ -190,7 +190,9 @@ void eigh(double* A, size_t n, double* w) {
 // a quiet host, tens of milliseconds while other processes of the host are in
 // it, against 2.5 us for a launch.  So:
 //  * it is asked at most once per evaluation; afterwards the pool's own counters
-//    say how much of that free memory the evaluation has taken;
+//    say how much of that free memory the evaluation has taken.  Where the caller's code
+//    runs inside the evaluation (producers, gradient sinks, the all-reduce) and may take
+//    device memory itself, it is asked at every phase;
 //  * an evaluation whose chunks all fit whole in 64 MiB, or in 1/32 of the
 //    device's memory where it may be repeated (assume_memory), asks nothing
 //    (`need`: an upper bound of every size that is compared with a budget, so any
@@ -198,8 +200,9 @@ void eigh(double* A, size_t n, double* w) {
 //    latter fail, the caller runs it again without the assumption.
 class Budget {
  public:
-  Budget(const FockRequest& rq, size_t need)
-      : requested_(rq.mem_budget), need_(need), sharers_(std::max<size_t>(1, rq.sharers)) {
+  Budget(const FockRequest& rq, size_t need, bool callers_code)
+      : requested_(rq.mem_budget), need_(need), sharers_(std::max<size_t>(1, rq.sharers)),
+        callers_code_(callers_code) {
     if (!requested_ && rq.assume_memory) whole_ = std::max(whole_, assumed_doubles());
   }
 
@@ -210,7 +213,7 @@ class Budget {
     unsigned long long reserved = 0, used = 0;  // 64-bit pool attributes
     UW12_CUDA(cudaMemPoolGetAttribute(library_pool(), cudaMemPoolAttrReservedMemCurrent, &reserved));
     UW12_CUDA(cudaMemPoolGetAttribute(library_pool(), cudaMemPoolAttrUsedMemCurrent, &used));
-    if (free0_ < 0.0) {
+    if (free0_ < 0.0 || callers_code_) {
       size_t free_b = 0, total_b = 0;
       UW12_CUDA(cudaMemGetInfo(&free_b, &total_b));
       free0_ = double(free_b);
@@ -225,6 +228,7 @@ class Budget {
  private:
   static constexpr size_t kFloor = (size_t(64) << 20) / sizeof(double);
   size_t requested_, need_, sharers_, whole_ = kFloor;
+  bool callers_code_;
   double free0_ = -1.0, reserved0_ = 0.0;
 };
 
@@ -784,18 +788,24 @@ bool pair_form_cheaper(const FockRequest& rq, const std::vector<SpinDims>& sd, b
 }
 }  // namespace
 
+namespace {
+// Whether every three-index tensor that an evaluation reads is stored.
+bool all_stored(const FockRequest& rq) {
+  return rq.W->J3_0.get() && rq.V->J3_0.get() && rq.WV->J3_0.get() && rq.W->J3_ri_0.get() &&
+         rq.V->J3_ri_0.get();
+}
+}  // namespace
+
 size_t budget_need(const FockRequest& rq, bool adjoint, bool streamed) {
   const size_t N = rq.n_ao, np = packed_size(N), R = rq.W->n_ri, Rp = N + R;
   const size_t M = std::max({rq.W->n_df, rq.V->n_df, rq.WV->n_df});
-  bool stored = rq.W->J3_0.get() && rq.V->J3_0.get() && rq.WV->J3_0.get() &&
-                rq.W->J3_ri_0.get() && rq.V->J3_ri_0.get();
   size_t o = 0, o1 = 0;  // occupied orbitals of all spins, of the larger spin
   for (size_t n : rq.n_occ) {
     o += n;
     o1 = std::max(o1, n);
   }
   // aux blocks of unstored tensors and of streamed gradients
-  const size_t blocks = stored && !streamed ? 0 : 16 * (np + R * N) * M;
+  const size_t blocks = all_stored(rq) && !streamed ? 0 : 16 * (np + R * N) * M;
   size_t need = blocks + 2 * (N * N + np) * M;                           // unpacked AO blocks
   need = std::max(need, (2 * (N + o1) + 3 * Rp) * o * M);                // whole transforms
   if (rq.calc_fock) need = std::max(need, blocks + (4 * Rp * N + np + R * N) * M);
@@ -825,7 +835,7 @@ void form_fock(const FockRequest& rq) {
   const double two = (ns == 1) ? 2.0 : 1.0;
   const double kap4 = 2.0 * half;
   cudaStream_t st = current_stream();
-  Budget budgets(rq, budget_need(rq, false, false));
+  Budget budgets(rq, budget_need(rq, false, false), !all_stored(rq) || rq.n_shards > 1);
   size_t budget = budgets.doubles();
   // Sharding: aux functions and occupied orbitals are dealt out in
   // contiguous, balanced ranges (part).  The fitted densities, the MO
@@ -1887,7 +1897,7 @@ void form_fock_adjoint(const FockRequest& rq_in, const AdjointOutputs& out) {
   cudaStream_t st = current_stream();
   const bool streamed = out.sink3[0] || out.sink3[1] || out.sink3[2] || out.sink3_ri[0] ||
                         out.sink3_ri[1];
-  Budget budgets(rq, budget_need(rq, true, streamed));
+  Budget budgets(rq, budget_need(rq, true, streamed), !all_stored(rq) || streamed);
   size_t budget = budgets.doubles();
   double F[2][2] = {{0, 0}, {0, 0}};
   for (int s = 0; s < ns; ++s)
