@@ -693,14 +693,6 @@ struct SpinDims {
   size_t o = 0, a = 0, c = 0, ooff = 0, aoff = 0;
 };
 
-// Pairs (j, k) of active orbitals j and occupied orbitals k < k_end in pair order: k
-// ascending and j ascending within it, every j for a core orbital, j <= k - c for
-// an active one.
-size_t pair_count(size_t a, size_t c, size_t k_end) {
-  const size_t i = k_end > c ? k_end - c : 0;
-  return a * std::min(k_end, c) + i * (i + 1) / 2;
-}
-
 // Occupation-weighted occupied orbitals Co (utils.hpp:289-310) of both spins side
 // by side (N x o_tot) and their active (last n_active) columns Ca (freeze_core,
 // utils.hpp:235-253; N x a_tot), one after the other on the device.
@@ -842,11 +834,13 @@ void form_fock(const FockRequest& rq) {
   // transforms and the 2-el Fock run over this shard's aux range, and the
   // partial intermediates (fitted densities, B1, the stacked RI rows) are
   // summed over the shards by rq.allreduce before use; X_AB and t are summed
-  // from orbital ranges the same way.  The t~ dX Fock term runs over a range
-  // of W's aux functions, the direct Fock and the same-spin 3-el energy and
-  // Fock over ranges of occupied k.  The energies built from the reduced
-  // intermediates and the same-spin 2-el / 4-el terms come from shard 0.  The
-  // caller sums the partial energies and Fock matrices over the shards.
+  // from orbital ranges the same way.  The direct Fock and the same-spin 3-el
+  // energy run over ranges of occupied k, the Fock terms over orbital pairs
+  // over ranges of k with equal numbers of pairs (pair_bound), and t~ dX over
+  // aux functions, where that form is the cheaper one, over a range of W's.
+  // The energies built from the reduced intermediates and the same-spin 2-el /
+  // 4-el terms come from shard 0.  The caller sums the partial energies and
+  // Fock matrices over the shards.
   const size_t n_shards = std::max<size_t>(1, rq.n_shards);
   const size_t shard = rq.shard;
   const bool lead = shard == 0;
@@ -1580,7 +1574,8 @@ void form_fock(const FockRequest& rq) {
         xscr = std::max(xscr, (Xi->J3_0.get() ? 0 : np * aux_step(*Xi, false, budget / 2)) +
                                   (Xi->J3_ri_0.get() ? 0 : R * N * aux_step(*Xi, true, budget / 2)));
       const size_t pair = Rp * N;  // doubles of one pair's matrix
-      const auto [klo, khi] = part(o);
+      const size_t klo = pair_bound(a, c, shard, n_shards);
+      const size_t khi = pair_bound(a, c, shard + 1, n_shards);
       const size_t kavail = budget > xscr ? budget - xscr : 0;
       // A chunk of occupied orbitals [k0, k0 + nk): its pairs are [p0, p0 + np_) in
       // pair order.  Y of its pairs lies in two blocks: Y[j, k], j < nj, is matrix

@@ -67,6 +67,25 @@ struct PairColumns {
   }
 };
 
+// Pairs (j, k) of active orbitals j and occupied orbitals k < k_end in pair order: k
+// ascending and j ascending within it, every j for a core orbital, j <= k - c for
+// an active one.
+inline size_t pair_count(size_t a, size_t c, size_t k_end) {
+  const size_t i = k_end > c ? k_end - c : 0;
+  return a * (k_end < c ? k_end : c) + i * (i + 1) / 2;
+}
+
+// First occupied orbital of shard i of n (i = n: o = c + a): the shards' ranges have about
+// the same number of pairs each, within the pairs of one orbital.  Even ranges of orbitals
+// give the last of 8 shards 23 % of the pairs instead of 12.5 (no core).
+inline size_t pair_bound(size_t a, size_t c, size_t i, size_t n) {
+  const size_t o = c + a, total = pair_count(a, c, o) * i;
+  size_t k = 0;
+  while (k < o && pair_count(a, c, k) * n < total) ++k;
+  if (k > 0 && pair_count(a, c, k) * n - total > total - pair_count(a, c, k - 1) * n) --k;
+  return k;
+}
+
 // Sums of wdot, permdot_4el and permdot_3el: acc is a device array of
 // kAccDoubles, zeroed before its first use; slots below kAccSlots hold sums, the
 // last double is the ticket of the reductions' last block.
