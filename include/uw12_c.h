@@ -346,10 +346,11 @@ int uw12c_profile_read_kind(int kind, unsigned long long* launches, double* ms, 
 /* Split-K autotuner of the FP64 GEMM engine (no counterpart in libuw12, which
  * leaves its BLAS to choose its own blocking).  The engine splits the
  * contraction of a GEMM whose output has too few tiles to fill the GPU; by
- * default a wave-occupancy rule picks the split.  mode 1 (tune): the first
+ * default a cost model picks the split.  mode 1 (tune): the first
  * GEMM with beta = 0 and an automatic split of each shape class (output CTA
- * count, power-of-two bucket of the k tiles over all reduction batches; output
- * CTA counts of at least 8 waves never split) is launched once with each
+ * count in tiles of 128 x 128, power-of-two buckets of the k tiles over all
+ * reduction batches and of the 32 x 8 blocks of the output; output
+ * CTA counts of at least 8 waves are not tuned) is launched once with each
  * candidate split (1 .. 64, at least 4 k tiles per part, split-K partials
  * within 256 MiB or the rule's own), each timed on the
  * library's stream, which synchronises it; the fastest is recorded and the
@@ -357,8 +358,10 @@ int uw12c_profile_read_kind(int kind, unsigned long long* launches, double* ms, 
  * for every class it has, the rule otherwise, no timing.  mode 0: the rule
  * (default).  When path names an existing file (written by
  * uw12c_autotune_save: a comment line, then "output_ctas k_tile_bucket split
- * ms" per class) its classes are merged into the table first; a malformed file
- * is UW12C_ERR_INVALID.  The table and the mode are process-wide and apply to
+ * ms output_block_bucket" per class) its classes are merged into the table
+ * first; a line without the last number stands for every output of its CTA
+ * count that has no line of its own, and mode 1 still measures those; a
+ * malformed file is UW12C_ERR_INVALID.  The table and the mode are process-wide and apply to
  * every thread and device; tune on one device of the kind that will use the
  * table, with one evaluation at a time (timings overlapped by other work are
  * not representative).  Splits change the summation order only: results agree

@@ -9,6 +9,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "dgemm_tile.cuh"
@@ -304,7 +305,10 @@ void profile_record(int kind, cudaEvent_t a, cudaEvent_t b, double work, std::st
 // choose_plan predicts the split-K factor of a launch.  The autotuner replaces
 // it by measurement: a shape class is (output CTAs = 128 x 128 output tiles x
 // output batches, power-of-two bucket of the k tiles over all reduction
-// batches); in tuning mode the first automatic-split GEMM of a class not yet in
+// batches, power-of-two bucket of the 32 x 8 blocks that cover the output: launches
+// use tiles from 64 x 64 down to 32 x 32 and 128 x 8, so 24 x 24 and 128 x 128, one
+// CTA of 128 x 128 both, want different splits); in tuning mode the first
+// automatic-split GEMM of a class not yet in
 // the table is launched once with every candidate split (1, 2, 3, 4, 6, 8, 12,
 // 16, 24, 32, 48, 64 while each CTA keeps >= 4 k tiles and the partial tiles stay
 // within 256 MiB or the rule's), each with the tile the cost model picks for it
@@ -313,12 +317,16 @@ void profile_record(int kind, cudaEvent_t a, cudaEvent_t b, double work, std::st
 // (their repeated launches overwrite C); the others, and every GEMM in "use"
 // mode, take the table's split for their class when it has one and the rule's
 // otherwise.  Outputs of at least 8 waves of 128 x 128 tiles are not tuned.
+// A file's line without the last bucket (tables of one-tile kernels) stands for every
+// output of its CTA count that has no entry of its own, and does not keep tuning mode
+// from measuring one.
 namespace {
 struct TuneKey {
   long long ctas;
   int kbucket;
+  int blocks;  // bucket of the output's 32 x 8 blocks, -1: any
   bool operator<(const TuneKey& o) const {
-    return ctas != o.ctas ? ctas < o.ctas : kbucket < o.kbucket;
+    return std::tie(ctas, kbucket, blocks) < std::tie(o.ctas, o.kbucket, o.blocks);
   }
 };
 struct TuneEntry {
@@ -337,18 +345,27 @@ int kbucket_of(long long ktiles_total) {
 
 TuneKey tune_key(long long m, long long n, long long k, long long nbo, long long nbr) {
   const long long tiles = ((m + 127) / 128) * ((n + 127) / 128);
-  return TuneKey{tiles * nbo, kbucket_of(((k + BK - 1) / BK) * nbr)};
+  const long long blocks = ((m + 31) / 32) * ((n + 7) / 8);
+  return TuneKey{tiles * nbo, kbucket_of(((k + BK - 1) / BK) * nbr), kbucket_of(blocks * nbo)};
 }
 TuneKey tune_key(const GemmDesc& d) {
   return tune_key(d.m, d.n, d.k, d.nbo1 * d.nbo2, d.nbr1 * d.nbr2);
 }
 
+// the table's split for a class, or 0 (the caller holds g_tune_mu)
+int table_split(TuneKey key) {
+  auto it = g_tune.find(key);
+  if (it == g_tune.end()) {
+    key.blocks = -1;
+    it = g_tune.find(key);
+  }
+  return it == g_tune.end() ? 0 : it->second.split;
+}
+
 // the table's split for d's class, or 0
 int tuned_split(const GemmDesc& d) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  if (g_tune_mode == 0) return 0;
-  auto it = g_tune.find(tune_key(d));
-  return it == g_tune.end() ? 0 : it->second.split;
+  return g_tune_mode == 0 ? 0 : table_split(tune_key(d));
 }
 
 bool tuning_wanted(const GemmDesc& d) {
@@ -427,15 +444,16 @@ void autotune_set(int mode, const char* path) {
         ++lineno;
         if (line[0] == '#' || line[0] == '\n') continue;
         long long ctas = 0;
-        int kb = 0, split = 0;
+        int kb = 0, split = 0, blocks = -1;
         double ms = 0.0;
-        if (std::sscanf(line, "%lld %d %d %lf", &ctas, &kb, &split, &ms) != 4 || ctas <= 0 ||
-            kb < 0 || kb > 62 || split < 1 || split > 64) {
+        if (std::sscanf(line, "%lld %d %d %lf %d", &ctas, &kb, &split, &ms, &blocks) < 4 ||
+            ctas <= 0 || kb < 0 || kb > 62 || split < 1 || split > 64 || blocks < -1 ||
+            blocks > 62) {
           std::fclose(f);
           throw Error(kErrInvalid, std::string("autotune: malformed line ") +
                                        std::to_string(lineno) + " in " + path);
         }
-        loaded[TuneKey{ctas, kb}] = TuneEntry{split, ms};
+        loaded[TuneKey{ctas, kb, blocks}] = TuneEntry{split, ms};
       }
       std::fclose(f);
     }
@@ -450,10 +468,13 @@ void autotune_save(const char* path) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
   FILE* f = std::fopen(path, "w");
   if (!f) throw Error(kErrInvalid, std::string("autotune: cannot write ") + path);
-  std::fprintf(f, "# output_ctas k_tile_bucket split ms\n");
-  for (const auto& kv : g_tune)
-    std::fprintf(f, "%lld %d %d %.6f\n", kv.first.ctas, kv.first.kbucket, kv.second.split,
+  std::fprintf(f, "# output_ctas k_tile_bucket split ms output_block_bucket\n");
+  for (const auto& kv : g_tune) {
+    std::fprintf(f, "%lld %d %d %.6f", kv.first.ctas, kv.first.kbucket, kv.second.split,
                  kv.second.ms);
+    if (kv.first.blocks >= 0) std::fprintf(f, " %d", kv.first.blocks);
+    std::fprintf(f, "\n");
+  }
   std::fclose(f);
 }
 
@@ -470,8 +491,7 @@ long long autotune_size() {
 int autotune_lookup(long long m, long long n, long long k, long long nbo, long long nbr) {
   if (m <= 0 || n <= 0 || k <= 0 || nbo <= 0 || nbr <= 0) return 0;
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  auto it = g_tune.find(tune_key(m, n, k, nbo, nbr));
-  return it == g_tune.end() ? 0 : it->second.split;
+  return table_split(tune_key(m, n, k, nbo, nbr));
 }
 
 void gemm(const GemmDesc& d) {
