@@ -282,10 +282,23 @@ def reference_inputs(w):
 # --------------------------------------------------------------------------
 # CPU baseline: libuw12 itself, sampled (timing build of oracle/ref.mk)
 # --------------------------------------------------------------------------
+def cpu_reference_missing():
+    """Why libuw12's timing build cannot run here, or None (it is built when its
+    sources are there)."""
+    from oracle import ref_lib as R
+    if R.available(timing=True):
+        return None
+    try:
+        R.build()
+    except RuntimeError as exc:
+        return str(exc).splitlines()[0]
+    if R.available(timing=True):
+        return None
+    return "libuw12 is not built (oracle/_ref) and its sources are not on this machine"
+
+
 def cpu_reference_problem(w, h):
     from oracle import ref_lib as R
-    if not R.available(timing=True):
-        R.build()
     cores = os.cpu_count() or 1
     R.set_threads(cores, 1, timing=True)
     p = R.RefProblem(h["W3"], h["W2"], h["W3_ri"], h["V3"], h["V2"], h["V3_ri"], h["WV3"],
@@ -315,6 +328,10 @@ def cpu_model() -> str:
 def run_reference(args, rank, world):
     """The reference arm: libuw12 (timing build) on the host cores, rank 0 only."""
     if rank != 0:
+        return
+    missing = cpu_reference_missing()
+    if missing:
+        print(json.dumps({"impl": "reference", "unavailable": missing}), flush=True)
         return
     from oracle import ref_lib as R, synth
     w = workload_of(args)
@@ -813,8 +830,10 @@ def main():
         del gh, host_out
 
     # ---- CPU baseline: libuw12 itself on the same inputs (rank 0, N = 1)
-    cpu = None
+    cpu = cpu_missing = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
+        cpu_missing = cpu_reference_missing()
+    if rank == 0 and world == 1 and not args.no_cpu_baseline and not cpu_missing:
         p, cores = cpu_reference_problem(w, host)
         est, wall, nloops, _ = p.timed_evaluate(1, *cpu_reference_args(w, host, args.s_os,
                                                                        args.s_ss))
@@ -855,6 +874,7 @@ def main():
             "phases_ms_split_step": phases_split,
             "phases_ms_fp64_forward": phases_fwd,
             "cpu_baseline": cpu,
+            **({"cpu_baseline_unavailable": cpu_missing} if cpu_missing else {}),
             "e2e": e2e,
             "gpu_launches": int(launches),
             "clocks": clk,
