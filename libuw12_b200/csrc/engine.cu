@@ -588,7 +588,12 @@ void fitted_density_raw(const IntegralsHandle& X, const double* dmat, int ns, do
 }
 
 // Largest product (operations) of W and V in one launch, and largest evaluation (doubles of
-// both potentials' transforms) that forms them side by side.
+// both potentials' transforms) that forms them side by side.  Closed-shell Fock matrices
+// with 3 DF and 4 RI functions per AO, o = N / 10, in turn on one box, with these limits / one
+// after the other / side by side without limits: 0.26 / 0.31 / 0.26 ms at N = 24, 0.43 / 0.50
+// / 0.43 at 61, 1.30 / 1.37 / 1.28 at 100, 2.32 / 2.38 / 2.28 at 120 (16 M doubles), 4.77 /
+// 4.80 / 4.68 at 143, 6.98 / 7.00 / 6.89 at 160, 19.7 / 19.8 / 19.6 at 200: what lies above
+// the limits gains 1 to 2 %, against twice the memory of the transforms.
 constexpr double kJointFlops = 2e9;
 constexpr size_t kJointDoubles = size_t(1) << 24;
 
@@ -746,7 +751,9 @@ namespace {
 // residue bytes written at 5.8 TB/s) and a result element its reconstruction (L + 8
 // bytes at 3.4 TB/s), in units of a multiply-add (L of them at 2.88 POPS): the forms'
 // operations are equal at N=500, M=1500, R=2000, o=40/38, opposite spin, but the pairs
-// prepare the three-index tensors once per spin: 339 ms, over aux functions 321.
+// prepare the three-index tensors once per spin: 338 ms, over aux functions 321 (in turn on
+// one box).  Every product is priced as if it ran split, which small and long ones
+// do not; the routing rule has rates of its own (ozaki_profitable, where the reason stands).
 bool pair_form_cheaper(const FockRequest& rq, const std::vector<SpinDims>& sd, bool same_spin) {
   const int ns = rq.n_spin;
   const double N = double(rq.n_ao), R = double(rq.W->n_ri), Rp = N + R;
@@ -1432,96 +1439,100 @@ void form_fock(const FockRequest& rq) {
       const size_t ao = a * o, No = N * o;
       DevBuf b2wl, b2vl, b1wl, b1vl;
       if (do_ind) {
-      b2wl.alloc(ao * MW);
-      b2vl.alloc(ao * MV);
-      scale_rc(XW.B2[s].get(), LL(ao), LL(ao), LL(MW), nullptr, W.lam.get(), 1.0, b2wl.get(), LL(ao));
-      scale_rc(XV.B2[s].get(), LL(ao), LL(ao), LL(MV), nullptr, V.lam.get(), 1.0, b2vl.get(), LL(ao));
-      clock.mark("ss_4el_energy");
-      // ---- 4-el indirect energy (four_electron.cpp:143-179)
-      if (lead) {
-        DevBuf W4(ao * ao), V4(ao * ao);
-        GemmDesc gw = gemm_nn(LL(ao), LL(ao), LL(MW), 1.0, b2wl.get(), LL(ao), XW.B2[s].get(),
-                              LL(ao), 0.0, W4.get(), LL(ao));
-        gw.b_ncontig = true;
-        GemmDesc gv = gemm_nn(LL(ao), LL(ao), LL(MV), 1.0, b2vl.get(), LL(ao), XV.B2[s].get(),
-                              LL(ao), 0.0, V4.get(), LL(ao));
-        gv.b_ncontig = true;
-        gemm_both(gw, gv);
-        permdot_4el(W4.get(), V4.get(), LL(a), LL(o), -0.5 * two, acc.get(), kE4i);
-      }
-      clock.mark("ss_3el_energy");
-      // ---- 3-el indirect energy (indirect_utils.cpp:101-133), chunked over k, YW and ZV
-      // formed once per pair of a chunk (B2 is symmetric in the active pair): N=300 Fock
-      // 129.5 -> 125.9 ms
-      {
-        budget = budgets.doubles();
-        const size_t per_k = 2 * Rp * a * a + a * (MW + MV);
-        const auto [klo, khi] = part(o);
-        const size_t kc = tile_chunk(khi - klo, a,
-                                     std::max<size_t>(1, std::min(khi - klo, budget / per_k)));
-        DevBuf YW, ZV, b2p;
-        for (size_t k0 = klo; k0 < khi; k0 += kc) {
-          const PairColumns q = PairColumns::of(LL(a), LL(c), LL(k0), LL(std::min(kc, khi - k0)));
-          const size_t n = static_cast<size_t>(q.count());
-          if (YW.size() < Rp * a * n) {
-            YW.alloc(Rp * a * n);
-            ZV.alloc(Rp * a * n);
-            b2p.alloc(n * (MW + MV));
-          }
-          double* b2v = b2p.get() + n * MW;
-          pack_pairs(XW.B2[s].get(), q, LL(o), LL(MW), W.lam.get(), 0.5, b2p.get());
-          pack_pairs(XV.B2[s].get(), q, LL(o), LL(MV), V.lam.get(), 0.5, b2v);
-          GemmDesc gw = gemm_nn(LL(Rp * a), LL(n), LL(MW), 1.0, XW.Wst[s].get(), LL(Rp * a),
-                                b2p.get(), LL(n), 0.0, YW.get(), LL(Rp * a));
+        b2wl.alloc(ao * MW);
+        b2vl.alloc(ao * MV);
+        scale_rc(XW.B2[s].get(), LL(ao), LL(ao), LL(MW), nullptr, W.lam.get(), 1.0, b2wl.get(),
+                 LL(ao));
+        scale_rc(XV.B2[s].get(), LL(ao), LL(ao), LL(MV), nullptr, V.lam.get(), 1.0, b2vl.get(),
+                 LL(ao));
+        clock.mark("ss_4el_energy");
+        // ---- 4-el indirect energy (four_electron.cpp:143-179)
+        if (lead) {
+          DevBuf W4(ao * ao), V4(ao * ao);
+          GemmDesc gw = gemm_nn(LL(ao), LL(ao), LL(MW), 1.0, b2wl.get(), LL(ao), XW.B2[s].get(),
+                                LL(ao), 0.0, W4.get(), LL(ao));
           gw.b_ncontig = true;
-          GemmDesc gv = gemm_nn(LL(Rp * a), LL(n), LL(MV), 1.0, XV.SV[s].get(), LL(Rp * a), b2v,
-                                LL(n), 0.0, ZV.get(), LL(Rp * a));
+          GemmDesc gv = gemm_nn(LL(ao), LL(ao), LL(MV), 1.0, b2vl.get(), LL(ao), XV.B2[s].get(),
+                                LL(ao), 0.0, V4.get(), LL(ao));
           gv.b_ncontig = true;
           gemm_both(gw, gv);
-          permdot_3el(YW.get(), ZV.get(), LL(Rp), q, two, acc.get(), kE3i);
+          permdot_4el(W4.get(), V4.get(), LL(a), LL(o), -0.5 * two, acc.get(), kE4i);
+        }
+        clock.mark("ss_3el_energy");
+        // ---- 3-el indirect energy (indirect_utils.cpp:101-133), chunked over k, YW and ZV
+        // formed once per pair of a chunk (B2 is symmetric in the active pair): N=300 Fock
+        // 129.5 -> 125.9 ms
+        {
+          budget = budgets.doubles();
+          const size_t per_k = 2 * Rp * a * a + a * (MW + MV);
+          const auto [klo, khi] = part(o);
+          const size_t kc = tile_chunk(khi - klo, a,
+                                       std::max<size_t>(1, std::min(khi - klo, budget / per_k)));
+          DevBuf YW, ZV, b2p;
+          for (size_t k0 = klo; k0 < khi; k0 += kc) {
+            const PairColumns q = PairColumns::of(LL(a), LL(c), LL(k0), LL(std::min(kc, khi - k0)));
+            const size_t n = static_cast<size_t>(q.count());
+            if (YW.size() < Rp * a * n) {
+              YW.alloc(Rp * a * n);
+              ZV.alloc(Rp * a * n);
+              b2p.alloc(n * (MW + MV));
+            }
+            double* b2v = b2p.get() + n * MW;
+            pack_pairs(XW.B2[s].get(), q, LL(o), LL(MW), W.lam.get(), 0.5, b2p.get());
+            pack_pairs(XV.B2[s].get(), q, LL(o), LL(MV), V.lam.get(), 0.5, b2v);
+            GemmDesc gw = gemm_nn(LL(Rp * a), LL(n), LL(MW), 1.0, XW.Wst[s].get(), LL(Rp * a),
+                                  b2p.get(), LL(n), 0.0, YW.get(), LL(Rp * a));
+            gw.b_ncontig = true;
+            GemmDesc gv = gemm_nn(LL(Rp * a), LL(n), LL(MV), 1.0, XV.SV[s].get(), LL(Rp * a), b2v,
+                                  LL(n), 0.0, ZV.get(), LL(Rp * a));
+            gv.b_ncontig = true;
+            gemm_both(gw, gv);
+            permdot_3el(YW.get(), ZV.get(), LL(Rp), q, two, acc.get(), kE3i);
+          }
+        }
+        if (!calc) continue;
+        b1wl.alloc(No * MW);
+        b1vl.alloc(No * MV);
+        scale_rc(XW.B1[s].get(), LL(No), LL(No), LL(MW), nullptr, W.lam.get(), 1.0, b1wl.get(),
+                 LL(No));
+        scale_rc(XV.B1[s].get(), LL(No), LL(No), LL(MV), nullptr, V.lam.get(), 1.0, b1vl.get(),
+                 LL(No));
+        clock.mark("ss_4el_fock");
+        // ---- 4-el indirect Fock (four_electron.cpp:181-249)
+        if (lead) {
+          DevBuf W43(No * ao), V43(No * ao);
+          GemmDesc gw = gemm_nn(LL(No), LL(ao), LL(MW), 1.0, b1wl.get(), LL(No), XW.B2[s].get(),
+                                LL(ao), 0.0, W43.get(), LL(No));
+          gw.b_ncontig = true;
+          GemmDesc gv = gemm_nn(LL(No), LL(ao), LL(MV), 1.0, b1vl.get(), LL(No), XV.B2[s].get(),
+                                LL(ao), 0.0, V43.get(), LL(No));
+          gv.b_ncontig = true;
+          gemm_both(gw, gv);
+          GemmDesc gi = gemm_nn(LL(N), LL(N), LL(a), s_ss * (c > 0 ? -1.0 : -2.0),
+                                W43.get() + N * c, LL(No), V43.get() + N * c, LL(N), 1.0,
+                                Fp[s], LL(N));
+          gi.b_ncontig = true;
+          gi.nbr1 = LL(a);
+          gi.nbr2 = LL(o);
+          gi.sAr1 = LL(N);
+          gi.sAr2 = LL(No * a);
+          gi.sBr1 = LL(No);
+          gi.sBr2 = LL(No * a);
+          gemm(gi);
+          if (c > 0) {
+            GemmDesc gf = gemm_nn(LL(N), LL(N), LL(a), -s_ss, W43.get(), LL(No), V43.get(), LL(No),
+                                  1.0, Fp[s], LL(N));
+            gf.b_ncontig = true;
+            gf.nbr1 = LL(o);
+            gf.nbr2 = LL(o);
+            gf.sAr1 = LL(N);
+            gf.sAr2 = LL(No * a);
+            gf.sBr1 = LL(No * a);
+            gf.sBr2 = LL(N);
+            gemm(gf);
+          }
         }
       }
-      if (!calc) continue;
-      b1wl.alloc(No * MW);
-      b1vl.alloc(No * MV);
-      scale_rc(XW.B1[s].get(), LL(No), LL(No), LL(MW), nullptr, W.lam.get(), 1.0, b1wl.get(), LL(No));
-      scale_rc(XV.B1[s].get(), LL(No), LL(No), LL(MV), nullptr, V.lam.get(), 1.0, b1vl.get(), LL(No));
-      clock.mark("ss_4el_fock");
-      // ---- 4-el indirect Fock (four_electron.cpp:181-249)
-      if (lead) {
-        DevBuf W43(No * ao), V43(No * ao);
-        GemmDesc gw = gemm_nn(LL(No), LL(ao), LL(MW), 1.0, b1wl.get(), LL(No), XW.B2[s].get(),
-                              LL(ao), 0.0, W43.get(), LL(No));
-        gw.b_ncontig = true;
-        GemmDesc gv = gemm_nn(LL(No), LL(ao), LL(MV), 1.0, b1vl.get(), LL(No), XV.B2[s].get(),
-                              LL(ao), 0.0, V43.get(), LL(No));
-        gv.b_ncontig = true;
-        gemm_both(gw, gv);
-        GemmDesc gi = gemm_nn(LL(N), LL(N), LL(a), s_ss * (c > 0 ? -1.0 : -2.0),
-                              W43.get() + N * c, LL(No), V43.get() + N * c, LL(N), 1.0,
-                              Fp[s], LL(N));
-        gi.b_ncontig = true;
-        gi.nbr1 = LL(a);
-        gi.nbr2 = LL(o);
-        gi.sAr1 = LL(N);
-        gi.sAr2 = LL(No * a);
-        gi.sBr1 = LL(No);
-        gi.sBr2 = LL(No * a);
-        gemm(gi);
-        if (c > 0) {
-          GemmDesc gf = gemm_nn(LL(N), LL(N), LL(a), -s_ss, W43.get(), LL(No), V43.get(), LL(No),
-                                1.0, Fp[s], LL(N));
-          gf.b_ncontig = true;
-          gf.nbr1 = LL(o);
-          gf.nbr2 = LL(o);
-          gf.sAr1 = LL(N);
-          gf.sAr2 = LL(No * a);
-          gf.sBr1 = LL(No * a);
-          gf.sBr2 = LL(N);
-          gemm(gf);
-        }
-      }
-      }  // do_ind
       clock.mark("pair_fock");
       // ---- Fock terms over pairs of an active orbital j and an occupied
       // orbital k, in chunks of k.  With G_X[jk] = sum_A [sq(J3_0^X[:,A]);

@@ -51,7 +51,7 @@ struct Consts {
   int L = 0, nch = 0, cw = 0, beta = 0;
   uint32_t p[kOzakiMaxModuli];
   uint32_t barrett[kOzakiMaxModuli];  // floor(2^32 / p)
-  double pd[kOzakiMaxModuli], inv_p[kOzakiMaxModuli];
+  double inv_p[kOzakiMaxModuli];
   double w[kOzakiMaxModuli][kMaxChunks];  // chunks of (M/p_l) * ((M/p_l)^-1 mod p_l) mod M
   double mc[kMaxChunks];                  // chunks of M
   double inv_m;
@@ -87,7 +87,6 @@ Consts make_consts(int L) {
     c.log2_m += std::log2(double(p));
     c.p[l] = p;
     c.barrett[l] = static_cast<uint32_t>((1ULL << 32) / p);
-    c.pd[l] = double(p);
     c.inv_p[l] = 1.0 / double(p);
   }
   int bits = 0;
@@ -1870,12 +1869,15 @@ int ozaki_bits(int n_moduli, long long k_total) {
 #endif
 
 bool ozaki_profitable(const GemmDesc& d, int n_moduli) {
-  // Estimated times on a B200 (fitted to measured kernels): operand
-  // preparation streams each operand element twice in FP64 and writes L
-  // residue bytes (UW12_COST_PREP_TBS TB/s); the CRT reads L residue bytes
-  // (and C when beta != 0) and writes C (UW12_COST_CRT_TBS); the int8
-  // products run at UW12_COST_I8_POPS; the FP64 DMMA GEMM at
-  // UW12_COST_FP64_TFS TFLOP/s.  Split when it is clearly faster.
+  // Estimated times on a B200: operand preparation streams each operand
+  // element twice in FP64 and writes L residue bytes (UW12_COST_PREP_TBS
+  // TB/s); the CRT reads L residue bytes (and C when beta != 0) and writes C
+  // (UW12_COST_CRT_TBS); the int8 products run at UW12_COST_I8_POPS; the FP64
+  // DMMA GEMM at UW12_COST_FP64_TFS TFLOP/s.  Split when it is clearly faster.
+  // The rates are those of earlier kernels (today 5.8 and 3.4 TB/s, 2.9 POPS,
+  // 32 TFLOP/s), kept because they decide which products keep FP64's bits:
+  // today's would send sums of K = 7e5 to the split path, where 14 moduli hold
+  // 44 bits of an operand (48 at K = 1500).
   const double L = double(n_moduli);
   const double k_total = double(d.k) * double(d.nbr1) * double(d.nbr2);
   const double nbatch = double(d.nbo1) * double(d.nbo2);
