@@ -192,7 +192,8 @@ void eigh(double* A, size_t n, double* w) {
 //  * it is asked at most once per evaluation; afterwards the pool's own counters
 //    say how much of that free memory the evaluation has taken.  Where the caller's code
 //    runs inside the evaluation (producers, gradient sinks, the all-reduce) and may take
-//    device memory itself, it is asked at every phase;
+//    device memory itself, it is asked at every phase of an evaluation that is not
+//    repeated when an allocation fails, or is the repeat;
 //  * an evaluation whose chunks all fit whole in 64 MiB, or in 1/32 of the
 //    device's memory where it may be repeated (assume_memory), asks nothing
 //    (`need`: an upper bound of every size that is compared with a budget, so any
@@ -202,7 +203,7 @@ class Budget {
  public:
   Budget(const FockRequest& rq, size_t need, bool callers_code)
       : requested_(rq.mem_budget), need_(need), sharers_(std::max<size_t>(1, rq.sharers)),
-        callers_code_(callers_code) {
+        callers_code_(callers_code && !rq.assume_memory) {
     if (!requested_ && rq.assume_memory) whole_ = std::max(whole_, assumed_doubles());
   }
 
