@@ -285,30 +285,36 @@ void setup_metric(IntegralsHandle* h, const double* X2, bool device_mem) {
 
 // Columns [a0, a0 + na) of X's AO (ri = false: Np rows) or RI (ri = true:
 // R N rows) three-index tensor, column-major with leading dimension = rows: a
-// pointer into the stored tensor, or the producer's output in `scratch`
-// (integral-direct mode).
-const double* aux_block(const IntegralsHandle& X, bool ri, size_t a0, size_t na,
-                        DevBuf& scratch) {
+// pointer into the stored tensor, or the producer's output in `room`
+// (integral-direct mode; rows * na doubles).
+const double* aux_block(const IntegralsHandle& X, bool ri, size_t a0, size_t na, double* room) {
   const size_t rows = ri ? X.n_ri * X.n_ao : packed_size(X.n_ao);
   const DeviceArray& stored = ri ? X.J3_ri_0 : X.J3_0;
   if (stored.get()) return stored.get() + rows * a0;
   const AuxProducer& fn = ri ? X.ri_fn : X.ao_fn;
   if (!fn) throw_runtime(ri ? "J3_ri_0 not stored" : "J3_0 not stored");
-  if (scratch.size() < rows * na) scratch.alloc(rows * na);
   cudaStream_t s = current_stream();
   if (profile_enabled()) {
     cudaEvent_t a, b;
     UW12_CUDA(cudaEventCreate(&a));
     UW12_CUDA(cudaEventCreate(&b));
     UW12_CUDA(cudaEventRecord(a, s));
-    fn(a0, na, scratch.get(), rows, s);
+    fn(a0, na, room, rows, s);
     UW12_CUDA(cudaEventRecord(b, s));
     profile_record(kProfProducer, a, b, 8.0 * double(rows) * double(na),
                    std::string(ri ? "produce ri " : "produce ao ") + std::to_string(na));
   } else {
-    fn(a0, na, scratch.get(), rows, s);
+    fn(a0, na, room, rows, s);
   }
-  return scratch.get();
+  return room;
+}
+
+// The same with the producer's output in `scratch`, which grows to hold it.
+const double* aux_block(const IntegralsHandle& X, bool ri, size_t a0, size_t na,
+                        DevBuf& scratch) {
+  const size_t rows = ri ? X.n_ri * X.n_ao : packed_size(X.n_ao);
+  if (!(ri ? X.J3_ri_0 : X.J3_0).get() && scratch.size() < rows * na) scratch.alloc(rows * na);
+  return aux_block(X, ri, a0, na, scratch.get());
 }
 
 // Aux functions per block when looping over a tensor: all of them when it is
@@ -1358,13 +1364,12 @@ void form_fock(const FockRequest& rq) {
       // produced again for every chunk of W's aux functions: V's RI blocks
       // take up to a quarter of the budget (their aux functions are the
       // contraction length of the p GEMM, whose output is large), its AO
-      // blocks up to a sixteenth, the chunk the rest; unstored W blocks add
-      // to the chunk's share.
+      // blocks up to a sixteenth, the chunk the rest.
       budget = budgets.doubles(0.7);
       const size_t vstep = aux_step(V, false, budget / 4), vrstep = aux_step(V, true, budget);
       const size_t vscr = (V.J3_0.get() ? 0 : np * vstep) + (V.J3_ri_0.get() ? 0 : R * N * vrstep);
       const size_t nq = tdx_spins.size(), gsz = Rp * N;
-      const size_t per_a = (2 + nq) * gsz + (W.J3_0.get() ? 0 : np) + (W.J3_ri_0.get() ? 0 : R * N);
+      const size_t per_a = (1 + nq) * gsz + nq * np;
       const size_t avail = budget > vscr ? budget - vscr : 0;
       const auto [alo, ahi] = part(MW);
       const size_t ac = tile_chunk(ahi - alo, 1,
@@ -1380,32 +1385,36 @@ void form_fock(const FockRequest& rq) {
         T2 = T2i.get();
       }
       // Per chunk of W's aux functions a: G = [sq(J3_0^W[:, a]); J3ri_0^W[:, a]]
-      // (R' x N per a; afterwards the packed s columns), L = S^-1 G and H (R' x N
-      // per a and spin).  Stacked AO + RI operands and stacked spins prepare (in
+      // (R' x N per a), L = S^-1 G, the packed columns s, and H (R' x N per a and
+      // spin).  Stacked AO + RI operands and stacked spins prepare (in
       // split precision) and read every operand once per chunk, and each product
       // is written once: the opposite-spin Fock at N = 500, M = 1500, R = 2000, open
-      // shell, 14 moduli 369 -> 332 ms.
-      DevBuf G(gsz * ac), Lb(gsz * ac), H(gsz * ac * nq), scrW, scrWr, scrV, scrVr;
+      // shell, 14 moduli 369 -> 332 ms.  What is larger per a makes chunks shorter and
+      // the producers of V run more often, so memory is shared: W's blocks are produced
+      // where L is written next, and H takes G's place, which only L reads.  Buffers for
+      // each would be 28.0 instead of 15.1 M doubles per a at N = 1200, R = 4800 (closed
+      // shell): 1.8 times the passes over V's integrals.
+      DevBuf Lb(gsz * ac), H(gsz * ac * nq), sbuf(np * ac * nq), scrV, scrVr;
+      double* const G = H.get();
       for (size_t a0 = alo; a0 < ahi; a0 += ac) {
         const size_t na = std::min(ac, ahi - a0);
-        unpack_sym(aux_block(W, false, a0, na, scrW), LL(np), LL(N), LL(na), G.get(), LL(Rp),
+        unpack_sym(aux_block(W, false, a0, na, Lb.get()), LL(np), LL(N), LL(na), G, LL(Rp),
                    LL(gsz));
-        copy3d(aux_block(W, true, a0, na, scrWr), LL(R), LL(R * N), G.get() + N, LL(Rp), LL(gsz),
+        copy3d(aux_block(W, true, a0, na, Lb.get()), LL(R), LL(R * N), G + N, LL(Rp), LL(gsz),
                LL(R), LL(N), LL(na));
-        gemm(gemm_nn(LL(Rp), LL(N * na), LL(Rp), 1.0, AB.Sinv.get(), LL(Rp), G.get(), LL(Rp), 0.0,
+        gemm(gemm_nn(LL(Rp), LL(N * na), LL(Rp), 1.0, AB.Sinv.get(), LL(Rp), G, LL(Rp), 0.0,
                      Lb.get(), LL(Rp)));
         // s = J3_0^V T2^T and p = J3_ri_0^V T2^T, accumulated over V's aux blocks
-        double* sbuf = G.get();
         const double* t2 = T2 + nq * a0;
         for (size_t b0 = 0; b0 < MV; b0 += vstep) {
           const size_t nb = std::min(vstep, MV - b0);
           GemmDesc gs = gemm_nn(LL(np), LL(na * nq), LL(nb), 1.0,
                                 aux_block(V, false, b0, nb, scrV), LL(np), t2 + nq * MW * b0,
-                                LL(nq * MW), b0 ? 1.0 : 0.0, sbuf, LL(np));
+                                LL(nq * MW), b0 ? 1.0 : 0.0, sbuf.get(), LL(np));
           gs.b_ncontig = true;
           gemm(gs);
         }
-        unpack_sym(sbuf, LL(np), LL(N), LL(na * nq), H.get(), LL(Rp), LL(gsz));
+        unpack_sym(sbuf.get(), LL(np), LL(N), LL(na * nq), H.get(), LL(Rp), LL(gsz));
         for (size_t b0 = 0; b0 < MV; b0 += vrstep) {
           const size_t nb = std::min(vrstep, MV - b0);
           GemmDesc gp = gemm_nn(LL(R), LL(na * nq), LL(nb), 1.0,
