@@ -761,6 +761,7 @@ int uw12c_integrals_create_callback(const double* X2, int x2_mem_kind,
     h->h.reset(uw12b::integrals_create_producer(X2, x2_mem_kind == UW12C_MEM_DEVICE,
                                                 std::move(ao), std::move(ri), n_ao,
                                                 n_df, n_ri, store_ao != 0, store_ri != 0));
+    h->h->host_producers = host;
     *out = h.release();
   });
 }

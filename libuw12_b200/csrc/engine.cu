@@ -747,6 +747,12 @@ void upload_orbitals(const FockRequest& rq, std::vector<SpinDims>& sd, size_t& o
 // form_fock
 // --------------------------------------------------------------------------
 namespace {
+// Whether every three-index tensor that an evaluation reads is stored.
+bool all_stored(const FockRequest& rq) {
+  return rq.W->J3_0.get() && rq.V->J3_0.get() && rq.WV->J3_0.get() && rq.W->J3_ri_0.get() &&
+         rq.V->J3_ri_0.get();
+}
+
 // Whether the t~ dX Fock term takes fewer operations over orbital pairs than over
 // aux functions (halves of the FLOPs of both forms' products; a tie goes to
 // the pairs).  Over aux functions: S^-1 G_W, and per spin J3^V T2^T and the sum
@@ -761,7 +767,17 @@ namespace {
 // prepare the three-index tensors once per spin: 338 ms, over aux functions 321 (in turn on
 // one box).  Every product is priced as if it ran split, which small and long ones
 // do not; the routing rule has rates of its own (ozaki_profitable, where the reason stands).
-bool pair_form_cheaper(const FockRequest& rq, const std::vector<SpinDims>& sd, bool same_spin) {
+//
+// Unstored tensors are produced again for every chunk: V's over aux functions, W's and V's
+// of every spin over pairs, where the same-spin terms do so anyway.  An element produced
+// costs its 8 bytes at 2.9 TB/s on the device (a copy; slower producers would want aux
+// functions earlier, but at 1 TB/s N=240, o=24/22 in split precision with a copying producer
+// took 32.3 instead of 29.4 ms) or at 50 GB/s from the host, and the chunks are those that
+// the budgets b_pairs and b_aux hold now.  Shards must agree on the form, whatever each has
+// stored and free, so they leave this out.  N=160, M=480, R=640, o=16/15, opposite spin,
+// host producers: 172 ms over pairs, 132 over aux functions.
+bool pair_form_cheaper(const FockRequest& rq, const std::vector<SpinDims>& sd, bool same_spin,
+                       double b_pairs, double b_aux) {
   const int ns = rq.n_spin;
   const double N = double(rq.n_ao), R = double(rq.W->n_ri), Rp = N + R;
   const double MW = double(rq.W->n_df), MV = double(rq.V->n_df);
@@ -790,15 +806,33 @@ bool pair_form_cheaper(const FockRequest& rq, const std::vector<SpinDims>& sd, b
     else
       pairs += product(J, ap, MW) + product(J, ap, MV) + ap * (MW * MW + MV * MV);
   }
+  // cost of producing what is not stored of X once
+  const double per_second = L > 0.0 ? 1.44e15 / L : 16e12;
+  auto once = [&](const IntegralsHandle& X) {
+    const double elements =
+        (X.J3_0.get() ? 0.0 : 0.5 * N * (N + 1.0)) + (X.J3_ri_0.get() ? 0.0 : R * N);
+    return elements * double(X.n_df) * 8.0 / (X.host_producers ? 50e9 : 2.9e12) * per_second;
+  };
+  const double once_w = once(*rq.W), once_v = once(*rq.V);
+  if (once_w + once_v > 0.0 && rq.n_shards <= 1) {
+    const double np = 0.5 * N * (N + 1.0), gsz = Rp * N;
+    auto chunks = [](double doubles, double budget) {
+      return doubles > 0.0 ? std::ceil(doubles / budget) : 0.0;
+    };
+    // at most two eighths of the budget (a quarter and a sixteenth over aux functions) hold
+    // the produced blocks
+    auto pair_chunks = [&](const SpinDims& d, double n_s) {
+      const double ap = double(pair_count(d.a, d.c, d.o));
+      const double y = same_spin ? 2.0 * double(d.a) * double(d.o) : 0.0;
+      return chunks(ap * ((1.0 + n_s) * gsz + np) + y * gsz, 0.75 * b_pairs);
+    };
+    aux += once_w + once_v * chunks(MW * ((1.0 + nq) * gsz + nq * np), 0.69 * b_aux);
+    for (const SpinDims& d : sd) {
+      pairs += pair_chunks(d, same_spin && ns == 2 ? 2.0 : 1.0) * (once_w + once_v);
+      if (same_spin) aux += pair_chunks(d, 1.0) * (once_w + once_v);
+    }
+  }
   return pairs <= aux;
-}
-}  // namespace
-
-namespace {
-// Whether every three-index tensor that an evaluation reads is stored.
-bool all_stored(const FockRequest& rq) {
-  return rq.W->J3_0.get() && rq.V->J3_0.get() && rq.WV->J3_0.get() && rq.W->J3_ri_0.get() &&
-         rq.V->J3_ri_0.get();
 }
 }  // namespace
 
@@ -972,7 +1006,10 @@ void form_fock(const FockRequest& rq) {
   PerX XW, XV;
   // The t~ dX Fock term through orbital pairs (below) or aux functions; the
   // pairs need B2 whole.
-  const bool pairs_cheaper = calc && pair_form_cheaper(rq, sd, do_ind);
+  const bool pairs_cheaper =
+      calc && (all_stored(rq) || sharded ? pair_form_cheaper(rq, sd, do_ind, 1.0, 1.0)
+                              : pair_form_cheaper(rq, sd, do_ind, double(budgets.doubles()),
+                                                  double(budgets.doubles(0.7))));
   const bool need_sv_w = calc && do_ind && !pairs_cheaper;
   // Without same-spin terms the stacked transforms serve only X_AB, t and the
   // direct Fock, which are sums over orbitals: when the whole intermediates

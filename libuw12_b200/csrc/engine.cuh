@@ -51,6 +51,7 @@ struct IntegralsHandle {
   DeviceArray J3_0, J3_ri_0, P2, lam;
   std::vector<double> lam_host;
   AuxProducer ao_fn, ri_fn;  // set when J3_0 / J3_ri_0 are not stored
+  bool host_producers = false;  // their output crosses the host link
 };
 
 // ABS+ projectors (ri_utils.hpp:45-74) stored as one (N+R) x (N+R) matrix
