@@ -21,7 +21,7 @@
 // Measured (one B200, kernel alone), against the same pipeline depth at one
 // 128 x 128 CTA per SM without fragment double buffering (30.3 TFLOP/s at
 // 45000 x 9000 x 900): 64 x 64 33.0 TFLOP/s there, 64 x 32 31.0, 32 x 32 30.0
-// (2 % more on the fastest boxes); 360 x 360 x 360 64 -> 10 us (32 x 32);
+// (2 % more on other devices); 360 x 360 x 360 64 -> 10 us (32 x 32);
 // 480 x 12 x 120, 360 batches, 242 -> 44 us (128 x 16); 125250 x 2 x 1500
 // 1.62 -> 0.24 ms (128 x 8, 6.4 TB/s of operand).
 #pragma once

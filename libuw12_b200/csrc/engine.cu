@@ -596,7 +596,7 @@ void fitted_density_raw(const IntegralsHandle& X, const double* dmat, int ns, do
 
 // Largest product (operations) of W and V in one launch, and largest evaluation (doubles of
 // both potentials' transforms) that forms them side by side.  Closed-shell Fock matrices
-// with 3 DF and 4 RI functions per AO, o = N / 10, in turn on one box, with these limits / one
+// with 3 DF and 4 RI functions per AO, o = N / 10, in turn on one B200, with these limits / one
 // after the other / side by side without limits: 0.26 / 0.31 / 0.26 ms at N = 24, 0.43 / 0.50
 // / 0.43 at 61, 1.30 / 1.37 / 1.28 at 100, 2.32 / 2.38 / 2.28 at 120 (16 M doubles), 4.77 /
 // 4.80 / 4.68 at 143, 6.98 / 7.00 / 6.89 at 160, 19.7 / 19.8 / 19.6 at 200: what lies above
@@ -765,7 +765,7 @@ bool all_stored(const FockRequest& rq) {
 // bytes at 3.4 TB/s), in units of a multiply-add (L of them at 2.88 POPS): the forms'
 // operations are equal at N=500, M=1500, R=2000, o=40/38, opposite spin, but the pairs
 // prepare the three-index tensors once per spin: 338 ms, over aux functions 321 (in turn on
-// one box).  Every product is priced as if it ran split, which small and long ones
+// one B200).  Every product is priced as if it ran split, which small and long ones
 // do not; the routing rule has rates of its own (ozaki_profitable, where the reason stands).
 //
 // Unstored tensors are produced again for every chunk: V's over aux functions, W's and V's
