@@ -573,9 +573,29 @@ double* noalloc_scratch_for_current_device() {
   }
   return g_scratch_ptr[dev];
 }
+
+// At a device's first call: the fixed array and every kernel that a later call may launch
+// (all layouts of all tiles, the split reduction, the empty contraction), so that no later
+// one loads device code, which takes device memory.
+void load_all_for_current_device() {
+  static bool loaded[64] = {};
+  static std::mutex mu;
+  int dev = 0;
+  UW12_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  if (dev < 0 || dev >= 64 || loaded[dev]) return;
+  noalloc_scratch_for_current_device();
+  for (int layout = 0; layout < 16; ++layout) load_layout(layout);
+  cudaFuncAttributes fa{};
+  UW12_CUDA(cudaFuncGetAttributes(&fa, splitk_reduce<unsigned>));
+  UW12_CUDA(cudaFuncGetAttributes(&fa, splitk_reduce<long long>));
+  UW12_CUDA(cudaFuncGetAttributes(&fa, scale_only));
+  loaded[dev] = true;
+}
 }  // namespace
 
 void gemm_noalloc(const GemmDesc& d) {
+  load_all_for_current_device();
   KParams p;
   bool empty_k = false;
   if (!prepare(d, p, &empty_k)) return;
