@@ -48,7 +48,7 @@ assert call(*shapes[0], 0, 0, 0) == 0
 torch.cuda.synchronize()
 fill = []
 size = 8 << 30
-while size >= 1 << 20:
+while size >= 1 << 20 and torch.cuda.mem_get_info()[0] > 8 << 20:  # half of the array's size
     try:
         fill.append(torch.empty(size, dtype=torch.uint8, device=dev))
     except torch.OutOfMemoryError:
